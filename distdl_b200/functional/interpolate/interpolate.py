@@ -27,7 +27,7 @@ def _call(x, y, adjoint, mode, x_off, y_off, in_global, out_global, scale, align
     nd = x.dim() - 2
     BC = x.shape[0] * x.shape[1]
     cuda = int(x.is_cuda)
-    dtype = {torch.float32: 0, torch.float64: 1}[x.dtype]
+    dtype = {torch.float32: 0, torch.float64: 1, torch.bfloat16: 2}[x.dtype]
     stream = torch.cuda.current_stream().cuda_stream if cuda else 0
     sc = (ctypes.c_double * nd)(*[float(s) for s in scale])
     _native.launch_count += cuda
@@ -44,6 +44,11 @@ def _steps(in_global, out_global, scale_factor, align_corners):
         sf = None if scale_factor is None else (scale_factor[d] if np.ndim(scale_factor) else scale_factor)
         out.append(1.0 / float(sf) if (sf is not None and sf > 0 and not align_corners) else float(n_in) / float(n_out))
     return out
+
+
+def _direct(t):
+    """True for the types that the kernels read themselves; others go through fp32."""
+    return t.dtype in (torch.float32, torch.float64) or (t.is_cuda and t.dtype == torch.bfloat16)
 
 
 class InterpolateFunction(torch.autograd.Function):
@@ -63,7 +68,7 @@ class InterpolateFunction(torch.autograd.Function):
         in_g, out_g = tail(x_global_shape), tail(y_global_shape)
         out_local = [b - a for a, b in zip(y_off, tail(y_local_stop))]
         xc = x.contiguous()
-        if xc.dtype not in (torch.float32, torch.float64):
+        if not _direct(xc):
             xc = xc.float()
         y = torch.empty(list(x.shape[:2]) + out_local, dtype=xc.dtype, device=x.device)
         steps = _steps(in_g, out_g, scale_factor, align_corners)
@@ -75,9 +80,10 @@ class InterpolateFunction(torch.autograd.Function):
     def backward(ctx, gy):
         mode, x_off, y_off, in_g, out_g, steps, align_corners, xshape, xdtype = ctx.cfg
         g = gy.contiguous()
-        if g.dtype not in (torch.float32, torch.float64):
+        if not _direct(g):
             g = g.float()
-        gx = torch.zeros(xshape, dtype=g.dtype, device=g.device)
+        # the CUDA kernel writes every element, the CPU code adds to what is there
+        gx = (torch.empty if g.is_cuda else torch.zeros)(xshape, dtype=g.dtype, device=g.device)
         _call(gx, g, True, mode, x_off, y_off, in_g, out_g, steps, align_corners)
         return (gx.to(xdtype),) + (None,) * 9
 

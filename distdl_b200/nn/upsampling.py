@@ -87,6 +87,7 @@ class DistributedUpsample(Module, InterpolateMixin):
     def forward(self, input):
         if not self.P_x.active:
             return input
-        x = F.pad(input, self.pad_tuple, mode="constant", value=0)
+        # (without padding the copy is spared: interpolation keeps nothing of its input for the backward pass)
+        x = F.pad(input, self.pad_tuple, mode="constant", value=0) if any(self.pad_tuple) else input
         x = self.halo_layer(x)
         return self.interp_layer(x)

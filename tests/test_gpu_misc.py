@@ -168,3 +168,36 @@ def test_pooling_kernels_match_torch_on_a_cropped_view(nd, kind, kernel, stride,
     y.backward(dy.to(dtype))
     yr.backward(dy)
     assert (x.grad.float() - xr.grad).abs().max().item() <= tol * (1 + xr.grad.abs().max().item()) * 4
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16])
+@pytest.mark.parametrize("mode,ac,n_in,n_out", [
+    ("linear", False, (7, 9, 11), (14, 18, 22)),       # two outputs per input: four take an inner input
+    ("linear", True, (5, 6, 7), (8, 9, 10)),
+    ("linear", False, (9, 8, 6), (4, 5, 3)),           # fewer outputs than inputs: some inputs are taken by none
+    ("linear", True, (3, 4, 2), (40, 60, 90)),         # more outputs per input than a thread keeps weights for
+    ("linear", False, (1, 5, 3), (6, 1, 16)),          # extents of one
+    ("nearest", False, (5, 3, 4), (10, 7, 33))])
+def test_interpolation_kernels_over_scales(mode, ac, n_in, n_out, dtype):
+    """1-, 2- and 3-dimensional, few planes and more planes than a thread takes at once, sub-ranges of the output,
+    against the CPU code in fp64; an infinity reaches the outputs whose weight for it is not zero, and no other."""
+    from distdl_b200.functional.interpolate import interpolate
+    torch.manual_seed(5)
+    tol = {torch.float32: 2e-6, torch.float64: 1e-13, torch.bfloat16: 8e-3}[dtype]     # a few roundings of the type
+    for nd, planes, cut in ((1, 3, 0), (2, 70, 1), (3, 5, 1)):
+        gi, go = list(n_in[3 - nd:]), list(n_out[3 - nd:])
+        lo = [0] * nd
+        hi = [max(1, n - cut) for n in go]
+        x = torch.randn(1, planes, *gi).to(dtype)
+        args = (lo, gi, gi, lo, hi, go, None, mode, ac)
+        xc, xg = x.double().clone().requires_grad_(), x.cuda().requires_grad_()
+        yc, yg = interpolate(xc, *args), interpolate(xg, *args)
+        assert yg.dtype == dtype and yg.shape == yc.shape
+        assert (yg.double().cpu() - yc).abs().max() <= tol * yc.abs().max()
+        dy = torch.randn(yc.shape).to(dtype)
+        yc.backward(dy.double())
+        yg.backward(dy.cuda())
+        assert (xg.grad.double().cpu() - xc.grad).abs().max() <= tol * (1 + xc.grad.abs().max())
+        bad = x.clone()
+        bad[:, :, -1] = float("inf")
+        assert torch.equal(interpolate(bad.cuda(), *args).isfinite().cpu(), interpolate(bad.double(), *args).isfinite())
