@@ -70,7 +70,10 @@ class DistributedPoolBase(Module, HaloMixin, PoolingMixin):
     def forward(self, input):
         if not self.P_x.active:
             return input
-        x = F.pad(input, self.pad_tuple, mode="constant", value=self.pad_value)
+        # (without padding the copy is spared: pooling keeps nothing of its input for the backward pass)
+        x = input
+        if any(self.pad_tuple) or not input.is_contiguous():
+            x = F.pad(input, self.pad_tuple, mode="constant", value=self.pad_value)
         x = self.halo_layer(x)
         x = x[self.needed_slices]
         k = tuple(int(v) for v in self.kernel_size)
