@@ -122,11 +122,35 @@ class DistributedBatchNorm(Module):
         mine = float(self.P_x.index[1])
         self.global_count = float(sum(c[0] for c in counts if c[1] == mine))
 
+    def _affine_weights(self):
+        if not self.affine:
+            return None, None
+        if self.gamma_buffer is None:
+            self.prefetch_weights()
+        gamma, beta = self.gamma_buffer, self.beta_buffer
+        self.gamma_buffer = self.beta_buffer = None
+        return gamma, beta
+
+    def _alone(self, input, bn_ops):
+        """One worker holds the whole batch that the layer was set up for: nothing travels between the passes,
+        so that they run fused (the statistics then stay in fp32 instead of the input's type in between)."""
+        if self.P_x.size != 1 or self.global_count != float(np.prod(input.shape) / input.shape[1]):
+            return False
+        features = ([self.gamma, self.beta] if self.affine else []) + \
+            ([self.running_mean, self.running_var] if self.track_running_stats else [])
+        return bn_ops.train_usable(input, self.momentum, *features)
+
     def forward(self, input):
         if not self.P_x.active:
             return input
         from ..ops import batchnorm as bn_ops
-        if self.training or not self.track_running_stats:
+        batch_stats = self.training or not self.track_running_stats
+        update = self.training and self.track_running_stats
+        if batch_stats and self._alone(input, bn_ops):
+            gamma, beta = self._affine_weights()
+            return bn_ops.train_batch_norm(input, gamma, beta, self.eps, self.running_mean if update else None,
+                                           self.running_var if update else None, self.momentum)
+        if batch_stats:
             # local per-feature sums: one reduction kernel each (fp32 accumulation)
             s = self.sr(bn_ops.channel_sum(input))
             mean_root = s / self.global_count if self.P_sum.active else s
@@ -143,12 +167,7 @@ class DistributedBatchNorm(Module):
         else:
             mean = self.bc_rm(self.running_mean)
             var = self.bc_rv(self.running_var)
-        gamma = beta = None
-        if self.affine:
-            if self.gamma_buffer is None:
-                self.prefetch_weights()
-            gamma, beta = self.gamma_buffer, self.beta_buffer
-            self.gamma_buffer = self.beta_buffer = None
+        gamma, beta = self._affine_weights()
         # normalisation and affine map in one element-wise kernel (and one reduction + one element-wise
         # kernel in its backward pass)
         return bn_ops.normalize(input, mean, var, gamma, beta, self.eps)

@@ -15,6 +15,10 @@ from ._util import ptr, stream_ptr, use_native
 _v, _i, _ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
 _native.declare("dd_bn_reduce", [_v, _v, _v, _i, _i, _ll, _i, _i, _v, _v, _v])
 _native.declare("dd_bn_affine", [_v, _v, _v, _v, _v, _v, _i, _i, _ll, _i, _v, _v])
+_native.declare("dd_bn_train_workspace", [_i, _i, _ll])
+_native.declare("dd_bn_train_fwd", [_v, _v, _v, _i, _i, _i, _i, _ll, _i, ctypes.c_float, _v, _v, _i, ctypes.c_float,
+                                    _v, _v, _v, _v])
+_native.declare("dd_bn_train_bwd", [_v, _v, _v, _i, _i, _i, _i, _ll, _i, _v, _v, _v, _v, _v, _v, _v])
 _DT = {torch.bfloat16: 0, torch.float32: 1}
 
 
@@ -101,6 +105,60 @@ class _Normalize(torch.autograd.Function):
         dgamma = (rstd * sdyx).reshape(gmeta[0]).to(gmeta[1]) if has_g and ctx.needs_input_grad[3] else None
         dbeta = sdy.reshape(bmeta[0]).to(bmeta[1]) if has_b and ctx.needs_input_grad[4] else None
         return dx, dmean, dvar, dgamma, dbeta, None
+
+
+class _TrainBatchNorm(torch.autograd.Function):
+    """Statistics, running statistics, normalisation and their joint gradient, for a batch that one
+    worker holds whole: the backward pass goes through the mean and the variance in one map."""
+
+    @staticmethod
+    def forward(ctx, x, gamma, beta, eps, running_mean, running_var, momentum):
+        B, F, R = _geometry(x)
+        ws = torch.empty(_native.lib().dd_bn_train_workspace(B, F, R), dtype=torch.float32, device=x.device)
+        stat = torch.empty(2, F, dtype=torch.float32, device=x.device)
+        y = torch.empty_like(x)
+        _native.call("dd_bn_train_fwd", x.data_ptr(), ptr(gamma), ptr(beta), 1 if gamma is None else _DT[gamma.dtype],
+                     1 if beta is None else _DT[beta.dtype], B, F, R, _DT[x.dtype], eps, ptr(running_mean),
+                     ptr(running_var), 1 if running_mean is None else _DT[running_mean.dtype], momentum,
+                     ws.data_ptr(), stat.data_ptr(), y.data_ptr(), stream_ptr())
+        ctx.save_for_backward(x, stat, gamma)
+        ctx.beta_meta = None if beta is None else (beta.shape, beta.dtype)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, stat, gamma = ctx.saved_tensors
+        B, F, R = _geometry(x)
+        dy = dy.contiguous()
+        ws = torch.empty(_native.lib().dd_bn_train_workspace(B, F, R) + 3 * F, dtype=torch.float32, device=x.device)
+        need = ctx.needs_input_grad
+        dx = torch.empty_like(x) if need[0] else None
+        dgamma = torch.empty_like(gamma) if gamma is not None and need[1] else None
+        dbeta = None
+        if ctx.beta_meta is not None and need[2]:
+            dbeta = torch.empty(ctx.beta_meta[0], dtype=ctx.beta_meta[1], device=x.device)
+        _native.call("dd_bn_train_bwd", x.data_ptr(), dy.data_ptr(), ptr(gamma), 1 if gamma is None else _DT[gamma.dtype],
+                     1 if dbeta is None else _DT[dbeta.dtype], B, F, R, _DT[x.dtype], stat.data_ptr(),
+                     ws[3 * F:].data_ptr(), ws.data_ptr(), ptr(dx), ptr(dgamma), ptr(dbeta), stream_ptr())
+        return dx, dgamma, dbeta, None, None, None, None
+
+
+def train_usable(x, momentum, *features):
+    """True where :func:`train_batch_norm` may stand for ``channel_sum`` ... ``normalize``: kernels' types, and
+    per-feature tensors that are contiguous on ``x``'s device."""
+    if not usable(x) or not isinstance(momentum, (int, float)):
+        return False
+    return all(t is None or (t.dtype in _DT and t.device == x.device and t.is_contiguous() and t.numel() == x.shape[1])
+               for t in features)
+
+
+def train_batch_norm(x, gamma, beta, eps, running_mean=None, running_var=None, momentum=0.0):
+    """Batch norm with the statistics of ``x`` itself; updates the running statistics in place."""
+    y = _TrainBatchNorm.apply(x, gamma, beta, eps, running_mean, running_var, momentum)
+    for t in (running_mean, running_var):
+        if t is not None and not t.is_inference():
+            torch._C._increment_version([t])          # written by the kernel
+    return y
 
 
 def channel_sum(x):

@@ -201,3 +201,51 @@ def test_interpolation_kernels_over_scales(mode, ac, n_in, n_out, dtype):
         bad = x.clone()
         bad[:, :, -1] = float("inf")
         assert torch.equal(interpolate(bad.cuda(), *args).isfinite().cpu(), interpolate(bad.double(), *args).isfinite())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape,affine,track", [
+    ((6, 5, 7, 9), True, True),             # planes of 63: units shared between neighbours
+    ((4, 3, 64), True, False),
+    ((3, 70, 2), False, True),              # many features, planes smaller than a unit
+    ((2, 2, 37, 41, 13), True, True),       # several CTAs per plane
+    ((5, 4), True, True)])                  # no dimension besides batch and feature
+def test_batch_norm_layer_fused_on_one_worker(shape, affine, track, dtype):
+    """Output, gradients and running statistics of the layer against PyTorch in fp64, with a mean far from zero."""
+    import distdl_b200
+    from distdl_b200 import backends
+    from distdl_b200.nn import DistributedBatchNorm
+    distdl_b200.config.set_backend("native", "cupy")
+    torch.manual_seed(9)
+    P = backends.backend.Partition().create_partition_inclusive([0]).create_cartesian_topology_partition([1] * len(shape))
+    F = shape[1]
+    layer = DistributedBatchNorm(P, F, affine=affine, track_running_stats=track, device="cuda", dtype=dtype)
+    x = (torch.randn(shape, device="cuda") * 2 + 50).to(dtype).requires_grad_()
+    w = torch.ones(F, dtype=torch.float64, device="cuda")
+    b = torch.zeros(F, dtype=torch.float64, device="cuda")
+    if affine:
+        with torch.no_grad():
+            layer.gamma.add_(torch.randn_like(layer.gamma), alpha=0.3)
+            layer.beta.add_(torch.randn_like(layer.beta), alpha=0.3)
+        w, b = layer.gamma.detach().double().flatten(), layer.beta.detach().double().flatten()
+    xr, w, b = x.detach().double().requires_grad_(), w.requires_grad_(), b.requires_grad_()
+    rm, rv = torch.zeros(F, device="cuda").double(), torch.ones(F, device="cuda").double()
+    yr = torch.nn.functional.batch_norm(xr, rm, rv, w, b, True, 0.1, layer.eps)
+    y = layer(x)
+    dy = torch.randn(shape, device="cuda").to(dtype)
+    y.backward(dy)
+    yr.backward(dy.double())
+    # fp32: subtracting a mean of 50 from values of spread 2 leaves 25 eps; bf16: the rounding of the results
+    tol = 2e-5 if dtype == torch.float32 else 8e-3
+
+    def close(a, r, floor=0.0):
+        assert (a.double().flatten() - r.flatten()).abs().max() <= tol * (r.abs().max() + floor)
+
+    close(y, yr)
+    close(x.grad, xr.grad, floor=float(dy.double().abs().max()))
+    if affine:
+        close(layer.gamma.grad, w.grad, floor=1.0)
+        close(layer.beta.grad, b.grad, floor=1.0)
+    if track:
+        close(layer.running_mean, rm)
+        close(layer.running_var, rv)
