@@ -11,11 +11,11 @@ reference performs the same conversions with einops patterns
 """
 from __future__ import annotations
 
-import os
-
 import numpy as np
 import torch
 
+from ..ops._util import env
+from ..utilities import streams
 from ..utilities.slicing import compute_subshape, worker_layout
 
 
@@ -75,6 +75,11 @@ def local_out_features(out_features, num_gpu, index, num_heads=None, num_heads_k
     return int(sum(blocks[index]))
 
 
+def through(module, x):
+    """``module(x)`` of a data-movement module, without the call where the module is the identity."""
+    return x if module.identity else module(x)
+
+
 def deliver_grad(param, g):
     """Adds the gradient shard ``g`` to ``param``: into the optimizer's fp32
     accumulator when the parameter has one (``main_grad_view``), else into
@@ -101,7 +106,7 @@ def direct_main_grad(param, gather, shape):
     Autograd then sees no gradient for the gathered weight, so the per-micro-batch
     reduce-scatter adjoint of the all-gather does not run."""
     acc = getattr(param, "main_grad_view", None)
-    if acc is None or not param.is_cuda or os.environ.get("DISTDL_DIRECT_MAIN_GRAD", "1") == "0":
+    if acc is None or not param.is_cuda or env("DISTDL_DIRECT_MAIN_GRAD", "1") == "0":
         return None
     if gather.scale_backward is not None:
         return None
@@ -171,13 +176,12 @@ class PrefetchStream:
     def run(self, fn):
         if not self.cuda:
             return fn()
-        from ..utilities import streams
+        before = streams.queued()
         with streams.deferred():
             out = fn()
-        side = streams.side_stream()
-        if side is not None:
+        if streams.queued() != before:          # (where every gather is the identity there is nothing to wait for)
             self._event = torch.cuda.Event()
-            self._event.record(side)
+            self._event.record(streams.side_stream())
         return out
 
     def wait(self):

@@ -6,7 +6,7 @@ import torch
 
 from ..utilities.slicing import compute_subshape
 from ..utilities.torch import zero_volume_tensor
-from ._linear_common import KeptBufferGuard, PrefetchStream, deliver_grad, root_partition
+from ._linear_common import KeptBufferGuard, PrefetchStream, deliver_grad, root_partition, through
 from .all_gather import AllGather
 from .module import Module
 from .reduce_scatter import ReduceScatter
@@ -95,7 +95,7 @@ class _ZeroNormBase(Module):
     def _collect(self):
         out = {}
         for n in self.param_names:
-            full = self.allgather(getattr(self, n)).reshape(self.num_features)
+            full = through(self.allgather, getattr(self, n)).reshape(self.num_features)
             if not self.auto_clear_buffer:
                 full = full.detach().requires_grad_(True)
                 if full.is_cuda and full.dtype == torch.bfloat16:

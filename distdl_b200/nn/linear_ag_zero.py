@@ -10,7 +10,7 @@ from ..utilities import recompute
 from ..utilities.slicing import compute_subshape
 from ..utilities.torch import zero_volume_tensor
 from ._linear_common import (KeptBufferGuard, PrefetchStream, deliver_grad, direct_main_grad, local_out_features,
-                             reduce_scatter_grad, relayout, root_partition, var_blocks)
+                             reduce_scatter_grad, relayout, root_partition, through, var_blocks)
 from .all_gather import AllGather
 from .module import Module
 from .reduce_scatter import ReduceScatter
@@ -208,7 +208,7 @@ class DistributedLinearAllGatherZero(Module):
 
     # ---------------------------------------------------------------- forward
     def _collect_weights(self):
-        w = self.allgather_weight(self.weight)            # [in, 1.., out/M, 1]
+        w = through(self.allgather_weight, self.weight)   # [in, 1.., out/M, 1]
         self.weight_buffer = w.reshape(self.in_features, self.out_features_local)
         if self.bias is not None:
             self.bias_buffer = self.allgather_bias_over_dp(self.bias).reshape(self.out_features_local)
@@ -277,7 +277,7 @@ class DistributedLinearAllGatherZero(Module):
                 from ..parallel import fused
                 y = fused.maybe_ag_linear(self, input, wt, b)
             if y is None:
-                x = self.all_gather(input)
+                x = through(self.all_gather, input)
                 y = ops.linear(x, wt, b)
         if self.auto_clear_buffer:
             self.clear_weight_buffer()

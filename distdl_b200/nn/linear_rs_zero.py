@@ -10,7 +10,7 @@ from ..utilities import recompute
 from ..utilities.slicing import compute_subshape
 from ..utilities.torch import zero_volume_tensor
 from ._linear_common import (KeptBufferGuard, PrefetchStream, deliver_grad, derived_partition, direct_main_grad,
-                             reduce_scatter_grad, root_partition)
+                             reduce_scatter_grad, root_partition, through)
 from .all_gather import AllGather
 from .module import Module
 from .reduce_scatter import ReduceScatter
@@ -154,7 +154,7 @@ class DistributedLinearReduceScatterZero(Module):
         return destination
 
     def _collect_weights(self):
-        w = self.allgather_weight(self.weight)                 # [out, 1.., in/M]
+        w = through(self.allgather_weight, self.weight)        # [out, 1.., in/M]
         self.weight_buffer = w.reshape(self.out_features, self.in_features_local)
         if self.use_bias and self.P_bias.active:
             self.bias_buffer = self.allgather_bias(self.bias).reshape(self.out_features)
@@ -203,7 +203,7 @@ class DistributedLinearReduceScatterZero(Module):
             if y is not None:
                 return y
         y = ops.linear(input, w, b)
-        return self.reduce_scatter(y)
+        return through(self.reduce_scatter, y)
 
     def forward(self, input):
         if not self.P_x.active:

@@ -1,6 +1,6 @@
 """Base class of every distributed layer.
 
-A forward pre-hook runs the layer's set-up lazily, on the first call and again
+The call runs the layer's set-up lazily, on the first call and again
 whenever the structure of the input (shape, dtype, requires_grad) changes
 (``src/distdl/nn/module.py:34-56``, ``:101-112``); set
 ``DISTDL_CHECK_INPUT_CHANGED=0`` to skip the re-check.  The backend that is
@@ -16,7 +16,23 @@ class Module(torch.nn.Module):
         super().__init__()
         self._distdl_backend = backends.backend
         self._distdl_is_setup = False
-        self.register_forward_pre_hook(self._distdl_forward_pre_hook)
+
+    # Set in every forward pass: plain attributes, never parameters, buffers or sub-modules (also where a gather
+    # that is the identity hands the Parameter itself on), so that they skip torch.nn.Module's registration.
+    _distdl_plain = frozenset(("weight_buffer", "bias_buffer", "buffers_gathered", "gamma_buffer", "beta_buffer",
+                               "_distdl_is_setup", "_input_tensor_structure"))
+
+    def __setattr__(self, name, value):
+        if name in Module._distdl_plain:
+            object.__setattr__(self, name, value)
+        else:
+            super().__setattr__(name, value)
+
+    def __call__(self, *input, **kwargs):
+        # (not a registered pre-hook: a module without hooks takes torch.nn.Module's short way)
+        if self._distdl_module_requires_reset(input):
+            Module._distdl_forward_pre_hook(self, input)
+        return super().__call__(*input, **kwargs)
 
     @staticmethod
     def _distdl_forward_pre_hook(self, input):

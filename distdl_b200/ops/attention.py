@@ -10,12 +10,11 @@ output of a fused QKV projection is consumed in place (strided views).
 from __future__ import annotations
 
 import math
-import os
 
 import torch
 
 from .. import _native
-from ._util import stream_ptr, use_native
+from ._util import env, stream_ptr, use_native
 
 _native.declare("dd_attn_fwd", [_native.c_void_p, _native.c_ll, _native.c_ll, _native.c_void_p, _native.c_ll,
                                 _native.c_ll, _native.c_void_p, _native.c_ll, _native.c_ll, _native.c_void_p,
@@ -57,7 +56,7 @@ def attention_forward(q, k, v, batch, seq, causal=True, scale=None):
     lse = torch.empty(batch, Hq, seq, dtype=torch.float32, device=q.device)
     # head dim 128 / 64 and sequences of whole 256-row pairs run the two-tile kernel (scores and
     # probabilities in tensor memory, two query tiles alternating on the tensor cores)
-    two_tile = D in (64, 128) and seq % 256 == 0 and os.environ.get("DISTDL_ATTN_FWD2", "1") != "0"
+    two_tile = D in (64, 128) and seq % 256 == 0 and env("DISTDL_ATTN_FWD2", "1") != "0"
     _native.call("dd_attn_fwd2" if two_tile else "dd_attn_fwd", q.data_ptr(), *_strides(q), k.data_ptr(), *_strides(k),
                  v.data_ptr(), *_strides(v), out.data_ptr(), lse.data_ptr(), batch, seq, Hq, Hkv, D, int(causal),
                  float(scale), stream_ptr())
@@ -77,7 +76,7 @@ def attention_backward(dout, q, k, v, out, lse, batch, seq, causal=True, scale=N
         dv = torch.empty(tokens, Hkv, D, dtype=q.dtype, device=q.device)
     dout = dout.contiguous()
     # the kernels that keep P / dS in tensor memory (scratch: delta and the base-2 lse)
-    in_tmem = D in (64, 128) and os.environ.get("DISTDL_ATTN_BWD2", "1") != "0"
+    in_tmem = D in (64, 128) and env("DISTDL_ATTN_BWD2", "1") != "0"
     delta = torch.empty(2 if in_tmem else 1, batch, Hq, seq, dtype=torch.float32, device=q.device)
     _native.call("dd_attn_bwd2" if in_tmem else "dd_attn_bwd", q.data_ptr(), *_strides(q), k.data_ptr(), *_strides(k),
                  v.data_ptr(), *_strides(v), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), delta.data_ptr(),
@@ -122,7 +121,7 @@ def attention(q, k, v, batch: int, seq: int, causal: bool = True, scale: float =
     tensors (strided views allowed); ``k``/``v`` may have fewer heads (GQA)."""
     D = q.shape[-1]
     native = (use_native(q) and q.dtype == torch.bfloat16 and D in (64, 128) and seq % 128 == 0
-              and os.environ.get("DISTDL_ATTN_IMPL", "native") == "native")
+              and env("DISTDL_ATTN_IMPL", "native") == "native")
     if native:
         return _AttnFn.apply(q, k, v, batch, seq, causal, scale)
     return _reference(q, k, v, batch, seq, causal, scale)
@@ -156,7 +155,7 @@ def attention_packed(qkv, Hq: int, Hkv: int, batch: int, seq: int, causal: bool 
     ordered q..., k..., v...).  Returns ``[tokens, Hq, head_dim]``."""
     D = qkv.shape[-1]
     native = (use_native(qkv) and qkv.dtype == torch.bfloat16 and D in (64, 128) and seq % 128 == 0
-              and qkv.is_contiguous() and os.environ.get("DISTDL_ATTN_IMPL", "native") == "native")
+              and qkv.is_contiguous() and env("DISTDL_ATTN_IMPL", "native") == "native")
     if native:
         return _PackedAttnFn.apply(qkv, Hq, Hkv, batch, seq, causal, scale)
     return _reference(qkv[:, :Hq], qkv[:, Hq:Hq + Hkv], qkv[:, Hq + Hkv:], batch, seq, causal, scale)

@@ -194,6 +194,7 @@ def gather_in_place(x: torch.Tensor, ranks):
     # `out` may have been in use by earlier kernels of this stream)
     side.wait_stream(main)
     _pull(P, first, srcs, out, nbytes, side.cuda_stream)
+    streams.note_queued()
     out.record_stream(side)
     if not streams.is_deferred():
         main.wait_stream(side)

@@ -60,7 +60,10 @@ class Trainer:
             from ..nn import reset_setup
             reset_setup(self.model)
         self._last_shape = tuple(tokens.shape)
-        self.model.train()
+        for m in self.model.modules():
+            if not m.training:
+                self.model.train()
+                break
         self.opt.set_lr(cosine_lr(self.steps_done, self.base_lr, self.warmup_steps, self.total_steps))
         total = torch.zeros((), dtype=torch.float32, device=tokens.device)
         scale = 1.0 / float(self.global_tokens)

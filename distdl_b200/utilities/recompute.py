@@ -107,14 +107,20 @@ def _unpack(obj):
     return obj
 
 
-@contextlib.contextmanager
+_nothing = contextlib.nullcontext()
+
+
 def saved_as_recipe(tensor, fn):
     """Inside the block, autograd saves ``fn`` wherever it would save ``tensor`` (any view of its
     storage).  ``fn`` must return a tensor with the layout of ``tensor``.  Does nothing when recipes
     are off, when ``fn`` is None or when ``tensor`` is empty."""
     if not active() or fn is None or not isinstance(tensor, torch.Tensor) or tensor.numel() == 0:
-        yield None
-        return
+        return _nothing
+    return _saved_as_recipe(tensor, fn)
+
+
+@contextlib.contextmanager
+def _saved_as_recipe(tensor, fn):
     recipe = Recipe(fn)
     _targets.append((tensor.untyped_storage().data_ptr(), tensor.dtype, tensor.device, tensor.storage_offset(), recipe))
     try:

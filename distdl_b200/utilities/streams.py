@@ -9,7 +9,6 @@ both.  Wait-free copies have no such problem, so they may overlap the compute st
 ``deferred()`` marks a region (a weight prefetch) in which the consumer promises to call
 ``join()`` before it touches the results; outside such a region every side-stream operation
 is joined immediately."""
-import contextlib
 import threading
 
 import torch
@@ -36,13 +35,25 @@ def is_deferred() -> bool:
     return getattr(_state, "deferred", 0) > 0
 
 
-@contextlib.contextmanager
-def deferred():
-    _state.deferred = getattr(_state, "deferred", 0) + 1
-    try:
-        yield
-    finally:
+def note_queued():
+    """To be called by whoever puts work on the side stream: lets a prefetch see whether its gathers did."""
+    _state.queued = getattr(_state, "queued", 0) + 1
+
+
+def queued() -> int:
+    """How often this thread has put work on a side stream so far."""
+    return getattr(_state, "queued", 0)
+
+
+class deferred:
+    __slots__ = ()
+
+    def __enter__(self):
+        _state.deferred = getattr(_state, "deferred", 0) + 1
+
+    def __exit__(self, *exc):
         _state.deferred -= 1
+        return False
 
 
 def join():

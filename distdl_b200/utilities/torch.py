@@ -33,8 +33,10 @@ class TensorStructure:
     def __eq__(self, other):
         if not isinstance(other, TensorStructure):
             return NotImplemented
-        a = None if self.shape is None else tuple(int(s) for s in self.shape)
-        b = None if other.shape is None else tuple(int(s) for s in other.shape)
+        a, b = self.shape, other.shape
+        if not (isinstance(a, tuple) and isinstance(b, tuple)):          # (a torch.Size is a tuple)
+            a = None if a is None else tuple(int(s) for s in a)
+            b = None if b is None else tuple(int(s) for s in b)
         return a == b and self.dtype == other.dtype and self.requires_grad == other.requires_grad
 
     def __repr__(self):
