@@ -119,6 +119,17 @@ def direct_main_grad(param, gather, shape):
     return None
 
 
+def attach_main_grad(tensor, param, broadcast):
+    """Gives ``tensor`` (a view of ``param`` that came through the data-parallel ``broadcast``) the optimizer's
+    accumulator of ``param`` as its ``main_grad``, where the broadcast is the identity: the gradient is then
+    added there in fp32 instead of being written in bf16, handed through autograd and added up."""
+    acc = getattr(param, "main_grad_view", None)
+    if acc is None or not param.is_cuda or not broadcast.identity or broadcast.scale_backward is not None \
+            or acc.numel() != tensor.numel() or env("DISTDL_DIRECT_MAIN_GRAD", "1") == "0":
+        return
+    tensor.main_grad = acc.view(tensor.shape)
+
+
 def reduce_scatter_grad(rs, full_grad, param, scale_backward=None):
     """Reduce-scatters the gradient accumulated on a gathered parameter and
     delivers the slice to ``param`` (fused into the fp32 accumulator when the

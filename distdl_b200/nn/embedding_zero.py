@@ -6,7 +6,7 @@ import torch
 from .. import ops
 from ..utilities.slicing import compute_subshape
 from ..utilities.torch import zero_volume_tensor
-from ._linear_common import KeptBufferGuard, PrefetchStream, reduce_scatter_grad
+from ._linear_common import KeptBufferGuard, PrefetchStream, direct_main_grad, reduce_scatter_grad
 from .all_gather import AllGather
 from .module import Module
 from .reduce_scatter import ReduceScatter
@@ -117,6 +117,12 @@ class DistributedEmbeddingZero(Module):
         self.collect_weights()
         self.wait_for_streams()
         w = self.weight_buffer
+        mg = direct_main_grad(self.weight, self.allgather, w.shape)
+        if mg is not None:
+            # the scatter-add goes straight into the optimizer's fp32 accumulator: no gradient of the table's size
+            # is cleared, rounded to bf16 and added up again for the few rows that the tokens name
+            w = w.view(w.shape)              # a fresh tensor object to carry the attribute
+            w.main_grad = mg
         if self.max_norm is None and not self.scale_grad_by_freq and not self.sparse:
             y = ops.embedding(input, w, self.padding_idx)
         else:

@@ -8,7 +8,8 @@ import torch
 from .. import ops
 from ..utilities.torch import zero_volume_tensor
 from . import init
-from ._linear_common import PrefetchStream, derived_partition, local_out_features, relayout, root_partition, var_blocks
+from ._linear_common import (PrefetchStream, attach_main_grad, derived_partition, local_out_features, relayout,
+                             root_partition, var_blocks)
 from .all_gather import AllGather
 from .broadcast import Broadcast
 from .module import Module
@@ -191,6 +192,9 @@ class DistributedLinearAllGather(Module):
         if self.weight_buffer is None:
             weight = self.broadcast_weight(self.weight).view(-1, self.in_features)
             bias = self.broadcast_bias(self.bias).view(-1) if self.bias is not None else None
+            attach_main_grad(weight, self.weight, self.broadcast_weight)
+            if bias is not None:
+                attach_main_grad(bias, self.bias, self.broadcast_bias)
         else:
             self.prefetch.wait()
             weight, bias = self.weight_buffer, self.bias_buffer

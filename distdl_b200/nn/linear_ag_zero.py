@@ -269,6 +269,10 @@ class DistributedLinearAllGatherZero(Module):
         mg = direct_main_grad(self.weight, self.allgather_weight, w.shape)
         if mg is not None:
             wt.main_grad = mg.t()
+        mgb = direct_main_grad(self.bias, self._bias_ag, b.shape) if b is not None else None
+        if mgb is not None:
+            b = b.view(b.shape)              # a fresh tensor object to carry the attribute
+            b.main_grad = mgb
         y = None
         # where recipes are on, the backward pass gathers the weight shards again instead of
         # holding the gathered weight since the forward pass

@@ -9,7 +9,7 @@ from .. import ops
 from ..utilities.slicing import compute_subshape
 from ..utilities.torch import zero_volume_tensor
 from . import init
-from ._linear_common import PrefetchStream, derived_partition, root_partition
+from ._linear_common import PrefetchStream, attach_main_grad, derived_partition, root_partition
 from .broadcast import Broadcast
 from .module import Module
 from .reduce_scatter import ReduceScatter
@@ -167,6 +167,9 @@ class DistributedLinearReduceScatter(Module):
         if self.weight_buffer is None:
             weight = self.broadcast_weight(self.weight).view(self.out_features, -1)
             bias = self.broadcast_bias(self.bias).view(self.out_features) if self.bias is not None else None
+            attach_main_grad(weight, self.weight, self.broadcast_weight)
+            if bias is not None:
+                attach_main_grad(bias, self.bias, self.broadcast_bias)
         else:
             self.prefetch.wait()
             weight, bias = self.weight_buffer, self.bias_buffer

@@ -219,11 +219,16 @@ class DistributedLinearReduceScatterZero(Module):
         if mg is not None:
             w = w.view(w.shape)              # a fresh tensor object to carry the attribute
             w.main_grad = mg
+        b = self.bias_buffer
+        mgb = direct_main_grad(self.bias, self.allgather_bias, b.shape) if b is not None else None
+        if mgb is not None:
+            b = b.view(b.shape)
+            b.main_grad = mgb
         # where recipes are on, the backward pass gathers the weight shards again instead of
         # holding the gathered weight since the forward pass
         resharded = self.auto_clear_buffer and int(self.allgather_weight.P_x.shape[self.allgather_weight.axes_all_gather[0]]) > 1
         with recompute.saved_as_recipe(base, self._regather if resharded else None):
-            y = self._linear_then_scatter(input, w, self.bias_buffer)
+            y = self._linear_then_scatter(input, w, b)
         if self.auto_clear_buffer:
             self.clear_weight_buffer()
         return y

@@ -11,10 +11,16 @@ transposition copies.  It stands where the reference calls
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from .. import _native
 from ._util import ptr, stream_ptr, use_native
+
+_v, _i, _ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
+_native.declare("dd_colsum_parts", [_ll, _i])
+_native.declare("dd_colsum", [_v, _ll, _i, _v, _v, _i, _v])
 
 F_OUT_F32 = 1
 F_ACCUMULATE = 2
@@ -109,6 +115,19 @@ def weight_grad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor = None, tar
     return gemm(dy2.t(), x2.t())
 
 
+def column_sum(x2: torch.Tensor, acc: torch.Tensor = None) -> torch.Tensor:
+    """``x2.sum(0)`` of a contiguous bf16 matrix in fp32; with ``acc`` (flat fp32) added to it in place."""
+    rows, n = x2.shape
+    if rows == 0 or n % 8 or x2.data_ptr() % 16 or x2.dtype != torch.bfloat16 \
+            or not (acc is None or (acc.dtype == torch.float32 and acc.is_contiguous())):
+        s = x2.sum(0, dtype=torch.float32)
+        return s if acc is None else acc.add_(s)
+    out = acc if acc is not None else torch.empty(n, dtype=torch.float32, device=x2.device)
+    parts = torch.empty(_native.lib().dd_colsum_parts(rows, n), n, dtype=torch.float32, device=x2.device)
+    _native.call("dd_colsum", x2.data_ptr(), rows, n, parts.data_ptr(), out.data_ptr(), int(acc is not None), stream_ptr())
+    return out
+
+
 class _LinearFn(torch.autograd.Function):
     """y = x @ w.T + b with all three GEMMs on the native kernel.
 
@@ -145,10 +164,8 @@ class _LinearFn(torch.autograd.Function):
             dw = weight_grad(dy2, x2, target=ctx.wgrad)
         if ctx.has_bias and ctx.needs_input_grad[2]:
             mg = ctx.b_main_grad
-            s = dy2.sum(0, dtype=torch.float32)
-            if mg is not None:
-                mg.add_(s)
-            else:
+            s = column_sum(dy2, mg)
+            if mg is None:
                 db = s.to(dy.dtype)
         return dx, dw, db
 

@@ -197,3 +197,59 @@ def test_accumulate_into_fp32_buffer():
     acc2 = torch.zeros(1000, device="cuda")
     accumulate_f32_(acc2, g32)
     assert torch.equal(acc2, g32)
+
+
+@pytest.mark.parametrize("rows,n", [(1, 8), (33, 264), (7, 6400), (4096, 256), (5000, 1600)])
+def test_column_sum(rows, n):
+    """Fewer rows than a CTA takes, columns beyond the last full group of 256, accumulation; the same bits in
+    every run."""
+    from distdl_b200.ops.gemm import column_sum
+    torch.manual_seed(4)
+    x = torch.randn(rows, n, device="cuda").bfloat16()
+    ref = x.double().sum(0)
+    tol = 2e-6 * x.double().abs().sum(0).max()            # fp32 sums of bf16 values, in blocks
+    out = column_sum(x)
+    assert (out.double() - ref).abs().max() <= tol and torch.equal(out, column_sum(x))
+    acc = torch.randn(n, device="cuda")
+    want = acc.double() + ref
+    assert column_sum(x, acc) is acc and (acc.double() - want).abs().max() <= tol + 1e-6
+
+
+@pytest.mark.parametrize("zero,kept", [(True, False), (True, True), (False, False)])
+def test_embedding_and_linear_gradients_reach_the_fp32_accumulator(zero, kept):
+    """Parameters with an optimizer's accumulator: two backward passes add up there in fp32 and leave no .grad;
+    repeated ids, an accumulator that is not 16-byte aligned."""
+    import distdl_b200
+    from distdl_b200 import backends, nn
+    distdl_b200.config.set_backend("native", "cupy")
+    torch.manual_seed(6)
+    world = backends.backend.Partition().create_partition_inclusive([0])
+    P = world.create_cartesian_topology_partition([1, 1, 1])
+    V, d, out = 50, 24, 40
+    kw = dict(dtype=torch.bfloat16, auto_clear_buffer=not kept)
+    embed = nn.DistributedEmbeddingZero(P, V, d, **kw)
+    if zero:
+        ag = nn.DistributedLinearAllGatherZero(P, d, out, bias=True, **kw)
+        rs = nn.DistributedLinearReduceScatterZero(P, out, d, bias=True, **kw)
+    else:
+        ag = nn.DistributedLinearAllGather(P, d, out, bias=True, dtype=torch.bfloat16)
+        rs = nn.DistributedLinearReduceScatter(P, out, d, bias=True, dtype=torch.bfloat16)
+    params = [embed.weight, ag.weight, ag.bias, rs.weight, rs.bias]
+    for p in params:
+        shift = 1 if p is embed.weight else 0
+        p.main_grad_view = torch.zeros(p.numel() + 8, device="cuda")[shift:shift + p.numel()]
+    ids = torch.randint(0, 7, (2, 64), device="cuda")
+    gs = [torch.randn(2, 64, d, device="cuda").bfloat16() for _ in range(2)]
+    w = [p.detach().double().requires_grad_() for p in params]
+    w1 = (lambda t: t.reshape(d, out)) if zero else (lambda t: t.reshape(out, d).t())
+    for g in gs:
+        rs(ag(embed(ids))).backward(g)
+        h = torch.nn.functional.embedding(ids, w[0].reshape(V, d)) @ w1(w[1]) + w[2].reshape(out)
+        (h @ w[3].reshape(d, out).t() + w[4].reshape(d)).backward(g.double())
+    for m in (embed, ag, rs):
+        if hasattr(m, "clear_weight_buffer"):
+            m.clear_weight_buffer()
+    for p, r in zip(params, w):
+        assert p.grad is None
+        err = (p.main_grad_view.double() - r.grad.flatten()).norm() / r.grad.norm()
+        assert err < 1e-2, err                  # bf16 activations and incoming gradients
