@@ -88,10 +88,9 @@ inline void process_output(const InterpGeom& g, T* x, T* y, long long bc, int o0
 
 // ---------------------------------------------------------------------------------- GPU kernels
 // Both directions move each element once and are meant to run at memory speed, so a thread fixes ONE
-// spatial position, works out its source rows, columns and weights in double precision once, and then
-// walks the batch x channel planes: the index arithmetic (64-bit divisions, fp64) is paid once per
-// gridDim.y-th of the planes instead of per element.  [8, 64, 128, 128] -> 256^2 in bf16: forward
-// 437 -> 75 us, adjoint 420 -> 158 us (before: one element at a time with fp64 index
+// spatial position, takes its source rows, columns and weights (fp64 arithmetic) from a table that the CTA
+// fills together, and then walks the batch x channel planes.  [8, 64, 128, 128] -> 256^2 in bf16: forward
+// 437 -> 76 us, adjoint 420 -> 65 us; [1, 32, 46^3] -> 69^3 in fp32: 208 -> 50 and 205 -> 82 us (before: one element at a time with fp64 index
 // arithmetic and fp32 copies of the tensors around the kernel; the adjoint scattered with atomics).
 // The adjoint GATHERS: an input position collects the outputs whose support covers it, which makes it
 // deterministic and needs neither a cleared gradient nor atomics.
@@ -101,77 +100,138 @@ template <typename T> struct Acc { using type = T; };
 template <> struct Acc<__nv_bfloat16> { using type = float; };
 __device__ __forceinline__ float ld(const float* p) { return __ldg(p); }
 __device__ __forceinline__ double ld(const double* p) { return __ldg(p); }
-__device__ __forceinline__ float ld(const __nv_bfloat16* p) { return __bfloat162float(__ldg(p)); }
+__device__ __forceinline__ float ld(const __nv_bfloat16* p) {
+  return __uint_as_float((uint32_t)__ldg(reinterpret_cast<const unsigned short*>(p)) << 16);
+}
 __device__ __forceinline__ void st(float* p, float v) { *p = v; }
 __device__ __forceinline__ void st(double* p, double v) { *p = v; }
 __device__ __forceinline__ void st(__nv_bfloat16* p, float v) { *p = __float2bfloat16(v); }
-// a zero weight takes nothing from its operand, not even an infinity or a NaN
+// acc + w v, where a zero weight takes nothing from its operand, not even an infinity or a NaN: in fp32 by a mask
+// that is made once (two instructions per term), in fp64 by selection
+template <typename A> struct Weight;
+template <> struct Weight<float> {
+  float w;
+  uint32_t mask;
+  __device__ __forceinline__ void set(float v) { w = v; mask = v != 0.f ? 0xffffffffu : 0u; }
+  __device__ __forceinline__ float add(float acc, float v) const {
+    return fmaf(w, __uint_as_float(__float_as_uint(v) & mask), acc);
+  }
+};
+template <> struct Weight<double> {
+  double w;
+  __device__ __forceinline__ void set(double v) { w = v; }
+  __device__ __forceinline__ double add(double acc, double v) const { return w != 0.0 ? acc + w * v : acc; }
+};
 template <typename A> __device__ __forceinline__ A term(A w, A v) { return w != (A)0 ? w * v : (A)0; }
 
+// Where the positions of one CTA lie: consecutive positions of a plane, so that a CTA meets few different
+// columns, rows and sheets, and their source indices and weights go into a table in shared memory that the
+// CTA's threads fill together (fp64 arithmetic for tens of entries instead of three per thread).
+struct Span {
+  int col0, row0, sheet0;      // of the CTA's first position
+  int cols, rows, sheets;      // entries: columns from col0 on (around the end), rows from row0 on, sheets
+};
+__device__ __forceinline__ Span span_of(const int* n, int per_cta) {
+  const long long plane = (long long)n[0] * n[1] * n[2];
+  const long long first = blockIdx.x * (long long)per_cta;
+  const int count = (int)min((long long)per_cta, plane - first);
+  Span sp;
+  const long long row = first / n[2];
+  sp.col0 = (int)(first - row * n[2]);
+  sp.sheet0 = (int)(row / n[1]);
+  sp.row0 = (int)(row - (long long)sp.sheet0 * n[1]);
+  sp.cols = min(per_cta, n[2]);
+  sp.rows = (sp.col0 + count - 1) / n[2] + 1;
+  sp.sheets = (sp.row0 + sp.rows - 1) / n[1] + 1;
+  return sp;
+}
+// entry t of the table -> (dimension, index)
+__device__ __forceinline__ void span_entry(const Span& sp, const int* n, int t, int& d, int& i) {
+  if (t < sp.cols) { d = 2; i = sp.col0 + t; if (i >= n[2]) i -= n[2]; return; }
+  t -= sp.cols;
+  if (t < sp.rows) { d = 1; i = (sp.row0 + t) % n[1]; return; }
+  d = 0; i = sp.sheet0 + t - sp.rows;
+}
+// position number `off` of the CTA -> its entries and its indices
+__device__ __forceinline__ void span_locate(const Span& sp, const int* n, int off, int* entry, int* i) {
+  const int c = sp.col0 + off, row = c / n[2];
+  i[2] = c - row * n[2];
+  entry[2] = off < sp.cols ? off : (i[2] >= sp.col0 ? i[2] - sp.col0 : i[2] - sp.col0 + n[2]);
+  const int h = sp.row0 + row, sheet = h / n[1];
+  i[1] = h - sheet * n[1];
+  entry[1] = sp.cols + row;
+  i[0] = sp.sheet0 + sheet;
+  entry[0] = sp.cols + sp.rows + sheet;
+}
+constexpr int kMaxEntries(int per_cta) { return per_cta + 2 * (kThreads + 2); }
+
+// planes that this CTA walks
+__device__ __forceinline__ int planes_left(long long BC) { return (int)((BC - blockIdx.y + gridDim.y - 1) / gridDim.y); }
+
 // V consecutive outputs of one row per thread (V divides the row, so that a pair of bf16 leaves as one word).
-template <typename T, int ND, int V>
+// I: offsets within a plane of x, 32 bits unless a plane is larger than that.
+template <typename T, int ND, int V, typename I>
 __global__ void __launch_bounds__(kThreads)
 interp_fwd_kernel(const InterpGeom g, const T* __restrict__ x, T* __restrict__ y, long long BC) {
   using A = typename Acc<T>::type;
+  __shared__ int s_i[2][kMaxEntries(kThreads * V)];
+  __shared__ A s_w[2][kMaxEntries(kThreads * V)];
   const long long out_plane = (long long)g.out_local[0] * g.out_local[1] * g.out_local[2];
   const long long in_plane = (long long)g.in_local[0] * g.in_local[1] * g.in_local[2];
+  const Span sp = span_of(g.out_local, (int)blockDim.x * V);
+  for (int t = threadIdx.x; t < sp.cols + sp.rows + sp.sheets; t += blockDim.x) {
+    int d, o, a[2];
+    span_entry(sp, g.out_local, t, d, o);
+    A lam;
+    source_index<A>(g, d, o, a[0], a[1], lam);
+    const A w[2] = {(A)1 - lam, lam};
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const bool in = a[s] >= 0 && a[s] < g.in_local[d];
+      s_i[s][t] = in ? a[s] : 0;
+      s_w[s][t] = in ? w[s] : (A)0;
+    }
+  }
+  __syncthreads();
   const long long first = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * V;
   if (first >= out_plane) return;
-  int o[3];
-  long long r = first;
-  o[2] = (int)(r % g.out_local[2]); r /= g.out_local[2];
-  o[1] = (int)(r % g.out_local[1]);
-  o[0] = (int)(r / g.out_local[1]);
-  constexpr int D0 = 3 - ND;                       // leading dimensions of extent 1 are not interpolated
-  constexpr int NR = 1 << (ND - 1);                // source rows
-  long long row[NR];
-  A wr[NR];
-  {
-    int a[3][2] = {{0, 0}, {0, 0}, {0, 0}};
-    A w[3][2] = {{(A)1, (A)0}, {(A)1, (A)0}, {(A)1, (A)0}};
-#pragma unroll
-    for (int d = D0; d < 2; ++d) {
-      A lam;
-      source_index<A>(g, d, o[d], a[d][0], a[d][1], lam);
-      w[d][0] = (A)1 - lam; w[d][1] = lam;
-#pragma unroll
-      for (int s = 0; s < 2; ++s)
-        if (a[d][s] < 0 || a[d][s] >= g.in_local[d]) { a[d][s] = 0; w[d][s] = (A)0; }
-    }
-#pragma unroll
-    for (int i = 0; i < NR; ++i) {
-      const int s1 = i & 1, s0 = (i >> 1) & 1;
-      row[i] = ((long long)a[0][s0] * g.in_local[1] + a[1][s1]) * g.in_local[2];
-      wr[i] = w[0][s0] * w[1][s1];
-    }
-  }
-  int col[V][2];
-  A wc[V][2];
+  int entry[3], o[3];
+  span_locate(sp, g.out_local, (int)threadIdx.x * V, entry, o);
+  constexpr int NR = 1 << (ND - 1);                // source rows (leading dimensions of extent 1 are not interpolated)
+  I at[NR][V][2];
+  Weight<A> wr[NR], wc[V][2];
+  I col[V][2];
 #pragma unroll
   for (int v = 0; v < V; ++v) {
-    A lam;
-    source_index<A>(g, 2, o[2] + v, col[v][0], col[v][1], lam);
-    wc[v][0] = (A)1 - lam; wc[v][1] = lam;
+    const int e = entry[2] + v < sp.cols ? entry[2] + v : entry[2] + v - sp.cols;   // (V > 1: the row goes on)
 #pragma unroll
-    for (int s = 0; s < 2; ++s)
-      if (col[v][s] < 0 || col[v][s] >= g.in_local[2]) { col[v][s] = 0; wc[v][s] = (A)0; }
+    for (int s = 0; s < 2; ++s) { col[v][s] = s_i[s][e]; wc[v][s].set(s_w[s][e]); }
   }
-#pragma unroll 2
-  for (long long bc = blockIdx.y; bc < BC; bc += gridDim.y) {
-    const T* xb = x + bc * in_plane;
+#pragma unroll
+  for (int i = 0; i < NR; ++i) {
+    const int s1 = i & 1, s0 = (i >> 1) & 1;
+    const I row = ((I)s_i[s0][entry[0]] * g.in_local[1] + s_i[s1][entry[1]]) * g.in_local[2];
+    wr[i].set((ND >= 3 ? s_w[s0][entry[0]] : (A)1) * (ND >= 2 ? s_w[s1][entry[1]] : (A)1));
+#pragma unroll
+    for (int v = 0; v < V; ++v) { at[i][v][0] = row + col[v][0]; at[i][v][1] = row + col[v][1]; }
+  }
+  // (pointers that step from plane to plane: a 64-bit product per plane and tensor costs more than the taps)
+  const T* xb = x + blockIdx.y * in_plane;
+  T* yo = y + blockIdx.y * out_plane + first;
+  const long long xstep = gridDim.y * in_plane, ystep = gridDim.y * out_plane;
+#pragma unroll (ND >= 3 ? 1 : 2)
+  for (int left = planes_left(BC); left > 0; --left, xb += xstep, yo += ystep) {
     A acc[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) acc[v] = (A)0;
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
-      const T* p = xb + row[i];
 #pragma unroll
       for (int v = 0; v < V; ++v) {
-        const A t = term<A>(wc[v][0], ld(p + col[v][0])) + term<A>(wc[v][1], ld(p + col[v][1]));
-        acc[v] += term<A>(wr[i], t);
+        const A t = wc[v][1].add(wc[v][0].add((A)0, ld(xb + at[i][v][0])), ld(xb + at[i][v][1]));
+        acc[v] = wr[i].add(acc[v], t);
       }
     }
-    T* yo = y + bc * out_plane + first;
     if constexpr (V == 2) *reinterpret_cast<uint32_t*>(yo) = dd::pack_bf16x2(acc[0], acc[1]);
     else st(yo, acc[0]);
   }
@@ -228,72 +288,119 @@ __device__ __noinline__ typename Acc<T>::type adjoint_any(const InterpGeom& g, c
   return acc;
 }
 
-// K: outputs per dimension whose weights a thread keeps (2 and 4 unrolled in registers; 32 in local memory)
+// Outputs of dimension d that take input i: lo .. lo + n - 1 with their weights; n = -1 where more than K do.
+// WINDOW: the taps are moved to a window of K outputs that all exist (out_local[d] >= K), unused ones weigh zero.
+template <typename A, int K, bool WINDOW>
+__device__ __forceinline__ int adjoint_taps(const InterpGeom& g, int d, int i, int& lo, A* w) {
+  int hi;
+  adjoint_candidates(g, d, i, lo, hi);
+  while (lo <= hi && adjoint_weight<A>(g, d, lo, i) == (A)0) ++lo;
+  while (hi >= lo && adjoint_weight<A>(g, d, hi, i) == (A)0) --hi;
+  const int n = hi - lo + 1;
+  if (n <= 0) lo = 0;                            // nothing takes this input
+  const int shift = WINDOW && lo + K > g.out_local[d] ? lo + K - g.out_local[d] : 0;
+  lo -= shift;
+  for (int j = 0; j < K; ++j) w[j] = j >= shift && j - shift < n ? adjoint_weight<A>(g, d, lo + j, i) : (A)0;
+  return n > K ? -1 : n > 0 ? n : 0;
+}
+
+// K: outputs per dimension whose weights a thread keeps: up to four in registers, unrolled, from a table that the
+// CTA fills together, as a window of outputs whose rows and columns lie at the same offsets for every thread; 32
+// in a thread's own (local) memory, for scales above two and outputs smaller than the window.
 template <typename T, int ND, int K>
 __global__ void __launch_bounds__(kThreads)
 interp_adjoint_kernel(const InterpGeom g, T* __restrict__ x, const T* __restrict__ y, long long BC) {
   using A = typename Acc<T>::type;
+  constexpr bool TABLE = K <= 4;
+  constexpr int E = TABLE ? kMaxEntries(kThreads) : 1;
+  __shared__ int s_lo[E], s_n[E];
+  __shared__ A s_w[TABLE ? K : 1][E];
   const long long out_plane = (long long)g.out_local[0] * g.out_local[1] * g.out_local[2];
   const long long in_plane = (long long)g.in_local[0] * g.in_local[1] * g.in_local[2];
+  const Span sp = span_of(g.in_local, (int)blockDim.x);
+  if constexpr (TABLE) {
+    for (int t = threadIdx.x; t < sp.cols + sp.rows + sp.sheets; t += blockDim.x) {
+      int d, i;
+      span_entry(sp, g.in_local, t, d, i);
+      A w[K];
+      int lo = 0, n = 1;
+      if (d < 3 - ND) {                           // a leading dimension of extent 1
+#pragma unroll
+        for (int j = 0; j < K; ++j) w[j] = (A)(j == 0 ? 1 : 0);
+      } else {
+        n = adjoint_taps<A, K, true>(g, d, i, lo, w);
+      }
+      s_lo[t] = lo;
+      s_n[t] = n;
+#pragma unroll
+      for (int j = 0; j < K; ++j) s_w[j][t] = w[j];
+    }
+    __syncthreads();
+  }
   const long long pos = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (pos >= in_plane) return;
-  int i[3], lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0}, n[3] = {1, 1, 1};
-  long long r = pos;
-  i[2] = (int)(r % g.in_local[2]); r /= g.in_local[2];
-  i[1] = (int)(r % g.in_local[1]);
-  i[0] = (int)(r / g.in_local[1]);
-  constexpr int D0 = 3 - ND;
+  int entry[3], i[3], lo[3], n[3];
   A w[3][K];
-  bool fits = true;
+  span_locate(sp, g.in_local, (int)threadIdx.x, entry, i);
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
+    if constexpr (TABLE) {
+      lo[d] = s_lo[entry[d]];
+      n[d] = s_n[entry[d]];
 #pragma unroll
-    for (int j = 0; j < K; ++j) w[d][j] = (A)(j == 0 && d < D0 ? 1 : 0);
+      for (int j = 0; j < K; ++j) w[d][j] = s_w[j][entry[d]];
+    } else if (d < 3 - ND) {
+      lo[d] = 0; n[d] = 1; w[d][0] = (A)1;
+    } else {
+      n[d] = adjoint_taps<A, K, false>(g, d, i[d], lo[d], w[d]);
+    }
   }
-#pragma unroll
-  for (int d = D0; d < 3; ++d) {
-    adjoint_candidates(g, d, i[d], lo[d], hi[d]);
-    while (lo[d] <= hi[d] && adjoint_weight<A>(g, d, lo[d], i[d]) == (A)0) ++lo[d];
-    while (hi[d] >= lo[d] && adjoint_weight<A>(g, d, hi[d], i[d]) == (A)0) --hi[d];
-    n[d] = hi[d] - lo[d] + 1;
-    if (n[d] > K) { fits = false; continue; }
-    if (n[d] <= 0) { n[d] = 0; lo[d] = 0; }         // nothing takes this input: all weights stay zero
-#pragma unroll (K <= 4 ? K : 1)
-    for (int j = 0; j < K; ++j)
-      if (j < n[d]) w[d][j] = adjoint_weight<A>(g, d, lo[d] + j, i[d]);
-  }
-  if (!fits) {
+  if (n[0] < 0 || n[1] < 0 || n[2] < 0) {
+    int from[3], to[3];
+    for (int d = 0; d < 3; ++d) adjoint_candidates(g, d, i[d], from[d], to[d]);
     for (long long bc = blockIdx.y; bc < BC; bc += gridDim.y)
-      st(x + bc * in_plane + pos, adjoint_any<T>(g, y + bc * out_plane, i, lo, hi));
+      st(x + bc * in_plane + pos, adjoint_any<T>(g, y + bc * out_plane, i, from, to));
     return;
   }
   const long long base = ((long long)lo[0] * g.out_local[1] + lo[1]) * g.out_local[2] + lo[2];
-  const int s1 = g.out_local[2];
   const long long s0 = (long long)g.out_local[1] * g.out_local[2];
-#pragma unroll 1
-  for (long long bc = blockIdx.y; bc < BC; bc += gridDim.y) {
-    const T* yb = y + bc * out_plane + base;
-    A acc = (A)0;
-    if constexpr (K <= 4) {
+  if constexpr (TABLE) {
+    Weight<A> wc[K];
 #pragma unroll
-      for (int a = 0; a < (ND >= 3 ? K : 1); ++a)
+    for (int c = 0; c < K; ++c) wc[c].set(w[2][c]);
+    const T* yb = y + blockIdx.y * out_plane + base;
+    T* xo = x + blockIdx.y * in_plane + pos;
+    const long long xstep = gridDim.y * in_plane, ystep = gridDim.y * out_plane;
+#pragma unroll (ND >= 3 ? 1 : 2)
+    for (int left = planes_left(BC); left > 0; --left, xo += xstep, yb += ystep) {
+      A acc = (A)0;
+#pragma unroll
+      for (int a = 0; a < (ND >= 3 ? K : 1); ++a) {
+        A sheet = (A)0;
 #pragma unroll
         for (int b = 0; b < (ND >= 2 ? K : 1); ++b) {
+          const T* row = yb + (a * s0 + (long long)b * g.out_local[2]);
           A t = (A)0;
 #pragma unroll
-          for (int c = 0; c < K; ++c)
-            if (a < n[0] && b < n[1] && c < n[2]) t += term<A>(w[2][c], ld(yb + a * s0 + (long long)b * s1 + c));
-          acc += term<A>(w[0][a] * w[1][b], t);
+          for (int c = 0; c < K; ++c) t = wc[c].add(t, ld(row + c));
+          if (ND >= 2) { Weight<A> wb; wb.set(w[1][b]); sheet = wb.add(sheet, t); } else sheet = t;
         }
-    } else {
+        if (ND >= 3) { Weight<A> wa; wa.set(w[0][a]); acc = wa.add(acc, sheet); } else acc = sheet;
+      }
+      st(xo, acc);
+    }
+  } else {
+    for (long long bc = blockIdx.y; bc < BC; bc += gridDim.y) {
+      const T* yb = y + bc * out_plane + base;
+      A acc = (A)0;
       for (int a = 0; a < n[0]; ++a)
         for (int b = 0; b < n[1]; ++b) {
           A t = (A)0;
-          for (int c = 0; c < n[2]; ++c) t += term<A>(w[2][c], ld(yb + a * s0 + (long long)b * s1 + c));
+          for (int c = 0; c < n[2]; ++c) t += term<A>(w[2][c], ld(yb + a * s0 + (long long)b * g.out_local[2] + c));
           acc += term<A>(w[0][a] * w[1][b], t);
         }
+      st(x + bc * in_plane + pos, acc);
     }
-    st(x + bc * in_plane + pos, acc);
   }
 }
 
@@ -316,22 +423,26 @@ int run_cuda(int adjoint, const InterpGeom& g, T* x, T* y, long long BC, cudaStr
   const long long out_plane = (long long)g.out_local[0] * g.out_local[1] * g.out_local[2];
   if (!adjoint) {
     if (BC * out_plane <= 0) return 0;
+    const bool small = in_plane < 0x7fffffffLL;
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-      if (g.out_local[2] % 2 == 0 && (reinterpret_cast<uintptr_t>(y) & 3) == 0) {
+      if (small && g.out_local[2] % 2 == 0 && (reinterpret_cast<uintptr_t>(y) & 3) == 0) {
         const int t = plane_threads(out_plane / 2);
-        interp_fwd_kernel<T, ND, 2><<<plane_grid(out_plane / 2, BC, t), t, 0, s>>>(g, x, y, BC);
+        interp_fwd_kernel<T, ND, 2, int><<<plane_grid(out_plane / 2, BC, t), t, 0, s>>>(g, x, y, BC);
         return (int)cudaGetLastError();
       }
     }
     const int t = plane_threads(out_plane);
-    interp_fwd_kernel<T, ND, 1><<<plane_grid(out_plane, BC, t), t, 0, s>>>(g, x, y, BC);
+    if (small) interp_fwd_kernel<T, ND, 1, int><<<plane_grid(out_plane, BC, t), t, 0, s>>>(g, x, y, BC);
+    else       interp_fwd_kernel<T, ND, 1, long long><<<plane_grid(out_plane, BC, t), t, 0, s>>>(g, x, y, BC);
     return (int)cudaGetLastError();
   }
   if (BC * in_plane <= 0) return 0;
   if (out_plane <= 0) return (int)cudaMemsetAsync(x, 0, (size_t)(BC * in_plane) * sizeof(T), s);
   // outputs per input and dimension, as a hint: a position that has more takes the slow way by itself
   double per = 1.0;
+  int least = g.out_local[2];                       // the smallest extent must hold a whole window
   for (int d = 3 - ND; d < 3; ++d) {
+    if (g.out_local[d] < least) least = g.out_local[d];
     double step = g.scale[d];
     if (g.linear && g.align_corners)
       step = g.out_global[d] > 1 ? (double)(g.in_global[d] - 1) / (double)(g.out_global[d] - 1) : 0.0;
@@ -340,8 +451,9 @@ int run_cuda(int adjoint, const InterpGeom& g, T* x, T* y, long long BC, cudaStr
   }
   const int t = plane_threads(in_plane);
   const dim3 grid = plane_grid(in_plane, BC, t);
-  if (per <= 2.0)      interp_adjoint_kernel<T, ND, 2><<<grid, t, 0, s>>>(g, x, y, BC);
-  else if (per <= 4.0) interp_adjoint_kernel<T, ND, 4><<<grid, t, 0, s>>>(g, x, y, BC);
+  if (per <= 2.0 && least >= 2)      interp_adjoint_kernel<T, ND, 2><<<grid, t, 0, s>>>(g, x, y, BC);
+  else if (per <= 3.0 && least >= 3) interp_adjoint_kernel<T, ND, 3><<<grid, t, 0, s>>>(g, x, y, BC);
+  else if (per <= 4.0 && least >= 4) interp_adjoint_kernel<T, ND, 4><<<grid, t, 0, s>>>(g, x, y, BC);
   else                 interp_adjoint_kernel<T, ND, 32><<<grid, t, 0, s>>>(g, x, y, BC);
   return (int)cudaGetLastError();
 }

@@ -26,6 +26,10 @@ struct PoolGeom {
 template <typename T> __device__ __forceinline__ float pf(T v);
 template <> __device__ __forceinline__ float pf<float>(float v) { return v; }
 template <> __device__ __forceinline__ float pf<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+// planes that this CTA walks
+__device__ __forceinline__ int planes_left(const PoolGeom& g) {
+  return (int)((g.planes - blockIdx.y + gridDim.y - 1) / gridDim.y);
+}
 template <typename T> __device__ __forceinline__ T pt(float v);
 template <> __device__ __forceinline__ float pt<float>(float v) { return v; }
 template <> __device__ __forceinline__ __nv_bfloat16 pt<__nv_bfloat16>(float v) { return __float2bfloat16(v); }
@@ -33,10 +37,12 @@ template <> __device__ __forceinline__ __nv_bfloat16 pt<__nv_bfloat16>(float v) 
 // Both kernels are bound by memory once the index arithmetic is out of the way, so a thread fixes one
 // position of the plane, decodes it once (64-bit divisions) and walks the planes with it; windows of the
 // common sizes are unrolled so that their loads are in flight together (K / C = 0: sizes at run time).
-// [8, 64, 256, 256] bf16, max 2x2 stride 2: forward 119 -> 35 us, backward 585 -> 95 us;
-// [1, 32, 93, 93, 93] fp32, average 3^3 stride 2: 130 -> 84 and 725 -> 60 us (before: every
+// [8, 64, 256, 256] bf16, max 2x2 stride 2: forward 119 -> 26 us, backward 585 -> 28 us;
+// [1, 32, 93, 93, 93] fp32, average 3^3 stride 2: 130 -> 44 and 725 -> 61 us (before: every
 // element decoded by itself).
-template <typename T, bool MAX, int K0, int K1, int K2>
+// UNIT: neighbours along the last dimension of the window are neighbours in memory, and a plane's offsets fit
+// 32 bits, so that a row of the window is one address.
+template <typename T, bool MAX, int K0, int K1, int K2, bool UNIT>
 __global__ void __launch_bounds__(256)
 pool_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, int* __restrict__ arg, const PoolGeom g, float inv_vol) {
   const long long per_plane = (long long)g.out[0] * g.out[1] * g.out[2];
@@ -51,8 +57,12 @@ pool_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, int* __restrict__ ar
                         (long long)o2 * g.s[2] * g.xs[2];
   const long long st0 = g.d[0] * g.xs[0], st1 = g.d[1] * g.xs[1], st2 = g.d[2] * g.xs[2];
   const int ix0 = g.d[0] * g.in[1] * g.in[2], ix1 = g.d[1] * g.in[2], ix2 = g.d[2];
-  for (long long pl = blockIdx.y; pl < g.planes; pl += gridDim.y) {
-    const T* xp = x + pl * g.xs_plane + off;
+  const T* xp = x + blockIdx.y * g.xs_plane + off;
+  T* yp = y + blockIdx.y * per_plane + pos;
+  int* ap = MAX ? arg + blockIdx.y * per_plane + pos : nullptr;
+  const long long xstep = gridDim.y * g.xs_plane, ystep = gridDim.y * per_plane;
+#pragma unroll (K0 * K1 * K2 == 0 || K0 * K1 * K2 > 9 ? 1 : 4)
+  for (int left = planes_left(g); left > 0; --left, xp += xstep, yp += ystep, ap += MAX ? ystep : 0) {
     float acc = MAX ? -INFINITY : 0.f;
     int best = first;
 #pragma unroll
@@ -61,15 +71,15 @@ pool_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, int* __restrict__ ar
       for (int b = 0; b < k1; ++b)
 #pragma unroll
         for (int c = 0; c < k2; ++c) {
-          const float v = pf<T>(xp[a * st0 + b * st1 + c * st2]);
+          const float v = pf<T>(UNIT ? xp[a * (int)st0 + b * (int)st1 + c] : xp[a * st0 + b * st1 + c * st2]);
           if (MAX) {
             if (v > acc || v != v) { acc = v; best = first + a * ix0 + b * ix1 + c * ix2; }
           } else {
             acc += v;
           }
         }
-    y[pl * per_plane + pos] = pt<T>(MAX ? acc : acc * inv_vol);
-    if (MAX) arg[pl * per_plane + pos] = best;
+    *yp = pt<T>(MAX ? acc : acc * inv_vol);
+    if (MAX) *ap = best;
   }
 }
 
@@ -99,9 +109,12 @@ pool_bwd_kernel(const T* __restrict__ dy, const int* __restrict__ arg, T* __rest
   const long long base = ((long long)lo0 * g.out[1] + lo1) * g.out[2] + lo2;
   const long long row0 = (long long)g.out[1] * g.out[2];
   const int n0 = hi0 - lo0 + 1, n1 = hi1 - lo1 + 1, n2 = hi2 - lo2 + 1;
-  for (long long pl = blockIdx.y; pl < g.planes; pl += gridDim.y) {
-    const T* dyp = dy + pl * out_plane + base;
-    const int* ap = MAX ? arg + pl * out_plane + base : nullptr;
+  const T* dyp = dy + blockIdx.y * out_plane + base;
+  const int* ap = MAX ? arg + blockIdx.y * out_plane + base : nullptr;
+  T* dxp = dx + blockIdx.y * per_plane + pos;
+  const long long istep = gridDim.y * per_plane, ostep = gridDim.y * out_plane;
+#pragma unroll (C0 * C1 * C2 == 0 || C0 * C1 * C2 > 4 ? 1 : 4)
+  for (int left = planes_left(g); left > 0; --left, dyp += ostep, ap += MAX ? ostep : 0, dxp += istep) {
     float acc = 0.f;
     if constexpr (C0 > 0) {
 #pragma unroll
@@ -128,7 +141,53 @@ pool_bwd_kernel(const T* __restrict__ dy, const int* __restrict__ arg, T* __rest
         }
       }
     }
-    dx[pl * per_plane + pos] = pt<T>(MAX ? acc : acc * inv_vol);
+    *dxp = pt<T>(MAX ? acc : acc * inv_vol);
+  }
+}
+
+// Windows of 2 at stride 2 along the last dimension that tile it: two neighbouring inputs belong to the same
+// outputs, so a thread takes the pair: one position, one argument and one gradient for two results that leave
+// together.  C0, C1 as above (1 or at run time).
+template <typename T, bool MAX, int C0, int C1>
+__global__ void __launch_bounds__(256)
+pool_bwd_pair_kernel(const T* __restrict__ dy, const int* __restrict__ arg, T* __restrict__ dx, const PoolGeom g,
+                     float inv_vol) {
+  const long long per_plane = (long long)g.in[0] * g.in[1] * g.in[2];
+  const long long out_plane = (long long)g.out[0] * g.out[1] * g.out[2];
+  const long long pos = 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x);
+  if (pos >= per_plane) return;
+  const int here = (int)pos;
+  const int i2 = here % g.in[2], i1 = here / g.in[2] % g.in[1], i0 = here / g.in[2] / g.in[1];
+  int lo0, hi0, lo1, hi1;
+  cover(i0, g.k[0], g.s[0], 1, g.out[0], lo0, hi0);
+  cover(i1, g.k[1], g.s[1], 1, g.out[1], lo1, hi1);
+  const long long base = ((long long)lo0 * g.out[1] + lo1) * g.out[2] + (i2 >> 1);
+  const long long row0 = (long long)g.out[1] * g.out[2];
+  const int n0 = hi0 - lo0 + 1, n1 = hi1 - lo1 + 1;
+  const T* dyp = dy + blockIdx.y * out_plane + base;
+  const int* ap = MAX ? arg + blockIdx.y * out_plane + base : nullptr;
+  T* d = dx + blockIdx.y * per_plane + pos;
+  const long long istep = gridDim.y * per_plane, ostep = gridDim.y * out_plane;
+#pragma unroll (C0 == 1 && C1 == 1 ? 4 : 1)
+  for (int left = planes_left(g); left > 0; --left, dyp += ostep, ap += MAX ? ostep : 0, d += istep) {
+    float a0 = 0.f, a1 = 0.f;
+    for (int a = 0; a < (C0 ? C0 : n0); ++a)
+      for (int b = 0; b < (C1 ? C1 : n1); ++b)
+        if (a < n0 && b < n1) {
+          const long long o = a * row0 + (long long)b * g.out[2];
+          const float v = pf<T>(dyp[o]);
+          if (MAX) {
+            const int best = ap[o];
+            if (best == here) a0 += v;
+            if (best == here + 1) a1 += v;
+          } else {
+            a0 += v;
+            a1 += v;
+          }
+        }
+    if (!MAX) { a0 *= inv_vol; a1 *= inv_vol; }
+    if constexpr (sizeof(T) == 2) *reinterpret_cast<uint32_t*>(d) = pack_bf16x2(a0, a1);
+    else *reinterpret_cast<float2*>(d) = make_float2(a0, a1);
   }
 }
 
@@ -166,12 +225,20 @@ void launch_fwd(const void* x, void* y, int* arg, const PoolGeom& g, float inv, 
   const int t = threads_for(n), *k = g.k;
   const T* xp = reinterpret_cast<const T*>(x);
   T* yp = reinterpret_cast<T*>(y);
-  if (k[0] == 1 && k[1] == 2 && k[2] == 2)      pool_fwd_kernel<T, MAX, 1, 2, 2><<<grid, t, 0, st>>>(xp, yp, arg, g, inv);
-  else if (k[0] == 1 && k[1] == 3 && k[2] == 3) pool_fwd_kernel<T, MAX, 1, 3, 3><<<grid, t, 0, st>>>(xp, yp, arg, g, inv);
-  else if (k[0] == 2 && k[1] == 2 && k[2] == 2) pool_fwd_kernel<T, MAX, 2, 2, 2><<<grid, t, 0, st>>>(xp, yp, arg, g, inv);
-  else if (k[0] == 3 && k[1] == 3 && k[2] == 3) pool_fwd_kernel<T, MAX, 3, 3, 3><<<grid, t, 0, st>>>(xp, yp, arg, g, inv);
-  else                                          pool_fwd_kernel<T, MAX, 0, 0, 0><<<grid, t, 0, st>>>(xp, yp, arg, g, inv);
+  long long reach = 0;
+  for (int i = 0; i < 3; ++i) reach += (long long)(g.in[i] - 1) * (g.xs[i] < 0 ? -g.xs[i] : g.xs[i]);
+  const bool unit = g.xs[2] * g.d[2] == 1 && reach < 0x7fffffffLL;
+#define DD_POOL_FWD(A, B, C) do { \
+    if (unit) pool_fwd_kernel<T, MAX, A, B, C, true><<<grid, t, 0, st>>>(xp, yp, arg, g, inv); \
+    else      pool_fwd_kernel<T, MAX, A, B, C, false><<<grid, t, 0, st>>>(xp, yp, arg, g, inv); } while (0)
+  if (k[0] == 1 && k[1] == 2 && k[2] == 2)      DD_POOL_FWD(1, 2, 2);
+  else if (k[0] == 1 && k[1] == 3 && k[2] == 3) DD_POOL_FWD(1, 3, 3);
+  else if (k[0] == 2 && k[1] == 2 && k[2] == 2) DD_POOL_FWD(2, 2, 2);
+  else if (k[0] == 3 && k[1] == 3 && k[2] == 3) DD_POOL_FWD(3, 3, 3);
+  else                                          DD_POOL_FWD(0, 0, 0);
 }
+
+#undef DD_POOL_FWD
 
 template <typename T, bool MAX>
 void launch_bwd(const void* dy, const int* arg, void* dx, const PoolGeom& g, float inv, cudaStream_t st) {
@@ -184,6 +251,15 @@ void launch_bwd(const void* dy, const int* arg, void* dx, const PoolGeom& g, flo
   bool dilated = false;
   for (int i = 0; i < 3; ++i) { c[i] = (g.k[i] + g.s[i] - 1) / g.s[i]; dilated = dilated || (g.d[i] != 1 && g.k[i] > 1); }
   const int most = c[0] > c[1] ? (c[0] > c[2] ? c[0] : c[2]) : (c[1] > c[2] ? c[1] : c[2]);
+  const bool pair = g.k[2] == 2 && g.s[2] == 2 && !dilated && g.in[2] == 2 * g.out[2] &&
+                    (reinterpret_cast<uintptr_t>(dx) & 7) == 0;
+  if (pair) {
+    const dim3 half = grid_for(n / 2, g.planes);
+    const int th = threads_for(n / 2);
+    if (c[0] == 1 && c[1] == 1) pool_bwd_pair_kernel<T, MAX, 1, 1><<<half, th, 0, st>>>(dyp, arg, dxp, g, inv);
+    else                        pool_bwd_pair_kernel<T, MAX, 0, 0><<<half, th, 0, st>>>(dyp, arg, dxp, g, inv);
+    return;
+  }
   if (dilated || most > 3) pool_bwd_kernel<T, MAX, 0, 0, 0><<<grid, t, 0, st>>>(dyp, arg, dxp, g, inv);
   else if (most == 1)      pool_bwd_kernel<T, MAX, 1, 1, 1><<<grid, t, 0, st>>>(dyp, arg, dxp, g, inv);
   else if (most == 2 && c[0] == 1) pool_bwd_kernel<T, MAX, 1, 2, 2><<<grid, t, 0, st>>>(dyp, arg, dxp, g, inv);

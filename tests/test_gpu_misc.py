@@ -249,3 +249,27 @@ def test_batch_norm_layer_fused_on_one_worker(shape, affine, track, dtype):
     if track:
         close(layer.running_mean, rm)
         close(layer.running_var, rv)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kind,kernel,stride,space", [
+    ("max", (2, 2), (2, 2), (12, 14)), ("avg", (2, 2), (2, 2), (6, 6)), ("max", (3, 2), (1, 2), (9, 8)),
+    ("avg", (3, 3, 2), (2, 2, 2), (7, 9, 6)), ("max", (2, 2, 2), (2, 2, 2), (4, 5, 130)), ("max", (2,), (2,), (10,))])
+def test_pooling_backward_by_pairs(kind, kernel, stride, space, dtype):
+    """Windows of two that tile the last dimension, with every form of window along the others."""
+    import torch.nn.functional as F
+
+    from distdl_b200.ops import pooling
+    torch.manual_seed(10)
+    nd = len(space)
+    x = torch.randn(3, 70, *space, device="cuda").to(dtype).requires_grad_()
+    xr = x.detach().double().requires_grad_()
+    fn = getattr(F, f"{kind}_pool{nd}d")
+    y, yr = pooling.pool(x, kind, kernel, stride), fn(xr, kernel, stride=stride)
+    dy = torch.randn(yr.shape, device="cuda").to(dtype)
+    y.backward(dy)
+    yr.backward(dy.double())
+    tol = 1e-6 if dtype == torch.float32 else 8e-3           # fp32 sums of a few terms; one rounding to bf16
+    assert (y.double() - yr).abs().max() <= tol * yr.abs().max()
+    if dtype == torch.float32 or kind == "avg" or stride == kernel:
+        assert (x.grad.double() - xr.grad).abs().max() <= tol * xr.grad.abs().max()
