@@ -5,6 +5,7 @@ import numpy as np
 import torch
 import torch.nn.functional as F
 
+from ..ops.pad import pad
 from ..utilities.slicing import assemble_slices
 from ..utilities.torch import TensorStructure, distdl_padding_to_torch_padding, zero_volume_tensor
 from .broadcast import Broadcast
@@ -163,7 +164,7 @@ class DistributedFeatureConvBase(Module, HaloMixin, ConvMixin):
             return input
         w = self.w_broadcast(self.weight)
         b = self.b_broadcast(self.bias) if self.use_bias else None
-        x = F.pad(input, self.pad_tuple, mode="constant", value=0)
+        x = pad(input, self.pad_tuple)
         x = self.halo_layer(x)
         x = x[self.needed_slices]
         return self._local_conv(x, w, b)

@@ -2,6 +2,7 @@
 import numpy as np
 import torch.nn.functional as F
 
+from ..ops.pad import pad
 from ..utilities.slicing import assemble_slices
 from ..utilities.torch import TensorStructure, distdl_padding_to_torch_padding
 from .conv_feature import _per_dim
@@ -73,7 +74,7 @@ class DistributedPoolBase(Module, HaloMixin, PoolingMixin):
         # (without padding the copy is spared: pooling keeps nothing of its input for the backward pass)
         x = input
         if any(self.pad_tuple) or not input.is_contiguous():
-            x = F.pad(input, self.pad_tuple, mode="constant", value=self.pad_value)
+            x = pad(input, self.pad_tuple, self.pad_value)
         x = self.halo_layer(x)
         x = x[self.needed_slices]
         k = tuple(int(v) for v in self.kernel_size)

@@ -1,7 +1,7 @@
 """Upsampling of spatially partitioned tensors (``src/distdl/nn/upsampling.py:16-258``)."""
 import numpy as np
-import torch.nn.functional as F
 
+from ..ops.pad import pad
 from ..utilities.slicing import compute_start_index, compute_stop_index
 from ..utilities.torch import TensorStructure, distdl_padding_to_torch_padding
 from .halo_exchange import HaloExchange
@@ -88,6 +88,6 @@ class DistributedUpsample(Module, InterpolateMixin):
         if not self.P_x.active:
             return input
         # (without padding the copy is spared: interpolation keeps nothing of its input for the backward pass)
-        x = F.pad(input, self.pad_tuple, mode="constant", value=0) if any(self.pad_tuple) else input
+        x = pad(input, self.pad_tuple) if any(self.pad_tuple) else input
         x = self.halo_layer(x)
         return self.interp_layer(x)

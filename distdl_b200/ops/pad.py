@@ -1,0 +1,54 @@
+"""Constant padding of the spatial dimensions of ``[batch, channel, *space]`` tensors and its adjoint, the crop,
+on this library's kernel (``csrc/pad.cu``).  Stands where the reference calls ``torch.nn.functional.pad``
+(``src/distdl/nn/conv_feature.py``, ``src/distdl/nn/pooling.py``)."""
+from __future__ import annotations
+
+import ctypes
+
+import torch
+
+from .. import _native
+from ._util import stream_ptr, use_native
+
+_i3 = ctypes.c_int * 3
+_v, _ll, _i = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
+_native.declare("dd_shift_copy", [_v, _v, _i, _ll, _i3, _i3, _i3, ctypes.c_uint, _v])
+# the bits of 0 and -inf
+_FILL = {torch.bfloat16: (0, 0xFF80), torch.float16: (0, 0xFC00), torch.float32: (0, 0xFF800000)}
+
+
+def _three(v, fill):
+    v = [int(a) for a in v]
+    return _i3(*([fill] * (3 - len(v)) + v))
+
+
+class _ShiftCopyFn(torch.autograd.Function):
+    """``y[o] = x[o - lo]`` in a tensor of spatial shape ``space``, ``fill`` outside ``x``; its adjoint is the
+    shift back, filled with zeros."""
+
+    @staticmethod
+    def forward(ctx, x, lo, space, lowest):
+        ctx.lo, ctx.space = lo, tuple(x.shape[2:])
+        x = x.contiguous()
+        y = torch.empty(tuple(x.shape[:2]) + space, dtype=x.dtype, device=x.device)
+        _native.call("dd_shift_copy", x.data_ptr(), y.data_ptr(), x.element_size(), x.shape[0] * x.shape[1],
+                     _three(x.shape[2:], 1), _three(space, 1), _three(lo, 0), _FILL[x.dtype][int(lowest)], stream_ptr())
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        return _ShiftCopyFn.apply(dy, tuple(-a for a in ctx.lo), ctx.space, False), None, None, None
+
+
+def pad(x: torch.Tensor, pad_tuple, value: float = 0.0) -> torch.Tensor:
+    """``torch.nn.functional.pad(x, pad_tuple, value=value)``; function transforms and forward-mode
+    differentiation, which the kernel does not know, keep the library's operator."""
+    nd = x.dim() - 2
+    spatial, rest = pad_tuple[:2 * nd], pad_tuple[2 * nd:]
+    if (1 <= nd <= 3 and use_native(x) and x.dtype in _FILL and value in (0.0, float("-inf")) and x.numel() > 0
+            and x.is_contiguous() and any(spatial) and min(spatial) >= 0 and not any(rest)
+            and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0):
+        lo = tuple(int(a) for a in spatial[::2][::-1])
+        hi = tuple(int(a) for a in spatial[1::2][::-1])
+        return _ShiftCopyFn.apply(x, lo, tuple(int(n) + a + b for n, a, b in zip(x.shape[2:], lo, hi)), value != 0.0)
+    return torch.nn.functional.pad(x, pad_tuple, mode="constant", value=value)

@@ -251,6 +251,31 @@ def test_batch_norm_layer_fused_on_one_worker(shape, affine, track, dtype):
         close(layer.running_var, rv)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("space,pads", [((7,), (0, 1)), ((5, 8), (1, 1, 1, 1)), ((6, 5), (0, 3, 2, 0)),
+                                        ((3, 4, 13), (2, 1, 0, 0, 1, 0)), ((4, 300), (4, 0, 0, 0))])
+def test_padding_kernel_moves_the_same_bits(space, pads, dtype):
+    """Widths on either side, row lengths of every divisibility, few and many planes, 0 and -inf; gradients of
+    the first and second order; an input that is not contiguous and a function transform take the library's way."""
+    import torch.nn.functional as F
+
+    from distdl_b200.ops.pad import pad
+    torch.manual_seed(8)
+    for planes in (1, 37):
+        x = torch.randn(2, planes, *space, device="cuda").to(dtype).requires_grad_()
+        xr = x.detach().clone().requires_grad_()
+        for value in (0.0, float("-inf")):
+            y, yr = pad(x, pads, value), F.pad(xr, pads, value=value)
+            assert "ShiftCopy" in type(y.grad_fn).__name__ and torch.equal(y, yr)
+        dy = torch.randn_like(yr)
+        g, = torch.autograd.grad((pad(x, pads) * 1).pow(2).mul(dy).sum(), x, create_graph=True)
+        gr, = torch.autograd.grad((F.pad(xr, pads) * 1).pow(2).mul(dy).sum(), xr, create_graph=True)
+        assert torch.equal(g, gr)
+        assert torch.equal(torch.autograd.grad(g.sum(), x)[0], torch.autograd.grad(gr.sum(), xr)[0])
+    assert torch.equal(pad(x.transpose(0, 1), pads), F.pad(x.transpose(0, 1), pads))
+    assert torch.equal(torch.func.vmap(lambda t: pad(t, pads))(x.detach()[None]), F.pad(x.detach(), pads)[None])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("kind,kernel,stride,space", [
     ("max", (2, 2), (2, 2), (12, 14)), ("avg", (2, 2), (2, 2), (6, 6)), ("max", (3, 2), (1, 2), (9, 8)),
