@@ -49,10 +49,10 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
 //   flags       : dd::gemm::Flags
 //   max_ctas    : 0 = one CTA per SM; otherwise an upper bound (used to leave
 //                 SMs to a concurrent communication kernel)
-DD_API int dd_gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const void* B, int b_mn,
-                        long long ldb, long long strideB, void* D, long long ldd, long long strideD,
-                        const void* bias, int M, int N, int K, int batch, int flags, int max_ctas,
-                        void* stream) {
+namespace {
+int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const void* B, int b_mn, long long ldb,
+              long long strideB, void* D, long long ldd, long long strideD, const void* bias, int M, int N, int K,
+              int batch, int flags, int max_ctas, const int* rows, int bound_k, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return DD_ERR_BAD_ARG;
   if ((lda % 8) || (ldb % 8)) return DD_ERR_ALIGN;
   if (batch > 1 && ((strideA % 8) || (strideB % 8))) return DD_ERR_ALIGN;
@@ -78,6 +78,7 @@ DD_API int dd_gemm_bf16(const void* A, int a_mn, long long lda, long long stride
     q.M = M; q.N = N; q.K = K; q.batch = batch;
     q.D = D; q.ldd = ldd; q.strideD = strideD; q.bias = bias; q.flags = flags; q.group_m = 4;
     q.status = device_status(&err2);
+    q.rows = rows; q.bound_k = bound_k;
     if (err2) return err2;
     const int ptiles = ((M + 2 * g2::BM - 1) / (2 * g2::BM)) * ((N + g2::BN - 1) / g2::BN) * batch;
     int ctas = current_sm_count() & ~1;
@@ -130,4 +131,23 @@ DD_API int dd_gemm_bf16(const void* A, int a_mn, long long lda, long long stride
   if (a_mn) return launch<true, false>(ta, tb, p, grid, s);
   if (b_mn) return launch<false, true>(ta, tb, p, grid, s);
   return launch<false, false>(ta, tb, p, grid, s);
+}
+}  // namespace
+
+DD_API int dd_gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const void* B, int b_mn,
+                        long long ldb, long long strideB, void* D, long long ldd, long long strideD,
+                        const void* bias, int M, int N, int K, int batch, int flags, int max_ctas,
+                        void* stream) {
+  return gemm_bf16(A, a_mn, lda, strideA, B, b_mn, ldb, strideB, D, ldd, strideD, bias, M, N, K, batch, flags, max_ctas,
+                   nullptr, 0, stream);
+}
+
+// The same for a batch whose entry b has zeros in A after its first rows[b] rows (bound_k: whose terms of the
+// contraction after the first rows[b] are zero); rows [batch] on the device.  The result is the same: what is known
+// to be zero is not read and not multiplied, in tiles of 256 rows or blocks of 64 terms (by the CTA-pair kernel).
+DD_API int dd_gemm_bf16_rows(const void* A, int a_mn, long long lda, long long strideA, const void* B, int b_mn,
+                             long long ldb, long long strideB, void* D, long long ldd, long long strideD, int M, int N,
+                             int K, int batch, int flags, const int* rows, int bound_k, void* stream) {
+  return gemm_bf16(A, a_mn, lda, strideA, B, b_mn, ldb, strideB, D, ldd, strideD, nullptr, M, N, K, batch, flags, 0, rows,
+                   bound_k, stream);
 }

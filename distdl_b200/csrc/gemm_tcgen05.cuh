@@ -57,6 +57,10 @@ struct Params {
   int flags;
   int group_m;         // tile-order grouping (rows of tiles swept per column sweep)
   StatusRecord* status;
+  // CTA-pair kernel, batched products: A's rows after the first rows[b] (on the device, null = all live) are zero;
+  // with bound_k the terms of the contraction after the first rows[b] are.
+  const int* rows = nullptr;
+  int bound_k = 0;
 };
 
 struct SharedStorage {

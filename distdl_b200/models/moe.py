@@ -27,23 +27,25 @@ class _BatchedLinearFn(torch.autograd.Function):
     """y[e] = x[e] @ w[e].T for bf16 CUDA tensors, all three GEMMs on the native kernel."""
 
     @staticmethod
-    def forward(ctx, x, w):
-        ctx.save_for_backward(x, w)
-        return gemm(x, w)
+    def forward(ctx, x, w, rows):
+        ctx.save_for_backward(x, w, rows)
+        return gemm(x, w, rows=rows)
 
     @staticmethod
     def backward(ctx, dy):
-        x, w = ctx.saved_tensors
+        x, w, rows = ctx.saved_tensors
         dy = dy.contiguous()
-        dx = gemm(dy, w.transpose(1, 2))
-        dw = gemm(dy.transpose(1, 2), x.transpose(1, 2))
-        return dx, dw
+        dx = gemm(dy, w.transpose(1, 2), rows=rows)
+        dw = gemm(dy.transpose(1, 2), x.transpose(1, 2), rows=rows, bound_k=True)
+        return dx, dw, None
 
 
-def batched_linear(x, w):
-    """x [E, rows, in], w [E, out, in] -> [E, rows, out]."""
+def batched_linear(x, w, rows=None):
+    """x [E, rows, in], w [E, out, in] -> [E, rows, out].  ``rows`` (int32 [E]): the rows of an expert's capacity
+    that tokens take; the rows after them are zero, in ``x`` and in the gradient that comes back, and no work is
+    spent on them."""
     if x.is_cuda and x.dtype == torch.bfloat16 and w.shape[1] % 8 == 0 and w.shape[2] % 8 == 0 and x.shape[1] % 8 == 0:
-        return _BatchedLinearFn.apply(x.contiguous(), w)
+        return _BatchedLinearFn.apply(x.contiguous(), w, rows)
     return torch.einsum("ecm,enm->ecn", x, w)
 
 
@@ -169,9 +171,11 @@ class MoEFeedForward(torch.nn.Module):
         send = moe_ops.dispatch(xt, ids, slot, E, C, k)                       # [E, C, d]
         recv = _AllToAllFn.apply(send.reshape(P, El * C, d), self.ep_ranks)   # [P(src), El*C, d]
         h = recv.reshape(P, El, C, d).transpose(0, 1).reshape(El, P * C, d)
-        h = batched_linear(h, self.w_up)
+        # on one worker an expert's tokens are the first rows of its capacity: the empty rest is not multiplied
+        rows = counts if P == 1 else None
+        h = batched_linear(h, self.w_up, rows)
         h = ops.swiglu(h)
-        h = batched_linear(h, self.w_down)                                    # [El, P*C, d]
+        h = batched_linear(h, self.w_down, rows)                              # [El, P*C, d]
         back = h.reshape(El, P, C, d).transpose(0, 1).reshape(P, El * C, d)
         back = _AllToAllFn.apply(back.contiguous(), self.ep_ranks).reshape(E, C, d)
         y = moe_ops.combine(back, topw, ids, slot, T, k)

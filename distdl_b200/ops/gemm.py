@@ -19,6 +19,7 @@ from .. import _native
 from ._util import ptr, stream_ptr, use_native
 
 _v, _i, _ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
+_native.declare("dd_gemm_bf16_rows", [_v, _i, _ll, _ll, _v, _i, _ll, _ll, _v, _ll, _ll, _i, _i, _i, _i, _i, _v, _i, _v])
 _native.declare("dd_colsum_parts", [_ll, _i])
 _native.declare("dd_colsum", [_v, _ll, _i, _v, _v, _i, _v])
 
@@ -38,13 +39,18 @@ def _major(t: torch.Tensor):
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, *, bias: torch.Tensor = None,
-         accumulate: bool = False, out_dtype: torch.dtype = None, max_ctas: int = 0) -> torch.Tensor:
+         accumulate: bool = False, out_dtype: torch.dtype = None, max_ctas: int = 0, rows: torch.Tensor = None,
+         bound_k: bool = False) -> torch.Tensor:
     """``out[.., m, n] (+)= a[.., m, k] @ b[.., n, k].T (+ bias)`` on bf16 operands.
 
     ``a`` and ``b`` are *views*: pass ``w`` for ``x @ w.T``, ``w.t()`` for
     ``dy @ w``, and ``dy.t(), x.t()`` for ``dy.T @ x``; any combination of
     row-/column-contiguous views with 16-byte-aligned leading dimensions is
     accepted.  ``out`` may be bf16 or fp32 and may be a strided row-major view.
+
+    ``rows`` (int32 ``[batch]`` on the device, for 3-D operands without a bias) promises that ``a[b]`` is zero after
+    its first ``rows[b]`` rows, or, with ``bound_k``, that the terms of the contraction after the first ``rows[b]``
+    are zero: the result is the same, the work on those zeros is left out.
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16, "bf16 operands required"
     assert a.dim() == b.dim() and a.dim() in (2, 3)
@@ -79,6 +85,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, *, bias: to
         assert bias.is_contiguous() and bias.numel() == N
     ldd = out.stride(-2)
     sd = out.stride(0) if out.dim() == 3 else 0
+    if rows is not None:
+        assert bias is None and rows.dtype == torch.int32 and rows.numel() == batch and rows.is_contiguous()
+        _native.call("dd_gemm_bf16_rows", a.data_ptr(), a_mn, lda, sa, b.data_ptr(), b_mn, ldb, sb, out.data_ptr(), ldd,
+                     sd, M, N, K, batch, flags, rows.data_ptr(), int(bound_k), stream_ptr())
+        return out
     _native.call("dd_gemm_bf16", a.data_ptr(), a_mn, lda, sa, b.data_ptr(), b_mn, ldb, sb, out.data_ptr(), ldd, sd,
                  ptr(bias), M, N, K, batch, flags, max_ctas, stream_ptr())
     return out

@@ -118,3 +118,30 @@ def test_gemm_error_bound_scales_with_the_contraction_length(M, N, K):
     reft = at.double().t() @ bt.double()
     outt = gemm(at.t(), bt.t(), out_dtype=torch.float32)
     assert (outt.double() - reft).abs().max().item() < acc_term
+
+
+@pytest.mark.parametrize("C,counts", [(384, (0, 1, 256, 257, 500)), (96, (0, 5, 96, 64, 33)), (1000, (1000, 512, 0, 64, 999))])
+def test_batched_gemm_skips_zero_rows(C, counts):
+    """Rows and terms that are known to be zero: the bits are those of the full product, for no live row, counts on
+    and off the edges of tiles and k-blocks, and counts beyond the capacity; both output types."""
+    from distdl_b200 import _native
+    from distdl_b200.models.moe import batched_linear
+    from distdl_b200.ops import gemm
+    torch.manual_seed(3)
+    E, d, f = len(counts), 136, 328
+    rows = torch.tensor(counts, dtype=torch.int32, device="cuda")
+    keep = (torch.arange(C, device="cuda")[None] < rows[:, None])[..., None]
+    x = torch.where(keep, torch.randn(E, C, d, device="cuda"), torch.zeros((), device="cuda")).bfloat16()
+    dy = torch.where(keep, torch.randn(E, C, f, device="cuda"), torch.zeros((), device="cuda")).bfloat16()
+    w = torch.randn(E, f, d, device="cuda", dtype=torch.bfloat16)
+    got, want = [], []
+    for r, out in ((rows, got), (None, want)):
+        a, b = x.clone().requires_grad_(), w.clone().requires_grad_()
+        y = batched_linear(a, b, r)
+        out += [y.detach(), *torch.autograd.grad(y, (a, b), dy), gemm(x, w, out_dtype=torch.float32, rows=r),
+                gemm(dy.transpose(1, 2), x.transpose(1, 2), out_dtype=torch.float32, rows=r, bound_k=True) if r is not None
+                else gemm(dy.transpose(1, 2), x.transpose(1, 2), out_dtype=torch.float32)]
+    for g, v in zip(got, want):
+        assert torch.equal(g, v)
+    torch.cuda.synchronize()
+    assert _native.read_status()[0] == 0
