@@ -5,7 +5,7 @@ import numpy as np
 import torch
 import torch.nn.functional as F
 
-from ..ops.pad import pad
+from ..ops.pad import channels_first, channels_last_usable, pad, pad_channels_last
 from ..utilities.slicing import assemble_slices
 from ..utilities.torch import TensorStructure, distdl_padding_to_torch_padding, zero_volume_tensor
 from .broadcast import Broadcast
@@ -145,6 +145,9 @@ class DistributedFeatureConvBase(Module, HaloMixin, ConvMixin):
         lo = needed[:, 0]
         hi = needed[:, 1] + local_pad[:, 0] + local_pad[:, 1]
         self.needed_slices = assemble_slices(lo, hi)
+        # one worker whose windows read all of the padded input
+        self.whole = self.P_x.size == 1 and not np.any(lo) and \
+            bool(np.all(hi == np.asarray(input[0].shape, dtype=int) + total.sum(axis=1)))
 
     def _distdl_module_teardown(self, input):
         self.halo_layer = None
@@ -164,6 +167,9 @@ class DistributedFeatureConvBase(Module, HaloMixin, ConvMixin):
             return input
         w = self.w_broadcast(self.weight)
         b = self.b_broadcast(self.bias) if self.use_bias else None
+        if self.whole and self.groups == 1 and channels_last_usable(input, self.pad_tuple, w.shape[0]):
+            # nothing to exchange or to crop: padding and change of layout in one pass, the result back in another
+            return channels_first(self._local_conv(pad_channels_last(input, self.pad_tuple), w, b))
         x = pad(input, self.pad_tuple)
         x = self.halo_layer(x)
         x = x[self.needed_slices]

@@ -12,6 +12,7 @@ from ._util import stream_ptr, use_native
 
 _i3 = ctypes.c_int * 3
 _v, _ll, _i = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
+_native.declare("dd_shift_channels", [_v, _v, _i, _i, _i, _i, _i3, _i3, _i3, _v])
 _native.declare("dd_shift_copy", [_v, _v, _i, _ll, _i3, _i3, _i3, ctypes.c_uint, _v])
 # the bits of 0 and -inf
 _FILL = {torch.bfloat16: (0, 0xFF80), torch.float16: (0, 0xFC00), torch.float32: (0, 0xFF800000)}
@@ -38,6 +39,68 @@ class _ShiftCopyFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         return _ShiftCopyFn.apply(dy, tuple(-a for a in ctx.lo), ctx.space, False), None, None, None
+
+
+_LAST = {2: torch.channels_last, 3: torch.channels_last_3d}
+
+
+def _shift_channels(x, to_last, lo, space):
+    nd = len(space)
+    y = torch.empty(tuple(x.shape[:2]) + space, dtype=x.dtype, device=x.device,
+                    memory_format=_LAST[nd] if to_last else torch.contiguous_format)
+    _native.call("dd_shift_channels", x.data_ptr(), y.data_ptr(), int(to_last), x.element_size(), x.shape[0], x.shape[1],
+                 _three(x.shape[2:], 1), _three(space, 1), _three(lo, 0), stream_ptr())
+    return y
+
+
+class _ToChannelsLastFn(torch.autograd.Function):
+    """``y[o] = x[o - lo]``, zero outside ``x``, in channels-last memory; the adjoint of
+    :class:`_FromChannelsLastFn` with the opposite shift."""
+
+    @staticmethod
+    def forward(ctx, x, lo, space):
+        ctx.lo, ctx.space = lo, tuple(x.shape[2:])
+        return _shift_channels(x.contiguous(), True, lo, space)
+
+    @staticmethod
+    def backward(ctx, dy):
+        return _FromChannelsLastFn.apply(dy, tuple(-a for a in ctx.lo), ctx.space), None, None
+
+
+class _FromChannelsLastFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, lo, space):
+        ctx.lo, ctx.space = lo, tuple(x.shape[2:])
+        return _shift_channels(x.contiguous(memory_format=_LAST[len(space)]), False, lo, space)
+
+    @staticmethod
+    def backward(ctx, dy):
+        return _ToChannelsLastFn.apply(dy, tuple(-a for a in ctx.lo), ctx.space), None, None
+
+
+def channels_last_usable(x: torch.Tensor, pad_tuple, out_channels: int) -> bool:
+    """Whether a convolution of ``x`` should run in channels-last memory: its tensor-core kernels work in that layout
+    and convert every operand on the way in and every result on the way out otherwise."""
+    nd = x.dim() - 2
+    if nd not in _LAST or not use_native(x) or not x.is_contiguous() or x.numel() == 0 or x.shape[0] > 65535:
+        return False
+    if not (x.dtype in (torch.bfloat16, torch.float16) or (x.dtype == torch.float32 and torch.backends.cudnn.allow_tf32)):
+        return False
+    return (x.shape[1] % 8 == 0 and out_channels % 8 == 0 and min(pad_tuple) >= 0 and not any(pad_tuple[2 * nd:])
+            and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0)
+
+
+def pad_channels_last(x: torch.Tensor, pad_tuple) -> torch.Tensor:
+    """``x`` padded with zeros, in channels-last memory (see :func:`channels_last_usable`)."""
+    nd = x.dim() - 2
+    lo = tuple(int(a) for a in pad_tuple[:2 * nd:2][::-1])
+    hi = tuple(int(a) for a in pad_tuple[1:2 * nd:2][::-1])
+    return _ToChannelsLastFn.apply(x, lo, tuple(int(n) + a + b for n, a, b in zip(x.shape[2:], lo, hi)))
+
+
+def channels_first(y: torch.Tensor) -> torch.Tensor:
+    """``y.contiguous()`` of a channels-last tensor."""
+    return _FromChannelsLastFn.apply(y, (0,) * (y.dim() - 2), tuple(int(n) for n in y.shape[2:]))
 
 
 def pad(x: torch.Tensor, pad_tuple, value: float = 0.0) -> torch.Tensor:

@@ -298,3 +298,59 @@ def test_pooling_backward_by_pairs(kind, kernel, stride, space, dtype):
     assert (y.double() - yr).abs().max() <= tol * yr.abs().max()
     if dtype == torch.float32 or kind == "avg" or stride == kernel:
         assert (x.grad.double() - xr.grad).abs().max() <= tol * xr.grad.abs().max()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("space,pads,C", [((5, 7), (1, 1, 1, 1), 8), ((64, 3), (0, 2, 1, 0), 72), ((3, 4, 13), (1, 1, 0, 0, 2, 1), 136),
+                                          ((9, 9, 9), (0, 0, 0, 0, 0, 0), 24)])
+def test_padding_into_channels_last_and_back(space, pads, C, dtype):
+    """Channels below, on and beyond a tile, positions beyond a tile; the bits of padding and crop, to the second
+    order."""
+    import torch.nn.functional as F
+
+    from distdl_b200.ops.pad import channels_first, channels_last_usable, pad_channels_last
+    torch.manual_seed(12)
+    x = torch.randn(3, C, *space, device="cuda").to(dtype).requires_grad_()
+    xr = x.detach().clone().requires_grad_()
+    assert channels_last_usable(x, pads, 8)
+    y, yr = pad_channels_last(x, pads), F.pad(xr, pads)
+    fmt = torch.channels_last if len(space) == 2 else torch.channels_last_3d
+    assert y.is_contiguous(memory_format=fmt) and torch.equal(y, yr)
+    z = channels_first(y)
+    assert z.is_contiguous() and torch.equal(z, yr)
+    dy = torch.randn_like(yr)
+    g, = torch.autograd.grad((z * 1).pow(2).mul(dy).sum(), x, create_graph=True)
+    gr, = torch.autograd.grad((yr * 1).pow(2).mul(dy).sum(), xr, create_graph=True)
+    assert g.is_contiguous() and torch.equal(g, gr)
+    assert torch.equal(torch.autograd.grad(g.sum(), x)[0], torch.autograd.grad(gr.sum(), xr)[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("space,cin,cout,kernel,stride,bias", [((13, 17), 16, 24, 3, 1, True), ((12, 12), 8, 8, 1, 1, False),
+                                                               ((11, 9, 10), 24, 16, 3, 1, True), ((14, 14), 16, 16, 3, 2, False),
+                                                               ((9, 9), 12, 8, 3, 1, True)])
+def test_feature_convolution_on_one_worker(space, cin, cout, kernel, stride, bias, dtype):
+    """Layouts in and out, and all gradients, against PyTorch in fp64; channel counts that keep the old way too."""
+    import torch.nn.functional as F
+
+    import distdl_b200
+    from distdl_b200 import backends, nn
+    distdl_b200.config.set_backend("native", "cupy")
+    torch.manual_seed(13)
+    nd = len(space)
+    P = backends.backend.Partition().create_partition_inclusive([0]).create_cartesian_topology_partition([1] * (nd + 2))
+    cls = {2: nn.DistributedFeatureConv2d, 3: nn.DistributedFeatureConv3d}[nd]
+    layer = cls(P, cin, cout, kernel, stride=stride, padding=kernel // 2, bias=bias, device="cuda", dtype=dtype)
+    x = torch.randn(2, cin, *space, device="cuda").to(dtype).requires_grad_()
+    params = [layer.weight] + ([layer.bias] if bias else [])
+    ref = [t.detach().double().requires_grad_() for t in [x] + params]
+    y = layer(x)
+    yr = getattr(F, f"conv{nd}d")(ref[0], ref[1], ref[2] if bias else None, stride=stride, padding=kernel // 2)
+    assert y.is_contiguous() and y.dtype == dtype and y.shape == yr.shape
+    dy = torch.randn(yr.shape, device="cuda").to(dtype)
+    got = torch.autograd.grad(y, [x] + params, dy)
+    want = torch.autograd.grad(yr, ref, dy.double())
+    assert got[0].is_contiguous()
+    for a, b in zip([y, *got], [yr, *want]):
+        # products of tf32 (2^-11) or bf16 operands in fp32, bf16 results rounded once
+        assert (a.double() - b).norm() <= (1e-3 if dtype == torch.float32 else 4e-3) * b.norm()
