@@ -323,9 +323,10 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
       const int vi = threadIdx.x + i * kNormThreads;
       if (vi < nvec) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          pw[vi * 8 + j] = dw[i][j];
-          if (WANT_DB) pb[vi * 8 + j] = db[i][j];
+        for (int j = 0; j < 8; j += 4) {
+          *reinterpret_cast<float4*>(pw + vi * 8 + j) = make_float4(dw[i][j], dw[i][j + 1], dw[i][j + 2], dw[i][j + 3]);
+          if (WANT_DB)
+            *reinterpret_cast<float4*>(pb + vi * 8 + j) = make_float4(db[i][j], db[i][j + 1], db[i][j + 2], db[i][j + 3]);
         }
       }
     }
@@ -333,31 +334,32 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
 }
 
 // dw[c] (+)= sum_p partial[p][0][c];  db[c] (+)= sum_p partial[p][1][c]
-// Block = 32 columns x 16 part-lanes: the parts are split over the lanes and
-// folded through shared memory, so the serial chain per thread is nparts / 16.
-constexpr int kRedCols = 32, kRedLanes = 16;
+// Block = 32 columns x 32 part-lanes: the parts are split over the lanes and folded through shared memory, so the
+// serial chain of loads per thread is nparts / 32, four in flight; db's half is read only where it is wanted.
+// 2048 columns: 10.6 -> 3.4 us (16 lanes, twice the parts, both halves).
+constexpr int kRedCols = 32, kRedLanes = 32;
+__device__ __forceinline__ float fold_lane(const float* __restrict__ src, int nparts, size_t step) {
+  float s = 0.f;
+#pragma unroll 4
+  for (int p = threadIdx.y; p < nparts; p += kRedLanes) s += __ldg(src + p * step);
+  return s;
+}
 __global__ void __launch_bounds__(kRedCols * kRedLanes)
 norm_bwd_reduce_kernel(const float* __restrict__ partial, int nparts, int d,
                        float* __restrict__ dw, float* __restrict__ db, int accumulate) {
   __shared__ float s_w[kRedLanes][kRedCols + 1], s_b[kRedLanes][kRedCols + 1];
   const int col = threadIdx.x, lane = threadIdx.y;
   const int c = blockIdx.x * kRedCols + col;
-  float sw = 0.f, sb = 0.f;
-  if (c < d) {
-    for (int p = lane; p < nparts; p += kRedLanes) {
-      sw += partial[(size_t)p * 2 * d + c];
-      sb += partial[(size_t)p * 2 * d + d + c];
-    }
-  }
-  s_w[lane][col] = sw;
-  s_b[lane][col] = sb;
+  if (dw != nullptr) s_w[lane][col] = c < d ? fold_lane(partial + c, nparts, 2 * (size_t)d) : 0.f;
+  if (db != nullptr) s_b[lane][col] = c < d ? fold_lane(partial + d + c, nparts, 2 * (size_t)d) : 0.f;
   __syncthreads();
-  if (lane == 0 && c < d) {
+  if (c >= d || lane > 1) return;
+  float* out = lane == 0 ? dw : db;                        // one warp folds dw, another db
+  if (out == nullptr) return;
+  float s = 0.f;
 #pragma unroll
-    for (int l = 1; l < kRedLanes; ++l) { sw += s_w[l][col]; sb += s_b[l][col]; }
-    if (dw != nullptr) dw[c] = accumulate ? dw[c] + sw : sw;
-    if (db != nullptr) db[c] = accumulate ? db[c] + sb : sb;
-  }
+  for (int l = 0; l < kRedLanes; ++l) s += lane == 0 ? s_w[l][col] : s_b[l][col];
+  out[c] = accumulate ? out[c] + s : s;
 }
 
 // ---------------------------------------------------------------------------
@@ -765,8 +767,10 @@ static void launch_norm_bwd_any(int rms, bool want_db, int grid, cudaStream_t s,
 
 // CTAs of the backward kernel = slices of its partial-sum scratch.
 DD_API int dd_norm_bwd_parts(int rows) {
+  // two CTAs per SM are resident (about 126 registers per thread): more of them would only run one after the
+  // other and write more partial sums (3000 x 2048: 592 CTAs 20.2 us, 296 19.5 us; 4096 x 1600 with bias 29.4 and 24.4 us)
   const int groups = (rows + 1) / 2;
-  return groups < 148 * 4 ? (groups > 0 ? groups : 1) : 148 * 4;
+  return groups < 148 * 2 ? (groups > 0 ? groups : 1) : 148 * 2;
 }
 
 DD_API int dd_norm_fwd(int rms, const void* x, const void* res, void* xsum, const void* w, const void* b, void* y,
@@ -785,6 +789,7 @@ DD_API int dd_norm_bwd(int rms, const void* dy, const void* x, const void* w, co
                        void* dx, float* dw, float* db, float* partial, int accumulate, int rows, int d,
                        void* stream) {
   if (d % 8 != 0 || d > kNormThreads * kMaxVec * 8 || rows <= 0) return DD_ERR_BAD_ARG;
+  if (reinterpret_cast<uintptr_t>(partial) & 15) return DD_ERR_ALIGN;
   const int grid = dd_norm_bwd_parts(rows);
   launch_norm_bwd_any(rms, db != nullptr && partial != nullptr, grid, STREAM(stream), dy, x, w, stats, dres, dx,
                       partial, rows, d);
