@@ -567,46 +567,81 @@ colsum_fold_kernel(const float* __restrict__ partial, int parts, int n, float* _
 // Fused softmax cross-entropy over bf16 logits [rows, ld] (first V columns
 // valid).  loss[row] = lse - logit[target]; logits are overwritten by
 // (softmax - onehot) * grad_scale (columns >= V get 0).  target < 0 = ignored.
+//
+// One CTA per row, two passes (the second finds the row in L2).  Bound by instruction issue before the memory,
+// so the whole vectors run without column tests, powers of two with the scale folded into one multiply-add stand
+// for exp, and the target is looked for per vector: 8192 x 128256 1015 -> 843 us, 4096 x 50257: 227 ->
+// 187 us (two exponentials per logit alone: 470 and 93 us).
 // ---------------------------------------------------------------------------
+constexpr float kLog2e = 1.4426950408889634f;
+__device__ __forceinline__ void softmax_step(const uint4& u, float& m, float& s) {
+  float a[8];
+  unpack8(u, a);
+  float lm = fmaxf(fmaxf(fmaxf(a[0], a[1]), fmaxf(a[2], a[3])), fmaxf(fmaxf(a[4], a[5]), fmaxf(a[6], a[7])));
+  if (lm > m) { s *= exp2f((m - lm) * kLog2e); m = lm; }
+  const float ref = m == -INFINITY ? 0.f : m * kLog2e;      // (nothing but -inf so far: its powers are zero)
+  float t = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) t += exp2f(fmaf(a[j], kLog2e, -ref));
+  s += t;
+}
 __global__ void __launch_bounds__(1024)
 xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
             float* __restrict__ loss, int V, int ld, float grad_scale) {
   __shared__ float red[32];
   const long long row = blockIdx.x;
   __nv_bfloat16* lr = logits + row * (long long)ld;
-  const int nvec = ld >> 3;
+  uint4* lv = reinterpret_cast<uint4*>(lr);
+  const int nvec = ld >> 3, nfull = V >> 3, step = blockDim.x;
   float m = -INFINITY, s = 0.f;
-  for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
-    float a[8];
-    load8(lr + vi * 8, a);
-    float lm = m;
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (vi * 8 + j < V) lm = fmaxf(lm, a[j]);
-    if (lm > m) { s *= __expf(m - lm); m = lm; }
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (vi * 8 + j < V) s += __expf(a[j] - m);
+  int vi = threadIdx.x;
+  for (; vi + step < nfull; vi += 2 * step) {
+    const uint4 u0 = lv[vi], u1 = lv[vi + step];
+    softmax_step(u0, m, s);
+    softmax_step(u1, m, s);
+  }
+  if (vi < nfull) softmax_step(lv[vi], m, s);
+  if (threadIdx.x < V - nfull * 8) {                        // the columns of a last, partial vector
+    const float a = __bfloat162float(lr[nfull * 8 + threadIdx.x]);
+    if (a > m) { s *= exp2f((m - a) * kLog2e); m = a; }
+    s += exp2f(fmaf(a, kLog2e, m == -INFINITY ? 0.f : -m * kLog2e));
   }
   const float gm = block_max(m, red);
-  s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
+  s = (m == -INFINITY) ? 0.f : s * exp2f((m - gm) * kLog2e);
   s = block_sum(s, red);
   const float lse = gm + logf(s);
   const long long tgt = targets[row];
   if (threadIdx.x == 0) loss[row] = (tgt >= 0 && tgt < V) ? lse - __bfloat162float(lr[tgt]) : 0.f;
   __syncthreads();
-  const float sc = (tgt >= 0 && tgt < V) ? grad_scale : 0.f;
-  for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
+  const bool valid = tgt >= 0 && tgt < V;
+  const float sc = valid ? grad_scale : 0.f, ref = lse * kLog2e;
+  const int tv = valid ? (int)(tgt >> 3) : -1, tj = (int)(tgt & 7);
+#pragma unroll 2
+  for (vi = threadIdx.x; vi < nfull; vi += step) {
+    float a[8];
+    unpack8(lv[vi], a);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] = exp2f(fmaf(a[j], kLog2e, -ref));
+    if (vi == tv) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j == tj) a[j] -= 1.f;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] *= sc;
+    lv[vi] = pack8(a);
+  }
+  for (vi = nfull + threadIdx.x; vi < nvec; vi += step) {
     float a[8], o[8];
-    load8(lr + vi * 8, a);
+    unpack8(lv[vi], a);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int c = vi * 8 + j;
-      float p = (c < V) ? __expf(a[j] - lse) : 0.f;
+      float p = (c < V) ? exp2f(fmaf(a[j], kLog2e, -ref)) : 0.f;
       if (c == tgt) p -= 1.f;
       o[j] = p * sc;
     }
-    store8(lr + vi * 8, o);
+    lv[vi] = pack8(o);
   }
 }
 
