@@ -23,6 +23,14 @@ def _three(v, fill):
     return _i3(*([fill] * (3 - len(v)) + v))
 
 
+def _plain(x) -> bool:
+    """A tensor and a moment at which a kernel may stand for the library's operators: no subclass, no dispatch
+    mode, tracer, compiler, function transform or forward-mode differentiation, which know the operators only."""
+    return (type(x) in (torch.Tensor, torch.nn.Parameter) and torch._C._len_torch_dispatch_stack() == 0
+            and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+
+
 class _ShiftCopyFn(torch.autograd.Function):
     """``y[o] = x[o - lo]`` in a tensor of spatial shape ``space``, ``fill`` outside ``x``; its adjoint is the
     shift back, filled with zeros."""
@@ -87,7 +95,7 @@ def channels_last_usable(x: torch.Tensor, pad_tuple, out_channels: int) -> bool:
     if not (x.dtype in (torch.bfloat16, torch.float16) or (x.dtype == torch.float32 and torch.backends.cudnn.allow_tf32)):
         return False
     return (x.shape[1] % 8 == 0 and out_channels % 8 == 0 and min(pad_tuple) >= 0 and not any(pad_tuple[2 * nd:])
-            and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0)
+            and _plain(x))
 
 
 def pad_channels_last(x: torch.Tensor, pad_tuple) -> torch.Tensor:
@@ -104,13 +112,11 @@ def channels_first(y: torch.Tensor) -> torch.Tensor:
 
 
 def pad(x: torch.Tensor, pad_tuple, value: float = 0.0) -> torch.Tensor:
-    """``torch.nn.functional.pad(x, pad_tuple, value=value)``; function transforms and forward-mode
-    differentiation, which the kernel does not know, keep the library's operator."""
+    """``torch.nn.functional.pad(x, pad_tuple, value=value)``."""
     nd = x.dim() - 2
     spatial, rest = pad_tuple[:2 * nd], pad_tuple[2 * nd:]
     if (1 <= nd <= 3 and use_native(x) and x.dtype in _FILL and value in (0.0, float("-inf")) and x.numel() > 0
-            and x.is_contiguous() and any(spatial) and min(spatial) >= 0 and not any(rest)
-            and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0):
+            and x.is_contiguous() and any(spatial) and min(spatial) >= 0 and not any(rest) and _plain(x)):
         lo = tuple(int(a) for a in spatial[::2][::-1])
         hi = tuple(int(a) for a in spatial[1::2][::-1])
         return _ShiftCopyFn.apply(x, lo, tuple(int(n) + a + b for n, a, b in zip(x.shape[2:], lo, hi)), value != 0.0)

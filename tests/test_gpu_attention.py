@@ -66,12 +66,12 @@ def test_attention_backward(batch, seq, Hq, Hkv, D, causal):
 @pytest.mark.parametrize("D,Hq,Hkv,B,S", [(64, 3, 1, 2, 128), (128, 4, 2, 1, 384), (64, 25, 25, 1, 256)])
 def test_backward_with_an_output_that_is_not_16_byte_aligned(D, Hq, Hkv, B, S):
     """The row sums of O * dO read O in whatever width its address allows: the same bits either way."""
-    from distdl_b200.ops import attention as A
+    from distdl_b200.ops.attention import attention_backward, attention_forward
     torch.manual_seed(14)
     q, k, v = (torch.randn(B * S, h, D, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv))
     dout = torch.randn(B * S, Hq, D, device="cuda").bfloat16()
-    out, lse = A.attention_forward(q, k, v, B, S, True)
+    out, lse = attention_forward(q, k, v, B, S, True)
     shifted = torch.empty(out.numel() + 4, device="cuda", dtype=torch.bfloat16)[4:].view(out.shape).copy_(out)
     assert shifted.data_ptr() % 16 == 8
-    for a, b in zip(A.attention_backward(dout, q, k, v, out, lse, B, S), A.attention_backward(dout, q, k, v, shifted, lse, B, S)):
+    for a, b in zip(attention_backward(dout, q, k, v, out, lse, B, S), attention_backward(dout, q, k, v, shifted, lse, B, S)):
         assert torch.equal(a, b)
