@@ -40,6 +40,52 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   kern<<<grid, dd::gemm2::NUM_THREADS, dd::gemm2::SMEM_BYTES, stream>>>(ta, tb, td, p);
   return (int)cudaGetLastError();
 }
+
+// Second half of a split contraction: D (+)= sum_s part[s] (+ bias), the parts in order (the same bits in every
+// run).  Bound by the read of the parts, which the GEMM has just left in L2; four columns per thread.
+__global__ void __launch_bounds__(256)
+split_reduce_kernel(const float* __restrict__ part, int split, long long part_stride, int ldw, const Params p) {
+  const int quads = ldw >> 2;
+  const long long total = (long long)p.M * quads;
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= total) return;
+  const int row = (int)(i / quads), col = (int)(i - (long long)row * quads) * 4;
+  const float* src = part + (long long)row * ldw + col;
+  float4 s = __ldg(reinterpret_cast<const float4*>(src));
+#pragma unroll 4
+  for (int k = 1; k < split; ++k) {
+    const float4 t = __ldg(reinterpret_cast<const float4*>(src + k * part_stride));
+    s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
+  }
+  float v[4] = {s.x, s.y, s.z, s.w};
+  const bool add = (p.flags & F_ACCUMULATE) != 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (col + j >= p.N) break;
+    if (p.flags & F_BIAS)
+      v[j] += (p.flags & F_BIAS_F32) ? __ldg(reinterpret_cast<const float*>(p.bias) + col + j)
+                                     : __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(p.bias) + col + j));
+  }
+  const long long at = (long long)row * p.ldd + col;
+  const bool vec = col + 4 <= p.N && p.ldd % 4 == 0 && (reinterpret_cast<uintptr_t>(p.D) & 15) == 0;
+  if (p.flags & F_OUT_F32) {
+    float* d = reinterpret_cast<float*>(p.D) + at;
+    if (vec) {
+      const float4 o = add ? *reinterpret_cast<const float4*>(d) : make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(d) = make_float4(v[0] + o.x, v[1] + o.y, v[2] + o.z, v[3] + o.w);
+    } else {
+      for (int j = 0; j < 4 && col + j < p.N; ++j) d[j] = add ? d[j] + v[j] : v[j];
+    }
+  } else {
+    __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.D) + at;
+    if (vec && !add) {
+      *reinterpret_cast<uint2*>(d) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+    } else {
+      for (int j = 0; j < 4 && col + j < p.N; ++j)
+        d[j] = __float2bfloat16(add ? __bfloat162float(d[j]) + v[j] : v[j]);
+    }
+  }
+}
 }  // namespace
 
 // D[b,m,n] (+)= sum_k A[b,m,k] B[b,n,k] (+ bias[n]);  bf16 operands, fp32 accumulation.
@@ -150,4 +196,48 @@ DD_API int dd_gemm_bf16_rows(const void* A, int a_mn, long long lda, long long s
                              int K, int batch, int flags, const int* rows, int bound_k, void* stream) {
   return gemm_bf16(A, a_mn, lda, strideA, B, b_mn, ldb, strideB, D, ldd, strideD, nullptr, M, N, K, batch, flags, 0, rows,
                    bound_k, stream);
+}
+
+// Into how many parts dd_gemm_bf16_split should cut the contraction (1: not at all).  A GEMM with few output tiles
+// leaves SMs idle while each of its own walks all of K, and an SM takes in no more than about 85 GB/s, so that even
+// the read of the weights goes at a fifth of the memory rate with 16 tiles.  The parts run as a batch of the same
+// kernels into an fp32 workspace.  Measured: 33 x 4096 x 14336 split 8 ways 85.5 -> 29.0 us, 300 x 1600 x 6400 5 ways
+// 35.4 -> 19.0 us, 64 x 8 x 4096 16 ways 21.7 -> 9.7 us, error against fp64 2 to 10 times smaller (shorter sums).  A
+// k-block of 64 costs a CTA about 0.36 us, the parts and their sum about 5 us, the second launch 8 us on the host,
+// which a short GEMM does not hide: split from a gain of 8 us beyond both on.
+DD_API int dd_gemm_split(int M, int N, int K) {
+  const int sms = current_sm_count(), num_k = K / 64;
+  if (K % 64 || M <= 0 || N <= 0) return 1;
+  const bool pair = M > BM;
+  const long long tiles = (long long)((M + (pair ? 2 * BM - 1 : BM - 1)) / (pair ? 2 * BM : BM)) * ((N + BN - 1) / BN);
+  const long long slots = pair ? sms / 2 : sms;
+  int best = 1;
+  double best_gain = 8.0;
+  for (int s = 2; s <= 16 && tiles * s <= slots && num_k / s >= 4; ++s) {
+    if (num_k % s) continue;
+    const double gain = 0.36 * (num_k - num_k / s) - 13.0 - (double)s * M * N * 8.0 / 6e6;
+    if (gain > best_gain) { best_gain = gain; best = s; }
+  }
+  return best;
+}
+
+// dd_gemm_bf16 for one product whose contraction runs in `split` parts (K a multiple of 64 * split).
+// ws: split * M * (N rounded up to 4) floats, 16-byte aligned.
+DD_API int dd_gemm_bf16_split(const void* A, int a_mn, long long lda, const void* B, int b_mn, long long ldb, void* D,
+                              long long ldd, const void* bias, int M, int N, int K, int flags, int split, float* ws,
+                              void* stream) {
+  if (M <= 0 || N <= 0 || split < 1 || K <= 0 || K % (64 * split) || ws == nullptr) return DD_ERR_BAD_ARG;
+  if (reinterpret_cast<uintptr_t>(ws) & 15) return DD_ERR_ALIGN;
+  const long long kc = K / split;
+  const int ldw = (N + 3) & ~3;
+  const int r = gemm_bf16(A, a_mn, lda, a_mn ? kc * lda : kc, B, b_mn, ldb, b_mn ? kc * ldb : kc, ws, ldw,
+                          (long long)M * ldw, nullptr, M, N, (int)kc, split, F_OUT_F32, 0, nullptr, 0, stream);
+  if (r) return r;
+  Params p;
+  p.M = M; p.N = N; p.K = K; p.batch = 1;
+  p.D = D; p.ldd = ldd; p.strideD = 0; p.bias = bias; p.flags = flags; p.group_m = 1; p.status = nullptr;
+  const long long total = (long long)M * (ldw / 4);
+  split_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      ws, split, (long long)M * ldw, ldw, p);
+  return (int)cudaGetLastError();
 }

@@ -12,6 +12,7 @@ transposition copies.  It stands where the reference calls
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 
@@ -20,6 +21,8 @@ from ._util import ptr, stream_ptr, use_native
 
 _v, _i, _ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
 _native.declare("dd_gemm_bf16_rows", [_v, _i, _ll, _ll, _v, _i, _ll, _ll, _v, _ll, _ll, _i, _i, _i, _i, _i, _v, _i, _v])
+_native.declare("dd_gemm_split", [_i, _i, _i])
+_native.declare("dd_gemm_bf16_split", [_v, _i, _ll, _v, _i, _ll, _v, _ll, _v, _i, _i, _i, _i, _i, _v, _v])
 _native.declare("dd_colsum_parts", [_ll, _i])
 _native.declare("dd_colsum", [_v, _ll, _i, _v, _v, _i, _v])
 
@@ -36,6 +39,15 @@ def _major(t: torch.Tensor):
     if t.stride(-2) == 1:
         return 1, t.stride(-1), (t.stride(0) if t.dim() == 3 else 0)
     raise ValueError("GEMM operand needs unit stride in one of its last two dimensions")
+
+
+# outputs of more elements than this have tiles for half the SMs: the contraction is never split
+_SPLIT_MAX_MN = 37 * 256 * 256
+
+
+@functools.lru_cache(maxsize=1024)
+def _split(M, N, K):
+    return _native.lib().dd_gemm_split(M, N, K)
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, *, bias: torch.Tensor = None,
@@ -90,6 +102,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, *, bias: to
         _native.call("dd_gemm_bf16_rows", a.data_ptr(), a_mn, lda, sa, b.data_ptr(), b_mn, ldb, sb, out.data_ptr(), ldd,
                      sd, M, N, K, batch, flags, rows.data_ptr(), int(bound_k), stream_ptr())
         return out
+    if K >= 4096 and batch == 1 and max_ctas == 0 and M * N <= _SPLIT_MAX_MN:
+        split = _split(M, N, K)
+        if split > 1:
+            ws = torch.empty(split * M * ((N + 3) & ~3), dtype=torch.float32, device=a.device)
+            _native.call("dd_gemm_bf16_split", a.data_ptr(), a_mn, lda, b.data_ptr(), b_mn, ldb, out.data_ptr(), ldd,
+                         ptr(bias), M, N, K, flags, split, ws.data_ptr(), stream_ptr())
+            return out
     _native.call("dd_gemm_bf16", a.data_ptr(), a_mn, lda, sa, b.data_ptr(), b_mn, ldb, sb, out.data_ptr(), ldd, sd,
                  ptr(bias), M, N, K, batch, flags, max_ctas, stream_ptr())
     return out

@@ -145,3 +145,34 @@ def test_batched_gemm_skips_zero_rows(C, counts):
         assert torch.equal(g, v)
     torch.cuda.synchronize()
     assert _native.read_status()[0] == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 256, 8192), (33, 520, 6400), (128, 264, 14336), (129, 512, 8192), (200, 88, 6144),
+                                   (300, 1000, 8192), (16, 8, 4096)])
+@pytest.mark.parametrize("b_mn", [0, 1])
+def test_gemm_split_contraction(M, N, K, b_mn):
+    """Few tiles and a long contraction: bias, both output types, accumulation, strided outputs; the same bits in
+    every run, nothing written beside the output."""
+    from distdl_b200 import _native
+    from distdl_b200.ops import gemm
+    assert _native.lib().dd_gemm_split(M, N, K) > 1
+    torch.manual_seed(2)
+    a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(K, N, device="cuda", dtype=torch.bfloat16).t() if b_mn else \
+        torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
+    bias = torch.randn(N, device="cuda")
+    ref = _ref(a, b)
+    for out in (torch.full((M, N + 8), 7.0, device="cuda", dtype=torch.bfloat16), torch.full((M, N + 4), 7.0, device="cuda"),
+                torch.full((M, N + 1), 7.0, device="cuda")):
+        view = out[:, :N]
+        gemm(a, b, out=view, bias=bias)
+        # bf16 results round once (2^-8); fp32 sums of K products in another order
+        tol = 2 ** -8 if out.dtype == torch.bfloat16 else 2e-5
+        _check(view, ref + bias, tol=tol)
+        first = view.clone()
+        gemm(a, b, out=view, bias=bias)
+        assert torch.equal(view, first) and (out[:, N:] == 7.0).all()
+        gemm(a, b, out=view, accumulate=True)
+        _check(view, 2 * ref + bias, tol=2 * tol)
+    torch.cuda.synchronize()
+    assert _native.read_status()[0] == 0
