@@ -35,6 +35,9 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float
 __device__ __forceinline__ float load_as(const void* p, int dtype, int i) {
   return dtype == 0 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]) : reinterpret_cast<const float*>(p)[i];
 }
+__device__ __forceinline__ float round_as(float v, int dtype) {
+  return dtype == 0 ? __bfloat162float(__float2bfloat16(v)) : v;
+}
 __device__ __forceinline__ void store_as(void* p, int dtype, int i, float v) {
   if (dtype == 0) reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16(v);
   else reinterpret_cast<float*>(p)[i] = v;
@@ -211,10 +214,13 @@ bn_moments_kernel(const T* __restrict__ x, int B, int F, long long R, Split sp, 
   }
 }
 
-// One warp per feature: statistics of the batch, running statistics.  stat = [mean | rstd] x F.
+// One warp per feature: statistics of the batch, running statistics.  stat = [mean | rstd | sum (x - mean)] x F.
+// Sums, mean and variance take the type of x on their way, as they do where they travel between workers: the
+// results (and which of two equal values a following max pooling picks) do not depend on the number of workers.
+// The gradient kernels below round in the same places.
 __global__ void bn_moments_final_kernel(const float* __restrict__ part, int splits, int F, float count, float eps,
-                                        float* __restrict__ stat, void* run_mean, void* run_var, int run_dtype,
-                                        float momentum, float unbias) {
+                                        float* __restrict__ stat, int dtype, void* run_mean, void* run_var,
+                                        int run_dtype, float momentum, float unbias) {
   const int f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (f >= F) return;
   Moments m{0.f, 0.f, 0.f};
@@ -224,18 +230,25 @@ __global__ void bn_moments_final_kernel(const float* __restrict__ part, int spli
   }
   m = warp_merge(m);
   if (lane) return;
-  const float var = m.m2 / count;
-  stat[f] = m.mean;
+  const float mean = dtype == 0 ? round_as(round_as(m.mean * count, 0) / count, 0) : m.mean;
+  const float off = m.mean - mean;
+  const float var = round_as(round_as(m.m2 + count * off * off, dtype) / count, dtype);
+  stat[f] = mean;
   stat[F + f] = 1.f / sqrtf(var + eps);
+  stat[2 * F + f] = count * off;
   if (run_mean != nullptr) {
-    store_as(run_mean, run_dtype, f, (1.f - momentum) * load_as(run_mean, run_dtype, f) + momentum * m.mean);
-    store_as(run_var, run_dtype, f, (1.f - momentum) * load_as(run_var, run_dtype, f) + momentum * var * unbias);
+    const float keep = 1.f - momentum;
+    store_as(run_mean, run_dtype, f, round_as(keep * load_as(run_mean, run_dtype, f), run_dtype) +
+                                         round_as(momentum * mean, dtype));
+    store_as(run_var, run_dtype, f, round_as(keep * load_as(run_var, run_dtype, f), run_dtype) +
+                                        round_as(momentum * round_as(var * unbias, dtype), dtype));
   }
 }
 
-// One warp per feature: coef = [a | b | c] x F of dx = a dy + b (x - mean) + c, and the parameter gradients.
+// One warp per feature: coef = [a | b | c] x F of dx = a dy + b (x - mean) + c (through the normalisation, the
+// squared deviations and the sum), and the parameter gradients.
 __global__ void bn_grad_final_kernel(const float* __restrict__ part, int splits, int F, float count,
-                                     const float* __restrict__ stat, const void* gamma, int gamma_dtype,
+                                     const float* __restrict__ stat, int dtype, const void* gamma, int gamma_dtype,
                                      float* __restrict__ coef, void* dgamma, void* dbeta, int beta_dtype) {
   const int f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (f >= F) return;
@@ -248,15 +261,19 @@ __global__ void bn_grad_final_kernel(const float* __restrict__ part, int splits,
   if (lane) return;
   const float rstd = stat[F + f], g = gamma == nullptr ? 1.f : load_as(gamma, gamma_dtype, f);
   const float a = g * rstd;
+  const float dv = round_as(round_as(-0.5f * g * rstd * rstd * rstd * s2, dtype) / count, dtype);
+  const float dmean = round_as(round_as(-a * s1, dtype) + round_as(-2.f * dv * stat[2 * F + f], dtype), dtype);
   coef[f] = a;
-  coef[F + f] = -a * rstd * rstd * s2 / count;
-  coef[2 * F + f] = -a * s1 / count;
+  coef[F + f] = 2.f * dv;
+  coef[2 * F + f] = round_as(dmean / count, dtype);
   if (dgamma != nullptr) store_as(dgamma, gamma_dtype, f, rstd * s2);
   if (dbeta != nullptr) store_as(dbeta, beta_dtype, f, s1);
 }
 
-// Per-feature coefficients of  y = a (x - m) + c (+ e z):  given (AFFINE), or gamma * rstd, mean, beta from the
-// batch statistics (NORMALIZE).
+// Per-feature coefficients of  y = a (x - m) + c (+ e z):  given (kAffine), gamma * rstd, mean, beta from the batch
+// statistics (kNormalize), or given, the terms rounded to T one by one and added in the order e z, a (x - m), c
+// (kGradient).
+enum MapMode { kAffine, kNormalize, kGradient };
 struct Coef {
   const float *a, *m, *c, *e;
   const void *gamma, *beta;
@@ -265,7 +282,17 @@ struct Coef {
 
 // blockIdx.x walks the units of a plane (one more than fit, since a plane need not start on the grid),
 // blockIdx.y the planes.
-template <typename T, int VEC, bool NORMALIZE>
+template <typename T, MapMode MODE>
+__device__ __forceinline__ float map_value(float x, float z, bool has_z, float a, float m, float c, float ez) {
+  if (MODE == kGradient) {
+    constexpr int dt = sizeof(T) == 2 ? 0 : 1;
+    return round_as(round_as(ez * z, dt) + round_as(a * (x - m), dt), dt) + c;
+  }
+  float v = a * (x - m) + c;
+  if (has_z) v += ez * z;
+  return v;
+}
+template <typename T, int VEC, MapMode MODE>
 __global__ void __launch_bounds__(kBnThreads)
 bn_map_kernel(const T* __restrict__ x, const T* __restrict__ z, const Coef k, int F, int planes, long long R,
               T* __restrict__ y) {
@@ -278,7 +305,7 @@ bn_map_kernel(const T* __restrict__ x, const T* __restrict__ z, const Coef k, in
     float a = k.a[f];
     const float m = k.m ? k.m[f] : 0.f;
     float c = 0.f;
-    if (NORMALIZE) {
+    if (MODE == kNormalize) {
       if (k.gamma != nullptr) a *= load_as(k.gamma, k.gamma_dtype, f);
       if (k.beta != nullptr) c = load_as(k.beta, k.beta_dtype, f);
     } else if (k.c) {
@@ -286,23 +313,17 @@ bn_map_kernel(const T* __restrict__ x, const T* __restrict__ z, const Coef k, in
     }
     const float ez = z != nullptr ? k.e[f] : 0.f;
     if (VEC == 1 || (e >= p0 && e + VEC <= p1)) {
-      float v[VEC];
+      float v[VEC], w[VEC];
       load_unit<T, VEC>(x + e, v);
+      if (z != nullptr) load_unit<T, VEC>(z + e, w);
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) v[i] = a * (v[i] - m) + c;
-      if (z != nullptr) {
-        float w[VEC];
-        load_unit<T, VEC>(z + e, w);
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) v[i] += ez * w[i];
-      }
+      for (int i = 0; i < VEC; ++i) v[i] = map_value<T, MODE>(v[i], w[i], z != nullptr, a, m, c, ez);
       store_unit<T, VEC>(y + e, v);
     } else {
       for (int i = 0; i < VEC; ++i)
         if (e + i >= p0 && e + i < p1) {
-          float v = a * (to_f<T>(x[e + i]) - m) + c;
-          if (z != nullptr) v += ez * to_f<T>(z[e + i]);
-          y[e + i] = from_f<T>(v);
+          const float w = z != nullptr ? to_f<T>(z[e + i]) : 0.f;
+          y[e + i] = from_f<T>(map_value<T, MODE>(to_f<T>(x[e + i]), w, z != nullptr, a, m, c, ez));
         }
     }
   }
@@ -328,8 +349,8 @@ Split split_for(int B, int F, long long R, int vec) {
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-template <typename T>
-int map(bool normalize, const T* x, const T* z, const Coef& k, int B, int F, long long R, T* y, cudaStream_t s) {
+template <typename T, MapMode MODE>
+int map(const T* x, const T* z, const Coef& k, int B, int F, long long R, T* y, cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
   const bool vec = aligned16(x) && aligned16(y) && (z == nullptr || aligned16(z));
   const long long units = vec ? (R + V - 1) / V + 1 : R;
@@ -341,10 +362,8 @@ int map(bool normalize, const T* x, const T* z, const Coef& k, int B, int F, lon
   if (by > planes) by = planes;
   if (by > 65535) by = 65535;
   const dim3 grid((unsigned)bx, (unsigned)by);
-  if (vec && normalize)  bn_map_kernel<T, V, true><<<grid, t, 0, s>>>(x, z, k, F, (int)planes, R, y);
-  else if (vec)          bn_map_kernel<T, V, false><<<grid, t, 0, s>>>(x, z, k, F, (int)planes, R, y);
-  else if (normalize)    bn_map_kernel<T, 1, true><<<grid, t, 0, s>>>(x, z, k, F, (int)planes, R, y);
-  else                   bn_map_kernel<T, 1, false><<<grid, t, 0, s>>>(x, z, k, F, (int)planes, R, y);
+  if (vec) bn_map_kernel<T, V, MODE><<<grid, t, 0, s>>>(x, z, k, F, (int)planes, R, y);
+  else     bn_map_kernel<T, 1, MODE><<<grid, t, 0, s>>>(x, z, k, F, (int)planes, R, y);
   return (int)cudaGetLastError();
 }
 
@@ -371,10 +390,11 @@ int train_fwd(const T* x, const void* gamma, const void* beta, int gamma_dtype, 
   if (vec) bn_moments_kernel<T, V><<<grid, kBnThreads, 0, s>>>(x, B, F, R, sp, ws);
   else     bn_moments_kernel<T, 1><<<grid, kBnThreads, 0, s>>>(x, B, F, R, sp, ws);
   const double n = (double)B * (double)R;
-  bn_moments_final_kernel<<<(F + 7) / 8, 256, 0, s>>>(ws, splits, F, (float)n, eps, stat, run_mean, run_var, run_dtype,
-                                                      momentum, (float)(n / (n - 1.0 > 1.0 ? n - 1.0 : 1.0)));
+  bn_moments_final_kernel<<<(F + 7) / 8, 256, 0, s>>>(ws, splits, F, (float)n, eps, stat,
+                                                      sizeof(T) == 2 ? 0 : 1, run_mean, run_var, run_dtype, momentum,
+                                                      (float)(n / (n - 1.0 > 1.0 ? n - 1.0 : 1.0)));
   Coef k{stat + F, stat, nullptr, nullptr, gamma, beta, gamma_dtype, beta_dtype};
-  return map<T>(true, x, nullptr, k, B, F, R, y, s);
+  return map<T, kNormalize>(x, nullptr, k, B, F, R, y, s);
 }
 
 template <typename T>
@@ -384,12 +404,12 @@ int train_bwd(const T* x, const T* dy, const void* gamma, int gamma_dtype, int b
   const Split sp = split_for(B, F, R, vec ? 16 / (int)sizeof(T) : 1);
   int r = reduce<T, true>(x, dy, stat, B, F, R, 2, sp, vec, ws, nullptr, s);
   if (r) return r;
-  bn_grad_final_kernel<<<(F + 7) / 8, 256, 0, s>>>(ws, sp.su * sp.sb, F, (float)((double)B * (double)R), stat, gamma,
-                                                   gamma_dtype, coef, dgamma, dbeta, beta_dtype);
+  bn_grad_final_kernel<<<(F + 7) / 8, 256, 0, s>>>(ws, sp.su * sp.sb, F, (float)((double)B * (double)R), stat,
+                                                   sizeof(T) == 2 ? 0 : 1, gamma, gamma_dtype, coef, dgamma, dbeta, beta_dtype);
   if (dx == nullptr) return (int)cudaGetLastError();
-  // dx = b (x - mean) + c + a dy
+  // dx = a dy + b (x - mean) + c
   Coef k{coef + F, stat, coef + 2 * F, coef, nullptr, nullptr, 1, 1};
-  return map<T>(false, x, dy, k, B, F, R, dx, s);
+  return map<T, kGradient>(x, dy, k, B, F, R, dx, s);
 }
 
 }  // namespace
@@ -418,9 +438,9 @@ DD_API int dd_bn_affine(const void* x, const void* z, const float* a, const floa
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   Coef k{a, m, c, e, nullptr, nullptr, 1, 1};
   if (dtype == 0)
-    return map<__nv_bfloat16>(false, reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(z),
+    return map<__nv_bfloat16, kAffine>(reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(z),
                               k, B, F, R, reinterpret_cast<__nv_bfloat16*>(y), s);
-  return map<float>(false, reinterpret_cast<const float*>(x), reinterpret_cast<const float*>(z), k, B, F, R,
+  return map<float, kAffine>(reinterpret_cast<const float*>(x), reinterpret_cast<const float*>(z), k, B, F, R,
                     reinterpret_cast<float*>(y), s);
 }
 
@@ -435,8 +455,8 @@ DD_API int dd_bn_train_workspace(int B, int F, long long R) {
   return 3 * most * F;
 }
 
-// Batch norm of one worker's whole batch.  stat: [2, F] fp32 (mean, 1 / sqrt(var + eps)), kept for the backward
-// pass; gamma / beta / run_*: [F] in their own types (0 = bf16, 1 = fp32) or null.
+// Batch norm of one worker's whole batch.  stat: [3, F] fp32 (mean, 1 / sqrt(var + eps), sum (x - mean)), kept for the
+// backward pass; gamma / beta / run_*: [F] in their own types (0 = bf16, 1 = fp32) or null.
 DD_API int dd_bn_train_fwd(const void* x, const void* gamma, const void* beta, int gamma_dtype, int beta_dtype, int B,
                            int F, long long R, int dtype, float eps, void* run_mean, void* run_var, int run_dtype,
                            float momentum, float* ws, float* stat, void* y, void* stream) {

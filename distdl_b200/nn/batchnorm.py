@@ -133,7 +133,7 @@ class DistributedBatchNorm(Module):
 
     def _alone(self, input, bn_ops):
         """One worker holds the whole batch that the layer was set up for: nothing travels between the passes,
-        so that they run fused (the statistics then stay in fp32 instead of the input's type in between)."""
+        so that they run fused."""
         if self.P_x.size != 1 or self.global_count != float(np.prod(input.shape) / input.shape[1]):
             return False
         features = ([self.gamma, self.beta] if self.affine else []) + \

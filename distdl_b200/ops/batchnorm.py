@@ -115,7 +115,7 @@ class _TrainBatchNorm(torch.autograd.Function):
     def forward(ctx, x, gamma, beta, eps, running_mean, running_var, momentum):
         B, F, R = _geometry(x)
         ws = torch.empty(_native.lib().dd_bn_train_workspace(B, F, R), dtype=torch.float32, device=x.device)
-        stat = torch.empty(2, F, dtype=torch.float32, device=x.device)
+        stat = torch.empty(3, F, dtype=torch.float32, device=x.device)
         y = torch.empty_like(x)
         _native.call("dd_bn_train_fwd", x.data_ptr(), ptr(gamma), ptr(beta), 1 if gamma is None else _DT[gamma.dtype],
                      1 if beta is None else _DT[beta.dtype], B, F, R, _DT[x.dtype], eps, ptr(running_mean),
