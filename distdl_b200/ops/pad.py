@@ -86,15 +86,23 @@ class _FromChannelsLastFn(torch.autograd.Function):
         return _ToChannelsLastFn.apply(dy, tuple(-a for a in ctx.lo), ctx.space), None, None
 
 
-def channels_last_usable(x: torch.Tensor, pad_tuple, out_channels: int) -> bool:
+def channels_last_usable(x: torch.Tensor, pad_tuple, weight: torch.Tensor, stride, dilation) -> bool:
     """Whether a convolution of ``x`` should run in channels-last memory: its tensor-core kernels work in that layout
     and convert every operand on the way in and every result on the way out otherwise."""
     nd = x.dim() - 2
     if nd not in _LAST or not use_native(x) or not x.is_contiguous() or x.numel() == 0 or x.shape[0] > 65535:
         return False
-    if not (x.dtype in (torch.bfloat16, torch.float16) or (x.dtype == torch.float32 and torch.backends.cudnn.allow_tf32)):
+    if x.dtype == torch.float32:
+        # channels-last fp32 runs in tf32.  Channels-first does so as well only for some shapes: for 3 x 3 x 3 windows
+        # on volumes with 16 channels or more always (errors against fp64 alike, 2.9e-4), for images, 1 x 1 windows or
+        # fewer channels it may take fp32 kernels (2e-7), which must stay
+        if not (nd == 3 and torch.backends.cudnn.allow_tf32 and min(x.shape[1], weight.shape[0]) >= 16
+                and tuple(weight.shape[2:]) == (3, 3, 3) and all(int(s) == 1 for s in stride)
+                and all(int(d) == 1 for d in dilation)):
+            return False
+    elif x.dtype not in (torch.bfloat16, torch.float16):
         return False
-    return (x.shape[1] % 8 == 0 and out_channels % 8 == 0 and min(pad_tuple) >= 0 and not any(pad_tuple[2 * nd:])
+    return (x.shape[1] % 8 == 0 and weight.shape[0] % 8 == 0 and min(pad_tuple) >= 0 and not any(pad_tuple[2 * nd:])
             and _plain(x))
 
 

@@ -314,7 +314,12 @@ def test_padding_into_channels_last_and_back(space, pads, C, dtype):
     torch.manual_seed(12)
     x = torch.randn(3, C, *space, device="cuda").to(dtype).requires_grad_()
     xr = x.detach().clone().requires_grad_()
-    assert channels_last_usable(x, pads, 8)
+    nd = len(space)
+    w = torch.empty(16, C, *[3] * nd, device="cuda", dtype=dtype)
+    one = (1,) * nd
+    # fp32 only where the library's channels-first kernels run in tf32 too
+    assert channels_last_usable(x, pads, w, one, one) == (dtype != torch.float32 or (nd == 3 and C >= 16))
+    assert not channels_last_usable(x.float(), pads, w[..., :1], one, one)
     y, yr = pad_channels_last(x, pads), F.pad(xr, pads)
     fmt = torch.channels_last if len(space) == 2 else torch.channels_last_3d
     assert y.is_contiguous(memory_format=fmt) and torch.equal(y, yr)
