@@ -253,3 +253,46 @@ def test_embedding_and_linear_gradients_reach_the_fp32_accumulator(zero, kept):
         assert p.grad is None
         err = (p.main_grad_view.double() - r.grad.flatten()).norm() / r.grad.norm()
         assert err < 1e-2, err                  # bf16 activations and incoming gradients
+
+
+@pytest.mark.parametrize("V,ld", [(5, 8), (4099, 4104), (40003, 40008), (16384, 16384)])
+@pytest.mark.parametrize("fill", [torch.finfo(torch.bfloat16).min, float("-inf"), torch.finfo(torch.bfloat16).max, -1e38])
+def test_xent_with_masked_and_extreme_logits(V, ld, fill):
+    """Masks over whole and partial vectors, over all columns but one, in front of and behind what a thread reads
+    first, masked targets and ignored rows, in rows of less and of more than one sweep of the CTA: loss and gradient
+    of each row against fp64."""
+    from distdl_b200 import _native
+    from distdl_b200.ops._util import stream_ptr
+    torch.manual_seed(11)
+    low, rows = fill < 0, 8
+    lg = torch.randn(rows, ld, device="cuda").mul_(3).bfloat16()
+    third = V // 3
+    if low:                                                 # (fp32 has no room for a log beside several of 3e38)
+        lg[0, :third] = fill                                # whole vectors and one in part, seen first; the target
+        lg[1, -(ld - V) - third - 1:] = fill                # seen last, up to the partial vector
+        lg[2, torch.rand(ld, device="cuda") < 0.9] = fill   # here and there
+        lg[3, :] = fill                                     # all but one column
+        lg[3, V - 1] = 2.0
+        lg[4, :third] = -torch.finfo(torch.bfloat16).max    # two kinds of mask beside each other
+        lg[4, third:2 * third] = float("-inf")
+    lg[5, 0] = fill                                         # one logit
+    tgt = torch.tensor([0, 0, V // 2, V - 1, V - 1, 0, -100, V], device="cuda")
+    lg[2, V // 2] = 1.0
+    scale = 0.5
+    a = lg[:, :V].double()
+    ok = (tgt >= 0) & (tgt < V)
+    t = tgt.clamp(0, V - 1)
+    lse = torch.logsumexp(a, 1)
+    want = torch.where(ok, lse - a.gather(1, t[:, None])[:, 0], 0.0)
+    grad = torch.softmax(a, 1)
+    grad[torch.arange(rows), t] -= 1.0
+    grad = torch.where(ok[:, None], grad * scale, 0.0)
+    loss = torch.empty(rows, device="cuda")
+    _native.call("dd_xent", lg.data_ptr(), tgt.data_ptr(), loss.data_ptr(), rows, V, ld, scale, stream_ptr())
+    same = (loss.double() == want) | (torch.isinf(want) & (loss == want.float()))
+    # fp32: a few roundings of the largest value that takes part, and of a sum of V terms added in blocks
+    assert (same | ((loss.double() - want).abs() <= 1e-6 * (lse.abs() + want.abs()) + 1e-5)).all(), (loss, want)
+    # probabilities carry the rounding of lse (2^-24 |lse|) and are rounded to bf16
+    tol = grad.abs() * (2 ** -8 + 4e-7 * lse.abs().clamp(max=1e4)[:, None]) + 1e-6
+    assert ((lg[:, :V].double() - grad).abs() <= tol).all()
+    assert (lg[:, V:] == 0).all()
