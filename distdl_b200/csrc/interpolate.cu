@@ -423,6 +423,9 @@ int run_cuda(int adjoint, const InterpGeom& g, T* x, T* y, long long BC, cudaStr
   const long long out_plane = (long long)g.out_local[0] * g.out_local[1] * g.out_local[2];
   if (!adjoint) {
     if (BC * out_plane <= 0) return 0;
+    // an empty slab of the input gives nothing to any output, and holds no element that the kernel could read with
+    // weight zero
+    if (in_plane <= 0) return (int)cudaMemsetAsync(y, 0, (size_t)(BC * out_plane) * sizeof(T), s);
     const bool small = in_plane < 0x7fffffffLL;
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
       if (small && g.out_local[2] % 2 == 0 && (reinterpret_cast<uintptr_t>(y) & 3) == 0) {

@@ -203,6 +203,23 @@ def test_interpolation_kernels_over_scales(mode, ac, n_in, n_out, dtype):
         assert torch.equal(interpolate(bad.cuda(), *args).isfinite().cpu(), interpolate(bad.double(), *args).isfinite())
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16])
+@pytest.mark.parametrize("mode", ["linear", "nearest"])
+@pytest.mark.parametrize("n_in", [(0,), (0, 5), (4, 0), (0, 3, 4), (3, 0, 4), (3, 4, 0)])
+def test_interpolation_of_an_empty_slab(n_in, mode, dtype):
+    """A worker may hold none of the input's entries along a dimension: zeros, as the CPU code writes them, and a
+    gradient without elements."""
+    from distdl_b200.functional.interpolate import interpolate
+    nd = len(n_in)
+    n_global, n_out = [6] * nd, [7] * nd
+    args = ([2] * nd, [2 + n for n in n_in], n_global, [0] * nd, n_out, n_out, None, mode, False)
+    x = torch.empty(2, 3, *n_in, device="cuda", dtype=dtype, requires_grad=True)
+    y = interpolate(x, *args)
+    assert y.dtype == dtype and torch.equal(y.double().cpu(), interpolate(x.detach().double().cpu(), *args))
+    assert y.shape == (2, 3, *n_out) and not y.any()
+    assert torch.autograd.grad(y.sum(), x)[0].shape == x.shape
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape,affine,track", [
     ((6, 5, 7, 9), True, True),             # planes of 63: units shared between neighbours
