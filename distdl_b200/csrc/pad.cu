@@ -82,19 +82,15 @@ int run(const void* src, void* dst, const ShiftGeom& g, W fill, cudaStream_t s) 
 
 // ------------------------------------------------------------------ between channels-first and channels-last
 // The same shifted copy into or out of the layout [batch, n0, n1, n2, C] that the tensor-core convolutions work in,
-// so that padding, crop and change of layout are one pass.  A CTA moves 64 positions of 32 words of channels (a
-// word: two 2-byte channels or one of 4 bytes) through shared memory: channels-first side 64 positions at a time,
-// channels-last side 16 bytes per thread, both without bank conflicts (pitch 65).  [8, 64, 256, 256] bf16, padded by
-// one: 48 us to channels-last, 34 us back (the library's own conversion inside the convolution: 64 and 46
-// behind 31 and 26 for padding and crop); [1, 32, 93^3] fp32: 70 and 43 us.
+// so that padding, crop and change of layout are one pass, for 2-byte elements.  A CTA moves 64 positions of 32 words
+// (pairs of channels) through shared memory: channels-first side 64 positions at a time, channels-last side 16 bytes
+// per thread, both without bank conflicts (pitch 65).  [8, 64, 256, 256] bf16, padded by one: 48 us to channels-last,
+// 34 us back (the library's own conversion inside the convolution: 64 and 46 behind 31 and 26 for padding and crop).
 constexpr int kPos = 64, kWords = 32, kPitch = kPos + 1;
 
-template <typename W> __device__ __forceinline__ uint32_t gather_word(const W* p, long long step, bool live, W fill);
-template <> __device__ __forceinline__ uint32_t gather_word<uint32_t>(const uint32_t* p, long long, bool live, uint32_t fill) {
-  return live ? __ldg(p) : fill;
-}
-template <> __device__ __forceinline__ uint32_t gather_word<uint16_t>(const uint16_t* p, long long step, bool live, uint16_t fill) {
-  const uint32_t a = live ? __ldg(p) : fill, b = live ? __ldg(p + step) : fill;
+// the pair of channels at p, zero outside
+__device__ __forceinline__ uint32_t gather_pair(const uint16_t* p, long long step, bool live) {
+  const uint32_t a = live ? __ldg(p) : 0, b = live ? __ldg(p + step) : 0;
   return a | (b << 16);
 }
 
@@ -107,29 +103,27 @@ __device__ __forceinline__ long long source_position(const ShiftGeom& g, long lo
   return live ? ((long long)i0 * g.in[1] + i1) * g.in[2] + i2 : -1;
 }
 
-template <typename W>
 __global__ void __launch_bounds__(256)
-to_channels_last_kernel(const W* __restrict__ src, W* __restrict__ dst, const ShiftGeom g, int C) {
-  constexpr int CPW = 4 / sizeof(W);                       // channels per word
+to_channels_last_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, const ShiftGeom g, int C) {
   __shared__ uint32_t tile[kWords][kPitch];
   const long long out_plane = (long long)g.out[0] * g.out[1] * g.out[2];
   const long long in_plane = (long long)g.in[0] * g.in[1] * g.in[2];
   const long long p0 = blockIdx.x * (long long)kPos;
-  const int c0 = blockIdx.y * kWords * CPW;
+  const int c0 = blockIdx.y * kWords * 2;
   {
     const int pos = threadIdx.x & (kPos - 1), w0 = threadIdx.x / kPos;
     const long long at = p0 + pos < out_plane ? source_position(g, p0 + pos) : -1;
-    const W* s = src + ((long long)blockIdx.z * C + c0 + w0 * CPW) * in_plane + (at < 0 ? 0 : at);
+    const uint16_t* s = src + ((long long)blockIdx.z * C + c0 + w0 * 2) * in_plane + (at < 0 ? 0 : at);
 #pragma unroll
     for (int w = w0; w < kWords; w += 256 / kPos) {
-      if (c0 + w * CPW < C) tile[w][pos] = gather_word<W>(s, in_plane, at >= 0, (W)0);
-      s += 256 / kPos * CPW * in_plane;
+      if (c0 + w * 2 < C) tile[w][pos] = gather_pair(s, in_plane, at >= 0);
+      s += 256 / kPos * 2 * in_plane;
     }
   }
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < kPos * 8 / 256; ++k) {
-    const int idx = threadIdx.x + 256 * k, chunk = idx & 7, pos = idx >> 3, c = c0 + chunk * 4 * CPW;
+    const int idx = threadIdx.x + 256 * k, chunk = idx & 7, pos = idx >> 3, c = c0 + chunk * 8;
     if (c >= C || p0 + pos >= out_plane) continue;
     const uint4 v = make_uint4(tile[chunk * 4][pos], tile[chunk * 4 + 1][pos], tile[chunk * 4 + 2][pos],
                                tile[chunk * 4 + 3][pos]);
@@ -137,18 +131,16 @@ to_channels_last_kernel(const W* __restrict__ src, W* __restrict__ dst, const Sh
   }
 }
 
-template <typename W>
 __global__ void __launch_bounds__(256)
-from_channels_last_kernel(const W* __restrict__ src, W* __restrict__ dst, const ShiftGeom g, int C) {
-  constexpr int CPW = 4 / sizeof(W);
+from_channels_last_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, const ShiftGeom g, int C) {
   __shared__ uint32_t tile[kWords][kPitch];
   const long long out_plane = (long long)g.out[0] * g.out[1] * g.out[2];
   const long long in_plane = (long long)g.in[0] * g.in[1] * g.in[2];
   const long long p0 = blockIdx.x * (long long)kPos;
-  const int c0 = blockIdx.y * kWords * CPW;
+  const int c0 = blockIdx.y * kWords * 2;
 #pragma unroll
   for (int k = 0; k < kPos * 8 / 256; ++k) {
-    const int idx = threadIdx.x + 256 * k, chunk = idx & 7, pos = idx >> 3, c = c0 + chunk * 4 * CPW;
+    const int idx = threadIdx.x + 256 * k, chunk = idx & 7, pos = idx >> 3, c = c0 + chunk * 8;
     if (c >= C || p0 + pos >= out_plane) continue;
     const long long at = source_position(g, p0 + pos);
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -159,15 +151,15 @@ from_channels_last_kernel(const W* __restrict__ src, W* __restrict__ dst, const 
   __syncthreads();
   const int pos = threadIdx.x & (kPos - 1), w0 = threadIdx.x / kPos;
   if (p0 + pos >= out_plane) return;
-  W* d = dst + ((long long)blockIdx.z * C + c0 + w0 * CPW) * out_plane + p0 + pos;
+  uint16_t* d = dst + ((long long)blockIdx.z * C + c0 + w0 * 2) * out_plane + p0 + pos;
 #pragma unroll
   for (int w = w0; w < kWords; w += 256 / kPos) {
-    if (c0 + w * CPW < C) {
+    if (c0 + w * 2 < C) {
       const uint32_t v = tile[w][pos];
-      d[0] = (W)v;
-      if constexpr (CPW == 2) d[out_plane] = (W)(v >> 16);
+      d[0] = (uint16_t)v;
+      d[out_plane] = (uint16_t)(v >> 16);
     }
-    d += 256 / kPos * CPW * out_plane;
+    d += 256 / kPos * 2 * out_plane;
   }
 }
 
@@ -187,13 +179,11 @@ DD_API int dd_shift_copy(const void* src, void* dst, int esize, long long planes
   return esize == 2 ? run<uint16_t>(src, dst, g, (uint16_t)fill, s) : run<uint32_t>(src, dst, g, fill, s);
 }
 
-// The same between [B, C, in...] and [B, out..., C] (to_last = 1) or [B, in..., C] and [B, C, out...] (to_last = 0),
-// filled with zeros.  C: a multiple of 8 (2-byte elements) or 4; the channels-last tensor 16-byte aligned.
-DD_API int dd_shift_channels(const void* src, void* dst, int to_last, int esize, int B, int C, const int* in,
-                             const int* out, const int* lo, void* stream) {
-  if (src == nullptr || dst == nullptr || B <= 0 || B > 65535 || C <= 0 || (esize != 2 && esize != 4) ||
-      C % (16 / esize))
-    return DD_ERR_BAD_ARG;
+// The same between [B, C, in...] and [B, out..., C] (to_last = 1) or [B, in..., C] and [B, C, out...] (to_last = 0) of
+// 2-byte elements, filled with zeros.  C: a multiple of 8; the channels-last tensor 16-byte aligned.
+DD_API int dd_shift_channels(const void* src, void* dst, int to_last, int B, int C, const int* in, const int* out,
+                             const int* lo, void* stream) {
+  if (src == nullptr || dst == nullptr || B <= 0 || B > 65535 || C <= 0 || C % 8) return DD_ERR_BAD_ARG;
   if (reinterpret_cast<uintptr_t>(to_last ? dst : src) & 15) return DD_ERR_ALIGN;
   ShiftGeom g;
   g.planes = 0;
@@ -202,12 +192,9 @@ DD_API int dd_shift_channels(const void* src, void* dst, int to_last, int esize,
     g.in[i] = in[i]; g.out[i] = out[i]; g.lo[i] = lo[i];
   }
   const long long n = (long long)out[0] * out[1] * out[2];
-  const int tc = kWords * 4 / esize;
-  const dim3 grid((unsigned)((n + kPos - 1) / kPos), (unsigned)((C + tc - 1) / tc), (unsigned)B);
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-#define DD_CL(K, W) K<W><<<grid, 256, 0, s>>>(reinterpret_cast<const W*>(src), reinterpret_cast<W*>(dst), g, C)
-  if (to_last) { if (esize == 2) DD_CL(to_channels_last_kernel, uint16_t); else DD_CL(to_channels_last_kernel, uint32_t); }
-  else         { if (esize == 2) DD_CL(from_channels_last_kernel, uint16_t); else DD_CL(from_channels_last_kernel, uint32_t); }
-#undef DD_CL
+  const dim3 grid((unsigned)((n + kPos - 1) / kPos), (unsigned)((C + kWords * 2 - 1) / (kWords * 2)), (unsigned)B);
+  const uint16_t* from = reinterpret_cast<const uint16_t*>(src);
+  auto kernel = to_last ? to_channels_last_kernel : from_channels_last_kernel;
+  kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(from, reinterpret_cast<uint16_t*>(dst), g, C);
   return (int)cudaGetLastError();
 }

@@ -167,7 +167,7 @@ class DistributedFeatureConvBase(Module, HaloMixin, ConvMixin):
             return input
         w = self.w_broadcast(self.weight)
         b = self.b_broadcast(self.bias) if self.use_bias else None
-        if self.whole and self.groups == 1 and channels_last_usable(input, self.pad_tuple, w, self.stride, self.dilation):
+        if self.whole and self.groups == 1 and channels_last_usable(input, self.pad_tuple, w):
             # nothing to exchange or to crop: padding and change of layout in one pass, the result back in another
             return channels_first(self._local_conv(pad_channels_last(input, self.pad_tuple), w, b))
         x = pad(input, self.pad_tuple)

@@ -319,7 +319,7 @@ def test_pooling_backward_by_pairs(kind, kernel, stride, space, dtype):
         assert (x.grad.double() - xr.grad).abs().max() <= tol * xr.grad.abs().max()
 
 
-@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("space,pads,C", [((5, 7), (1, 1, 1, 1), 8), ((64, 3), (0, 2, 1, 0), 72), ((3, 4, 13), (1, 1, 0, 0, 2, 1), 136),
                                           ((9, 9, 9), (0, 0, 0, 0, 0, 0), 24)])
 def test_padding_into_channels_last_and_back(space, pads, C, dtype):
@@ -333,10 +333,7 @@ def test_padding_into_channels_last_and_back(space, pads, C, dtype):
     xr = x.detach().clone().requires_grad_()
     nd = len(space)
     w = torch.empty(16, C, *[3] * nd, device="cuda", dtype=dtype)
-    one = (1,) * nd
-    # fp32 only where the library's channels-first kernels run in tf32 too
-    assert channels_last_usable(x, pads, w, one, one) == (dtype != torch.float32 or (nd == 3 and C >= 16))
-    assert not channels_last_usable(x.float(), pads, w[..., :1], one, one)
+    assert channels_last_usable(x, pads, w) and not channels_last_usable(x.float(), pads, w.float())
     y, yr = pad_channels_last(x, pads), F.pad(xr, pads)
     fmt = torch.channels_last if len(space) == 2 else torch.channels_last_3d
     assert y.is_contiguous(memory_format=fmt) and torch.equal(y, yr)
@@ -349,12 +346,16 @@ def test_padding_into_channels_last_and_back(space, pads, C, dtype):
     assert torch.equal(torch.autograd.grad(g.sum(), x)[0], torch.autograd.grad(gr.sum(), xr)[0])
 
 
-@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("space,cin,cout,kernel,stride,bias", [((13, 17), 16, 24, 3, 1, True), ((12, 12), 8, 8, 1, 1, False),
-                                                               ((11, 9, 10), 24, 16, 3, 1, True), ((14, 14), 16, 16, 3, 2, False),
-                                                               ((9, 9), 12, 8, 3, 1, True)])
-def test_feature_convolution_on_one_worker(space, cin, cout, kernel, stride, bias, dtype):
-    """Layouts in and out, and all gradients, against PyTorch in fp64; channel counts that keep the old way too."""
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("batch,space,cin,cout,kernel,stride,bias", [
+    (2, (13, 17), 16, 24, 3, 1, True), (2, (12, 12), 8, 8, 1, 1, False), (2, (14, 14), 16, 16, 3, 2, False),
+    (2, (9, 9), 12, 8, 3, 1, True), (5, (1, 40), 32, 16, 3, 1, False), (2, (11, 9, 10), 24, 16, 3, 1, True),
+    (16, (3, 3, 3), 48, 48, 3, 1, False), (1, (5, 86, 1), 32, 32, 3, 1, True), (1, (24, 84, 73), 64, 56, 3, 1, False),
+    (3, (16, 1, 24), 40, 128, 3, 1, False)])
+def test_feature_convolution_on_one_worker(batch, space, cin, cout, kernel, stride, bias, dtype):
+    """Layouts in and out, and output and gradients as close to fp64 as the library's convolution of the padded input,
+    channels first: whatever precision that has for this shape.  Channel counts that keep this way too, extents of one,
+    slabs, small volumes of a large batch."""
     import torch.nn.functional as F
 
     import distdl_b200
@@ -365,19 +366,39 @@ def test_feature_convolution_on_one_worker(space, cin, cout, kernel, stride, bia
     P = backends.backend.Partition().create_partition_inclusive([0]).create_cartesian_topology_partition([1] * (nd + 2))
     cls = {2: nn.DistributedFeatureConv2d, 3: nn.DistributedFeatureConv3d}[nd]
     layer = cls(P, cin, cout, kernel, stride=stride, padding=kernel // 2, bias=bias, device="cuda", dtype=dtype)
-    x = torch.randn(2, cin, *space, device="cuda").to(dtype).requires_grad_()
+    x = torch.randn(batch, cin, *space, device="cuda").to(dtype).requires_grad_()
     params = [layer.weight] + ([layer.bias] if bias else [])
-    ref = [t.detach().double().requires_grad_() for t in [x] + params]
+    conv = getattr(F, f"conv{nd}d")
+    results = []
     y = layer(x)
-    yr = getattr(F, f"conv{nd}d")(ref[0], ref[1], ref[2] if bias else None, stride=stride, padding=kernel // 2)
-    assert y.is_contiguous() and y.dtype == dtype and y.shape == yr.shape
-    dy = torch.randn(yr.shape, device="cuda").to(dtype)
-    got = torch.autograd.grad(y, [x] + params, dy)
-    want = torch.autograd.grad(yr, ref, dy.double())
-    assert got[0].is_contiguous()
-    for a, b in zip([y, *got], [yr, *want]):
-        # products of tf32 (2^-11) or bf16 operands in fp32, bf16 results rounded once
-        assert (a.double() - b).norm() <= (1e-3 if dtype == torch.float32 else 4e-3) * b.norm()
+    dy = torch.randn(y.shape, device="cuda").to(dtype)
+    results.append([y, *torch.autograd.grad(y, [x] + params, dy)])
+    assert y.is_contiguous() and y.dtype == dtype and results[0][1].is_contiguous()
+    for t in ([x] + params, [t.detach().double().requires_grad_() for t in [x] + params]):
+        z = conv(F.pad(t[0], (kernel // 2,) * 2 * nd), *t[1:], stride=stride)
+        results.append([z, *torch.autograd.grad(z, t, dy.to(z.dtype))])
+    for a, b, r in zip(*results):
+        assert a.shape == r.shape
+        # (sums in another order, where the layouts differ or the library adds atomically)
+        assert (a.double() - r).norm() <= 1.1 * (b.double() - r).norm() + 1e-7 * r.norm()
+
+
+def test_feature_convolution_with_the_precision_of_fp32_set_for_convolutions_alone():
+    """``torch.backends.cudnn.conv.fp32_precision``, beside which the older ``allow_tf32`` cannot be read."""
+    import distdl_b200
+    from distdl_b200 import backends, nn
+    distdl_b200.config.set_backend("native", "cupy")
+    P = backends.backend.Partition().create_partition_inclusive([0]).create_cartesian_topology_partition([1] * 5)
+    layer = nn.DistributedFeatureConv3d(P, 16, 16, 3, padding=1, device="cuda")
+    x = torch.randn(1, 16, 30, 30, 30, device="cuda")
+    want = torch.nn.functional.conv3d(x.double(), layer.weight.double(), layer.bias.double(), padding=1)
+    before = torch.backends.cudnn.conv.fp32_precision
+    try:
+        torch.backends.cudnn.conv.fp32_precision = "ieee"
+        y = layer(x)
+    finally:
+        torch.backends.cudnn.conv.fp32_precision = before
+    assert (y.double() - want).norm() <= 1e-6 * want.norm()
 
 
 def test_batch_norm_on_one_worker_matches_the_passes_between_workers():
