@@ -122,12 +122,13 @@ def direct_main_grad(param, gather, shape):
 def attach_main_grad(tensor, param, broadcast):
     """Gives ``tensor`` (a view of ``param`` that came through the data-parallel ``broadcast``) the optimizer's
     accumulator of ``param`` as its ``main_grad``, where the broadcast is the identity: the gradient is then
-    added there in fp32 instead of being written in bf16, handed through autograd and added up."""
+    added there in fp32 instead of being written in bf16, handed through autograd and added up (where nobody else
+    waits for it: see :func:`..ops._util.main_grad_now`)."""
     acc = getattr(param, "main_grad_view", None)
     if acc is None or not param.is_cuda or not broadcast.identity or broadcast.scale_backward is not None \
             or acc.numel() != tensor.numel() or env("DISTDL_DIRECT_MAIN_GRAD", "1") == "0":
         return
-    tensor.main_grad = acc.view(tensor.shape)
+    tensor.main_grad, tensor.main_grad_owner = acc.view(tensor.shape), param
 
 
 def reduce_scatter_grad(rs, full_grad, param, scale_backward=None):

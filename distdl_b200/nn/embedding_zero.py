@@ -121,8 +121,9 @@ class DistributedEmbeddingZero(Module):
         if mg is not None:
             # the scatter-add goes straight into the optimizer's fp32 accumulator: no gradient of the table's size
             # is cleared, rounded to bf16 and added up again for the few rows that the tokens name
-            w = w.view(w.shape)              # a fresh tensor object to carry the attribute
-            w.main_grad = mg
+            leaf = w                         # the parameter, or the gathered copy that is kept
+            w = w.view(w.shape)              # a fresh tensor object to carry the attributes
+            w.main_grad, w.main_grad_owner = mg, leaf
         if self.max_norm is None and not self.scale_grad_by_freq and not self.sparse:
             y = ops.embedding(input, w, self.padding_idx)
         else:

@@ -271,8 +271,9 @@ class DistributedLinearAllGatherZero(Module):
             wt.main_grad = mg.t()
         mgb = direct_main_grad(self.bias, self._bias_ag, b.shape) if b is not None else None
         if mgb is not None:
-            b = b.view(b.shape)              # a fresh tensor object to carry the attribute
-            b.main_grad = mgb
+            leaf = b if b.is_leaf else self.bias
+            b = b.view(b.shape)              # a fresh tensor object to carry the attributes
+            b.main_grad, b.main_grad_owner = mgb, leaf
         y = None
         # where recipes are on, the backward pass gathers the weight shards again instead of
         # holding the gathered weight since the forward pass

@@ -222,8 +222,9 @@ class DistributedLinearReduceScatterZero(Module):
         b = self.bias_buffer
         mgb = direct_main_grad(self.bias, self.allgather_bias, b.shape) if b is not None else None
         if mgb is not None:
+            leaf = b if b.is_leaf else self.bias
             b = b.view(b.shape)
-            b.main_grad = mgb
+            b.main_grad, b.main_grad_owner = mgb, leaf
         # where recipes are on, the backward pass gathers the weight shards again instead of
         # holding the gathered weight since the forward pass
         resharded = self.auto_clear_buffer and int(self.allgather_weight.P_x.shape[self.allgather_weight.axes_all_gather[0]]) > 1

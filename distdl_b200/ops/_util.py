@@ -31,6 +31,25 @@ def ptr(t):
     return 0 if t is None else t.data_ptr()
 
 
+def main_grad_now(acc, owner):
+    """``acc``, the fp32 accumulator that stands for the gradient of the leaf ``owner``, if the backward pass that is
+    running would hand that gradient to nobody but the optimizer's own hook; None where it has to go through autograd:
+    the leaf has hooks of the user's, or the pass does not accumulate into it (``torch.autograd.grad``, ``inputs=`` of
+    ``backward``) or builds a graph.  Asked in the backward pass, so that hooks of any moment count.  ``owner`` None: a
+    gathered weight, whose gradient is never autograd's."""
+    if acc is None or owner is None:
+        return acc
+    after = owner._post_accumulate_grad_hooks
+    if torch.is_grad_enabled() or owner._backward_hooks \
+            or (after and not all(getattr(h, "into_main_grad", False) for h in after.values())):
+        return None
+    try:
+        runs = torch._C._will_engine_execute_node(torch.autograd.graph.get_gradient_edge(owner).node)
+    except RuntimeError:            # the pass captures the gradient of this leaf
+        return None
+    return acc if runs else None
+
+
 def use_native(*tensors) -> bool:
     """True when the operands live on a CUDA device: the hand-written kernels run.
 

@@ -17,7 +17,7 @@ import functools
 import torch
 
 from .. import _native
-from ._util import ptr, stream_ptr, use_native
+from ._util import main_grad_now, ptr, stream_ptr, use_native
 
 _v, _i, _ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
 _native.declare("dd_gemm_bf16_rows", [_v, _i, _ll, _ll, _v, _i, _ll, _ll, _v, _ll, _ll, _i, _i, _i, _i, _i, _v, _i, _v])
@@ -117,8 +117,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, *, bias: to
 def grad_target(w: torch.Tensor):
     """What a weight-gradient GEMM needs to know about the weight ``w`` ([out, in], possibly a
     transposed view), as a small tuple that a backward pass can keep without keeping ``w``
-    itself alive: ``(main_grad, transposed_storage)``."""
-    return getattr(w, "main_grad", None), (not w.is_contiguous() and w.t().is_contiguous())
+    itself alive: ``(main_grad, transposed_storage, main_grad_owner)``."""
+    return (getattr(w, "main_grad", None), not w.is_contiguous() and w.t().is_contiguous(),
+            getattr(w, "main_grad_owner", None))
 
 
 def weight_grad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor = None, target=None):
@@ -128,12 +129,14 @@ def weight_grad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor = None, tar
 
     * ``w.main_grad`` (an fp32 tensor in the layout of ``w``, possibly a
       transposed view): the GEMM epilogue accumulates into it and ``None`` is
-      returned, so no bf16 gradient is ever written.
+      returned, so no bf16 gradient is ever written; with ``w.main_grad_owner``, the
+      leaf behind ``w``, only where :func:`main_grad_now` allows it.
     * ``w`` a transposed view of a contiguous ``[in, out]`` tensor: the gradient
       is produced in that storage order (``x^T dy``) and returned as the matching
       view, so autograd's transpose back is free instead of a strided copy.
     """
-    mg, transposed = target if target is not None else grad_target(w)
+    mg, transposed, owner = target if target is not None else grad_target(w)
+    mg = main_grad_now(mg, owner)
     if mg is not None:
         if mg.is_contiguous():
             gemm(dy2.t(), x2.t(), out=mg, accumulate=True)
@@ -177,7 +180,7 @@ class _LinearFn(torch.autograd.Function):
         ctx.has_bias = b is not None
         # (not the weight itself: a gathered ZeRO weight must not be held from forward to backward)
         ctx.wgrad = grad_target(w)
-        ctx.b_main_grad = getattr(b, "main_grad", None) if b is not None else None
+        ctx.b_main_grad = (getattr(b, "main_grad", None), getattr(b, "main_grad_owner", None))
         ctx.xshape = x.shape
         return y
 
@@ -193,7 +196,7 @@ class _LinearFn(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             dw = weight_grad(dy2, x2, target=ctx.wgrad)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            mg = ctx.b_main_grad
+            mg = main_grad_now(*ctx.b_main_grad)
             s = column_sum(dy2, mg)
             if mg is None:
                 db = s.to(dy.dtype)

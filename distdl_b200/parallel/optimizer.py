@@ -313,6 +313,7 @@ class FlatAdamW:
                 return
             ops.optim.accumulate_f32_(param.main_grad_view, g)
             param.grad = None
+        hook.into_main_grad = True
         return hook
 
     def set_lr(self, lr):

@@ -296,3 +296,68 @@ def test_xent_with_masked_and_extreme_logits(V, ld, fill):
     tol = grad.abs() * (2 ** -8 + 4e-7 * lse.abs().clamp(max=1e4)[:, None]) + 1e-6
     assert ((lg[:, :V].double() - grad).abs() <= tol).all()
     assert (lg[:, V:] == 0).all()
+
+
+@pytest.mark.parametrize("zero,kept", [(True, False), (True, True), (False, False)])
+def test_hooks_and_partial_backward_passes_see_the_gradients(zero, kept):
+    """Parameters with an optimizer's accumulator: hooks run, also those registered after the forward pass, and what
+    they return reaches the accumulator; ``torch.autograd.grad`` finds the gradients, and passes that are not asked
+    for them leave the accumulators alone."""
+    import distdl_b200
+    from distdl_b200 import backends, nn
+    from distdl_b200.parallel.optimizer import FlatAdamW
+    distdl_b200.config.set_backend("native", "cupy")
+    torch.manual_seed(6)
+    world = backends.backend.Partition().create_partition_inclusive([0])
+    P = world.create_cartesian_topology_partition([1, 1, 1])
+    V, d, out = 50, 24, 40
+    kw = dict(dtype=torch.bfloat16, auto_clear_buffer=not kept)
+    embed = nn.DistributedEmbeddingZero(P, V, d, **kw)
+    if zero:
+        ag = nn.DistributedLinearAllGatherZero(P, d, out, bias=True, **kw)
+        rs = nn.DistributedLinearReduceScatterZero(P, out, d, bias=True, **kw)
+    else:
+        ag = nn.DistributedLinearAllGather(P, d, out, bias=True, dtype=torch.bfloat16)
+        rs = nn.DistributedLinearReduceScatter(P, out, d, bias=True, dtype=torch.bfloat16)
+    model = torch.nn.ModuleList([embed, ag, rs])
+    opt = FlatAdamW(model)
+    params = [embed.weight, ag.bias, rs.bias] + ([] if zero else [ag.weight, rs.weight])
+    ids = torch.randint(0, 7, (2, 64), device="cuda")
+    g = torch.randn(2, 64, d, device="cuda").bfloat16()
+
+    def gradients():
+        for m in model:
+            if hasattr(m, "clear_weight_buffer"):
+                m.clear_weight_buffer()
+        got = [p.main_grad_view.clone() for p in params]
+        opt.grad.zero_()
+        return got
+
+    def leaves():                                # where autograd's gradients arrive
+        return [embed.weight_buffer, ag.bias_buffer, rs.bias_buffer] if kept else params
+
+    rs(ag(embed(ids))).backward(g)
+    want = gradients()
+    assert all(w.any() for w in want)
+    y = rs(ag(embed(ids)))
+    got = torch.autograd.grad(y, leaves(), g, retain_graph=True)
+    assert not any(p.main_grad_view.any() for p in params)
+    for a, w in zip(got, want):
+        assert (a.float().flatten() - w).norm() <= 2 ** -8 * w.norm()         # rounded to bf16 once
+    y.backward(g, inputs=[leaves()[0]])
+    assert all(p is params[0] or not v.any() for p, v in zip(params, gradients()))
+    if kept:
+        return
+    seen = []
+    handles = [p.register_hook(lambda t: 2 * t) for p in params[:2]]
+    y = rs(ag(embed(ids)))
+    handles += [p.register_post_accumulate_grad_hook(lambda p: seen.append(p.shape)) for p in params[2:]]
+    y.backward(g)
+    assert sorted(seen) == sorted(p.shape for p in params[2:])
+    for k, (a, w) in enumerate(zip(gradients(), want)):
+        w = 2 * w if k < 2 else w
+        assert (a - w).norm() <= 2 ** -8 * w.norm()
+    for h in handles:
+        h.remove()
+    rs(ag(embed(ids))).backward(g)
+    assert all(p.grad is None and torch.equal(a, w) for p, a, w in zip(params[1:], gradients()[1:], want[1:]))
