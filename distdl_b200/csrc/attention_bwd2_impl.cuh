@@ -113,8 +113,11 @@ attn_prepass_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __
   constexpr int LANES = D / 8, ROWS = 32 / LANES, ITERS = PRE_TOKENS / (PRE_WARPS * ROWS);
   __shared__ float s_delta[PRE_TOKENS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long first = (long long)blockIdx.z * S + blockIdx.x * PRE_TOKENS;
-  const int h = blockIdx.y, mine = warp * ROWS * ITERS + lane / LANES;
+  // a flat grid (tokens, then heads, then sequences): any number of sequences and heads, as in the kernels that follow
+  const int slices = S / PRE_TOKENS, slice = (int)(blockIdx.x % (unsigned)slices);
+  const int row = (int)(blockIdx.x / (unsigned)slices), b = row / Hq, h = row - b * Hq;
+  const long long first = (long long)b * S + slice * PRE_TOKENS;
+  const int mine = warp * ROWS * ITERS + lane / LANES;
   uint4 a[ITERS], g[ITERS];
 #pragma unroll
   for (int i = 0; i < ITERS; ++i) {
@@ -137,7 +140,7 @@ attn_prepass_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __
   }
   __syncthreads();
   if (threadIdx.x < PRE_TOKENS) {
-    const size_t o = ((size_t)blockIdx.z * Hq + h) * S + blockIdx.x * PRE_TOKENS + threadIdx.x;
+    const size_t o = (size_t)row * S + slice * PRE_TOKENS + threadIdx.x;
     delta[o] = s_delta[threadIdx.x];
     lse2[o] = lse[o] * kLog2e;
   }
@@ -588,12 +591,15 @@ int run(const void* q, long long q_row, long long q_head, const void* k, long lo
   float* delta = scratch;
   float* lse2 = scratch + (size_t)batch * Hq * S;
   if (reinterpret_cast<uintptr_t>(dout) & 15) return DD_ERR_ALIGN;
-  const dim3 pre((unsigned)(S / PRE_TOKENS), (unsigned)Hq, (unsigned)batch);
+  const long long pre = (long long)(S / PRE_TOKENS) * Hq * batch;
+  if (pre > 0x7fffffffLL) return DD_ERR_TOO_LARGE;
   auto prepass = (reinterpret_cast<uintptr_t>(out) & 15) == 0 ? attn_prepass_kernel<true> : attn_prepass_kernel<false>;
-  prepass<<<pre, 32 * PRE_WARPS, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(out),
-                                         reinterpret_cast<const __nv_bfloat16*>(dout), lse, delta, lse2, S, Hq);
+  prepass<<<(unsigned)pre, 32 * PRE_WARPS, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(out),
+                                                   reinterpret_cast<const __nv_bfloat16*>(dout), lse, delta, lse2, S, Hq);
+  int r = (int)cudaGetLastError();
+  if (r) return r;
   CUtensorMap tq, tk, tv, tdo;
-  int r = get_tensor_map_bf16_3d(&tq, q, D, tokens, Hq, q_row * 2, q_head * 2, 64, BT);
+  r = get_tensor_map_bf16_3d(&tq, q, D, tokens, Hq, q_row * 2, q_head * 2, 64, BT);
   if (r) return r;
   r = get_tensor_map_bf16_3d(&tk, k, D, tokens, Hkv, k_row * 2, k_head * 2, 64, BT);
   if (r) return r;

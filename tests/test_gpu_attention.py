@@ -75,3 +75,19 @@ def test_backward_with_an_output_that_is_not_16_byte_aligned(D, Hq, Hkv, B, S):
     assert shifted.data_ptr() % 16 == 8
     for a, b in zip(attention_backward(dout, q, k, v, out, lse, B, S), attention_backward(dout, q, k, v, shifted, lse, B, S)):
         assert torch.equal(a, b)
+def test_backward_of_more_sequences_than_a_grid_dimension_holds():
+    """65 537 windows of 128 tokens: the first, the last and those around the limit of a grid's second and third
+    dimension have the bits that a call of their own gives them."""
+    from distdl_b200 import _native
+    from distdl_b200.ops.attention import attention_backward, attention_forward
+    torch.manual_seed(15)
+    B, S, D = 65537, 128, 64
+    q, k, v, dout = (torch.randn(B * S, 1, D, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    out, lse = attention_forward(q, k, v, B, S, True)
+    grads = attention_backward(dout, q, k, v, out, lse, B, S)
+    for b in (0, 40000, 65534, 65535, 65536):
+        sl = slice(b * S, (b + 1) * S)
+        one = attention_backward(dout[sl], q[sl], k[sl], v[sl], out[sl], lse[b:b + 1], 1, S)
+        for a, r in zip(grads, one):
+            assert torch.equal(a[sl], r)
+    assert _native.read_status()[0] == 0
