@@ -531,6 +531,7 @@ DD_API int dd_attn_bwd(const void* q, long long q_row, long long q_head, const v
   if ((dq_row | dq_head | dk_row | dk_head | dv_row | dv_head) % 8) return DD_ERR_ALIGN;
   if ((reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) & 15)
     return DD_ERR_ALIGN;
+  if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout)) & 3) return DD_ERR_ALIGN;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const uint64_t tokens = (uint64_t)batch * S;
   const long long rows = (long long)tokens * Hq;

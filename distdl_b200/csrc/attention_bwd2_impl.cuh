@@ -97,7 +97,7 @@ __device__ __forceinline__ void issue_from_tmem(uint32_t tmem_d, uint32_t tmem_a
 // head, D / 8 lanes with 16 bytes each per row and all rows of a warp in flight, and writes its statistics as one run
 // (they lie token by token, the rows head by head).  4096 tokens x 25 x 64: 19.3 -> 5.2 us, 8192 x 32 x 128:
 // 53.6 -> 24.5 us (one row and 4 or 8 bytes per lane per warp, single words scattered).
-// WIDE: O is 16-byte aligned (dO always is, its tensor map asks for it).
+// WIDE: O is 16-byte aligned (dO always is, its tensor map asks for it); otherwise 4-byte aligned.
 // ---------------------------------------------------------------------------
 constexpr int PRE_TOKENS = 64, PRE_WARPS = 8;
 template <bool WIDE>
@@ -590,7 +590,7 @@ int run(const void* q, long long q_row, long long q_head, const void* k, long lo
   const uint64_t tokens = (uint64_t)batch * S;
   float* delta = scratch;
   float* lse2 = scratch + (size_t)batch * Hq * S;
-  if (reinterpret_cast<uintptr_t>(dout) & 15) return DD_ERR_ALIGN;
+  if ((reinterpret_cast<uintptr_t>(dout) & 15) || (reinterpret_cast<uintptr_t>(out) & 3)) return DD_ERR_ALIGN;
   const long long pre = (long long)(S / PRE_TOKENS) * Hq * batch;
   if (pre > 0x7fffffffLL) return DD_ERR_TOO_LARGE;
   auto prepass = (reinterpret_cast<uintptr_t>(out) & 15) == 0 ? attn_prepass_kernel<true> : attn_prepass_kernel<false>;

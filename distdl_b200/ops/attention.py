@@ -74,7 +74,7 @@ def attention_backward(dout, q, k, v, out, lse, batch, seq, causal=True, scale=N
         dk = torch.empty(tokens, Hkv, D, dtype=q.dtype, device=q.device)
     if dv is None:
         dv = torch.empty(tokens, Hkv, D, dtype=q.dtype, device=q.device)
-    dout = dout.contiguous()
+    dout, out = dout.contiguous(), out.contiguous()
     # the kernels that keep P / dS in tensor memory (scratch: delta and the base-2 lse)
     in_tmem = D in (64, 128) and env("DISTDL_ATTN_BWD2", "1") != "0"
     delta = torch.empty(2 if in_tmem else 1, batch, Hq, seq, dtype=torch.float32, device=q.device)

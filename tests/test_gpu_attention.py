@@ -75,6 +75,24 @@ def test_backward_with_an_output_that_is_not_16_byte_aligned(D, Hq, Hkv, B, S):
     assert shifted.data_ptr() % 16 == 8
     for a, b in zip(attention_backward(dout, q, k, v, out, lse, B, S), attention_backward(dout, q, k, v, shifted, lse, B, S)):
         assert torch.equal(a, b)
+
+
+def test_backward_with_an_output_of_any_stride_but_no_odd_address():
+    """Rows that lie apart are gathered first; an address between two 4-byte words is refused on the host."""
+    from distdl_b200 import _native
+    from distdl_b200.ops.attention import attention_backward, attention_forward
+    torch.manual_seed(16)
+    B, S, H, D = 2, 128, 3, 64
+    q, k, v, dout = (torch.randn(B * S, H, D, device="cuda").bfloat16() for _ in range(4))
+    out, lse = attention_forward(q, k, v, B, S, True)
+    apart = torch.cat([out, torch.randn_like(out)], dim=2)[..., :D]
+    for a, b in zip(attention_backward(dout, q, k, v, out, lse, B, S), attention_backward(dout, q, k, v, apart, lse, B, S)):
+        assert torch.equal(a, b)
+    odd = torch.empty(out.numel() + 8, device="cuda", dtype=torch.bfloat16)[1:1 + out.numel()].view(out.shape)
+    with pytest.raises(_native.NativeError):
+        attention_backward(dout, q, k, v, odd, lse, B, S)
+
+
 def test_backward_of_more_sequences_than_a_grid_dimension_holds():
     """65 537 windows of 128 tokens: the first, the last and those around the limit of a grid's second and third
     dimension have the bits that a call of their own gives them."""
