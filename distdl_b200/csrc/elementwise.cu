@@ -318,10 +318,17 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
   if (partial != nullptr) {
     float* pw = partial + (size_t)blockIdx.x * 2 * d;
     float* pb = pw + d;
+    const bool wide = (reinterpret_cast<uintptr_t>(partial) & 15) == 0;     // (a caller's scratch may start anywhere)
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
       const int vi = threadIdx.x + i * kNormThreads;
-      if (vi < nvec) {
+      if (vi < nvec && !wide) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          pw[vi * 8 + j] = dw[i][j];
+          if (WANT_DB) pb[vi * 8 + j] = db[i][j];
+        }
+      } else if (vi < nvec) {
 #pragma unroll
         for (int j = 0; j < 8; j += 4) {
           *reinterpret_cast<float4*>(pw + vi * 8 + j) = make_float4(dw[i][j], dw[i][j + 1], dw[i][j + 2], dw[i][j + 3]);
@@ -826,7 +833,6 @@ DD_API int dd_norm_bwd(int rms, const void* dy, const void* x, const void* w, co
                        void* dx, float* dw, float* db, float* partial, int accumulate, int rows, int d,
                        void* stream) {
   if (d % 8 != 0 || d > kNormThreads * kMaxVec * 8 || rows <= 0) return DD_ERR_BAD_ARG;
-  if (reinterpret_cast<uintptr_t>(partial) & 15) return DD_ERR_ALIGN;
   const int grid = dd_norm_bwd_parts(rows);
   launch_norm_bwd_any(rms, db != nullptr && partial != nullptr, grid, STREAM(stream), dy, x, w, stats, dres, dx,
                       partial, rows, d);

@@ -361,3 +361,25 @@ def test_hooks_and_partial_backward_passes_see_the_gradients(zero, kept):
         h.remove()
     rs(ag(embed(ids))).backward(g)
     assert all(p.grad is None and torch.equal(a, w) for p, a, w in zip(params[1:], gradients()[1:], want[1:]))
+
+
+@pytest.mark.parametrize("d", [264, 4096, 8192])
+def test_norm_backward_takes_a_scratch_that_starts_anywhere(d):
+    """The partial sums go to any 4-byte address of the caller's, with the same bits, and nothing beside them."""
+    from distdl_b200 import _native
+    from distdl_b200.ops._util import stream_ptr
+    torch.manual_seed(17)
+    rows = 37
+    x, dy, w = (torch.randn(n, d, device="cuda").bfloat16() for n in (rows, rows, 1))
+    stats = torch.stack([x.float().mean(1), (x.float().var(1, unbiased=False) + 1e-5).rsqrt()], 1).contiguous()
+    parts = _native.lib().dd_norm_bwd_parts(rows) * 2 * d
+    results = []
+    for shift in (0, 1, 2):
+        scratch = torch.full((parts + 4,), 7.0, device="cuda")
+        dx, dw, db = torch.empty_like(x), torch.empty(d, device="cuda"), torch.empty(d, device="cuda")
+        _native.call("dd_norm_bwd", 0, dy.data_ptr(), x.data_ptr(), w.data_ptr(), stats.data_ptr(), None, dx.data_ptr(),
+                     dw.data_ptr(), db.data_ptr(), scratch[shift:].data_ptr(), 0, rows, d, stream_ptr())
+        assert (scratch[:shift] == 7.0).all() and (scratch[shift + parts:] == 7.0).all()
+        results.append((dx, dw, db))
+    for other in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(results[0], other))
