@@ -165,7 +165,7 @@ __device__ __forceinline__ void merge(Moments& a, float n, float mean, float m2)
   if (n <= 0.f) return;
   const float t = a.n + n, d = mean - a.mean, w = n / t;
   a.mean += d * w;
-  a.m2 += m2 + d * d * a.n * w;
+  a.m2 += m2 + d * w * a.n * d;                           // (no square that overflows where it counts for nothing)
   a.n = t;
 }
 __device__ __forceinline__ Moments warp_merge(Moments m) {

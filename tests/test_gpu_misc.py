@@ -424,3 +424,21 @@ def test_batch_norm_on_one_worker_matches_the_passes_between_workers():
     for a, b in zip(*outs):
         assert (a != b).float().mean() < 0.1
         assert (a.double() - b.double()).norm() <= 8e-3 * b.double().norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(4, 3, 16), (2, 5, 3, 64)])
+def test_batch_norm_of_large_constant_features(shape, dtype):
+    """Values whose square is beyond fp32, but whose deviations from the mean are not."""
+    import distdl_b200
+    from distdl_b200 import backends
+    from distdl_b200.nn import DistributedBatchNorm
+    distdl_b200.config.set_backend("native", "cupy")
+    P = backends.backend.Partition().create_partition_inclusive([0]).create_cartesian_topology_partition([1] * len(shape))
+    layer = DistributedBatchNorm(P, shape[1], device="cuda", dtype=dtype)
+    x = torch.full(shape, 2.0 ** 66, device="cuda", dtype=dtype).requires_grad_()
+    y = layer(x)
+    assert not y.any()                                    # powers of two: sums and means are exact
+    y.backward(torch.ones_like(y))
+    assert x.grad.isfinite().all() and (layer.running_mean.float() - 0.1 * 2.0 ** 66).abs().max() < 2.0 ** 58
+    assert (layer.running_var.float() - 0.9).abs().max() < 0.01
