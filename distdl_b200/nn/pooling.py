@@ -71,18 +71,19 @@ class DistributedPoolBase(Module, HaloMixin, PoolingMixin):
     def forward(self, input):
         if not self.P_x.active:
             return input
-        # (without padding the copy is spared: pooling keeps nothing of its input for the backward pass)
+        from ..ops import pooling as pool_ops
+        native = not self.extra and input.is_cuda
+        # (without padding the copy is spared for this library's kernel, which keeps nothing of its input for the
+        # backward pass; the others keep theirs, so that it must not be the caller's tensor)
         x = input
-        if any(self.pad_tuple) or not input.is_contiguous():
+        if any(self.pad_tuple) or not input.is_contiguous() or not (native and pool_ops.usable(input)):
             x = pad(input, self.pad_tuple, self.pad_value)
         x = self.halo_layer(x)
         x = x[self.needed_slices]
         k = tuple(int(v) for v in self.kernel_size)
         s = tuple(int(v) for v in self.stride)
-        if not self.extra and x.is_cuda:
-            from ..ops import pooling as pool_ops
-            if pool_ops.usable(x):          # this library's kernel reads the cropped view in place
-                return pool_ops.pool(x, self.pool_kind, k, s, tuple(int(v) for v in self.dilation))
+        if native and pool_ops.usable(x):   # this library's kernel reads the cropped view in place
+            return pool_ops.pool(x, self.pool_kind, k, s, tuple(int(v) for v in self.dilation))
         if self.pool_kind == "avg":
             fn = {1: F.avg_pool1d, 2: F.avg_pool2d, 3: F.avg_pool3d}[self.num_dimensions]
             return fn(x, k, stride=s, padding=0, **self.extra)

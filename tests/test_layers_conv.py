@@ -591,3 +591,23 @@ def body_conv3d_channel_and_general(rank, world):
 
 def test_conv3d_channel_and_general_via_selector():
     run_ranks("test_layers_conv", "body_conv3d_channel_and_general", 4, timeout=300)
+
+
+def body_pool_of_a_tensor_that_changes(rank, world):
+    from distdl_b200 import nn as dnn
+    P = _cart([0], [1, 1, 1, 1])
+    for Pool, kw in ((dnn.DistributedMaxPool2d, {}), (dnn.DistributedAvgPool2d, {}),
+                     (dnn.DistributedAvgPool2d, {"divisor_override": 3})):
+        x = torch.randn(2, 3, 6, 8, requires_grad=True)
+        held = x * 1
+        y = Pool(P, 2, stride=2, **kw)(held)
+        want, = torch.autograd.grad(Pool(P, 2, stride=2, **kw)(x), x, torch.ones_like(y))
+        with torch.no_grad():
+            held.zero_()
+        assert torch.equal(torch.autograd.grad(y, x, torch.ones_like(y))[0], want)
+    return True
+
+
+def test_pooling_input_may_change_before_the_backward_pass():
+    """Pooling on one worker without padding keeps none of the caller's tensor."""
+    run_ranks("test_layers_conv", "body_pool_of_a_tensor_that_changes", 1)
