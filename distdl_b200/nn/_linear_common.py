@@ -17,6 +17,7 @@ import torch
 from ..ops._util import env
 from ..utilities import streams
 from ..utilities.slicing import compute_subshape, worker_layout
+from .module import hooked
 
 
 def derived_partition(P, index, shape):
@@ -76,8 +77,9 @@ def local_out_features(out_features, num_gpu, index, num_heads=None, num_heads_k
 
 
 def through(module, x):
-    """``module(x)`` of a data-movement module, without the call where the module is the identity."""
-    return x if module.identity else module(x)
+    """``module(x)`` of a data-movement module, without the call where the module is the identity and nobody has
+    hooked it."""
+    return x if module.identity and not hooked(module) else module(x)
 
 
 def deliver_grad(param, g):

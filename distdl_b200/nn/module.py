@@ -7,8 +7,15 @@ whenever the structure of the input (shape, dtype, requires_grad) changes
 active when the layer is built is captured on the instance.
 """
 import torch
+from torch.nn.modules import module as _torch_module
 
 from .. import backends, config
+
+
+def hooked(module):
+    """True where a call of ``module`` is more than its ``forward``: it, or every module, has hooks."""
+    return bool(module._forward_pre_hooks or module._forward_hooks or module._backward_pre_hooks
+                or module._backward_hooks or _torch_module._has_any_global_hook())
 
 
 class Module(torch.nn.Module):
@@ -29,10 +36,22 @@ class Module(torch.nn.Module):
             super().__setattr__(name, value)
 
     def __call__(self, *input, **kwargs):
-        # (not a registered pre-hook: a module without hooks takes torch.nn.Module's short way)
-        if self._distdl_module_requires_reset(input):
+        # a registered pre-hook only beside others, so that a module without hooks takes torch.nn.Module's short way
+        if self._forward_pre_hooks or _torch_module._global_forward_pre_hooks:
+            self._register_set_up()
+        elif self._distdl_module_requires_reset(input):
             Module._distdl_forward_pre_hook(self, input)
         return super().__call__(*input, **kwargs)
+
+    def register_forward_pre_hook(self, hook, *, prepend=False, with_kwargs=False):
+        self._register_set_up()
+        return super().register_forward_pre_hook(hook, prepend=prepend, with_kwargs=with_kwargs)
+
+    def _register_set_up(self):
+        """Set-up sees the input that global pre-hooks and those registered with ``prepend`` leave, and runs before the
+        module's other pre-hooks."""
+        if all(h is not Module._distdl_forward_pre_hook for h in self._forward_pre_hooks.values()):
+            super().register_forward_pre_hook(Module._distdl_forward_pre_hook)
 
     @staticmethod
     def _distdl_forward_pre_hook(self, input):

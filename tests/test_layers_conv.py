@@ -611,3 +611,37 @@ def body_pool_of_a_tensor_that_changes(rank, world):
 def test_pooling_input_may_change_before_the_backward_pass():
     """Pooling on one worker without padding keeps none of the caller's tensor."""
     run_ranks("test_layers_conv", "body_pool_of_a_tensor_that_changes", 1)
+
+
+def body_pre_hooks(rank, world):
+    from distdl_b200 import nn as dnn
+    from distdl_b200.nn._linear_common import through
+    from torch.nn.modules.module import register_module_forward_pre_hook
+    P = _cart([0], [1, 1, 1])
+    x = torch.randn(6, 4, 5)
+    half = lambda m, args: (args[0][:3],)  # noqa: E731
+    want = torch.nn.functional.batch_norm(x[:3], None, None, None, None, True)
+
+    def register_globally(layer, hook):
+        return register_module_forward_pre_hook(lambda m, a: hook(m, a) if m is layer else None)
+
+    for register in (register_globally, lambda layer, hook: layer.register_forward_pre_hook(hook, prepend=True)):
+        layer = dnn.DistributedBatchNorm(P, 4)
+        handle = register(layer, half)
+        assert torch.allclose(layer(x), want, atol=1e-5) and layer.global_count == 15
+        handle.remove()
+        assert layer(x[:3]).shape == want.shape
+    seen = []                                       # set-up comes before the module's other pre-hooks
+    layer = dnn.DistributedBatchNorm(P, 4)
+    layer.register_forward_pre_hook(lambda m, a: seen.append(m._distdl_is_setup))
+    layer(x)
+    assert seen == [True] and layer.global_count == 30
+    gather = dnn.AllGather(P, axes_all_gather=(0,))
+    assert gather.identity and through(gather, x) is x
+    gather.register_forward_hook(lambda m, a, y: 2 * y)
+    assert torch.equal(through(gather, x), 2 * x)
+    return True
+
+
+def test_set_up_keeps_its_place_among_forward_pre_hooks():
+    run_ranks("test_layers_conv", "body_pre_hooks", 1)
