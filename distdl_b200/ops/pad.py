@@ -27,8 +27,18 @@ def _plain(x) -> bool:
     """A tensor and a moment at which a kernel may stand for the library's operators: no subclass, no dispatch
     mode, tracer, compiler, function transform or forward-mode differentiation, which know the operators only."""
     return (type(x) in (torch.Tensor, torch.nn.Parameter) and torch._C._len_torch_dispatch_stack() == 0
-            and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
+            and not torch._C._are_functorch_transforms_active() and not torch._C._functorch.is_functorch_wrapped_tensor(x)
+            and not torch._C._functorch.is_legacy_batchedtensor(x) and torch.autograd.forward_ad._current_level < 0
             and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+
+
+def _operators(dy, lo, space):
+    """The shifted copy by the library's operators: for a backward pass under a function transform (batched gradients),
+    a dispatch mode or a tracer."""
+    pads = []
+    for n, a, m in reversed(list(zip(dy.shape[-len(space):], lo, space))):
+        pads += [a, m - n - a]
+    return torch.nn.functional.pad(dy, pads)
 
 
 class _ShiftCopyFn(torch.autograd.Function):
@@ -46,7 +56,9 @@ class _ShiftCopyFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        return _ShiftCopyFn.apply(dy, tuple(-a for a in ctx.lo), ctx.space, False), None, None, None
+        lo = tuple(-a for a in ctx.lo)
+        dx = _ShiftCopyFn.apply(dy, lo, ctx.space, False) if _plain(dy) else _operators(dy, lo, ctx.space)
+        return dx, None, None, None
 
 
 _LAST = {2: torch.channels_last, 3: torch.channels_last_3d}
@@ -72,7 +84,8 @@ class _ToChannelsLastFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        return _FromChannelsLastFn.apply(dy, tuple(-a for a in ctx.lo), ctx.space), None, None
+        lo = tuple(-a for a in ctx.lo)
+        return (_FromChannelsLastFn.apply if _plain(dy) else _operators)(dy, lo, ctx.space), None, None
 
 
 class _FromChannelsLastFn(torch.autograd.Function):
@@ -83,7 +96,8 @@ class _FromChannelsLastFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        return _ToChannelsLastFn.apply(dy, tuple(-a for a in ctx.lo), ctx.space), None, None
+        lo = tuple(-a for a in ctx.lo)
+        return (_ToChannelsLastFn.apply if _plain(dy) else _operators)(dy, lo, ctx.space), None, None
 
 
 def channels_last_usable(x: torch.Tensor, pad_tuple, weight: torch.Tensor) -> bool:

@@ -442,3 +442,29 @@ def test_batch_norm_of_large_constant_features(shape, dtype):
     y.backward(torch.ones_like(y))
     assert x.grad.isfinite().all() and (layer.running_mean.float() - 0.1 * 2.0 ** 66).abs().max() < 2.0 ** 58
     assert (layer.running_var.float() - 0.9).abs().max() < 0.01
+
+
+@pytest.mark.parametrize("nd,dtype", [(2, torch.bfloat16), (3, torch.bfloat16), (3, torch.float32)])
+def test_feature_convolution_with_batched_gradients(nd, dtype):
+    """Gradients of several incoming ones at once (a function transform around the backward pass only)."""
+    import distdl_b200
+    from distdl_b200 import backends, nn
+    from distdl_b200.ops.pad import pad
+    distdl_b200.config.set_backend("native", "cupy")
+    torch.manual_seed(18)
+    P = backends.backend.Partition().create_partition_inclusive([0]).create_cartesian_topology_partition([1] * (nd + 2))
+    cls = {2: nn.DistributedFeatureConv2d, 3: nn.DistributedFeatureConv3d}[nd]
+    layer = cls(P, 16, 16, 3, padding=1, device="cuda", dtype=dtype)
+    x = torch.randn(1, 16, *[5] * nd, device="cuda").to(dtype).requires_grad_()
+    y = layer(x)
+    dys = torch.randn(3, *y.shape, device="cuda").to(dtype)
+    got = torch.autograd.grad(y, (x, layer.weight), dys, is_grads_batched=True, retain_graph=True)
+    for k in range(3):
+        for a, b in zip(got, torch.autograd.grad(y, (x, layer.weight), dys[k], retain_graph=True)):
+            # the same products in another order: bf16 results, or tf32 operands
+            assert (a[k].double() - b.double()).norm() <= 8e-3 * b.double().norm()
+    p = pad(x, (1, 1, 0, 2, 1, 0)[:2 * nd])
+    dys = torch.randn(3, *p.shape, device="cuda").to(dtype)
+    got, = torch.autograd.grad(p, x, dys, is_grads_batched=True, retain_graph=True)
+    for k in range(3):
+        assert torch.equal(got[k], torch.autograd.grad(p, x, dys[k], retain_graph=True)[0])
