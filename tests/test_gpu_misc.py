@@ -291,6 +291,7 @@ def test_padding_kernel_moves_the_same_bits(space, pads, dtype):
         assert torch.equal(g, gr)
         assert torch.equal(torch.autograd.grad(g.sum(), x)[0], torch.autograd.grad(gr.sum(), xr)[0])
     assert torch.equal(pad(x.transpose(0, 1), pads), F.pad(x.transpose(0, 1), pads))
+    assert torch.equal(pad(x, pads[:2]), F.pad(x, pads[:2]))              # the last dimension alone
     assert torch.equal(torch.func.vmap(lambda t: pad(t, pads))(x.detach()[None]), F.pad(x.detach(), pads)[None])
     assert "pad" in str(torch.jit.trace(lambda t: pad(t, pads), x.detach()).graph)
 
