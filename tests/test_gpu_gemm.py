@@ -149,15 +149,18 @@ def test_batched_gemm_skips_zero_rows(C, counts):
 
 @pytest.mark.parametrize("M,N,K", [(1, 256, 8192), (33, 520, 6400), (128, 264, 14336), (129, 512, 8192), (200, 88, 6144),
                                    (300, 1000, 8192), (16, 8, 4096)])
+@pytest.mark.parametrize("a_mn", [0, 1])
 @pytest.mark.parametrize("b_mn", [0, 1])
-def test_gemm_split_contraction(M, N, K, b_mn):
-    """Few tiles and a long contraction: bias, both output types, accumulation, strided outputs; the same bits in
-    every run, nothing written beside the output."""
+def test_gemm_split_contraction(M, N, K, b_mn, a_mn):
+    """Few tiles and a long contraction, both layouts of both operands: bias, both output types, accumulation, strided
+    outputs; the same bits in every run, nothing written beside the output."""
     from distdl_b200 import _native
     from distdl_b200.ops import gemm
     assert _native.lib().dd_gemm_split(M, N, K) > 1
     torch.manual_seed(2)
-    a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    lead = (M + 7) // 8 * 8                                   # (a leading dimension that TMA can take)
+    a = torch.randn(K, lead, device="cuda", dtype=torch.bfloat16)[:, :M].t() if a_mn else \
+        torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
     b = torch.randn(K, N, device="cuda", dtype=torch.bfloat16).t() if b_mn else \
         torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
     bias = torch.randn(N, device="cuda")
@@ -174,5 +177,28 @@ def test_gemm_split_contraction(M, N, K, b_mn):
         assert torch.equal(view, first) and (out[:, N:] == 7.0).all()
         gemm(a, b, out=view, accumulate=True)
         _check(view, 2 * ref + bias, tol=2 * tol)
+    torch.cuda.synchronize()
+    assert _native.read_status()[0] == 0
+
+
+@pytest.mark.parametrize("n_out,n_in,tokens", [(64, 512, 8192), (384, 256, 8192)])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_weight_gradient_accumulates_over_a_split_contraction(n_out, n_in, tokens, transposed):
+    """A small weight and many tokens: two micro-batches into the fp32 accumulator, stored either way."""
+    from distdl_b200 import _native
+    from distdl_b200.ops.gemm import weight_grad
+    assert _native.lib().dd_gemm_split(*((n_in, n_out) if transposed else (n_out, n_in)), tokens) > 1
+    torch.manual_seed(19)
+    acc = torch.randn(*((n_in, n_out) if transposed else (n_out, n_in)), device="cuda")
+    mg = acc.t() if transposed else acc
+    want = mg.double()
+    w = torch.empty(n_out, n_in, device="cuda", dtype=torch.bfloat16)
+    w.main_grad = mg
+    for _ in range(2):
+        dy = torch.randn(tokens, n_out, device="cuda").bfloat16()
+        x = torch.randn(tokens, n_in, device="cuda").bfloat16()
+        want = want + dy.double().t() @ x.double()
+        assert weight_grad(dy, x, w) is None
+    assert (mg.double() - want).abs().max() < 1e-4 * tokens ** 0.5        # fp32 accumulation in any order
     torch.cuda.synchronize()
     assert _native.read_status()[0] == 0
