@@ -214,12 +214,14 @@ bn_moments_kernel(const T* __restrict__ x, int B, int F, long long R, Split sp, 
   }
 }
 
-// One warp per feature: statistics of the batch, running statistics.  stat = [mean | rstd | sum (x - mean)] x F.
+// One warp per feature: statistics of the batch, running statistics.  stat = [mean | rstd | sum (x - mean) | gamma] x F
+// (gamma as it is now: it may change before the backward pass).
 // Sums, mean and variance take the type of x on their way, as they do where they travel between workers: the
 // results (and which of two equal values a following max pooling picks) do not depend on the number of workers.
 // The gradient kernels below round in the same places.
 __global__ void bn_moments_final_kernel(const float* __restrict__ part, int splits, int F, float count, float eps,
-                                        float* __restrict__ stat, int dtype, void* run_mean, void* run_var,
+                                        float* __restrict__ stat, int dtype, const void* gamma, int gamma_dtype,
+                                        void* run_mean, void* run_var,
                                         int run_dtype, float momentum, float unbias) {
   const int f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (f >= F) return;
@@ -236,6 +238,7 @@ __global__ void bn_moments_final_kernel(const float* __restrict__ part, int spli
   stat[f] = mean;
   stat[F + f] = 1.f / sqrtf(var + eps);
   stat[2 * F + f] = count * off;
+  stat[3 * F + f] = gamma == nullptr ? 1.f : load_as(gamma, gamma_dtype, f);
   if (run_mean != nullptr) {
     const float keep = 1.f - momentum;
     store_as(run_mean, run_dtype, f, round_as(keep * load_as(run_mean, run_dtype, f), run_dtype) +
@@ -248,7 +251,7 @@ __global__ void bn_moments_final_kernel(const float* __restrict__ part, int spli
 // One warp per feature: coef = [a | b | c] x F of dx = a dy + b (x - mean) + c (through the normalisation, the
 // squared deviations and the sum), and the parameter gradients.
 __global__ void bn_grad_final_kernel(const float* __restrict__ part, int splits, int F, float count,
-                                     const float* __restrict__ stat, int dtype, const void* gamma, int gamma_dtype,
+                                     const float* __restrict__ stat, int dtype, int gamma_dtype,
                                      float* __restrict__ coef, void* dgamma, void* dbeta, int beta_dtype) {
   const int f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (f >= F) return;
@@ -259,7 +262,7 @@ __global__ void bn_grad_final_kernel(const float* __restrict__ part, int splits,
   }
   s1 = warp_sum(s1); s2 = warp_sum(s2);
   if (lane) return;
-  const float rstd = stat[F + f], g = gamma == nullptr ? 1.f : load_as(gamma, gamma_dtype, f);
+  const float rstd = stat[F + f], g = stat[3 * F + f];
   const float a = g * rstd;
   const float dv = round_as(round_as(-0.5f * g * rstd * rstd * rstd * s2, dtype) / count, dtype);
   const float dmean = round_as(round_as(-a * s1, dtype) + round_as(-2.f * dv * stat[2 * F + f], dtype), dtype);
@@ -391,21 +394,22 @@ int train_fwd(const T* x, const void* gamma, const void* beta, int gamma_dtype, 
   else     bn_moments_kernel<T, 1><<<grid, kBnThreads, 0, s>>>(x, B, F, R, sp, ws);
   const double n = (double)B * (double)R;
   bn_moments_final_kernel<<<(F + 7) / 8, 256, 0, s>>>(ws, splits, F, (float)n, eps, stat,
-                                                      sizeof(T) == 2 ? 0 : 1, run_mean, run_var, run_dtype, momentum,
+                                                      sizeof(T) == 2 ? 0 : 1, gamma, gamma_dtype, run_mean, run_var,
+                                                      run_dtype, momentum,
                                                       (float)(n / (n - 1.0 > 1.0 ? n - 1.0 : 1.0)));
   Coef k{stat + F, stat, nullptr, nullptr, gamma, beta, gamma_dtype, beta_dtype};
   return map<T, kNormalize>(x, nullptr, k, B, F, R, y, s);
 }
 
 template <typename T>
-int train_bwd(const T* x, const T* dy, const void* gamma, int gamma_dtype, int beta_dtype, int B, int F, long long R,
-              const float* stat, float* ws, float* coef, T* dx, void* dgamma, void* dbeta, cudaStream_t s) {
+int train_bwd(const T* x, const T* dy, int gamma_dtype, int beta_dtype, int B, int F, long long R, const float* stat,
+              float* ws, float* coef, T* dx, void* dgamma, void* dbeta, cudaStream_t s) {
   const bool vec = aligned16(x) && aligned16(dy);
   const Split sp = split_for(B, F, R, vec ? 16 / (int)sizeof(T) : 1);
   int r = reduce<T, true>(x, dy, stat, B, F, R, 2, sp, vec, ws, nullptr, s);
   if (r) return r;
   bn_grad_final_kernel<<<(F + 7) / 8, 256, 0, s>>>(ws, sp.su * sp.sb, F, (float)((double)B * (double)R), stat,
-                                                   sizeof(T) == 2 ? 0 : 1, gamma, gamma_dtype, coef, dgamma, dbeta, beta_dtype);
+                                                   sizeof(T) == 2 ? 0 : 1, gamma_dtype, coef, dgamma, dbeta, beta_dtype);
   if (dx == nullptr) return (int)cudaGetLastError();
   // dx = a dy + b (x - mean) + c
   Coef k{coef + F, stat, coef + 2 * F, coef, nullptr, nullptr, 1, 1};
@@ -455,8 +459,8 @@ DD_API int dd_bn_train_workspace(int B, int F, long long R) {
   return 3 * most * F;
 }
 
-// Batch norm of one worker's whole batch.  stat: [3, F] fp32 (mean, 1 / sqrt(var + eps), sum (x - mean)), kept for the
-// backward pass; gamma / beta / run_*: [F] in their own types (0 = bf16, 1 = fp32) or null.
+// Batch norm of one worker's whole batch.  stat: [4, F] fp32 (mean, 1 / sqrt(var + eps), sum (x - mean), gamma), kept
+// for the backward pass; gamma / beta / run_*: [F] in their own types (0 = bf16, 1 = fp32) or null.
 DD_API int dd_bn_train_fwd(const void* x, const void* gamma, const void* beta, int gamma_dtype, int beta_dtype, int B,
                            int F, long long R, int dtype, float eps, void* run_mean, void* run_var, int run_dtype,
                            float momentum, float* ws, float* stat, void* y, void* stream) {
@@ -472,15 +476,15 @@ DD_API int dd_bn_train_fwd(const void* x, const void* gamma, const void* beta, i
 }
 
 // coef: [3, F] fp32 scratch; dx, dgamma, dbeta may be null.
-DD_API int dd_bn_train_bwd(const void* x, const void* dy, const void* gamma, int gamma_dtype, int beta_dtype, int B, int F,
-                           long long R, int dtype, const float* stat, float* ws, float* coef, void* dx, void* dgamma,
-                           void* dbeta, void* stream) {
+DD_API int dd_bn_train_bwd(const void* x, const void* dy, int gamma_dtype, int beta_dtype, int B, int F, long long R,
+                           int dtype, const float* stat, float* ws, float* coef, void* dx, void* dgamma, void* dbeta,
+                           void* stream) {
   if (B <= 0 || F <= 0 || R <= 0 || ws == nullptr || stat == nullptr || coef == nullptr) return DD_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (dtype == 0)
     return train_bwd<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(dy),
-                                    gamma, gamma_dtype, beta_dtype, B, F, R, stat, ws, coef,
+                                    gamma_dtype, beta_dtype, B, F, R, stat, ws, coef,
                                     reinterpret_cast<__nv_bfloat16*>(dx), dgamma, dbeta, s);
-  return train_bwd<float>(reinterpret_cast<const float*>(x), reinterpret_cast<const float*>(dy), gamma, gamma_dtype,
-                          beta_dtype, B, F, R, stat, ws, coef, reinterpret_cast<float*>(dx), dgamma, dbeta, s);
+  return train_bwd<float>(reinterpret_cast<const float*>(x), reinterpret_cast<const float*>(dy), gamma_dtype, beta_dtype,
+                          B, F, R, stat, ws, coef, reinterpret_cast<float*>(dx), dgamma, dbeta, s);
 }

@@ -18,7 +18,7 @@ _native.declare("dd_bn_affine", [_v, _v, _v, _v, _v, _v, _i, _i, _ll, _i, _v, _v
 _native.declare("dd_bn_train_workspace", [_i, _i, _ll])
 _native.declare("dd_bn_train_fwd", [_v, _v, _v, _i, _i, _i, _i, _ll, _i, ctypes.c_float, _v, _v, _i, ctypes.c_float,
                                     _v, _v, _v, _v])
-_native.declare("dd_bn_train_bwd", [_v, _v, _v, _i, _i, _i, _i, _ll, _i, _v, _v, _v, _v, _v, _v, _v])
+_native.declare("dd_bn_train_bwd", [_v, _v, _i, _i, _i, _i, _ll, _i, _v, _v, _v, _v, _v, _v, _v])
 _DT = {torch.bfloat16: 0, torch.float32: 1}
 
 
@@ -115,29 +115,28 @@ class _TrainBatchNorm(torch.autograd.Function):
     def forward(ctx, x, gamma, beta, eps, running_mean, running_var, momentum):
         B, F, R = _geometry(x)
         ws = torch.empty(_native.lib().dd_bn_train_workspace(B, F, R), dtype=torch.float32, device=x.device)
-        stat = torch.empty(3, F, dtype=torch.float32, device=x.device)
+        stat = torch.empty(4, F, dtype=torch.float32, device=x.device)
         y = torch.empty_like(x)
         _native.call("dd_bn_train_fwd", x.data_ptr(), ptr(gamma), ptr(beta), 1 if gamma is None else _DT[gamma.dtype],
                      1 if beta is None else _DT[beta.dtype], B, F, R, _DT[x.dtype], eps, ptr(running_mean),
                      ptr(running_var), 1 if running_mean is None else _DT[running_mean.dtype], momentum,
                      ws.data_ptr(), stat.data_ptr(), y.data_ptr(), stream_ptr())
-        ctx.save_for_backward(x, stat, gamma)
+        ctx.save_for_backward(x, stat)         # (not gamma, which may change before the backward pass)
+        ctx.gamma_meta = None if gamma is None else (gamma.shape, gamma.dtype)
         ctx.beta_meta = None if beta is None else (beta.shape, beta.dtype)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, stat, gamma = ctx.saved_tensors
+        x, stat = ctx.saved_tensors
         B, F, R = _geometry(x)
         dy = dy.contiguous()
         ws = torch.empty(_native.lib().dd_bn_train_workspace(B, F, R) + 3 * F, dtype=torch.float32, device=x.device)
         need = ctx.needs_input_grad
         dx = torch.empty_like(x) if need[0] else None
-        dgamma = torch.empty_like(gamma) if gamma is not None and need[1] else None
-        dbeta = None
-        if ctx.beta_meta is not None and need[2]:
-            dbeta = torch.empty(ctx.beta_meta[0], dtype=ctx.beta_meta[1], device=x.device)
-        _native.call("dd_bn_train_bwd", x.data_ptr(), dy.data_ptr(), ptr(gamma), 1 if gamma is None else _DT[gamma.dtype],
+        dgamma, dbeta = (torch.empty(m[0], dtype=m[1], device=x.device) if m is not None and n else None
+                         for m, n in ((ctx.gamma_meta, need[1]), (ctx.beta_meta, need[2])))
+        _native.call("dd_bn_train_bwd", x.data_ptr(), dy.data_ptr(), 1 if dgamma is None else _DT[dgamma.dtype],
                      1 if dbeta is None else _DT[dbeta.dtype], B, F, R, _DT[x.dtype], stat.data_ptr(),
                      ws[3 * F:].data_ptr(), ws.data_ptr(), ptr(dx), ptr(dgamma), ptr(dbeta), stream_ptr())
         return dx, dgamma, dbeta, None, None, None, None

@@ -131,7 +131,8 @@ def pad(x: torch.Tensor, pad_tuple, value: float = 0.0) -> torch.Tensor:
     nd = x.dim() - 2
     spatial, rest = pad_tuple[:2 * nd], pad_tuple[2 * nd:]
     if (1 <= nd <= 3 and len(spatial) == 2 * nd and use_native(x) and x.dtype in _FILL
-            and value in (0.0, float("-inf")) and x.numel() > 0 and x.is_contiguous() and any(spatial) and min(spatial) >= 0 and not any(rest) and _plain(x)):
+            and value in (0.0, float("-inf")) and x.numel() > 0 and x.is_contiguous() and any(spatial)
+            and min(spatial) >= 0 and not any(rest) and _plain(x)):
         lo = tuple(int(a) for a in spatial[::2][::-1])
         hi = tuple(int(a) for a in spatial[1::2][::-1])
         return _ShiftCopyFn.apply(x, lo, tuple(int(n) + a + b for n, a, b in zip(x.shape[2:], lo, hi)), value != 0.0)

@@ -469,3 +469,24 @@ def test_feature_convolution_with_batched_gradients(nd, dtype):
     got, = torch.autograd.grad(p, x, dys, is_grads_batched=True, retain_graph=True)
     for k in range(3):
         assert torch.equal(got[k], torch.autograd.grad(p, x, dys[k], retain_graph=True)[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_batch_norm_weights_may_change_before_the_backward_pass(dtype):
+    """The gradient is that of the weights of the forward pass."""
+    import distdl_b200
+    from distdl_b200 import backends
+    from distdl_b200.nn import DistributedBatchNorm
+    distdl_b200.config.set_backend("native", "cupy")
+    torch.manual_seed(20)
+    P = backends.backend.Partition().create_partition_inclusive([0]).create_cartesian_topology_partition([1] * 4)
+    layer = DistributedBatchNorm(P, 6, device="cuda", dtype=dtype)
+    x = torch.randn(3, 6, 5, 7, device="cuda").to(dtype).requires_grad_()
+    dy = torch.randn(3, 6, 5, 7, device="cuda").to(dtype)
+    want = torch.autograd.grad(layer(x), (x, layer.gamma, layer.beta), dy)
+    y = layer(x)
+    with torch.no_grad():
+        layer.gamma.mul_(3)
+        layer.beta.add_(1)
+    for a, b in zip(torch.autograd.grad(y, (x, layer.gamma, layer.beta), dy), want):
+        assert torch.equal(a, b)
