@@ -897,7 +897,7 @@ DD_API int dd_colsum_parts(long long rows, int n) {
 }
 // out[c] (+)= sum over rows of x [rows, n] bf16 (16-byte aligned, n a multiple of 8)
 DD_API int dd_colsum(const void* x, long long rows, int n, float* partial, float* out, int accumulate, void* stream) {
-  if (rows <= 0 || n <= 0 || n % 8) return DD_ERR_BAD_ARG;
+  if (rows <= 0 || n <= 0 || n % 8 || x == nullptr || partial == nullptr || out == nullptr) return DD_ERR_BAD_ARG;
   if (reinterpret_cast<uintptr_t>(x) & 15) return DD_ERR_ALIGN;
   const int parts = dd_colsum_parts(rows, n);
   colsum_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)parts), 32 * kColWarps, 0, STREAM(stream)>>>(CBF(x), rows, n,

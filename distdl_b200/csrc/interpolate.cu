@@ -513,6 +513,10 @@ DD_API int dd_interpolate(int cuda, int linear, int adjoint, int dtype, int nd, 
   }
   g.align_corners = align_corners;
   g.linear = linear;
+  // (an empty tensor has no address, and so has one without storage, which must not reach a kernel)
+  long long n_in = BC, n_out = BC;
+  for (int d = 0; d < 3; ++d) { n_in *= g.in_local[d]; n_out *= g.out_local[d]; }
+  if ((x == nullptr && n_in > 0) || (y == nullptr && n_out > 0)) return DD_ERR_BAD_ARG;
   if (dtype == 0) return run<float>(cuda, adjoint, g, nd, x, y, BC, stream);
   if (dtype == 1) return run<double>(cuda, adjoint, g, nd, x, y, BC, stream);
   return run<__nv_bfloat16>(cuda, adjoint, g, nd, x, y, BC, stream);

@@ -168,3 +168,20 @@ def body_reset_setup(rank, world):
 
 def test_reset_setup_for_changes_one_worker_cannot_see():
     run_ranks("test_behaviour", "body_reset_setup", 2, timeout=120)
+
+
+def test_kernels_refuse_tensors_without_an_address():
+    """Fake tensors and the like: the entry points return an error before anything is launched."""
+    import ctypes
+
+    import distdl_b200.ops.gemm  # noqa: F401  (declares the entry point)
+    from distdl_b200 import _native
+    from distdl_b200.functional.interpolate import interpolate  # noqa: F401
+    lib, bad = _native.lib(), 1001
+    one, scale, some = (ctypes.c_int * 1)(4), (ctypes.c_double * 1)(1.0), ctypes.c_void_p(4096)
+    zero = (ctypes.c_int * 1)(0)
+    for x, y in ((None, some), (some, None)):
+        for adjoint in (0, 1):
+            assert lib.dd_interpolate(1, 1, adjoint, 0, 1, x, y, 2, one, one, zero, zero, one, one, scale, 0, None) == bad
+    for args in ((None, some, some), (some, None, some), (some, some, None)):
+        assert lib.dd_colsum(args[0], 8, 8, args[1], args[2], 0, None) == bad
