@@ -31,12 +31,26 @@ def ptr(t):
     return 0 if t is None else t.data_ptr()
 
 
-def main_grad_now(acc, owner):
+def _leaf_node(owner, ctx, k):
+    """The node that accumulates into the leaf ``owner``: the end of the views that lead from input ``k`` of the running
+    node ``ctx`` to it, a microsecond away; asked of the leaf itself, for four, where that is not the way."""
+    if ctx is not None:
+        node = ctx.next_functions[k][0]
+        further = node.next_functions
+        while len(further) == 1:
+            node = further[0][0]
+            further = node.next_functions
+        if getattr(node, "variable", None) is owner:
+            return node
+    return torch.autograd.graph.get_gradient_edge(owner).node
+
+
+def main_grad_now(acc, owner, ctx=None, k=0):
     """``acc``, the fp32 accumulator that stands for the gradient of the leaf ``owner``, if the backward pass that is
     running would hand that gradient to nobody but the optimizer's own hook; None where it has to go through autograd:
     the leaf has hooks of the user's, or the pass does not accumulate into it (``torch.autograd.grad``, ``inputs=`` of
-    ``backward``) or builds a graph.  Asked in the backward pass, so that hooks of any moment count.  ``owner`` None: a
-    gathered weight, whose gradient is never autograd's."""
+    ``backward``) or builds a graph.  Asked in the backward pass (of ``ctx``, whose input ``k`` the leaf became), so that
+    hooks of any moment count.  ``owner`` None: a gathered weight, whose gradient is never autograd's."""
     if acc is None or owner is None:
         return acc
     after = owner._post_accumulate_grad_hooks
@@ -44,7 +58,7 @@ def main_grad_now(acc, owner):
             or (after and not all(getattr(h, "into_main_grad", False) for h in after.values())):
         return None
     try:
-        runs = torch._C._will_engine_execute_node(torch.autograd.graph.get_gradient_edge(owner).node)
+        runs = torch._C._will_engine_execute_node(_leaf_node(owner, ctx, k))
     except RuntimeError:            # the pass captures the gradient of this leaf
         return None
     return acc if runs else None

@@ -27,7 +27,7 @@ class _EmbeddingFn(torch.autograd.Function):
         table = ctx.tref
         d = table.shape[-1]
         d2 = dout.reshape(-1, d).contiguous()
-        mg = main_grad_now(getattr(table, "main_grad", None), getattr(table, "main_grad_owner", None))
+        mg = main_grad_now(getattr(table, "main_grad", None), getattr(table, "main_grad_owner", None), ctx, 1)
         if mg is not None:
             _native.call("dd_embedding_bwd", flat.data_ptr(), d2.data_ptr(), mg.data_ptr(), flat.numel(), d,
                          table.shape[0], stream_ptr())

@@ -122,10 +122,10 @@ def grad_target(w: torch.Tensor):
             getattr(w, "main_grad_owner", None))
 
 
-def weight_grad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor = None, target=None):
+def weight_grad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor = None, target=None, ctx=None):
     """Gradient of ``y = x @ w.T`` with respect to ``w`` ([out, in]) from
     ``dy2 [tokens, out]`` and ``x2 [tokens, in]``; give either ``w`` or ``target =
-    grad_target(w)``.
+    grad_target(w)``, and the ``ctx`` of the running backward pass if ``w`` is its input 1.
 
     * ``w.main_grad`` (an fp32 tensor in the layout of ``w``, possibly a
       transposed view): the GEMM epilogue accumulates into it and ``None`` is
@@ -136,7 +136,7 @@ def weight_grad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor = None, tar
       view, so autograd's transpose back is free instead of a strided copy.
     """
     mg, transposed, owner = target if target is not None else grad_target(w)
-    mg = main_grad_now(mg, owner)
+    mg = main_grad_now(mg, owner, ctx, 1)
     if mg is not None:
         if mg.is_contiguous():
             gemm(dy2.t(), x2.t(), out=mg, accumulate=True)
@@ -194,9 +194,9 @@ class _LinearFn(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             dx = gemm(dy2, w.t()).view(ctx.xshape)
         if ctx.needs_input_grad[1]:
-            dw = weight_grad(dy2, x2, target=ctx.wgrad)
+            dw = weight_grad(dy2, x2, target=ctx.wgrad, ctx=ctx)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            mg = main_grad_now(*ctx.b_main_grad)
+            mg = main_grad_now(*ctx.b_main_grad, ctx, 2)
             s = column_sum(dy2, mg)
             if mg is None:
                 db = s.to(dy.dtype)
