@@ -33,12 +33,12 @@ def _plain(x) -> bool:
 
 
 def _operators(dy, lo, space):
-    """The shifted copy by the library's operators: for a backward pass under a function transform (batched gradients),
-    a dispatch mode or a tracer."""
+    """The shifted copy by the library's operators, contiguous: for a backward pass under a function transform (batched
+    gradients), a dispatch mode or a tracer."""
     pads = []
     for n, a, m in reversed(list(zip(dy.shape[-len(space):], lo, space))):
         pads += [a, m - n - a]
-    return torch.nn.functional.pad(dy, pads)
+    return torch.nn.functional.pad(dy, pads).contiguous()
 
 
 class _ShiftCopyFn(torch.autograd.Function):

@@ -460,6 +460,7 @@ def test_feature_convolution_with_batched_gradients(nd, dtype):
     y = layer(x)
     dys = torch.randn(3, *y.shape, device="cuda").to(dtype)
     got = torch.autograd.grad(y, (x, layer.weight), dys, is_grads_batched=True, retain_graph=True)
+    assert got[0].is_contiguous()
     for k in range(3):
         for a, b in zip(got, torch.autograd.grad(y, (x, layer.weight), dys[k], retain_graph=True)):
             # the same products in another order: bf16 results, or tf32 operands
