@@ -827,7 +827,7 @@ DD_API int dd_norm_fwd(int rms, const void* x, const void* res, void* xsum, cons
   return (int)cudaGetLastError();
 }
 
-// partial: scratch of dd_norm_bwd_parts(rows) * 2 * d floats (may be null when
+// partial: scratch of dd_norm_bwd_parts(rows) * 2 * d floats at any address (may be null when
 // neither dw nor db is wanted).
 DD_API int dd_norm_bwd(int rms, const void* dy, const void* x, const void* w, const void* stats, const void* dres,
                        void* dx, float* dw, float* db, float* partial, int accumulate, int rows, int d,

@@ -41,7 +41,8 @@ def _major(t: torch.Tensor):
     raise ValueError("GEMM operand needs unit stride in one of its last two dimensions")
 
 
-# outputs of more elements than this have tiles for half the SMs: the contraction is never split
+# Short cuts past the rule of dd_gemm_split, which answers 1 beyond them on a GPU of 148 SMs: outputs of more elements
+# have tiles for half the SMs, contractions of less than 4096 gain less than the second launch costs.
 _SPLIT_MAX_MN = 37 * 256 * 256
 
 
