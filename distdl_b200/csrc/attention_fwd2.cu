@@ -18,7 +18,8 @@ using namespace dd;
 #undef DD_HEAD_DIM
 #undef DD_FWD2_NS
 
-// Head dim 128 or 64, sequence length a multiple of 256.  Same argument convention as dd_attn_fwd.
+// softmax(scale * q k^T) v over [batch * S, heads, Dh] bf16 tensors, Dh = 128 or 64, any S: q / k / v by address, row and
+// head stride (in elements, unit stride within a row), out contiguous, lse [batch][Hq][S] (may be null).
 DD_API int dd_attn_fwd2(const void* q, long long q_row_stride, long long q_head_stride, const void* k,
                         long long k_row_stride, long long k_head_stride, const void* v, long long v_row_stride,
                         long long v_head_stride, void* out, float* lse, int batch, int S, int Hq, int Hkv, int Dh,

@@ -20,6 +20,8 @@
 // Issue order per KV block j:  PV_0(j), S_0(j+1), PV_1(j), S_1(j+1); products of
 // one thread execute in order, so S_t(j+1) may overwrite P_t(j) right after PV_t(j)
 // was issued.  Causal: tile t of query pair qp sees blocks 0 .. 2 qp + t.
+// Any sequence length: rows behind the end of a sequence are read as zeros (the tensor maps end there), keys there are
+// masked in the last block, queries there are not stored, and a pair's second tile may not exist at all.
 // All waits are bounded; a timeout drains and frees tensor memory.
 namespace DD_FWD2_NS {
 
@@ -66,18 +68,18 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   Barriers* bar = reinterpret_cast<Barriers*>(tiles + TILE_BYTES);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nQP = p.S / (2 * BQ);
+  const int nkv = (p.S + BKV - 1) / BKV;
+  const int nQP = (nkv + 1) / 2;
   // heaviest query pairs first; heads vary fastest (kv heads shared through L2)
   const int id = blockIdx.x;
   const int hb = id % (p.Hq * p.batch);
   const int qp = nQP - 1 - id / (p.Hq * p.batch);
   const int h = hb % p.Hq, b = hb / p.Hq;
   const int hkv = h / (p.Hq / p.Hkv);
-  const int nkv = p.S / BKV;
   const int n0 = p.causal ? 2 * qp + 1 : nkv;      // blocks seen by tile 0
-  const int n1 = p.causal ? 2 * qp + 2 : nkv;      // blocks seen by tile 1 (>= n0)
-  const int q_row0 = b * p.S + qp * 2 * BQ;
-  const int kv_row0 = b * p.S;
+  const int n1 = 2 * qp + 1 >= nkv ? 0 : p.causal ? 2 * qp + 2 : nkv;      // blocks seen by tile 1 (>= n0, or none)
+  const int blocks = n1 > n0 ? n1 : n0;
+  const int q_row0 = qp * 2 * BQ;                  // of this sequence
 
   if (threadIdx.x == 0) {
     mbar_init(&bar->q_full, 1);
@@ -108,9 +110,9 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       for (int t = 0; t < 2; ++t)
 #pragma unroll
         for (int c = 0; c < DCH; ++c)
-          tma_load_3d(sQ + t * Q_BYTES + c * (BQ * 128), &tmap_q, &bar->q_full, c * 64, q_row0 + t * BQ, h);
+          tma_load_4d(sQ + t * Q_BYTES + c * (BQ * 128), &tmap_q, &bar->q_full, c * 64, q_row0 + t * BQ, h, b);
       bool ok = true;
-      for (int j = 0; j < n1 && ok; ++j) {
+      for (int j = 0; j < blocks && ok; ++j) {
         const int st = j % KV_STAGES;
         const uint32_t ph = (j / KV_STAGES) & 1;
         ok = mbar_wait(&bar->k_empty[st], ph ^ 1, &bar->abort_flag, p.status, 31);
@@ -118,13 +120,13 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         mbar_expect_tx(&bar->k_full[st], KV_BYTES);
 #pragma unroll
         for (int c = 0; c < DCH; ++c)
-          tma_load_3d(sK + st * KV_BYTES + c * (BKV * 128), &tmap_k, &bar->k_full[st], c * 64, kv_row0 + j * BKV, hkv);
+          tma_load_4d(sK + st * KV_BYTES + c * (BKV * 128), &tmap_k, &bar->k_full[st], c * 64, j * BKV, hkv, b);
         ok = mbar_wait(&bar->v_empty[st], ph ^ 1, &bar->abort_flag, p.status, 32);
         if (!ok) break;
         mbar_expect_tx(&bar->v_full[st], KV_BYTES);
 #pragma unroll
         for (int c = 0; c < DCH; ++c)
-          tma_load_3d(sV + st * KV_BYTES + c * (BKV * 128), &tmap_v, &bar->v_full[st], c * 64, kv_row0 + j * BKV, hkv);
+          tma_load_4d(sV + st * KV_BYTES + c * (BKV * 128), &tmap_v, &bar->v_full[st], c * 64, j * BKV, hkv, b);
       }
       if (!ok) {
         const uint64_t t0 = globaltimer_ns();
@@ -163,9 +165,9 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       if (ok) {
         tc_fence_after();
         issue_S(0, 0);
-        issue_S(1, 0);
+        if (n1 > 0) issue_S(1, 0);
       }
-      for (int j = 0; j < n1 && ok; ++j) {
+      for (int j = 0; j < blocks && ok; ++j) {
         const int st = j % KV_STAGES;
         const uint32_t ph = (j / KV_STAGES) & 1;
         const int stn = (j + 1) % KV_STAGES;
@@ -207,6 +209,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const uint32_t tO = tmem_base + 256 + t * 128 + lane_off;
     const int nt = t == 0 ? n0 : n1;
     const int diag = p.causal ? 2 * qp + t : -1;
+    const int tail = p.S % BKV ? nkv - 1 : -1;      // block with keys behind the end of the sequence
     const float c = p.scale * 1.4426950408889634f;  // scores are exponentiated base 2
     float m_ref = -INFINITY, l = 0.f;
     bool ok = true;
@@ -221,10 +224,11 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       tmem_ld_32x32(tS + 96, *reinterpret_cast<uint32_t(*)[32]>(s + 96));
       tmem_ld_wait();
       float mx = m_ref;
-      if (j == diag) {
+      if (j == diag || j == tail) {
+        const int seen = min(j == diag ? row : BKV - 1, p.S - 1 - j * BKV);     // last key of this block that counts
 #pragma unroll
         for (int i = 0; i < 128; ++i) {
-          if (i > row) s[i] = 0xff800000u;          // -inf
+          if (i > seen) s[i] = 0xff800000u;          // -inf
           mx = fmaxf(mx, __uint_as_float(s[i]));
         }
       } else {
@@ -272,17 +276,19 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar->p_full[t]);
     }
-    if (ok) {
+    if (ok && nt > 0) {
       ok = mbar_wait(&bar->pv_done[t], (nt - 1) & 1, &bar->abort_flag, p.status, 40);
       if (ok) {
         tc_fence_after();
         const float inv = 1.f / l;
-        __nv_bfloat16* orow = p.O + ((size_t)(q_row0 + t * BQ + row) * p.Hq + h) * D;
+        const int q_row = q_row0 + t * BQ + row;
+        __nv_bfloat16* orow = p.O + (((size_t)b * p.S + q_row) * p.Hq + h) * D;
 #pragma unroll 1
         for (int ch = 0; ch < D / 32; ++ch) {
           uint32_t r[32];
           tmem_ld_32x32(tO + ch * 32, r);
           tmem_ld_wait();
+          if (q_row >= p.S) continue;
           uint4* dst = reinterpret_cast<uint4*>(orow + ch * 32);
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
@@ -294,8 +300,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             dst[g] = v;
           }
         }
-        if (p.lse != nullptr)
-          p.lse[((size_t)b * p.Hq + h) * p.S + qp * 2 * BQ + t * BQ + row] = m_ref * p.scale + logf(l);
+        if (p.lse != nullptr && q_row < p.S)
+          p.lse[((size_t)b * p.Hq + h) * p.S + q_row] = m_ref * p.scale + logf(l);
       }
     }
   }
@@ -305,19 +311,20 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
-// Two-tile forward kernel: sequence length a multiple of 256.  Same argument convention as dd_attn_fwd.
 int run(const void* q, long long q_row_stride, long long q_head_stride, const void* k,
                         long long k_row_stride, long long k_head_stride, const void* v, long long v_row_stride,
                         long long v_head_stride, void* out, float* lse, int batch, int S, int Hq, int Hkv, int Dh,
                         int causal, float scale, void* stream) {
-  if (S % 256 != 0 || Dh != D || Hq % Hkv != 0 || batch <= 0) return DD_ERR_BAD_ARG;
-  const uint64_t tokens = (uint64_t)batch * S;
+  if (S <= 0 || Dh != D || Hkv <= 0 || Hq <= 0 || Hq % Hkv != 0 || batch <= 0) return DD_ERR_BAD_ARG;
   CUtensorMap tq, tk, tv;
-  int r = get_tensor_map_bf16_3d(&tq, q, D, tokens, Hq, q_row_stride * 2, q_head_stride * 2, 64, BQ);
+  int r = get_tensor_map_bf16_4d(&tq, q, D, S, Hq, batch, q_row_stride * 2, q_head_stride * 2,
+                                 (uint64_t)S * q_row_stride * 2, 64, BQ);
   if (r) return r;
-  r = get_tensor_map_bf16_3d(&tk, k, D, tokens, Hkv, k_row_stride * 2, k_head_stride * 2, 64, BKV);
+  r = get_tensor_map_bf16_4d(&tk, k, D, S, Hkv, batch, k_row_stride * 2, k_head_stride * 2,
+                             (uint64_t)S * k_row_stride * 2, 64, BKV);
   if (r) return r;
-  r = get_tensor_map_bf16_3d(&tv, v, D, tokens, Hkv, v_row_stride * 2, v_head_stride * 2, 64, BKV);
+  r = get_tensor_map_bf16_4d(&tv, v, D, S, Hkv, batch, v_row_stride * 2, v_head_stride * 2,
+                             (uint64_t)S * v_row_stride * 2, 64, BKV);
   if (r) return r;
   int err = 0;
   Params2 p;
@@ -338,10 +345,11 @@ int run(const void* q, long long q_row_stride, long long q_head_stride, const vo
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = true;
   }
-  const int grid = (S / (2 * BQ)) * Hq * batch;
+  const long long grid = (S / (2 * BQ) + (S % (2 * BQ) != 0)) * (long long)Hq * batch;
+  if (grid > 0x7fffffffLL) return DD_ERR_TOO_LARGE;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (poly) attn_fwd2_kernel<true><<<grid, NUM_THREADS, SMEM_TOTAL, st>>>(tq, tk, tv, p);
-  else attn_fwd2_kernel<false><<<grid, NUM_THREADS, SMEM_TOTAL, st>>>(tq, tk, tv, p);
+  if (poly) attn_fwd2_kernel<true><<<(unsigned)grid, NUM_THREADS, SMEM_TOTAL, st>>>(tq, tk, tv, p);
+  else attn_fwd2_kernel<false><<<(unsigned)grid, NUM_THREADS, SMEM_TOTAL, st>>>(tq, tk, tv, p);
   return (int)cudaGetLastError();
 }
 

@@ -17,20 +17,20 @@ int g_sm_count[kMaxDevices] = {0};
 
 struct MapKey {
   const void* base;
-  uint64_t inner, outer, batch, s1, s2;
+  uint64_t inner, outer, batch, s1, s2, groups, s3;      // groups = 0: three dimensions
   uint32_t b0, b1;
   int dev;
   int f32;
   bool operator==(const MapKey& o) const {
     return f32 == o.f32 && base == o.base && inner == o.inner && outer == o.outer && batch == o.batch && s1 == o.s1 &&
-           s2 == o.s2 && b0 == o.b0 && b1 == o.b1 && dev == o.dev;
+           s2 == o.s2 && groups == o.groups && s3 == o.s3 && b0 == o.b0 && b1 == o.b1 && dev == o.dev;
   }
 };
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
     uint64_t h = reinterpret_cast<uint64_t>(k.base) * 0x9E3779B97F4A7C15ull;
     auto mix = [&h](uint64_t v) { h ^= v + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2); };
-    mix(k.inner); mix(k.outer); mix(k.batch); mix(k.s1); mix(k.s2); mix(k.b0); mix(k.b1); mix(k.dev); mix(k.f32);
+    mix(k.inner); mix(k.outer); mix(k.batch); mix(k.s1); mix(k.s2); mix(k.groups); mix(k.s3); mix(k.b0); mix(k.b1); mix(k.dev); mix(k.f32);
     return (size_t)h;
   }
 };
@@ -80,31 +80,39 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 namespace {
-int get_tensor_map_3d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t batch,
-                      uint64_t outer_stride_bytes, uint64_t batch_stride_bytes, uint32_t box_inner,
-                      uint32_t box_outer, int f32);
+int get_tensor_map(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t batch,
+                   uint64_t groups, uint64_t outer_stride_bytes, uint64_t batch_stride_bytes,
+                   uint64_t group_stride_bytes, uint32_t box_inner, uint32_t box_outer, int f32);
+}
+int get_tensor_map_bf16_4d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t heads,
+                           uint64_t sequences, uint64_t row_stride_bytes, uint64_t head_stride_bytes,
+                           uint64_t sequence_stride_bytes, uint32_t box_inner, uint32_t box_rows) {
+  return get_tensor_map(out, base, inner, rows, heads, sequences, row_stride_bytes, head_stride_bytes,
+                        sequence_stride_bytes, box_inner, box_rows, 0);
 }
 int get_tensor_map_bf16_3d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer,
                            uint64_t batch, uint64_t outer_stride_bytes, uint64_t batch_stride_bytes,
                            uint32_t box_inner, uint32_t box_outer) {
-  return get_tensor_map_3d(out, base, inner, outer, batch, outer_stride_bytes, batch_stride_bytes, box_inner,
-                           box_outer, 0);
+  return get_tensor_map(out, base, inner, outer, batch, 0, outer_stride_bytes, batch_stride_bytes, 0, box_inner,
+                        box_outer, 0);
 }
 int get_tensor_map_f32_3d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer,
                           uint64_t batch, uint64_t outer_stride_bytes, uint64_t batch_stride_bytes,
                           uint32_t box_inner, uint32_t box_outer) {
-  return get_tensor_map_3d(out, base, inner, outer, batch, outer_stride_bytes, batch_stride_bytes, box_inner,
-                           box_outer, 1);
+  return get_tensor_map(out, base, inner, outer, batch, 0, outer_stride_bytes, batch_stride_bytes, 0, box_inner,
+                        box_outer, 1);
 }
 namespace {
-int get_tensor_map_3d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t batch,
-                      uint64_t outer_stride_bytes, uint64_t batch_stride_bytes, uint32_t box_inner,
-                      uint32_t box_outer, int f32) {
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (outer_stride_bytes & 15) || (batch_stride_bytes & 15))
+int get_tensor_map(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t batch,
+                   uint64_t groups, uint64_t outer_stride_bytes, uint64_t batch_stride_bytes,
+                   uint64_t group_stride_bytes, uint32_t box_inner, uint32_t box_outer, int f32) {
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (outer_stride_bytes & 15) || (batch_stride_bytes & 15) ||
+      (group_stride_bytes & 15))
     return DD_ERR_ALIGN;
   int dev = 0;
   cudaGetDevice(&dev);
-  MapKey key{base, inner, outer, batch, outer_stride_bytes, batch_stride_bytes, box_inner, box_outer, dev, f32};
+  MapKey key{base, inner, outer, batch, outer_stride_bytes, batch_stride_bytes, groups, group_stride_bytes, box_inner,
+             box_outer, dev, f32};
   {
     std::lock_guard<std::mutex> lk(g_mu);
     auto it = g_maps.find(key);
@@ -121,19 +129,20 @@ int get_tensor_map_3d(CUtensorMap* out, const void* base, uint64_t inner, uint64
     cudaFree(nullptr);
     ctx_bound = true;
   }
-  cuuint64_t dims[3] = {inner, outer, batch};
-  cuuint64_t strides[2] = {outer_stride_bytes, batch_stride_bytes};
-  cuuint32_t box[3] = {box_inner, box_outer, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  cuuint64_t dims[4] = {inner, outer, batch, groups};
+  cuuint64_t strides[3] = {outer_stride_bytes, batch_stride_bytes, group_stride_bytes};
+  cuuint32_t box[4] = {box_inner, box_outer, 1, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = enc(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, groups ? 4 : 3,
+                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     fprintf(stderr,
-            "distdl_b200: cuTensorMapEncodeTiled failed (%d): base=%p dims={%llu,%llu,%llu} strides={%llu,%llu} "
-            "box={%u,%u,1}\n",
+            "distdl_b200: cuTensorMapEncodeTiled failed (%d): base=%p dims={%llu,%llu,%llu,%llu} strides={%llu,%llu,%llu} "
+            "box={%u,%u,1,1}\n",
             (int)r, base, (unsigned long long)inner, (unsigned long long)outer, (unsigned long long)batch,
-            (unsigned long long)outer_stride_bytes, (unsigned long long)batch_stride_bytes, box_inner, box_outer);
+            (unsigned long long)groups, (unsigned long long)outer_stride_bytes, (unsigned long long)batch_stride_bytes,
+            (unsigned long long)group_stride_bytes, box_inner, box_outer);
     return DD_ERR_DRIVER;
   }
   {

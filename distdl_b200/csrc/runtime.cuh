@@ -27,6 +27,12 @@ int get_tensor_map_f32_3d(CUtensorMap* out, const void* base, uint64_t inner, ui
                           uint64_t batch, uint64_t outer_stride_bytes, uint64_t batch_stride_bytes,
                           uint32_t box_inner, uint32_t box_outer);
 
+// A rank-4 bf16 tensor map of [rows, heads, D] tensors of several sequences: dims {inner, rows, heads, sequences}, box
+// {box_inner, box_rows, 1, 1}.  Rows behind the end of a sequence read as zeros.
+int get_tensor_map_bf16_4d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t heads,
+                           uint64_t sequences, uint64_t row_stride_bytes, uint64_t head_stride_bytes,
+                           uint64_t sequence_stride_bytes, uint32_t box_inner, uint32_t box_rows);
+
 int current_sm_count();
 
 }  // namespace dd

@@ -9,12 +9,14 @@ output of a fused QKV projection is consumed in place (strided views).
 """
 from __future__ import annotations
 
+import functools
 import math
 
 import torch
 
 from .. import _native
 from ._util import env, stream_ptr, use_native
+from .pad import _plain
 
 _native.declare("dd_attn_fwd", [_native.c_void_p, _native.c_ll, _native.c_ll, _native.c_void_p, _native.c_ll,
                                 _native.c_ll, _native.c_void_p, _native.c_ll, _native.c_ll, _native.c_void_p,
@@ -39,6 +41,13 @@ _native.declare("dd_attn_bwd", [_native.c_void_p, _native.c_ll, _native.c_ll, _n
                                 _native.c_void_p, _native.c_ll, _native.c_ll, _native.c_int, _native.c_int,
                                 _native.c_int, _native.c_int, _native.c_int, _native.c_int, _native.c_float,
                                 _native.c_void_p])
+_native.declare("dd_attn_bwd3", _BWD_ARGS[:13] + [_native.c_ll] + _BWD_ARGS[13:])
+_native.declare("dd_attn_bwd_one_pass", [_native.c_int] * 6)
+
+
+@functools.lru_cache(maxsize=1024)
+def _one_pass(batch, seq, Hq, Hkv, D, causal):
+    return bool(_native.lib().dd_attn_bwd_one_pass(batch, seq, Hq, Hkv, D, int(causal)))
 
 
 def _strides(t):
@@ -54,9 +63,8 @@ def attention_forward(q, k, v, batch, seq, causal=True, scale=None):
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     out = torch.empty(tokens, Hq, D, dtype=q.dtype, device=q.device)
     lse = torch.empty(batch, Hq, seq, dtype=torch.float32, device=q.device)
-    # head dim 128 / 64 and sequences of whole 256-row pairs run the two-tile kernel (scores and
-    # probabilities in tensor memory, two query tiles alternating on the tensor cores)
-    two_tile = D in (64, 128) and seq % 256 == 0 and env("DISTDL_ATTN_FWD2", "1") != "0"
+    # the two-tile kernel (scores and probabilities in tensor memory, two query tiles alternating on the tensor cores)
+    two_tile = D in (64, 128) and (env("DISTDL_ATTN_FWD2", "1") != "0" or seq % 128 != 0)
     _native.call("dd_attn_fwd2" if two_tile else "dd_attn_fwd", q.data_ptr(), *_strides(q), k.data_ptr(), *_strides(k),
                  v.data_ptr(), *_strides(v), out.data_ptr(), lse.data_ptr(), batch, seq, Hq, Hkv, D, int(causal),
                  float(scale), stream_ptr())
@@ -75,6 +83,22 @@ def attention_backward(dout, q, k, v, out, lse, batch, seq, causal=True, scale=N
     if dv is None:
         dv = torch.empty(tokens, Hkv, D, dtype=q.dtype, device=q.device)
     dout, out = dout.contiguous(), out.contiguous()
+    if seq % 128 and dout.data_ptr() % 16:
+        dout = dout.clone()
+    in_tmem = env("DISTDL_ATTN_BWD2", "1") != "0" or seq % 128 != 0
+    if in_tmem and D in (64, 128) and _one_pass(batch, seq, Hq, Hkv, D, bool(causal)):
+        # one kernel for all three gradients.  Scratch per 128 queries of a head: two statistics each and two counters;
+        # with more than one key tile the sums of dQ, with grouped-query heads those of dK and dV
+        tiles = batch * Hq * ((seq + 127) // 128)
+        words = 256 * tiles + 4 + (2 * tiles + 3) // 4 * 4 + (128 * D * tiles if seq > 128 else 0)
+        if Hq > Hkv:
+            words += 256 * D * (tiles // Hq * Hkv)
+        scratch = torch.empty(words, dtype=torch.float32, device=q.device)
+        _native.call("dd_attn_bwd3", q.data_ptr(), *_strides(q), k.data_ptr(), *_strides(k), v.data_ptr(), *_strides(v),
+                     out.data_ptr(), dout.data_ptr(), lse.data_ptr(), scratch.data_ptr(), words, dq.data_ptr(),
+                     *_strides(dq), dk.data_ptr(), *_strides(dk), dv.data_ptr(), *_strides(dv), batch, seq, Hq, Hkv, D,
+                     int(causal), float(scale), stream_ptr())
+        return dq, dk, dv
     # the kernels that keep P / dS in tensor memory (scratch: delta and the base-2 lse)
     in_tmem = D in (64, 128) and env("DISTDL_ATTN_BWD2", "1") != "0"
     delta = torch.empty(2 if in_tmem else 1, batch, Hq, seq, dtype=torch.float32, device=q.device)
@@ -127,6 +151,26 @@ def attention(q, k, v, batch: int, seq: int, causal: bool = True, scale: float =
     return _reference(q, k, v, batch, seq, causal, scale)
 
 
+def _operators(dout, qkv, Hq, Hkv, batch, seq, causal, scale):
+    """The packed gradient by the library's operators: for a backward pass that is itself differentiated, or runs under
+    a function transform (batched gradients), a dispatch mode or a tracer."""
+    with torch.enable_grad():
+        out = _reference(qkv[:, :Hq], qkv[:, Hq:Hq + Hkv], qkv[:, Hq + Hkv:], batch, seq, causal, scale)
+        return torch.autograd.grad(out, qkv, dout, create_graph=True)[0]
+
+
+def _ragged_ok(qkv, Hq, Hkv, batch, seq):
+    """Sequences that are not whole tiles of 128, in training at head dim 128: the kernels take over from the library's
+    operators, whose packed gradient is put together by copies (forward and backward, 3 x 1000 tokens, 16 / 4 heads:
+    189 -> 126 us on the GPU, 310 -> 185 on the host; 2 x 1531, 32 / 8: 370 -> 272; 8 x 333, 16 heads: 194 -> 89), where
+    nobody looks for the operators themselves and where the tensor maps can address the projection.  Without a gradient
+    (2 x 1531, 32 / 8: 54 against 68 us) and at head dim 64 the library's kernels are the faster ones."""
+    return (qkv.dim() == 3 and qkv.shape[2] == 128 and qkv.requires_grad and torch.is_grad_enabled() and batch > 0
+            and seq > 0 and Hkv > 0 and Hq > 0 and Hq % Hkv == 0 and qkv.shape[0] == batch * seq
+            and qkv.shape[1] == Hq + 2 * Hkv and qkv.data_ptr() % 16 == 0 and _plain(qkv)
+            and not (torch.is_autocast_enabled() and torch.get_autocast_dtype("cuda") != torch.bfloat16))
+
+
 class _PackedAttnFn(torch.autograd.Function):
     """Attention on a packed ``[tokens, Hq + 2*Hkv, D]`` projection output; the
     backward kernels write dq / dk / dv straight into one packed gradient."""
@@ -144,6 +188,8 @@ class _PackedAttnFn(torch.autograd.Function):
         qkv, out, lse = ctx.saved_tensors
         Hq, Hkv, batch, seq, causal, scale = ctx.cfg
         q, k, v = qkv[:, :Hq], qkv[:, Hq:Hq + Hkv], qkv[:, Hq + Hkv:]
+        if seq % 128 and (torch.is_grad_enabled() or not _plain(dout)):
+            return _operators(dout, qkv, Hq, Hkv, batch, seq, causal, scale), None, None, None, None, None, None
         dqkv = torch.empty_like(qkv)
         attention_backward(dout, q, k, v, out, lse, batch, seq, causal, scale, dq=dqkv[:, :Hq],
                            dk=dqkv[:, Hq:Hq + Hkv], dv=dqkv[:, Hq + Hkv:])
@@ -154,8 +200,9 @@ def attention_packed(qkv, Hq: int, Hkv: int, batch: int, seq: int, causal: bool 
     """Attention over a packed projection ``[tokens, Hq + 2*Hkv, head_dim]`` (heads
     ordered q..., k..., v...).  Returns ``[tokens, Hq, head_dim]``."""
     D = qkv.shape[-1]
-    native = (use_native(qkv) and qkv.dtype == torch.bfloat16 and D in (64, 128) and seq % 128 == 0
-              and qkv.is_contiguous() and env("DISTDL_ATTN_IMPL", "native") == "native")
+    native = (use_native(qkv) and qkv.dtype == torch.bfloat16 and D in (64, 128) and qkv.is_contiguous()
+              and env("DISTDL_ATTN_IMPL", "native") == "native"
+              and (seq % 128 == 0 or _ragged_ok(qkv, Hq, Hkv, batch, seq)))
     if native:
         return _PackedAttnFn.apply(qkv, Hq, Hkv, batch, seq, causal, scale)
     return _reference(qkv[:, :Hq], qkv[:, Hq:Hq + Hkv], qkv[:, Hq + Hkv:], batch, seq, causal, scale)

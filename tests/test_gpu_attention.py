@@ -109,3 +109,71 @@ def test_backward_of_more_sequences_than_a_grid_dimension_holds():
         for a, r in zip(grads, one):
             assert torch.equal(a[sl], r)
     assert _native.read_status()[0] == 0
+
+
+@pytest.mark.parametrize("batch,seq,Hq,Hkv,D,causal", [
+    (1, 7, 2, 2, 128, True),            # less than a tile
+    (2, 128, 40, 40, 64, False),        # one key tile: nothing is handed on
+    (3, 129, 4, 2, 128, True),          # one query and one key in the last tile, heads of a group on CTAs of their own
+    (2, 1000, 8, 4, 128, True),
+    (1, 641, 4, 1, 128, True),
+    (1, 512, 6, 2, 64, False),          # split groups, the last key tile finishes every query tile
+    (8, 384, 20, 20, 64, True),         # more key tiles than SMs: nobody starts together
+    (8, 640, 40, 20, 64, True),         # heads of a group one after the other
+    (1, 8192, 18, 9, 128, True),        # the same, the long sweeps at head dim 128
+    (2, 2048, 16, 16, 64, True)])       # four key tiles of a head start together
+def test_backward_in_one_pass(batch, seq, Hq, Hkv, D, causal):
+    """All three gradients from one kernel, against 64 bits.  P and dS are rounded to bf16 (2**-9 each at most) before the
+    products and the gradients after them: 2-norm errors of about 2**-9 * sqrt(2) = 0.28 %; 0.5 % allowed.  Twice the same
+    bits: the partial sums have an order."""
+    from distdl_b200 import _native
+    from distdl_b200.ops.attention import _one_pass, attention_backward, attention_forward
+    assert _one_pass(batch, seq, Hq, Hkv, D, causal)
+    torch.manual_seed(17)
+    T = batch * seq
+    qkv = torch.randn(T, Hq + 2 * Hkv, D, device="cuda", dtype=torch.bfloat16)
+    q, k, v = qkv[:, :Hq], qkv[:, Hq:Hq + Hkv], qkv[:, Hq + Hkv:]
+    dout = torch.randn(T, Hq, D, device="cuda", dtype=torch.bfloat16)
+    out, lse = attention_forward(q, k, v, batch, seq, causal)
+    grads = attention_backward(dout, q, k, v, out, lse, batch, seq, causal)
+    again = attention_backward(dout, q, k, v, out, lse, batch, seq, causal)
+    assert _native.read_status()[0] == 0
+    mask = torch.triu(torch.ones(seq, seq, device="cuda", dtype=torch.bool), 1) if causal else None
+    G, err, size = Hq // Hkv, [0.0] * 4, [0.0] * 4
+    for n in range(Hkv):                                      # one group of heads at a time: [batch, G or 1, seq, D]
+        heads = [slice(n * G, (n + 1) * G), slice(n, n + 1), slice(n, n + 1)]
+        four = lambda t, sl: t[:, sl].double().reshape(batch, seq, -1, D).transpose(1, 2)  # noqa: E731
+        ins = [four(t, sl).requires_grad_() for t, sl in zip((q, k, v), heads)]
+        s = ins[0] @ ins[1].transpose(-1, -2) / math.sqrt(D)
+        ref = (s if mask is None else s.masked_fill(mask, float("-inf"))).softmax(-1) @ ins[2]
+        want = [ref, *torch.autograd.grad(ref, ins, four(dout, heads[0]))]
+        for i, (t, w, sl) in enumerate(zip((out, *grads), want, [heads[0], *heads])):
+            err[i] += (four(t, sl) - w).pow(2).sum().item()
+            size[i] += w.pow(2).sum().item()
+    assert all(e < 5e-3 ** 2 * z for e, z in zip(err, size)), (err, size)
+    assert all(torch.equal(g, a) for g, a in zip(grads, again))
+
+
+def test_ragged_projection_in_training():
+    """Sequences that are not whole tiles run natively where a gradient is wanted, with a gradient at any address of
+    its own; without one they keep the library's operators."""
+    from distdl_b200.ops import attention_packed
+    from distdl_b200.ops.attention import _ragged_ok, _reference
+    torch.manual_seed(18)
+    B, S, Hq, Hkv, D = 2, 100, 4, 2, 128
+    x = torch.randn(B * S, Hq + 2 * Hkv, D, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    dout = torch.randn(B * S, Hq, D, device="cuda", dtype=torch.bfloat16)
+    y = attention_packed(x, Hq, Hkv, B, S)
+    assert type(y.grad_fn).__name__ == "_PackedAttnFnBackward"
+    w = x.detach().clone().requires_grad_()
+    h, = torch.autograd.grad(_reference(w[:, :Hq], w[:, Hq:Hq + Hkv], w[:, Hq + Hkv:], B, S, True, 1.0 / math.sqrt(D)), w, dout)
+    shifted = torch.empty(dout.numel() + 8, device="cuda", dtype=torch.bfloat16)[4:4 + dout.numel()].view(dout.shape).copy_(dout)
+    for d in (dout, shifted):
+        g, = torch.autograd.grad(y, x, d, retain_graph=True)
+        # two kernels, both with gradients of 0.28 % (see above)
+        assert (g.float() - h.float()).norm() < 8e-3 * h.float().norm()
+    with torch.no_grad():
+        assert attention_packed(x, Hq, Hkv, B, S).grad_fn is None
+        assert not _ragged_ok(x, Hq, Hkv, B, S)
+    odd = torch.empty(x.numel() + 8, device="cuda", dtype=torch.bfloat16)[1:1 + x.numel()].view(x.shape).requires_grad_()
+    assert not _ragged_ok(odd, Hq, Hkv, B, S)          # (and the library's kernels are not called with it here)
