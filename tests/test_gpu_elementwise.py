@@ -383,3 +383,17 @@ def test_norm_backward_takes_a_scratch_that_starts_anywhere(d):
         results.append((dx, dw, db))
     for other in results[1:]:
         assert all(torch.equal(a, b) for a, b in zip(results[0], other))
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 1023, 4099, (1 << 20) + 7])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_sum_of_squares_at_any_length_and_address(n, shift):
+    """16-byte loads where the address allows them, single ones otherwise and at the end.  fp32 sums of n non-negative
+    terms over thousands of threads: at most a few hundred roundings in a row, 512 * 2**-24."""
+    from distdl_b200.ops import sumsq_
+    torch.manual_seed(21)
+    x = torch.randn(n + shift, device="cuda")[shift:]
+    out = torch.full((1,), 2.0, device="cuda")
+    sumsq_(x, out)
+    want = x.double().pow(2).sum().item() + 2.0
+    assert abs(out.item() - want) <= 512 * 2 ** -24 * want
