@@ -301,7 +301,7 @@ class Block(torch.nn.Module):
 
 def _add_norm(norm, x, delta):
     """``(x + delta, norm(x + delta))``, fused where the norm layer can take a residual."""
-    if hasattr(norm, "_gathered"):
+    if hasattr(norm, "_gathered") or isinstance(norm, dnn.DistributedLayerNorm):
         return norm(x, residual=delta)
     s = x + delta
     return s, norm(s)

@@ -6,7 +6,7 @@ import torch
 from .. import ops
 from ..utilities.slicing import compute_subshape
 from ..utilities.torch import zero_volume_tensor
-from ._linear_common import derived_partition, root_partition
+from ._linear_common import attach_main_grad, derived_partition, root_partition, through
 from .all_sum_reduce import AllSumReduce
 from .broadcast import Broadcast
 from .module import Module
@@ -85,8 +85,8 @@ class DistributedLayerNorm(Module):
         """Broadcasts the affine parameters ahead of the next forward
         (``src/distdl/nn/layernorm.py:249-263``)."""
         if self.P_x.active and self.elementwise_affine:
-            self.weight_buffer = self.broadcast_weight(self.weight)
-            self.bias_buffer = self.broadcast_bias(self.bias)
+            self.weight_buffer = through(self.broadcast_weight, self.weight)
+            self.bias_buffer = through(self.broadcast_bias, self.bias)
 
     def gather_state_dict(self, module, destination, prefix, *args):
         if not (self.collect_state and self.P_x.active and self.elementwise_affine):
@@ -112,9 +112,11 @@ class DistributedLayerNorm(Module):
             destination[key] = self.scatter(t)
         return destination
 
-    def forward(self, input):
+    def forward(self, input, residual=None):
+        """With ``residual``: returns ``(input + residual, norm(input + residual))``, the add fused into the norm kernel
+        where the rows are whole on this worker."""
         if not self.P_x.active:
-            return input
+            return input if residual is None else (input, input)
         w = b = None
         if self.elementwise_affine:
             if self.weight_buffer is None:
@@ -122,10 +124,23 @@ class DistributedLayerNorm(Module):
             w, b = self.weight_buffer, self.bias_buffer
             self.weight_buffer = self.bias_buffer = None
         nn = len(self.normalized_shape)
+        if self.num_reduce == 1 and nn == 1:
+            if w is not None:
+                w, b = w.reshape(-1), b.reshape(-1)
+                if w is not self.weight and b is not self.bias:          # (views, which may carry attributes)
+                    attach_main_grad(w, self.weight, self.broadcast_weight)
+                    attach_main_grad(b, self.bias, self.broadcast_bias)
+            if residual is not None:
+                return ops.add_layer_norm(input, residual, w, b, self.eps)
+            return ops.layer_norm(input, w, b, self.eps)
+        if residual is not None:
+            input = input + residual
+            return input, self._normalize(input, w, b)
+        return self._normalize(input, w, b)
+
+    def _normalize(self, input, w, b):
+        nn = len(self.normalized_shape)
         if self.num_reduce == 1:
-            if nn == 1:
-                return ops.layer_norm(input, None if w is None else w.reshape(-1), None if b is None else b.reshape(-1),
-                                      self.eps)
             shape = tuple(input.shape[-nn:])
             return torch.nn.functional.layer_norm(input, shape, None if w is None else w.reshape(shape),
                                                   None if b is None else b.reshape(shape), self.eps)

@@ -8,7 +8,7 @@ import torch
 from .. import ops
 from ..utilities.torch import zero_volume_tensor
 from . import init
-from ._linear_common import (PrefetchStream, attach_main_grad, derived_partition, local_out_features, relayout,
+from ._linear_common import (PrefetchStream, attach_main_grad, derived_partition, local_out_features, relayout, through,
                              root_partition, var_blocks)
 from .all_gather import AllGather
 from .broadcast import Broadcast
@@ -181,17 +181,17 @@ class DistributedLinearAllGather(Module):
             return
 
         def work():
-            self.weight_buffer = self.broadcast_weight(self.weight).view(-1, self.in_features)
+            self.weight_buffer = through(self.broadcast_weight, self.weight).view(-1, self.in_features)
             if self.bias is not None:
-                self.bias_buffer = self.broadcast_bias(self.bias).view(-1)
+                self.bias_buffer = through(self.broadcast_bias, self.bias).view(-1)
         self.prefetch.run(work)
 
     def forward(self, input):
         if not self.P_y.active:
             return input
         if self.weight_buffer is None:
-            weight = self.broadcast_weight(self.weight).view(-1, self.in_features)
-            bias = self.broadcast_bias(self.bias).view(-1) if self.bias is not None else None
+            weight = through(self.broadcast_weight, self.weight).view(-1, self.in_features)
+            bias = through(self.broadcast_bias, self.bias).view(-1) if self.bias is not None else None
             attach_main_grad(weight, self.weight, self.broadcast_weight)
             if bias is not None:
                 attach_main_grad(bias, self.bias, self.broadcast_bias)
@@ -202,7 +202,7 @@ class DistributedLinearAllGather(Module):
         fused = _fused_ag_linear(self, input, weight, bias)
         if fused is not None:
             return fused
-        input = self.all_gather(input)
+        input = through(self.all_gather, input)
         return ops.linear(input, weight, bias)
 
 

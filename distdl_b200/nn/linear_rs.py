@@ -9,7 +9,7 @@ from .. import ops
 from ..utilities.slicing import compute_subshape
 from ..utilities.torch import zero_volume_tensor
 from . import init
-from ._linear_common import PrefetchStream, attach_main_grad, derived_partition, root_partition
+from ._linear_common import PrefetchStream, attach_main_grad, derived_partition, root_partition, through
 from .broadcast import Broadcast
 from .module import Module
 from .reduce_scatter import ReduceScatter
@@ -156,17 +156,17 @@ class DistributedLinearReduceScatter(Module):
             return
 
         def work():
-            self.weight_buffer = self.broadcast_weight(self.weight).view(self.out_features, -1)
+            self.weight_buffer = through(self.broadcast_weight, self.weight).view(self.out_features, -1)
             if self.bias is not None:
-                self.bias_buffer = self.broadcast_bias(self.bias).view(self.out_features)
+                self.bias_buffer = through(self.broadcast_bias, self.bias).view(self.out_features)
         self.prefetch.run(work)
 
     def forward(self, input):
         if not self.P_x.active:
             return input
         if self.weight_buffer is None:
-            weight = self.broadcast_weight(self.weight).view(self.out_features, -1)
-            bias = self.broadcast_bias(self.bias).view(self.out_features) if self.bias is not None else None
+            weight = through(self.broadcast_weight, self.weight).view(self.out_features, -1)
+            bias = through(self.broadcast_bias, self.bias).view(self.out_features) if self.bias is not None else None
             attach_main_grad(weight, self.weight, self.broadcast_weight)
             if bias is not None:
                 attach_main_grad(bias, self.bias, self.broadcast_bias)
@@ -178,7 +178,7 @@ class DistributedLinearReduceScatter(Module):
         if fused is not None:
             return fused
         y = ops.linear(input, weight, bias)
-        return self.reduce_scatter(y)
+        return through(self.reduce_scatter, y)
 
 
 def _fused_linear_rs(layer, input, weight, bias):

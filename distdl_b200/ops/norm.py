@@ -10,7 +10,7 @@ from __future__ import annotations
 import torch
 
 from .. import _native
-from ._util import ptr, stream_ptr, use_native
+from ._util import main_grad_now, ptr, stream_ptr, use_native
 
 _scratch = {}
 
@@ -24,6 +24,18 @@ def _partial_buffer(rows: int, d: int, device) -> torch.Tensor:
         buf = torch.empty(need, dtype=torch.float32, device=device)
         _scratch[device] = buf
     return buf
+
+
+def _main_grads(ctx, want_w, want_b, k):
+    """The fp32 accumulators of weight (input ``k`` of ``ctx``) and bias that the backward kernel may add to: those of
+    gathered parameters, or of leaves whose gradient nobody but the optimizer waits for (both or neither)."""
+    mgw = main_grad_now(getattr(ctx.wref, "main_grad", None), getattr(ctx.wref, "main_grad_owner", None), ctx, k) \
+        if want_w else None
+    mgb = main_grad_now(getattr(ctx.bref, "main_grad", None), getattr(ctx.bref, "main_grad_owner", None), ctx, k + 1) \
+        if want_b else None
+    if hasattr(ctx.wref, "main_grad_owner") and ((want_w and mgw is None) or (want_b and mgb is None)):
+        return None, None
+    return mgw, mgb
 
 
 class _NormFn(torch.autograd.Function):
@@ -61,8 +73,7 @@ class _NormFn(torch.autograd.Function):
         partial = None
         if want_w or want_b:
             partial = _partial_buffer(rows, d, x2.device)
-            mgw = getattr(ctx.wref, "main_grad", None) if want_w else None
-            mgb = getattr(ctx.bref, "main_grad", None) if want_b else None
+            mgw, mgb = _main_grads(ctx, want_w, want_b, 1)
             if mgw is not None or mgb is not None:
                 acc = 1
                 dw_buf, db_buf = mgw, mgb
@@ -133,8 +144,7 @@ class _AddNormFn(torch.autograd.Function):
         acc = 0
         if want_w or want_b:
             partial = _partial_buffer(rows, d, xs.device)
-            mgw = getattr(ctx.wref, "main_grad", None) if want_w else None
-            mgb = getattr(ctx.bref, "main_grad", None) if want_b else None
+            mgw, mgb = _main_grads(ctx, want_w, want_b, 2)
             if mgw is not None or mgb is not None:
                 acc = 1
                 dw_buf, db_buf = mgw, mgb

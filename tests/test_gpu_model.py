@@ -76,3 +76,79 @@ def test_decoder_trains_on_repeated_batch():
     losses = [trainer.step_device(tok).item() for _ in range(8)]
     assert all(v == v for v in losses)
     assert losses[-1] < losses[0] - 0.5, losses
+
+
+def _gpt2_grads(env, hook=False):
+    import distdl_b200
+    from distdl_b200 import models
+    from distdl_b200.parallel import FlatAdamW
+    distdl_b200.config.set_backend("native", "cupy")
+    old = {k: os.environ.get(k) for k in env}
+    os.environ.update(env)
+    try:
+        torch.manual_seed(3)
+        cfg = models.gpt2_xl(d_model=256, n_heads=4, n_kv_heads=4, ffn_dim=512, max_seq=128, vocab_size=1000, n_layers=2)
+        model = models.Decoder(cfg, models.ParallelLayout(1, 1))
+        with torch.no_grad():
+            for n, p in model.named_parameters():
+                if "norm" in n:
+                    p.add_(torch.randn_like(p) * 0.1)
+        seen = []
+        if hook:
+            for n, p in model.named_parameters():
+                if "norm2" in n:
+                    p.register_hook(lambda g, n=n: seen.append((n, g.float().norm().item())))
+        opt = FlatAdamW(model, lr=1e-3)
+        tok = _tokens(cfg)
+        for _ in range(2):
+            model.loss(tok[:, :-1], tok[:, 1:], scale=1.0 / tok[:, 1:].numel()).backward()
+        model.release_gathered()
+        torch.cuda.synchronize()
+        return opt.grad.clone(), opt.names, seen
+    finally:
+        for k, v in old.items():
+            if v is None:
+                os.environ.pop(k, None)
+            else:
+                os.environ[k] = v
+
+
+def test_layer_norms_of_a_decoder_accumulate_directly():
+    """LayerNorm weights and biases: straight into the fp32 accumulators, the same as through autograd (which rounds
+    the gradient of every micro-batch to bf16 first) and as the library path; a hook of the user's still sees them."""
+    a, names, _ = _gpt2_grads({"DISTDL_DIRECT_MAIN_GRAD": "1"})
+    for env in ({"DISTDL_DIRECT_MAIN_GRAD": "0"}, {"DISTDL_FORCE_TORCH": "1"}):
+        b, _, _ = _gpt2_grads(env)
+        for name, o, n in names:
+            x, y = a[o:o + n], b[o:o + n]
+            assert (x - y).abs().max().item() <= 3e-2 * y.abs().max().item() + 1e-7, (env, name)
+    c, _, seen = _gpt2_grads({"DISTDL_DIRECT_MAIN_GRAD": "1"}, hook=True)
+    assert len(seen) == 2 * 2 * 2 and all(v > 0 for _, v in seen)
+    for name, o, n in names:
+        x, y = a[o:o + n], c[o:o + n]
+        assert (x - y).abs().max().item() <= 2e-2 * y.abs().max().item() + 1e-7, name
+
+
+@pytest.mark.parametrize("affine,shape", [(True, (3, 37, 256)), (True, (1, 1, 1600)), (False, (2, 5, 264))])
+def test_layer_norm_layer_takes_a_residual(affine, shape):
+    import distdl_b200
+    from distdl_b200 import backends, nn
+    distdl_b200.config.set_backend("native", "cupy")
+    P = backends.backend.Partition().create_partition_inclusive([0]).create_cartesian_topology_partition([1, 1, 1])
+    torch.manual_seed(4)
+    layer = nn.DistributedLayerNorm(P, shape[-1], elementwise_affine=affine, device="cuda", dtype=torch.bfloat16)
+    if affine:
+        with torch.no_grad():
+            layer.weight.normal_()
+            layer.bias.normal_()
+    x, r = (torch.randn(shape, device="cuda").bfloat16().requires_grad_() for _ in range(2))
+    ds, dy = (torch.randn(shape, device="cuda").bfloat16() for _ in range(2))
+    leaves = [x, r, *layer.parameters()]
+    s, y = layer(x, residual=r)
+    got = torch.autograd.grad([s, y], leaves, [ds, dy])
+    s2 = x + r
+    want = torch.autograd.grad([s2, layer(s2)], leaves, [ds, dy])
+    assert torch.equal(s, s2)
+    for a, b in zip(got, want):
+        # the separate form rounds the two gradients of the sum to bf16 before it adds them
+        assert (a.float() - b.float()).norm() <= 1e-2 * b.float().norm()
