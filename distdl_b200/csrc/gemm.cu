@@ -25,19 +25,20 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int gr
   kern<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, p);
   return (int)cudaGetLastError();
 }
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int NB>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p, int grid,
                 cudaStream_t stream) {
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
-  auto kern = dd::gemm2::gemm2_bf16_kernel<A_MN, B_MN>;
+  auto kern = dd::gemm2::gemm2_bf16_kernel<A_MN, B_MN, NB>;
+  constexpr int bytes = dd::gemm2::Shape<NB>::SMEM;
   if (!configured[dev & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dd::gemm2::SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = true;
   }
-  kern<<<grid, dd::gemm2::NUM_THREADS, dd::gemm2::SMEM_BYTES, stream>>>(ta, tb, td, p);
+  kern<<<grid, dd::gemm2::NUM_THREADS, bytes, stream>>>(ta, tb, td, p);
   return (int)cudaGetLastError();
 }
 
@@ -113,11 +114,23 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
     CUtensorMap pa, pb;
     int rr;
     namespace g2 = dd::gemm2;
+    int ctas = current_sm_count() & ~1;
+    if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas & ~1;
+    if (ctas < 2) ctas = 2;
+    // Columns of a pair's tile: 128 where the waves of half tiles are the shorter time.  A half tile costs 1.25 times as
+    // much per column (its operands and what TMA brings are 192 bytes of shared memory a clock, a whole one's are 128).
+    // Forward, in us, 256 -> 128 columns: 4096 x 1600 x 6400 74.8 -> 69.7, 3000 x 2048 x 5632 67.6 -> 63.5, 512 x 1024 x 512
+    // 14.3 -> 11.2; but 4096 x 6400 x 1600 62.4 -> 71.7, 3000 x 11264 x 2048 98 -> 114.  Gradients that are added in fp32
+    // are bound by their epilogue besides (3000 x 2048 x 5632 70.6 -> 79.9): only where there is one wave either way.
+    const long long rows_of_tiles = (long long)((M + 2 * g2::BM - 1) / (2 * g2::BM)) * batch;
+    const long long whole = rows_of_tiles * ((N + 255) / 256), half = rows_of_tiles * ((N + 127) / 128), pairs = ctas / 2;
+    const bool narrow = rows == nullptr && ((flags & F_OUT_F32) ? half <= pairs
+                                            : (half + pairs - 1) / pairs * 125 < (whole + pairs - 1) / pairs * 200);
     if (a_mn) rr = get_tensor_map_bf16_3d(&pa, A, M, K, batch, lda * 2, strideA * 2, 64, g2::BK);
     else      rr = get_tensor_map_bf16_3d(&pa, A, K, M, batch, lda * 2, strideA * 2, g2::BK, g2::BM);
     if (rr) return rr;
     if (b_mn) rr = get_tensor_map_bf16_3d(&pb, B, N, K, batch, ldb * 2, strideB * 2, 64, g2::BK);
-    else      rr = get_tensor_map_bf16_3d(&pb, B, K, N, batch, ldb * 2, strideB * 2, g2::BK, g2::BNH);
+    else      rr = get_tensor_map_bf16_3d(&pb, B, K, N, batch, ldb * 2, strideB * 2, g2::BK, narrow ? 64 : g2::BNH);
     if (rr) return rr;
     int err2 = 0;
     Params q;
@@ -126,11 +139,8 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
     q.status = device_status(&err2);
     q.rows = rows; q.bound_k = bound_k;
     if (err2) return err2;
-    const int ptiles = ((M + 2 * g2::BM - 1) / (2 * g2::BM)) * ((N + g2::BN - 1) / g2::BN) * batch;
-    int ctas = current_sm_count() & ~1;
-    if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas & ~1;
-    if (ctas < 2) ctas = 2;
-    const int pgrid = 2 * ptiles < ctas ? 2 * ptiles : ctas;
+    const long long ptiles = narrow ? half : whole;
+    const int pgrid = 2 * ptiles < ctas ? (int)(2 * ptiles) : ctas;
     cudaStream_t ps = reinterpret_cast<cudaStream_t>(stream);
     // TMA epilogue where the output qualifies: bf16 store, fp32 store or fp32 add
     static const bool tma_epi = []() { const char* e = getenv("DISTDL_GEMM_TMA_EPI"); return !(e && e[0] == '0'); }();
@@ -145,10 +155,16 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
       if (rr) return rr;
       q.flags |= F_TMA_EPI;
     }
-    if (a_mn && b_mn) return launch_pair<true, true>(pa, pb, pd, q, pgrid, ps);
-    if (a_mn) return launch_pair<true, false>(pa, pb, pd, q, pgrid, ps);
-    if (b_mn) return launch_pair<false, true>(pa, pb, pd, q, pgrid, ps);
-    return launch_pair<false, false>(pa, pb, pd, q, pgrid, ps);
+    if (narrow) {
+      if (a_mn && b_mn) return launch_pair<true, true, 128>(pa, pb, pd, q, pgrid, ps);
+      if (a_mn) return launch_pair<true, false, 128>(pa, pb, pd, q, pgrid, ps);
+      if (b_mn) return launch_pair<false, true, 128>(pa, pb, pd, q, pgrid, ps);
+      return launch_pair<false, false, 128>(pa, pb, pd, q, pgrid, ps);
+    }
+    if (a_mn && b_mn) return launch_pair<true, true, 256>(pa, pb, pd, q, pgrid, ps);
+    if (a_mn) return launch_pair<true, false, 256>(pa, pb, pd, q, pgrid, ps);
+    if (b_mn) return launch_pair<false, true, 256>(pa, pb, pd, q, pgrid, ps);
+    return launch_pair<false, false, 256>(pa, pb, pd, q, pgrid, ps);
   }
   CUtensorMap ta, tb;
   int r;

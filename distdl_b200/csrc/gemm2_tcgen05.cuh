@@ -41,9 +41,21 @@ constexpr int OUT_WARP_BYTES = 2 * 32 * 128;
 constexpr int OUT_STAGE_BYTES = 4 * OUT_WARP_BYTES;          // 32 KB
 constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + OUT_STAGE_BYTES + 256;
 
+// The tile of a pair is 256 rows by NB columns.  256 columns move least through shared memory; 128 leave less of a last
+// wave idle (M = 4096, N = 1600: 112 tiles on 74 pairs are two waves, 208 tiles of half the size three halves).
+template <int NB>
+struct Shape {
+  static constexpr int NBH = NB / 2;                            // B rows staged per CTA
+  static constexpr int B_BYTES = NBH * BK * 2;
+  static constexpr int BYTES = A_STAGE_BYTES + B_BYTES;         // one stage
+  static constexpr int NSTAGES = NB == 256 ? STAGES : 8;
+  static constexpr int COLS = ACC_STAGES * NB;                  // of tensor memory
+  static constexpr int SMEM = 1024 + NSTAGES * BYTES + OUT_STAGE_BYTES + 256;
+};
+
 struct SharedStorage {
-  uint64_t full[STAGES];
-  uint64_t empty[STAGES];
+  uint64_t full[8];
+  uint64_t empty[8];
   uint64_t tmem_full[ACC_STAGES];
   uint64_t tmem_empty[ACC_STAGES];
   uint32_t tmem_base;
@@ -119,6 +131,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
 // the tensor are clipped by the hardware.  `write` = false skips the stores.
 // `add_src[0 .. n_add)`: optional bf16 matrices [rows][add_ld] (local memory) whose rows
 // row0 .. row0 + 31 are added to the tile before it is written (partials of other GPUs).
+template <int NB = BN>
 __device__ __forceinline__ void epilogue_tma(const Params& q, const CUtensorMap* map, uint32_t taddr, uint8_t* stage_w,
                                              int lane, int col_tile0, int row0, int tb, bool write,
                                              const __nv_bfloat16* const* add_src = nullptr, int n_add = 0,
@@ -128,7 +141,7 @@ __device__ __forceinline__ void epilogue_tma(const Params& q, const CUtensorMap*
   const int round_cols = f32 ? 64 : 128;
   const int box_cols = round_cols / 2;
 #pragma unroll 1
-  for (int rd = 0; rd < BN / round_cols; ++rd) {
+  for (int rd = 0; rd < NB / round_cols; ++rd) {
     const int colr = col_tile0 + rd * round_cols;
     if (colr >= q.N) break;
     if (lane == 0) tma_store_wait_read();
@@ -232,10 +245,12 @@ __device__ __forceinline__ int k_blocks(const Params& p, int tm, int tb) {
   return (k + BK - 1) / BK;
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int NB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ CUtensorMap tmap_d, const Params p) {
+  using T = Shape<NB>;
+  constexpr int STAGES = T::NSTAGES, STAGE_BYTES = T::BYTES, BN = NB, BNH = T::NBH, TMEM_COLS = T::COLS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* out_stage = tiles + STAGES * STAGE_BYTES;
@@ -365,7 +380,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const long long row_off = (long long)tb * p.strideD + (long long)row * p.ldd;
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
       if (p.flags & gemm::F_TMA_EPI) {
-        epilogue_tma(p, &tmap_d, taddr, out_stage + quarter * OUT_WARP_BYTES, lane, tn * BN,
+        epilogue_tma<NB>(p, &tmap_d, taddr, out_stage + quarter * OUT_WARP_BYTES, lane, tn * BN,
                      tm * 2 * BM + (int)rank * BM + quarter * 32, tb, true, nullptr, 0, 0, zero);
       } else {
 #pragma unroll 1
