@@ -1,6 +1,6 @@
 // bf16 GEMM on CTA pairs: tcgen05.mma.cta_group::2.
 //
-// Two CTAs of a cluster (two neighbouring SMs) share one 256x256 output tile:
+// Two CTAs of a cluster (two neighbouring SMs) share one 256x256 output tile (or 256x128, see Shape):
 // CTA r owns rows [128 r, 128 r + 128) of the tile (its TMEM holds that half of
 // the accumulator) and stages, per 64-deep k-block, its own 128x64 slice of A
 // and HALF of the 256x64 slice of B (rows [128 r, 128 r + 128) of B).  The
