@@ -29,6 +29,7 @@ import torch.utils.checkpoint
 
 from .. import nn as dnn
 from .. import ops
+from ..nn.module import hooked
 from ..utilities import recompute
 from ..utilities.slicing import compute_start_index, compute_subshape
 
@@ -299,9 +300,15 @@ class Block(torch.nn.Module):
                 fn()
 
 
+_layer_norm_forward = dnn.DistributedLayerNorm.forward
+
+
 def _add_norm(norm, x, delta):
-    """``(x + delta, norm(x + delta))``, fused where the norm layer can take a residual."""
-    if hasattr(norm, "_gathered") or isinstance(norm, dnn.DistributedLayerNorm):
+    """``(x + delta, norm(x + delta))``, fused where the norm layer can take a residual: a ``DistributedLayerNorm`` only
+    where a call of it is its own ``forward``, because hooks and a ``forward`` of the user's expect the sum and return
+    the norm alone."""
+    if hasattr(norm, "_gathered") or (getattr(norm.forward, "__func__", None) is _layer_norm_forward
+                                      and not hooked(norm)):
         return norm(x, residual=delta)
     s = x + delta
     return s, norm(s)

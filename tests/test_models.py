@@ -483,3 +483,58 @@ def test_blocks_that_keep_their_activations_train_like_blocks_that_recompute():
     run_ranks("test_models", "body_activation_policies", 4, args=("llama", 2), timeout=300)
     run_ranks("test_models", "body_activation_policies", 4, args=("gpt2", 2), timeout=300)
     run_ranks("test_models", "body_activation_policies", 2, args=("llama", 1), timeout=300)
+
+
+def body_hooked_layer_norms(rank, world):
+    """Hooks and subclasses of a block's LayerNorm meet the sum of stream and branch and return the norm alone."""
+    from distdl_b200 import models, nn
+    cfg = models.gpt2_tiny(dtype=torch.float32, max_seq=32, vocab_size=100, d_model=48, ffn_dim=96, eps=0.0)
+    model = models.Decoder(cfg, models.ParallelLayout(1, 1))
+    torch.manual_seed(1)
+    with torch.no_grad():
+        for p in model.parameters():
+            p.normal_(0.0, 0.3)
+    tokens = torch.randint(0, 100, (2, 32))
+    norm1, norm2 = model.blocks[1].norm1, model.blocks[0].norm2
+
+    def hidden():
+        with torch.no_grad():
+            return model(tokens)
+    want = hidden()
+    seen = []
+    handles = [n.register_forward_hook(lambda m, a, o: seen.append((m, a, o))) for n in (norm1, norm2)]
+    assert torch.equal(hidden(), want)
+    for h in handles:
+        h.remove()
+    assert len(seen) == 2
+    for m, a, o in seen:
+        assert len(a) == 1 and torch.is_tensor(o)
+        assert torch.equal(o, torch.nn.functional.layer_norm(a[0], (48,), m.weight.view(-1), m.bias.view(-1), 0.0))
+    # a norm does not see the scale of its input (a power of two, no eps: hardly a rounding), the stream none of the hook
+    for n in (norm1, norm2):
+        h = n.register_forward_pre_hook(lambda m, a: (a[0] * 4.0,))
+        assert torch.allclose(hidden(), want, rtol=1e-4, atol=1e-4)
+        h.remove()
+    # twice the output is twice the parameters
+    h = norm2.register_forward_hook(lambda m, a, o: o * 2.0)
+    doubled = hidden()
+    h.remove()
+    with torch.no_grad():
+        norm2.weight.mul_(2.0), norm2.bias.mul_(2.0)
+    assert torch.allclose(hidden(), doubled, rtol=1e-5, atol=1e-5) and not torch.allclose(doubled, want, rtol=1e-2, atol=1e-2)
+    with torch.no_grad():
+        norm2.weight.mul_(0.5), norm2.bias.mul_(0.5)
+
+    class Own(nn.DistributedLayerNorm):
+        def forward(self, input):
+            return super().forward(input)
+    norm2.__class__ = Own
+    assert torch.equal(hidden(), want)
+    norm2.__class__ = nn.DistributedLayerNorm
+    norm1.forward = lambda input: nn.DistributedLayerNorm.forward(norm1, input)
+    assert torch.equal(hidden(), want)
+    return True
+
+
+def test_hooked_layer_norms_of_a_decoder():
+    run_ranks("test_models", "body_hooked_layer_norms", 1)
