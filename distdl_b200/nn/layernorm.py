@@ -116,7 +116,10 @@ class DistributedLayerNorm(Module):
         """With ``residual``: returns ``(input + residual, norm(input + residual))``, the add fused into the norm kernel
         where the rows are whole on this worker."""
         if not self.P_x.active:
-            return input if residual is None else (input, input)
+            if residual is None:
+                return input
+            input = input + residual            # (without values, but both branches take part in the backward pass)
+            return input, input
         w = b = None
         if self.elementwise_affine:
             if self.weight_buffer is None:

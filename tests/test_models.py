@@ -538,3 +538,21 @@ def body_hooked_layer_norms(rank, world):
 
 def test_hooked_layer_norms_of_a_decoder():
     run_ranks("test_models", "body_hooked_layer_norms", 1)
+
+
+def body_residual_outside_the_partition(rank, world):
+    """A worker without a share of the rows still has both branches in its graph: collectives may hang on either."""
+    from distdl_b200 import backends, nn
+    P_world = backends.backend.Partition()
+    P_x = P_world.create_partition_inclusive([0]).create_cartesian_topology_partition([1, 1, 1])
+    layer = nn.DistributedLayerNorm(P_x, 8)
+    shape = (2, 3, 8) if rank == 0 else (0,)
+    x, delta = (torch.ones(shape, requires_grad=True) for _ in range(2))
+    s, y = layer(x, residual=delta)
+    assert s.shape == y.shape == shape
+    gx, gd = torch.autograd.grad((s.sum() + y.sum()), [x, delta])
+    assert gx.shape == gd.shape == shape and torch.equal(gx, gd)
+
+
+def test_residual_outside_the_partition():
+    run_ranks("test_models", "body_residual_outside_the_partition", 2)
