@@ -33,8 +33,11 @@ def _main_grads(ctx, want_w, want_b, k):
         if want_w else None
     mgb = main_grad_now(getattr(ctx.bref, "main_grad", None), getattr(ctx.bref, "main_grad_owner", None), ctx, k + 1) \
         if want_b else None
-    if hasattr(ctx.wref, "main_grad_owner") and ((want_w and mgw is None) or (want_b and mgb is None)):
-        return None, None
+    if (want_w and mgw is None) or (want_b and mgb is None):
+        # (one of the two leaves has hooks, or none of the optimizer's accumulators: it was frozen when that was built)
+        if all(getattr(t, "main_grad_owner", None) is not None
+               for t, acc in ((ctx.wref, mgw), (ctx.bref, mgb)) if acc is not None):
+            return None, None
     return mgw, mgb
 
 

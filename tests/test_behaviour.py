@@ -185,3 +185,42 @@ def test_kernels_refuse_tensors_without_an_address():
             assert lib.dd_interpolate(1, 1, adjoint, 0, 1, x, y, 2, one, one, zero, zero, one, one, scale, 0, None) == bad
     for args in ((None, some, some), (some, None, some), (some, some, None)):
         assert lib.dd_colsum(args[0], 8, 8, args[1], args[2], 0, None) == bad
+
+
+def test_norm_gradients_accumulate_for_both_parameters_or_neither():
+    """Weight and bias go into the optimizer's accumulators where both have one and nobody hooks them; otherwise both go
+    through autograd.  Gathered parameters (no owner) keep their accumulators."""
+    import types
+
+    from distdl_b200.ops.norm import _main_grads
+    got = []
+
+    class Probe(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x, w, b):
+            ctx.wref, ctx.bref = w, b
+            return x * 1.0
+
+        @staticmethod
+        def backward(ctx, dy):
+            got.append(_main_grads(ctx, True, True, 1))
+            return dy, torch.zeros(4), torch.zeros(4)
+
+    def ask(with_w, with_b, hook=None):
+        leaves = [torch.nn.Parameter(torch.ones(1, 4)) for _ in range(2)]
+        views = [p.view(4) for p in leaves]
+        for v, p, with_acc in zip(views, leaves, (with_w, with_b)):
+            if with_acc:
+                v.main_grad, v.main_grad_owner = torch.zeros(4), p
+        if hook is not None:
+            leaves[hook].register_hook(lambda g: None)
+        Probe.apply(torch.ones(4, requires_grad=True), *views).sum().backward()
+        return [None if a is None else a is v.main_grad for a, v in zip(got.pop(), views)]
+    assert ask(True, True) == [True, True]
+    for with_w, with_b in ((False, False), (True, False), (False, True)):
+        assert ask(with_w, with_b) == [None, None], (with_w, with_b)
+    assert ask(True, True, hook=0) == ask(True, True, hook=1) == [None, None]
+    w, b = torch.ones(4), torch.ones(4)
+    w.main_grad, b.main_grad = torch.zeros(4), torch.zeros(4)
+    ctx = types.SimpleNamespace(wref=w, bref=b)
+    assert _main_grads(ctx, True, True, 1) == (w.main_grad, b.main_grad)
