@@ -452,6 +452,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           if (j > 0) {
             ok = wait_turn(p.dq_turn + tile, j, p.ticket + 1, &bar->abort_flag, p.status);
             if (!ok) { bar->abort_flag = 1; break; }
+            fence_proxy_async();           // the sums it now adds to were written by another CTA's bulk copies
           }
           for (int ch = 0; ch < CHUNKS; ++ch) {
             ok = mbar_wait(&bar->chunk_full[it & 1][ch & 1], (phase + (ch >> 1)) & 1, &bar->abort_flag, p.status, 146);
@@ -576,6 +577,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     if (part > 0) {
       if (ok && lane == 0) ok = wait_turn(p.kv_turn + kv_tile, part, p.ticket + 1, &bar->abort_flag, p.status);
       ok = __all_sync(0xffffffffu, ok);
+      __syncwarp();             // orders the other lanes' accesses after lane 0's acquire, as the vote does not
       if (!ok) bar->abort_flag = 1;
     }
     if (ok) {
@@ -639,6 +641,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (lane == 0) ok = wait_turn(p.dq_turn + tile, j, p.ticket + 1, &bar->abort_flag, p.status);
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) { bar->abort_flag = 1; break; }
+        __syncwarp();           // orders the other lanes' reads after lane 0's acquire, as the shuffle does not
         fence_proxy_async();
       }
       if (i * BT + row < p.S) {

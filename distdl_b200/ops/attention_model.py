@@ -1,5 +1,6 @@
-"""A host model of the pipelines inside the attention kernels (``csrc/attention_bwd2_impl.cuh`` and the
-two-tile forward kernel ``csrc/attention_fwd2_impl.cuh``), for tests without a GPU.
+"""A host model of the pipelines inside the attention kernels (``csrc/attention_bwd2_impl.cuh``,
+``csrc/attention_bwd3_impl.cuh`` and the two-tile forward kernel ``csrc/attention_fwd2_impl.cuh``), for tests
+without a GPU.
 
 The kernels are warp-specialised: one thread issues TMA loads, one thread issues tensor-core products
 (which execute in issue order and signal completion through ``tcgen05.commit``), sixteen warps do the
@@ -88,6 +89,24 @@ class TensorPipe:
     def close(self):
         self._q.put(None)
         self._t.join()
+
+
+class Turn:
+    """A counter in global memory that CTAs hand on: ``wait(n)`` returns once it says ``n``."""
+
+    def __init__(self, name: str):
+        self.value, self.name = 0, name
+        self._cv = threading.Condition()
+
+    def wait(self, want: int):
+        with self._cv:
+            if not self._cv.wait_for(lambda: self.value == want, WAIT_LIMIT_S):
+                raise PipelineStuck(f"wait on {self.name} (turn {want}, at {self.value}) ran out")
+
+    def pass_on(self, value: int):
+        with self._cv:
+            self.value = value
+            self._cv.notify_all()
 
 
 def _jitter(rng):
@@ -446,3 +465,221 @@ def fwd_pair(Q, K, V, n, scale, diag=(None, None), row_warps=4, seed=0, grow_thr
     finally:
         pipe.close()
     return out, lse
+
+
+def one_pass(Q, dO, K, V, lse2, delta, scale, causal, roomy, split=1, resident=2, softmax_warps=2, drain_warps=2,
+             chunks=2, seed=0, wait_turns=True):
+    """The one-pass backward kernel for ONE kv head: ``Q``, ``dO`` are lists (query heads of the group) of lists
+    (query tiles) of ``[BT, D]`` arrays, ``lse2`` / ``delta`` the same of ``[BT]``, ``K`` / ``V`` lists with one
+    ``[BT, D]`` array per key tile.  One CTA per key tile and part of the group (``split`` parts), at most
+    ``resident`` of them at a time, started in the order of their tickets.  ``roomy``: the stages and the issue order
+    of head dim 64 (P and dQ have columns of their own), else those of 128 (P over S, dQ over dP).  What an
+    asynchronous bulk copy reads from shared memory it reads at the last moment that the kernel's waits allow.
+    ``wait_turns=False`` leaves out the order in which the parts of dQ are added.  Returns ``(dQ, dK, dV)`` in the
+    layout of the inputs."""
+    nT, (BT, D), heads_all = len(K), K[0].shape, len(Q)
+    W, heads = softmax_warps, heads_all // split
+    cols, width = BT // W, D // chunks
+    c = scale * 1.4426950408889634
+    QS, OS, DSB = (3, 2, 2) if roomy else (2, 1, 1)
+    nan = float("nan")
+    dQ = [[np.full((BT, D), nan) for _ in range(nT)] for _ in range(heads_all)]
+    dK, dV = ([np.full((BT, D), nan) for _ in range(nT)] for _ in range(2))
+    dq_sum = [[np.full((BT, D), nan) for _ in range(nT)] for _ in range(heads_all)]
+    dq_turn = [[Turn(f"dq_turn[{h}][{i}]") for i in range(nT)] for h in range(heads_all)]
+    kv_sum = [np.full((2, BT, D), nan) for _ in range(nT)]
+    kv_turn = [Turn(f"kv_turn[{j}]") for j in range(nT)]
+
+    def cta(place):
+        part, j = place % split, place // split
+        h0 = part * heads
+        per_head = nT - j if causal else nT
+        iters = heads * per_head
+
+        def tile_of(it):
+            return h0 + it // per_head, nT - 1 - it % per_head
+        bar = {n: MBarrier(1, n) for n in ("kv_full", "s_full", "dp_full", "dq_full", "acc_done")}
+        for n, count in (("q_full", QS), ("q_empty", QS), ("do_full", OS), ("do_empty", OS), ("chunk_empty", 2)):
+            bar[n] = [MBarrier(1, f"{n}[{s}]") for s in range(count)]
+        for n in ("s_read", "p_full", "ds_full"):
+            bar[n] = MBarrier(W, n)
+        bar["dq_empty"] = MBarrier(drain_warps, "dq_empty")
+        bar["chunk_full"] = [[MBarrier(drain_warps, f"chunk_full[{a}][{s}]") for s in range(2)] for a in range(2)]
+        joined = threading.Barrier(W)
+        smem = {"Q": [None] * QS, "stats": [None] * QS, "dO": [None] * OS,
+                "dS": [np.zeros((BT, BT)) for _ in range(DSB)], "chunk": [np.zeros((BT, width)) for _ in range(2)]}
+        tmem = {n: np.zeros((BT, BT)) for n in ("S", "dP")}
+        tmem["dV"], tmem["dK"] = np.zeros((BT, D)), np.zeros((BT, D))
+        tmem["P"] = np.zeros((BT, BT)) if roomy else tmem["S"]
+        tmem["dQ"] = np.zeros((BT, D)) if roomy else tmem["dP"][:, :D]       # (views: writing one is writing the other)
+        pipe = TensorPipe(random.Random(seed + 100 * place))
+
+        def tma():
+            rng = random.Random(seed + 100 * place + 1)
+            smem["K"], smem["V"] = K[j].copy(), V[j].copy()
+            bar["kv_full"].arrive()
+            for it in range(iters):
+                h, i = tile_of(it)
+                st, ot = it % QS, it % OS
+                bar["q_empty"][st].wait(((it // QS) & 1) ^ 1)
+                _jitter(rng)
+                smem["Q"][st], smem["stats"][st] = Q[h][i].copy(), (lse2[h][i].copy(), delta[h][i].copy())
+                bar["q_full"][st].arrive()
+                bar["do_empty"][ot].wait(((it // OS) & 1) ^ 1)
+                _jitter(rng)
+                smem["dO"][ot] = dO[h][i].copy()
+                bar["do_full"][ot].arrive()
+
+        def mma():
+            def put(name, fn, first=True):
+                def run():
+                    prod = fn()
+                    tmem[name][:] = prod if first else tmem[name] + prod
+                pipe.issue(run)
+
+            def s_of(it):
+                st = it % QS
+                bar["q_full"][st].wait((it // QS) & 1)
+                put("S", lambda: smem["K"] @ smem["Q"][st].T)
+                pipe.commit(bar["s_full"])
+
+            def dp_of(it):
+                ot = it % OS
+                bar["do_full"][ot].wait((it // OS) & 1)
+                put("dP", lambda: smem["V"] @ smem["dO"][ot].T)
+                pipe.commit(bar["dp_full"])
+            bar["kv_full"].wait(0)
+            s_of(0)
+            dp_of(0)
+            for it in range(iters):
+                st, ot, ds, more = it % QS, it % OS, it % DSB, it + 1 < iters
+                if roomy and more:
+                    bar["s_read"].wait(it & 1)
+                    s_of(it + 1)
+                bar["p_full"].wait(it & 1)
+                put("dV", lambda ot=ot: tmem["P"] @ smem["dO"][ot], it == 0)
+                pipe.commit(bar["do_empty"][ot])
+                if not roomy and more:
+                    s_of(it + 1)
+                bar["ds_full"].wait(it & 1)
+                if roomy:
+                    if more:
+                        dp_of(it + 1)
+                    if it > 0:
+                        bar["dq_empty"].wait((it - 1) & 1)
+                put("dQ", lambda ds=ds: smem["dS"][ds].T @ smem["K"])
+                pipe.commit(bar["dq_full"])
+                put("dK", lambda ds=ds, st=st: smem["dS"][ds] @ smem["Q"][st], it == 0)
+                pipe.commit(bar["q_empty"][st])
+                if not roomy and more:
+                    bar["dq_empty"].wait(it & 1)
+                    dp_of(it + 1)
+            pipe.commit(bar["acc_done"])
+
+        def adder(a):
+            def run():
+                rng = random.Random(seed + 100 * place + 30 + a)
+                phase = 0
+                for it in range(a, iters, 2):
+                    h, i = tile_of(it)
+                    if i == j if causal else j == nT - 1:
+                        continue
+                    if j > 0 and wait_turns:
+                        dq_turn[h][i].wait(j)
+
+                    def bulk(ch):
+                        _jitter(rng)
+                        at = dq_sum[h][i][:, ch * width:(ch + 1) * width]
+                        at[:] = at + smem["chunk"][ch & 1] if j > 0 else smem["chunk"][ch & 1]
+                    for ch in range(chunks):
+                        bar["chunk_full"][a][ch & 1].wait((phase + (ch >> 1)) & 1)
+                        if ch > 0:
+                            bulk(ch - 1)
+                            bar["chunk_empty"][(ch - 1) & 1].arrive()
+                    phase += chunks // 2
+                    bulk(chunks - 1)
+                    bar["chunk_empty"][(chunks - 1) & 1].arrive()
+                    dq_turn[h][i].pass_on(j + 1)
+            return run
+
+        def softmax(w):
+            def run():
+                rng = random.Random(seed + 100 * place + 10 + w)
+                mine = slice(w * cols, (w + 1) * cols)                  # this warp's query columns
+                later = np.arange(w * cols, (w + 1) * cols)[None, :] < np.arange(BT)[:, None]
+                for it in range(iters):
+                    st = it % QS
+                    bar["q_full"][st].wait((it // QS) & 1)
+                    bar["s_full"].wait(it & 1)
+                    _jitter(rng)
+                    s = tmem["S"][:, mine].copy()
+                    if roomy:
+                        bar["s_read"].arrive()
+                    p = np.exp2(s * c - smem["stats"][st][0][None, mine])
+                    if causal and it % per_head == per_head - 1:
+                        p = np.where(later, 0.0, p)
+                    if roomy and it > 0:
+                        bar["do_empty"][(it - 1) % OS].wait(((it - 1) // OS) & 1)
+                    _jitter(rng)
+                    tmem["P"][:, mine] = p
+                    bar["p_full"].arrive()
+                    bar["dp_full"].wait(it & 1)
+                    _jitter(rng)
+                    smem["dS"][it % DSB][:, mine] = p * (tmem["dP"][:, mine] - smem["stats"][st][1][None, mine])
+                    bar["ds_full"].arrive()
+                bar["acc_done"].wait(0)
+                if part > 0:
+                    kv_turn[j].wait(part)
+                rows = slice(w * cols, (w + 1) * cols)
+                for n, (name, out, mul) in enumerate((("dV", dV, 1.0), ("dK", dK, scale))):
+                    got = tmem[name][rows] if part == 0 else kv_sum[j][n][rows] + tmem[name][rows]
+                    if part == split - 1:
+                        out[j][rows] = got * mul
+                    else:
+                        kv_sum[j][n][rows] = got
+                if joined.wait(WAIT_LIMIT_S) == 0 and part < split - 1:
+                    kv_turn[j].pass_on(part + 1)
+            return run
+
+        def drain(w):
+            def run():
+                rng = random.Random(seed + 100 * place + 20 + w)
+                per = BT // drain_warps
+                rows = slice(w * per, (w + 1) * per)
+                chunk = 0
+                for it in range(iters):
+                    h, i = tile_of(it)
+                    bar["dq_full"].wait(it & 1)
+                    _jitter(rng)
+                    r = tmem["dQ"][rows].copy()
+                    bar["dq_empty"].arrive()
+                    if not (i == j if causal else j == nT - 1):
+                        for ch in range(chunks):
+                            bar["chunk_empty"][ch & 1].wait(((chunk >> 1) & 1) ^ 1)
+                            smem["chunk"][ch & 1][rows] = r[:, ch * width:(ch + 1) * width]
+                            bar["chunk_full"][it & 1][ch & 1].arrive()
+                            chunk += 1
+                        continue
+                    if j > 0:
+                        dq_turn[h][i].wait(j)
+                        r = dq_sum[h][i][rows] + r
+                    dQ[h][i][rows] = r * scale
+            return run
+        try:
+            _run_roles([tma, mma, adder(0), adder(1)] + [softmax(w) for w in range(W)]
+                       + [drain(w) for w in range(drain_warps)])
+        finally:
+            pipe.close()
+
+    ticket = iter(range(nT * split))
+    lock = threading.Lock()
+
+    def slot():
+        while True:
+            with lock:
+                place = next(ticket, None)
+            if place is None:
+                return
+            cta(place)
+    _run_roles([slot] * resident)
+    return dQ, dK, dV

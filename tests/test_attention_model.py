@@ -1,5 +1,6 @@
 """The schedules of the attention backward kernels, run as a host model (one thread per role, the same
-barriers, parities and issue order as ``csrc/attention_bwd2_impl.cuh``, random delays in every role):
+barriers, parities and issue order as ``csrc/attention_bwd2_impl.cuh`` and ``csrc/attention_bwd3_impl.cuh``,
+random delays in every role):
 every sweep length must terminate and give the directly computed gradients."""
 import numpy as np
 import pytest
@@ -137,3 +138,58 @@ def test_forward_pair_schedule_terminates_and_matches(qp, causal):
     # have written their probabilities, so nobody can run ahead of it
     o, lse = model.fwd_pair(Q, K, V, n, SCALE, diag=diag, grow_threshold=2.0, slow_warp=(1, 2))
     assert np.allclose(o, want_o, rtol=1e-9, atol=1e-9) and np.allclose(lse, want_l, rtol=1e-9, atol=1e-9)
+
+
+def _one_pass_case(nT, heads, causal, seed):
+    """Inputs of the one-pass kernel for one kv head and its gradients, computed directly."""
+    rng = np.random.default_rng(200 + seed)
+    D2 = 4
+    Q, dO = ([[rng.standard_normal((BT, D2)) for _ in range(nT)] for _ in range(heads)] for _ in range(2))
+    K, V = ([rng.standard_normal((BT, D2)) for _ in range(nT)] for _ in range(2))
+    l2, dl = ([[rng.standard_normal(BT) + add for _ in range(nT)] for _ in range(heads)] for add in (2.0, 0.0))
+    dQ = [[np.zeros((BT, D2)) for _ in range(nT)] for _ in range(heads)]
+    dK, dV = ([np.zeros((BT, D2)) for _ in range(nT)] for _ in range(2))
+    for h in range(heads):
+        for i in range(nT):
+            for j in range(i + 1 if causal else nT):
+                p = _p(Q[h][i], K[j], l2[h][i], UPPER if causal and i == j else None)
+                ds = p * (dO[h][i] @ V[j].T - dl[h][i][:, None]) * SCALE
+                dQ[h][i] += ds @ K[j]
+                dK[j] += ds.T @ Q[h][i]
+                dV[j] += p.T @ dO[h][i]
+    return (Q, dO, K, V, l2, dl, SCALE, causal), (dQ, dK, dV)
+
+
+def _agree(got, want):
+    return all(np.allclose(a, b, rtol=1e-9, atol=1e-9) for g, w in zip(got, want) for a, b in zip(g, w))
+
+
+@pytest.mark.parametrize("roomy", [True, False])
+@pytest.mark.parametrize("nT,heads,split,causal,resident", [
+    (1, 1, 1, True, 1), (1, 3, 3, False, 2), (2, 1, 1, True, 2), (3, 1, 1, False, 3), (5, 1, 1, True, 2),
+    (4, 2, 1, True, 4), (3, 4, 4, True, 3), (3, 4, 2, False, 6)])
+def test_one_pass_schedule_terminates_and_matches(nT, heads, split, causal, resident, roomy):
+    """Key tiles that start together or one after the other, heads of a group in one CTA or spread over several: every
+    wait ends, and no sum of dQ, dK or dV is read before it is complete or added out of turn."""
+    args, want = _one_pass_case(nT, heads, causal, nT)
+    for seed in range(2):
+        got = model.one_pass(*args, roomy, split=split, resident=resident, seed=seed)
+        assert _agree([sum(got[0], []), *got[1:]], [sum(want[0], []), *want[1:]]), seed
+
+
+def test_one_pass_without_turns_is_caught():
+    """The first key tile stores where the others add: without the order of the turns the sums are wrong, or whoever
+    waits for a number of parts never sees it."""
+    args, want = _one_pass_case(4, 1, False, 9)
+    old_limit, model.WAIT_LIMIT_S = model.WAIT_LIMIT_S, 0.5
+    try:
+        wrong = 0
+        for seed in range(4):
+            try:
+                got = model.one_pass(*args, True, resident=4, seed=seed, wait_turns=False)
+                wrong += not _agree([sum(got[0], []), *got[1:]], [sum(want[0], []), *want[1:]])
+            except (model.PipelineStuck, RuntimeError):
+                wrong += 1
+        assert wrong
+    finally:
+        model.WAIT_LIMIT_S = old_limit
