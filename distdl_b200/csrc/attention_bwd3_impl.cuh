@@ -106,6 +106,7 @@ __device__ __forceinline__ uint4 pack8(const uint32_t* r, float mul, float4 a, f
 __device__ __forceinline__ void put_cols32(uint32_t taddr, __nv_bfloat16* dst, float* sum, int ch, float mul, bool first,
                                            bool last, bool live) {
   uint32_t r[32];
+  __syncwarp();             // (after the stores of the rows that exist: the read is one of the whole warp)
   tmem_ld_32x32(taddr + ch, r);
   tmem_ld_wait();
 #pragma unroll
@@ -522,9 +523,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         for (int k = 0; k < COLS; ++k)
           if (cg * COLS + k < row) pr[k] = 0.f;
       }
-      if (!live) {
+      if (j * BT + BT > p.S) {
+        if (!live) {
 #pragma unroll
-        for (int k = 0; k < COLS; ++k) pr[k] = 0.f;
+          for (int k = 0; k < COLS; ++k) pr[k] = 0.f;
+        }
+        __syncwarp();             // (what follows is of the whole warp)
       }
       if (ROOMY && it > 0) {     // dV of the iteration before has read P
         ok = mbar_wait(&bar->do_empty[(it - 1) % DO_STAGES], ((it - 1) / DO_STAGES) & 1, &bar->abort_flag, p.status, 149);
@@ -657,6 +661,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           *reinterpret_cast<uint4*>(dq + 8 * g) = pack8(r + 8 * g, p.scale, a, e);
         }
       }
+      __syncwarp();               // (the next tile is read by the whole warp)
     }
   }
   tc_fence_before();

@@ -288,17 +288,19 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           uint32_t r[32];
           tmem_ld_32x32(tO + ch * 32, r);
           tmem_ld_wait();
-          if (q_row >= p.S) continue;
           uint4* dst = reinterpret_cast<uint4*>(orow + ch * 32);
+          if (q_row < p.S) {
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint4 v;
-            v.x = pack_bf16x2(__uint_as_float(r[8 * g]) * inv, __uint_as_float(r[8 * g + 1]) * inv);
-            v.y = pack_bf16x2(__uint_as_float(r[8 * g + 2]) * inv, __uint_as_float(r[8 * g + 3]) * inv);
-            v.z = pack_bf16x2(__uint_as_float(r[8 * g + 4]) * inv, __uint_as_float(r[8 * g + 5]) * inv);
-            v.w = pack_bf16x2(__uint_as_float(r[8 * g + 6]) * inv, __uint_as_float(r[8 * g + 7]) * inv);
-            dst[g] = v;
+            for (int g = 0; g < 4; ++g) {
+              uint4 v;
+              v.x = pack_bf16x2(__uint_as_float(r[8 * g]) * inv, __uint_as_float(r[8 * g + 1]) * inv);
+              v.y = pack_bf16x2(__uint_as_float(r[8 * g + 2]) * inv, __uint_as_float(r[8 * g + 3]) * inv);
+              v.z = pack_bf16x2(__uint_as_float(r[8 * g + 4]) * inv, __uint_as_float(r[8 * g + 5]) * inv);
+              v.w = pack_bf16x2(__uint_as_float(r[8 * g + 6]) * inv, __uint_as_float(r[8 * g + 7]) * inv);
+              dst[g] = v;
+            }
           }
+          __syncwarp();         // the lanes of rows behind the sequence take part in the next (aligned) read
         }
         if (p.lse != nullptr && q_row < p.S)
           p.lse[((size_t)b * p.Hq + h) * p.S + q_row] = m_ref * p.scale + logf(l);
