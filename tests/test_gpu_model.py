@@ -152,3 +152,27 @@ def test_layer_norm_layer_takes_a_residual(affine, shape):
     for a, b in zip(got, want):
         # the separate form rounds the two gradients of the sum to bf16 before it adds them
         assert (a.float() - b.float()).norm() <= 1e-2 * b.float().norm()
+
+
+@pytest.mark.parametrize("late", ["weight", "bias"])
+def test_norm_parameter_unfrozen_after_the_optimizer_was_built(late):
+    """The one without an accumulator gets its gradient from autograd, the other reaches the optimizer all the same."""
+    import distdl_b200
+    from distdl_b200 import backends, nn
+    from distdl_b200.parallel import FlatAdamW
+    distdl_b200.config.set_backend("native", "cupy")
+    P = backends.backend.Partition().create_partition_inclusive([0]).create_cartesian_topology_partition([1, 1, 1])
+    torch.manual_seed(6)
+    layer = nn.DistributedLayerNorm(P, 256, device="cuda", dtype=torch.bfloat16)
+    getattr(layer, late).requires_grad_(False)
+    opt = FlatAdamW(layer, lr=1e-3)
+    getattr(layer, late).requires_grad_(True)
+    x, dy = (torch.randn(2, 37, 256, device="cuda").bfloat16() for _ in range(2))
+    layer(x).backward(dy)
+    xh = torch.nn.functional.layer_norm(x.double(), (256,), eps=layer.eps)
+    want = {"weight": (xh * dy.double()).sum((0, 1)), "bias": dy.double().sum((0, 1))}
+    got = getattr(layer, late).grad.double().view(-1)
+    other = "bias" if late == "weight" else "weight"
+    # fp32 sums, then rounded to bf16 (2**-9 of a value at most)
+    assert (got - want[late]).norm() <= 4e-3 * want[late].norm()
+    assert (opt.grad[:256].double() - want[other]).norm() <= 4e-3 * want[other].norm()
