@@ -55,7 +55,10 @@ struct Params2 {
   StatusRecord* status;
 };
 
-template <bool POLY>
+// PAIRS: the sequence is whole pairs of tiles, so that nothing is masked but the diagonal.  The softmax threads are short of
+// registers; the general form spills a third more (head dim 64, causal, 32 / 8 heads, us, one form for all lengths -> PAIRS:
+// 8 x 1024 100.4 -> 94.3, 1 x 1024 22.5 -> 20.5, 1 x 16384 1 733 -> 1 644).
+template <bool POLY, bool PAIRS>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                  const __grid_constant__ CUtensorMap tmap_v, const Params2 p) {
@@ -77,8 +80,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   const int h = hb % p.Hq, b = hb / p.Hq;
   const int hkv = h / (p.Hq / p.Hkv);
   const int n0 = p.causal ? 2 * qp + 1 : nkv;      // blocks seen by tile 0
-  const int n1 = 2 * qp + 1 >= nkv ? 0 : p.causal ? 2 * qp + 2 : nkv;      // blocks seen by tile 1 (>= n0, or none)
-  const int blocks = n1 > n0 ? n1 : n0;
+  const int n1 = !PAIRS && 2 * qp + 1 >= nkv ? 0 : p.causal ? 2 * qp + 2 : nkv;      // blocks seen by tile 1 (>= n0, or none)
+  const int blocks = PAIRS || n1 > n0 ? n1 : n0;
   const int q_row0 = qp * 2 * BQ;                  // of this sequence
 
   if (threadIdx.x == 0) {
@@ -165,7 +168,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       if (ok) {
         tc_fence_after();
         issue_S(0, 0);
-        if (n1 > 0) issue_S(1, 0);
+        if (PAIRS || n1 > 0) issue_S(1, 0);
       }
       for (int j = 0; j < blocks && ok; ++j) {
         const int st = j % KV_STAGES;
@@ -208,8 +211,6 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const uint32_t tS = tmem_base + t * 128 + lane_off;
     const uint32_t tO = tmem_base + 256 + t * 128 + lane_off;
     const int nt = t == 0 ? n0 : n1;
-    const int diag = p.causal ? 2 * qp + t : -1;
-    const int tail = p.S % BKV ? nkv - 1 : -1;      // block with keys behind the end of the sequence
     const float c = p.scale * 1.4426950408889634f;  // scores are exponentiated base 2
     float m_ref = -INFINITY, l = 0.f;
     bool ok = true;
@@ -224,8 +225,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       tmem_ld_32x32(tS + 96, *reinterpret_cast<uint32_t(*)[32]>(s + 96));
       tmem_ld_wait();
       float mx = m_ref;
-      if (j == diag || j == tail) {
-        const int seen = min(j == diag ? row : BKV - 1, p.S - 1 - j * BKV);     // last key of this block that counts
+      const bool diag = p.causal && j == 2 * qp + t;
+      if (diag || (!PAIRS && (j + 1) * BKV > p.S)) {
+        // last key of this block that counts: up to the query itself, none behind the end of the sequence
+        const int seen = PAIRS ? row : min(diag ? row : BKV - 1, p.S - 1 - j * BKV);
 #pragma unroll
         for (int i = 0; i < 128; ++i) {
           if (i > seen) s[i] = 0xff800000u;          // -inf
@@ -276,20 +279,23 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar->p_full[t]);
     }
-    if (ok && nt > 0) {
+    if (ok && (PAIRS || nt > 0)) {
       ok = mbar_wait(&bar->pv_done[t], (nt - 1) & 1, &bar->abort_flag, p.status, 40);
       if (ok) {
         tc_fence_after();
         const float inv = 1.f / l;
-        const int q_row = q_row0 + t * BQ + row;
-        __nv_bfloat16* orow = p.O + (((size_t)b * p.S + q_row) * p.Hq + h) * D;
+        int place = blockIdx.x;                  // the head once more, instead of registers held over the loop
+        asm volatile("" : "+r"(place));
+        const int bh = place % (p.Hq * p.batch);
+        const int q_row = q_row0 + t * BQ + row;             // of this sequence
+        __nv_bfloat16* orow = p.O + (((size_t)(bh / p.Hq) * p.S + q_row) * p.Hq + bh % p.Hq) * D;
 #pragma unroll 1
         for (int ch = 0; ch < D / 32; ++ch) {
           uint32_t r[32];
           tmem_ld_32x32(tO + ch * 32, r);
           tmem_ld_wait();
           uint4* dst = reinterpret_cast<uint4*>(orow + ch * 32);
-          if (q_row < p.S) {
+          if (PAIRS || q_row < p.S) {
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
               uint4 v;
@@ -300,10 +306,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
               dst[g] = v;
             }
           }
-          __syncwarp();         // the lanes of rows behind the sequence take part in the next (aligned) read
+          if (!PAIRS) __syncwarp();         // the lanes of rows behind the sequence take part in the next (aligned) read
         }
-        if (p.lse != nullptr && q_row < p.S)
-          p.lse[((size_t)b * p.Hq + h) * p.S + q_row] = m_ref * p.scale + logf(l);
+        if (p.lse != nullptr && (PAIRS || q_row < p.S))
+          p.lse[(size_t)bh * p.S + q_row] = m_ref * p.scale + logf(l);
       }
     }
   }
@@ -340,18 +346,20 @@ int run(const void* q, long long q_row_stride, long long q_head_stride, const vo
   cudaGetDevice(&dev);
   // DISTDL_ATTN_EXP_POLY=1: a third of the exponentials on the FMA pipe (exp2_fma in common.cuh)
   static const bool poly = [] { const char* e = getenv("DISTDL_ATTN_EXP_POLY"); return e != nullptr && e[0] == '1'; }();
+  using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, Params2);
+  const Kernel kernels[4] = {attn_fwd2_kernel<false, false>, attn_fwd2_kernel<false, true>, attn_fwd2_kernel<true, false>,
+                             attn_fwd2_kernel<true, true>};
   if (!configured[dev & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd2_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attn_fwd2_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL);
-    if (e != cudaSuccess) return (int)e;
+    for (Kernel k : kernels) {
+      const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL);
+      if (e != cudaSuccess) return (int)e;
+    }
     configured[dev & 63] = true;
   }
   const long long grid = (S / (2 * BQ) + (S % (2 * BQ) != 0)) * (long long)Hq * batch;
   if (grid > 0x7fffffffLL) return DD_ERR_TOO_LARGE;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (poly) attn_fwd2_kernel<true><<<(unsigned)grid, NUM_THREADS, SMEM_TOTAL, st>>>(tq, tk, tv, p);
-  else attn_fwd2_kernel<false><<<(unsigned)grid, NUM_THREADS, SMEM_TOTAL, st>>>(tq, tk, tv, p);
+  kernels[(poly ? 2 : 0) + (S % (2 * BQ) == 0 ? 1 : 0)]<<<(unsigned)grid, NUM_THREADS, SMEM_TOTAL, st>>>(tq, tk, tv, p);
   return (int)cudaGetLastError();
 }
 
