@@ -14,6 +14,14 @@ int bwd3_split(int batch, int nT, int Hq, int Hkv, int causal) {
   const long long kv_heads = (long long)batch * Hkv, sweeps = causal ? kv_heads * (nT + 1) / 2 : kv_heads * nT;
   return Hq > Hkv && sweeps < current_sm_count() ? Hq / Hkv : 1;
 }
+// Words of scratch: per 128 queries of a head two statistics each and two counters; with more than one key tile the sums of
+// dQ, with the heads of a group split those of dK and dV.
+long long bwd3_words(int batch, int S, int Hq, int Hkv, int Dh, int causal) {
+  const int nT = S / 128 + (S % 128 != 0);
+  const long long tiles = (long long)batch * Hq * nT, kv_tiles = (long long)batch * Hkv * nT;
+  return 256 * tiles + 4 + (2 * tiles + 3) / 4 * 4 + (nT > 1 ? 128 * Dh * tiles : 0) +
+         (bwd3_split(batch, nT, Hq, Hkv, causal) > 1 ? 256 * Dh * kv_tiles : 0);
+}
 }  // namespace dd
 
 #define DD_HEAD_DIM 128
@@ -29,9 +37,7 @@ int bwd3_split(int batch, int nT, int Hq, int Hkv, int causal) {
 #undef DD_BWD3_NS
 
 // Gradients of softmax(scale * q k^T) v over [batch * S, heads, Dh] bf16 tensors given by address, row and head stride;
-// out and dout are contiguous, lse is [batch][Hq][S].  With tiles = batch * Hq * ceil(S / 128), `scratch` holds `words` =
-// 256 * tiles + 4 + ceil(2 * tiles / 4) * 4 words, for more than 128 tokens 128 * Dh * tiles words more, and for
-// Hq > Hkv another 256 * Dh * batch * Hkv * ceil(S / 128).
+// out and dout are contiguous, lse is [batch][Hq][S].  `scratch` holds `words` words, no fewer than dd_attn_bwd_one_pass says.
 DD_API int dd_attn_bwd3(const void* q, long long q_row, long long q_head, const void* k, long long k_row,
                        long long k_head, const void* v, long long v_row, long long v_head, const void* out,
                        const void* dout, const float* lse, float* scratch, long long words, void* dq, long long dq_row,
@@ -56,8 +62,12 @@ DD_API int dd_attn_bwd3(const void* q, long long q_row, long long q_head, const 
 //                  8 x 1024, 32, causal: 464 -> 507    2 x 2048, 16: 276 -> 314    2 x 4096, 32 / 8, causal: 1050 -> 1058
 // Hence: always where the group's heads are split over CTAs (the two kernels leave SMs idle there) and for one key tile;
 // otherwise where no more than a quarter of a head's key tiles start together, at head dim 128 for long sweeps only.
-DD_API int dd_attn_bwd_one_pass(int batch, int S, int Hq, int Hkv, int Dh, int causal) {
-  if (S % 128 || batch <= 0 || Hkv <= 0) return 1;
+// `words`: of scratch for the one kernel, on this device.
+DD_API int dd_attn_bwd_one_pass(int batch, int S, int Hq, int Hkv, int Dh, int causal, long long* words) {
+  *words = 4;
+  if (S <= 0 || batch <= 0 || Hkv <= 0 || Hq <= 0) return 1;         // (refused by the kernel's entry)
+  *words = dd::bwd3_words(batch, S, Hq, Hkv, Dh, causal);
+  if (S % 128) return 1;
   const int nT = S / 128;
   if (nT <= 1 || dd::bwd3_split(batch, nT, Hq, Hkv, causal) > 1) return 1;
   const long long fit = current_sm_count() / ((long long)Hkv * batch);

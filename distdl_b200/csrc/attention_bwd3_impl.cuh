@@ -695,7 +695,7 @@ int run(const void* q, long long q_row, long long q_head, const void* k, long lo
   p.kv_turn = p.dq_turn + tiles;
   p.dq_sum = reinterpret_cast<float*>(p.dq_turn + (2 * tiles + 3) / 4 * 4);
   p.kv_sum = p.dq_sum + (nT > 1 ? tiles * (BT * D) : 0);
-  if (p.kv_sum + (split > 1 ? kv_tiles * (2 * BT * D) : 0) > scratch + words) return DD_ERR_TOO_LARGE;
+  if (bwd3_words(batch, S, Hq, Hkv, D, causal) > words) return DD_ERR_TOO_LARGE;
   CUtensorMap tq, tk, tv, tdo;
   int r = get_tensor_map_bf16_4d(&tq, q, D, S, Hq, batch, q_row * 2, q_head * 2, (uint64_t)S * q_row * 2, 64, BT);
   if (!r) r = get_tensor_map_bf16_4d(&tk, k, D, S, Hkv, batch, k_row * 2, k_head * 2, (uint64_t)S * k_row * 2, 64, BT);

@@ -284,6 +284,8 @@ class Block(torch.nn.Module):
             # the library operators keep more: the rotary embedding is not in place (a second copy of the
             # projection), silu(gate) and its product are separate tensors, attention keeps fp32 statistics
             kept += 2 * qkv + h + 2 * x
+        # (while attention's backward pass runs, nothing of h is in use: its workspace, 4 bytes per element of dQ and with
+        # grouped heads split over CTAs of dK and dV, lies within 2 h)
         moment = 2 * h + 2 * qkv + 6 * tok * d * e
         # what storing the cheap outputs as well would add: the activation function's output, and
         # (where the projections save their input itself, i.e. without tensor parallelism) both norm outputs

@@ -9,6 +9,7 @@ output of a fused QKV projection is consumed in place (strided views).
 """
 from __future__ import annotations
 
+import ctypes
 import functools
 import math
 
@@ -42,12 +43,19 @@ _native.declare("dd_attn_bwd", [_native.c_void_p, _native.c_ll, _native.c_ll, _n
                                 _native.c_int, _native.c_int, _native.c_int, _native.c_int, _native.c_float,
                                 _native.c_void_p])
 _native.declare("dd_attn_bwd3", _BWD_ARGS[:13] + [_native.c_ll] + _BWD_ARGS[13:])
-_native.declare("dd_attn_bwd_one_pass", [_native.c_int] * 6)
+_native.declare("dd_attn_bwd_one_pass", [_native.c_int] * 6 + [_native.c_void_p])
 
 
 @functools.lru_cache(maxsize=1024)
+def _one_pass_words(device, batch, seq, Hq, Hkv, D, causal):
+    words = ctypes.c_longlong()
+    one = _native.lib().dd_attn_bwd_one_pass(batch, seq, Hq, Hkv, D, int(causal), ctypes.byref(words))
+    return words.value if one else 0
+
+
 def _one_pass(batch, seq, Hq, Hkv, D, causal):
-    return bool(_native.lib().dd_attn_bwd_one_pass(batch, seq, Hq, Hkv, D, int(causal)))
+    """Words of scratch for a backward pass in one kernel, 0 where two kernels are the faster way on this device."""
+    return _one_pass_words(torch._C._cuda_getDevice(), batch, seq, Hq, Hkv, D, bool(causal))
 
 
 def _strides(t):
@@ -86,13 +94,9 @@ def attention_backward(dout, q, k, v, out, lse, batch, seq, causal=True, scale=N
     if seq % 128 and dout.data_ptr() % 16:
         dout = dout.clone()
     in_tmem = env("DISTDL_ATTN_BWD2", "1") != "0" or seq % 128 != 0
-    if in_tmem and D in (64, 128) and _one_pass(batch, seq, Hq, Hkv, D, bool(causal)):
-        # one kernel for all three gradients.  Scratch per 128 queries of a head: two statistics each and two counters;
-        # with more than one key tile the sums of dQ, with grouped-query heads those of dK and dV
-        tiles = batch * Hq * ((seq + 127) // 128)
-        words = 256 * tiles + 4 + (2 * tiles + 3) // 4 * 4 + (128 * D * tiles if seq > 128 else 0)
-        if Hq > Hkv:
-            words += 256 * D * (tiles // Hq * Hkv)
+    words = _one_pass(batch, seq, Hq, Hkv, D, causal) if in_tmem and D in (64, 128) else 0
+    if words:
+        # one kernel for all three gradients
         scratch = torch.empty(words, dtype=torch.float32, device=q.device)
         _native.call("dd_attn_bwd3", q.data_ptr(), *_strides(q), k.data_ptr(), *_strides(k), v.data_ptr(), *_strides(v),
                      out.data_ptr(), dout.data_ptr(), lse.data_ptr(), scratch.data_ptr(), words, dq.data_ptr(),

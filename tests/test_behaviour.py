@@ -224,3 +224,22 @@ def test_norm_gradients_accumulate_for_both_parameters_or_neither():
     w.main_grad, b.main_grad = torch.zeros(4), torch.zeros(4)
     ctx = types.SimpleNamespace(wref=w, bref=b)
     assert _main_grads(ctx, True, True, 1) == (w.main_grad, b.main_grad)
+
+
+def test_scratch_of_the_one_pass_attention_backward():
+    """The sums of dK and dV take memory only where the heads of a group are split over CTAs."""
+    import ctypes
+
+    import distdl_b200.ops.attention  # noqa: F401  (declares the entry point)
+    from distdl_b200 import _native
+    words = ctypes.c_longlong()
+
+    def ask(batch, seq, hq, hkv, d):
+        _native.lib().dd_attn_bwd_one_pass(batch, seq, hq, hkv, d, 1, ctypes.byref(words))
+        return words.value
+    for batch, seq, hq, hkv, d, split in ((1, 16384, 32, 8, 128, False), (8, 1024, 32, 8, 64, False),
+                                          (3, 1000, 16, 4, 128, True), (1, 7, 4, 1, 64, True), (2, 256, 8, 8, 64, False)):
+        nT = -(-seq // 128)
+        tiles, kv_tiles = batch * hq * nT, batch * hkv * nT
+        want = 256 * tiles + 4 + -(-2 * tiles // 4) * 4 + (128 * d * tiles if nT > 1 else 0) + (256 * d * kv_tiles if split else 0)
+        assert ask(batch, seq, hq, hkv, d) == want

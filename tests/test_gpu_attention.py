@@ -196,3 +196,22 @@ def test_ragged_projection_with_a_scale_that_is_not_positive(scale):
     h, = torch.autograd.grad(ref, w, dout.double())
     # bf16 probabilities and results: 0.28 % (see above)
     assert (y.double() - ref).norm() < 5e-3 * ref.norm() and (g.double() - h).norm() < 5e-3 * h.norm()
+
+
+def test_backward_in_one_pass_holds_no_more_than_it_uses():
+    """Grouped-query heads that one CTA sweeps one after the other need no partial sums of dK and dV."""
+    from distdl_b200.ops.attention import _one_pass, attention_backward, attention_forward
+    B, S, Hq, Hkv, D = 8, 1024, 32, 8, 64
+    words = _one_pass(B, S, Hq, Hkv, D, True)
+    assert words
+    q, k, v, dout = (torch.randn(B * S, h, D, device="cuda", dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv, Hq))
+    out, lse = attention_forward(q, k, v, B, S, True)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    base = torch.cuda.memory_allocated()
+    grads = attention_backward(dout, q, k, v, out, lse, B, S, True)
+    held = torch.cuda.max_memory_allocated() - base
+    gradients = sum(g.numel() * 2 for g in grads)
+    # 4 bytes per element of dQ, statistics and counters; the allocator rounds each of four blocks up to 2 MB at most
+    assert held <= gradients + 4 * q.numel() + B * Hq * S * 8 + (1 << 20) + 4 * (2 << 20)
+    assert gradients + 4 * words <= held
