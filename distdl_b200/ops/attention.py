@@ -95,9 +95,15 @@ def attention_backward(dout, q, k, v, out, lse, batch, seq, causal=True, scale=N
         dout = dout.clone()
     in_tmem = env("DISTDL_ATTN_BWD2", "1") != "0" or seq % 128 != 0
     words = _one_pass(batch, seq, Hq, Hkv, D, causal) if in_tmem and D in (64, 128) else 0
+    scratch = None
     if words:
-        # one kernel for all three gradients
-        scratch = torch.empty(words, dtype=torch.float32, device=q.device)
+        try:
+            scratch = torch.empty(words, dtype=torch.float32, device=q.device)
+        except torch.OutOfMemoryError:
+            if seq % 128:
+                raise                       # (no other kernel takes such a length)
+    if scratch is not None:
+        # one kernel for all three gradients; without room for its sums, the two that need none
         _native.call("dd_attn_bwd3", q.data_ptr(), *_strides(q), k.data_ptr(), *_strides(k), v.data_ptr(), *_strides(v),
                      out.data_ptr(), dout.data_ptr(), lse.data_ptr(), scratch.data_ptr(), words, dq.data_ptr(),
                      *_strides(dq), dk.data_ptr(), *_strides(dk), dv.data_ptr(), *_strides(dv), batch, seq, Hq, Hkv, D,
