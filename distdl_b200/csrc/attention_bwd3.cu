@@ -50,18 +50,42 @@ DD_API int dd_attn_bwd3(const void* q, long long q_row, long long q_head, const 
              dk_row, dk_head, dv, dv_row, dv_head, batch, S, Hq, Hkv, causal, scale, stream);
 }
 
+// Whether the backward pass of a group that is split over CTAs is faster in one kernel than in two.  What the two kernels
+// leave idle shrinks with the pairs of kv head and key tile (`kv_tiles`), since they have one CTA for each; what the one
+// kernel loses is the hand-over.  Ratios one kernel : two, cold L2, by kv_tiles (800 sizes measured in all):
+//   head dim 128, causal   2 tiles, groups of 4:  48 0.82  112 1.03  176 1.17    2 tiles, groups of 8:  48 1.02  112 1.17
+//                          8 tiles, groups of 4:  80 0.76  144 0.94  208 1.16   16 tiles, groups of 8: 112 0.77  176 1.03
+//                         48 tiles, groups of 8: 144 0.69  240 0.94             32 tiles, groups of 2: 192 0.89  256 1.11
+//   head dim 128, full     groups of 4: 2 tiles 32 0.96 64 1.11, 8 tiles 32 1.19, 32 tiles 96 1.27
+//                          groups of 8: 4 tiles 32 0.96 64 1.06, 16 tiles 64 0.90 96 1.15
+//   head dim 64, full      groups of 2: 2 tiles 32 0.94 64 1.06, 8 tiles 32 1.29    groups of 3: 4 tiles 32 0.95, 24 tiles 24 1.12
+//                          groups of 4: 2 tiles 100 1.09, 16 tiles 96 0.89          (causal: 0.37 to 1.00)
+static bool split_in_one_pass(int nT, int group, long long kv_tiles, int Dh, int causal, long long sms) {
+  if (Dh == 64) {
+    if (causal) return true;
+    if (nT <= 4 && (nT <= 2 ? kv_tiles * 2 > sms : kv_tiles * 3 > sms * 2)) return false;
+    return group > 3 || nT <= (group == 3 ? 8 : 2);
+  }
+  if (causal) return kv_tiles * 5 * (nT + group) <= 8 * sms * nT || nT >= 64;
+  if (group >= 6 && nT * 4 >= group) return nT >= 8 ? kv_tiles * 5 <= sms * 2 : kv_tiles * 3 <= sms;
+  return (nT <= 2 || group == 5) && nT * 4 >= group && kv_tiles * 4 <= sms;
+}
+
 // Whether a backward pass should run in one kernel (attention_bwd3_impl.cuh) or in two (attention_bwd2_impl.cuh, whole
 // tiles only).  The one kernel forms the scores once and one exponential per score, but its CTAs hand the sums of dQ on to
-// one another (the key tiles of a head that start together follow one another at a distance of 3 us, and a delay of
-// one is a delay of all behind it), and at head dim 128 shared memory bounds it at nearly the time of the two.  In us, two
-// kernels -> one, batch x tokens, heads:
-//   head dim 64    8 x 1536, 16: 577 -> 392    4 x 1024, 25, causal: 173 -> 128    16 x 512, 16: 169 -> 149
-//                  1 x 16384, 16: 4963 -> 3486    1 x 4096, 8, causal, 18 of 32 key tiles together: 119 -> 136
-//   head dim 128   heads of a group split: 3 x 1024, 16 / 4, causal: 149 -> 112; 1 x 16384, 4 / 1, causal: 1379 -> 906
-//                  one key tile: 64 x 128, 16 / 4: 118 -> 75    1 x 16384, 32 / 8, causal: 6667 -> 6109
-//                  8 x 1024, 32, causal: 464 -> 507    2 x 2048, 16: 276 -> 314    2 x 4096, 32 / 8, causal: 1050 -> 1058
-// Hence: always where the group's heads are split over CTAs (the two kernels leave SMs idle there) and for one key tile;
-// otherwise where no more than a quarter of a head's key tiles start together, at head dim 128 for long sweeps only.
+// one another: the key tiles of a head that start together follow one another at the distance of a hand-over, which
+// full attention waits for (every sweep has the same length and starts at the same query tile) and causal attention
+// hides behind its longer sweeps.  At head dim 128 shared memory bounds it at nearly the time of the two besides.  Groups
+// that are split: above.  Otherwise, in us, two kernels -> one, batch x tokens, heads, each call alone and with a cold L2
+// (in brackets: back to back, where the power limit counts and with it the fewer products):
+//   head dim 64            8 x 1536, 16: 577 -> 392; 16 x 512, 16: 169 -> 149; 1 x 16384, 16: 5479 -> 3722; but 1 x 4096, 8, causal,
+//                          18 of 32 key tiles together: 112 -> 120; 1 x 1024, 16, full, all 8 together: 46 -> 77
+//   head dim 128, causal   1 x 16384, 32: 7412 -> 6791 (7581 -> 6679); 1 x 8192, 16: 873 -> 837 (965 -> 886); 1 x 16384, 32 / 8:
+//                          6170 -> 6632 (6988 -> 6403); but 8 x 1024, 32: 464 -> 503, 1 x 2048, 16: 93 -> 102
+//   head dim 128, full     1 x 16384, 32: 16190 -> 13422 (16588 -> 13371); but 1 x 4096, 8: 261 -> 489; 1 x 16384, 8: 3113 -> 4063;
+//                          1 x 16384, 32 / 8: 13976 -> 14919 (13897 -> 14790)
+//   one key tile           64 x 128, 16 / 4 of 128: 118 -> 75
+// Hence one kernel where no more than a quarter of a head's key tiles start together, at head dim 128 for long sweeps only.
 // `words`: of scratch for the one kernel, on this device.
 DD_API int dd_attn_bwd_one_pass(int batch, int S, int Hq, int Hkv, int Dh, int causal, long long* words) {
   *words = 4;
@@ -69,8 +93,13 @@ DD_API int dd_attn_bwd_one_pass(int batch, int S, int Hq, int Hkv, int Dh, int c
   *words = dd::bwd3_words(batch, S, Hq, Hkv, Dh, causal);
   if (S % 128) return 1;
   const int nT = S / 128;
-  if (nT <= 1 || dd::bwd3_split(batch, nT, Hq, Hkv, causal) > 1) return 1;
-  const long long fit = current_sm_count() / ((long long)Hkv * batch);
+  if (nT <= 1) return 1;
+  const long long sms = current_sm_count();
+  if (dd::bwd3_split(batch, nT, Hq, Hkv, causal) > 1 &&
+      split_in_one_pass(nT, Hq / Hkv, (long long)batch * Hkv * nT, Dh, causal, sms))
+    return 1;
+  const long long fit = sms / ((long long)Hkv * batch);
   const long long together = fit < 1 ? 1 : fit < nT ? fit : nT;
-  return (together == 1 || together * 4 <= nT) && (Dh == 64 || nT >= 64);
+  if (Dh == 64) return together == 1 || together * 4 <= nT;
+  return nT >= 64 && (causal ? together * 4 <= nT : Hq == Hkv && together * 32 <= nT);
 }

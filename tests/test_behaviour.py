@@ -243,3 +243,26 @@ def test_scratch_of_the_one_pass_attention_backward():
         tiles, kv_tiles = batch * hq * nT, batch * hkv * nT
         want = 256 * tiles + 4 + -(-2 * tiles // 4) * 4 + (128 * d * tiles if nT > 1 else 0) + (256 * d * kv_tiles if split else 0)
         assert ask(batch, seq, hq, hkv, d) == want
+
+
+def test_rule_of_the_attention_backward():
+    """Both sides of every line, at sizes where both ways were measured, on 148 SMs (batch, tokens, heads, kv heads, head
+    dim, causal)."""
+    import ctypes
+
+    import distdl_b200.ops.attention  # noqa: F401  (declares the entry point)
+    from distdl_b200 import _native
+    if _native.lib().dd_sm_count() != 148:
+        return
+    words = ctypes.c_longlong()
+    one = [(1, 1024, 16, 4, 64, 1), (1, 1024, 16, 4, 64, 0), (1, 4096, 8, 4, 64, 1), (16, 512, 16, 16, 64, 0),
+           (1, 256, 8, 4, 64, 0), (1, 512, 6, 2, 64, 0), (1, 16384, 16, 16, 64, 0), (64, 128, 16, 4, 128, 1),
+           (1, 2048, 4, 1, 128, 1), (2, 1024, 32, 8, 128, 1), (1, 8192, 16, 4, 128, 1), (1, 16384, 32, 32, 128, 1),
+           (1, 16384, 32, 8, 128, 1), (1, 8192, 16, 16, 128, 1), (4, 256, 16, 4, 128, 0), (1, 16384, 32, 32, 128, 0),
+           (3, 1000, 16, 4, 128, 1), (1, 7, 2, 2, 64, 0)]
+    two = [(1, 4096, 8, 4, 64, 0), (1, 4096, 8, 8, 64, 1), (1, 1024, 16, 16, 64, 0), (4, 1024, 32, 8, 128, 1),
+           (2, 2048, 32, 8, 128, 1), (8, 256, 32, 8, 128, 1), (2, 4096, 32, 8, 128, 1), (8, 1024, 32, 32, 128, 1),
+           (1, 2048, 16, 16, 128, 1), (1, 4096, 8, 4, 128, 0), (1, 16384, 8, 8, 128, 0), (1, 16384, 32, 8, 128, 0),
+           (4, 512, 8, 4, 128, 0), (4, 256, 32, 8, 128, 0)]
+    for sizes in one + two:
+        assert bool(_native.lib().dd_attn_bwd_one_pass(*sizes, ctypes.byref(words))) == (sizes in one), sizes
