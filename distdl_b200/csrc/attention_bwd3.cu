@@ -103,3 +103,19 @@ DD_API int dd_attn_bwd_one_pass(int batch, int S, int Hq, int Hkv, int Dh, int c
   if (Dh == 64) return together == 1 || together * 4 <= nT;
   return nT >= 64 && (causal ? together * 4 <= nT : Hq == Hkv && together * 32 <= nT);
 }
+
+// Whether training on a packed projection of a length that is not whole tiles (head dim 128) is faster on the kernels here
+// than on the library's operators, which put the packed gradient together by copies but whose backward pass waits for no
+// hand-over.  Forward and backward in us, library -> here, batch x tokens, heads:
+//   causal   1 x 900, 8: 183 -> 102; 3 x 1000, 32: 411 -> 224; 4 x 3000, 32 / 8: 1660 -> 1456; 1 x 4000, 32 / 8: 671 -> 605; 1 x 6000,
+//            32: 1450 -> 1290; but 1 x 4600, 32 / 8: 812 -> 886, 1 x 9000, 32 / 8: 2495 -> 3008, 1 x 12000, 32: 4512 -> 4803
+//   full     1 x 600, 32 / 8: 182 -> 105; 1 x 1000, 16: 197 -> 140; 3 x 1531, 32: 738 -> 657; 2 x 1000, 16 / 4: 323 -> 161;
+//            4 x 1000, 16 / 8: 368 -> 262; but 1 x 2100, 16: 279 -> 298, 1 x 4000, 8: 390 -> 528, 4 x 1000, 32 / 8: 448 -> 579,
+//            1 x 1300, 32 / 8: 220 -> 255, 2 x 3000, 16 / 4: 640 -> 1445
+DD_API int dd_attn_ragged(int batch, int S, int Hq, int Hkv, int causal) {
+  if (S <= 0 || batch <= 0 || Hkv <= 0 || Hq < Hkv) return 0;
+  const int nT = S / 128 + 1, group = Hq / Hkv;
+  if (causal) return nT <= (group == 1 ? 64 : 32);
+  if (group == 1) return nT <= 12;
+  return (long long)group * nT <= 20 || (nT <= 10 && dd::bwd3_split(batch, nT, Hq, Hkv, 0) > 1);
+}

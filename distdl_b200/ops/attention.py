@@ -43,6 +43,7 @@ _native.declare("dd_attn_bwd", [_native.c_void_p, _native.c_ll, _native.c_ll, _n
                                 _native.c_int, _native.c_int, _native.c_int, _native.c_int, _native.c_float,
                                 _native.c_void_p])
 _native.declare("dd_attn_bwd3", _BWD_ARGS[:13] + [_native.c_ll] + _BWD_ARGS[13:])
+_native.declare("dd_attn_ragged", [_native.c_int] * 5)
 _native.declare("dd_attn_bwd_one_pass", [_native.c_int] * 6 + [_native.c_void_p])
 
 
@@ -51,6 +52,11 @@ def _one_pass_words(device, batch, seq, Hq, Hkv, D, causal):
     words = ctypes.c_longlong()
     one = _native.lib().dd_attn_bwd_one_pass(batch, seq, Hq, Hkv, D, int(causal), ctypes.byref(words))
     return words.value if one else 0
+
+
+@functools.lru_cache(maxsize=1024)
+def _ragged_faster(device, batch, seq, Hq, Hkv, causal):
+    return bool(_native.lib().dd_attn_ragged(batch, seq, Hq, Hkv, int(causal)))
 
 
 def _one_pass(batch, seq, Hq, Hkv, D, causal):
@@ -169,18 +175,18 @@ def _operators(dout, qkv, Hq, Hkv, batch, seq, causal, scale):
         return torch.autograd.grad(out, qkv, dout, create_graph=True)[0]
 
 
-def _ragged_ok(qkv, Hq, Hkv, batch, seq, scale=None):
+def _ragged_ok(qkv, Hq, Hkv, batch, seq, scale=None, causal=True):
     """Sequences that are not whole tiles of 128, in training at head dim 128: the kernels take over from the library's
-    operators, whose packed gradient is put together by copies (forward and backward, 3 x 1000 tokens, 16 / 4 heads:
-    189 -> 126 us on the GPU, 310 -> 185 on the host; 2 x 1531, 32 / 8: 370 -> 272; 8 x 333, 16 heads: 194 -> 89), where
+    operators, whose packed gradient is put together by copies, where they are the faster way (``dd_attn_ragged``), where
     nobody looks for the operators themselves and where the tensor maps can address the projection.  The kernels mask with
-    -inf before they multiply by the scale: one of 0 or below is the library's.  Without a gradient
-    (2 x 1531, 32 / 8: 54 against 68 us) and at head dim 64 the library's kernels are the faster ones."""
+    -inf before they multiply by the scale: one of 0 or below is the library's.  Without a gradient (2 x 1531 tokens, 32 / 8
+    heads: 54 against 68 us) and at head dim 64 the library's kernels are the faster ones."""
     return (qkv.dim() == 3 and qkv.shape[2] == 128 and qkv.requires_grad and torch.is_grad_enabled() and batch > 0
             and seq > 0 and Hkv > 0 and Hq > 0 and Hq % Hkv == 0 and qkv.shape[0] == batch * seq
             and qkv.shape[1] == Hq + 2 * Hkv and (scale is None or (isinstance(scale, (int, float)) and 0 < scale < math.inf))
             and qkv.data_ptr() % 16 == 0 and _plain(qkv)
-            and not (torch.is_autocast_enabled() and torch.get_autocast_dtype("cuda") != torch.bfloat16))
+            and not (torch.is_autocast_enabled() and torch.get_autocast_dtype("cuda") != torch.bfloat16)
+            and _ragged_faster(torch._C._cuda_getDevice(), batch, seq, Hq, Hkv, bool(causal)))
 
 
 class _PackedAttnFn(torch.autograd.Function):
@@ -214,7 +220,7 @@ def attention_packed(qkv, Hq: int, Hkv: int, batch: int, seq: int, causal: bool 
     D = qkv.shape[-1]
     native = (use_native(qkv) and qkv.dtype == torch.bfloat16 and D in (64, 128) and qkv.is_contiguous()
               and env("DISTDL_ATTN_IMPL", "native") == "native"
-              and (seq % 128 == 0 or _ragged_ok(qkv, Hq, Hkv, batch, seq, scale)))
+              and (seq % 128 == 0 or _ragged_ok(qkv, Hq, Hkv, batch, seq, scale, causal)))
     if native:
         return _PackedAttnFn.apply(qkv, Hq, Hkv, batch, seq, causal, scale)
     return _reference(qkv[:, :Hq], qkv[:, Hq:Hq + Hkv], qkv[:, Hq + Hkv:], batch, seq, causal, scale)

@@ -266,3 +266,17 @@ def test_rule_of_the_attention_backward():
            (4, 512, 8, 4, 128, 0), (4, 256, 32, 8, 128, 0)]
     for sizes in one + two:
         assert bool(_native.lib().dd_attn_bwd_one_pass(*sizes, ctypes.byref(words))) == (sizes in one), sizes
+
+
+def test_rule_of_ragged_attention_in_training():
+    """Both sides of every line, at measured sizes (batch, tokens, heads, kv heads, causal), on 148 SMs."""
+    import distdl_b200.ops.attention  # noqa: F401  (declares the entry point)
+    from distdl_b200 import _native
+    here = [(1, 7, 8, 8, 1), (3, 1000, 16, 4, 1), (2, 1531, 32, 8, 1), (1, 4000, 32, 8, 1), (1, 6000, 32, 32, 1), (1, 7, 8, 8, 0),
+            (1, 600, 32, 8, 0), (1, 1000, 16, 16, 0), (3, 1531, 32, 32, 0), (2, 1000, 16, 4, 0), (4, 1000, 16, 8, 0)]
+    library = [(1, 4600, 32, 8, 1), (1, 9000, 32, 8, 1), (1, 12000, 32, 32, 1), (1, 2100, 16, 16, 0), (1, 4000, 8, 8, 0),
+               (4, 1000, 32, 8, 0), (1, 1300, 32, 8, 0), (2, 3000, 16, 4, 0)]
+    if _native.lib().dd_sm_count() != 148:
+        return
+    for sizes in here + library:
+        assert bool(_native.lib().dd_attn_ragged(*sizes)) == (sizes in here), sizes
