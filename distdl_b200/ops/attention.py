@@ -43,6 +43,7 @@ _native.declare("dd_attn_bwd", [_native.c_void_p, _native.c_ll, _native.c_ll, _n
                                 _native.c_int, _native.c_int, _native.c_int, _native.c_int, _native.c_float,
                                 _native.c_void_p])
 _native.declare("dd_attn_bwd3", _BWD_ARGS[:13] + [_native.c_ll] + _BWD_ARGS[13:])
+_native.declare("dd_attn_fwd_two_tiles", [_native.c_int] * 4)
 _native.declare("dd_attn_ragged", [_native.c_int] * 5)
 _native.declare("dd_attn_bwd_one_pass", [_native.c_int] * 6 + [_native.c_void_p])
 
@@ -52,6 +53,11 @@ def _one_pass_words(device, batch, seq, Hq, Hkv, D, causal):
     words = ctypes.c_longlong()
     one = _native.lib().dd_attn_bwd_one_pass(batch, seq, Hq, Hkv, D, int(causal), ctypes.byref(words))
     return words.value if one else 0
+
+
+@functools.lru_cache(maxsize=1024)
+def _two_tiles(device, batch, seq, Hq, causal):
+    return bool(_native.lib().dd_attn_fwd_two_tiles(batch, seq, Hq, int(causal)))
 
 
 @functools.lru_cache(maxsize=1024)
@@ -78,7 +84,8 @@ def attention_forward(q, k, v, batch, seq, causal=True, scale=None):
     out = torch.empty(tokens, Hq, D, dtype=q.dtype, device=q.device)
     lse = torch.empty(batch, Hq, seq, dtype=torch.float32, device=q.device)
     # the two-tile kernel (scores and probabilities in tensor memory, two query tiles alternating on the tensor cores)
-    two_tile = D in (64, 128) and (env("DISTDL_ATTN_FWD2", "1") != "0" or seq % 128 != 0)
+    two_tile = D in (64, 128) and (seq % 128 != 0 or (
+        env("DISTDL_ATTN_FWD2", "1") != "0" and _two_tiles(torch._C._cuda_getDevice(), batch, seq, Hq, bool(causal))))
     _native.call("dd_attn_fwd2" if two_tile else "dd_attn_fwd", q.data_ptr(), *_strides(q), k.data_ptr(), *_strides(k),
                  v.data_ptr(), *_strides(v), out.data_ptr(), lse.data_ptr(), batch, seq, Hq, Hkv, D, int(causal),
                  float(scale), stream_ptr())

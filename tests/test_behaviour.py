@@ -280,3 +280,15 @@ def test_rule_of_ragged_attention_in_training():
         return
     for sizes in here + library:
         assert bool(_native.lib().dd_attn_ragged(*sizes)) == (sizes in here), sizes
+
+
+def test_rule_of_the_attention_forward():
+    """Both sides of every line, at measured sizes (batch, tokens, heads, causal), on 148 SMs."""
+    import distdl_b200.ops.attention  # noqa: F401  (declares the entry point)
+    from distdl_b200 import _native
+    two = [(4, 128, 16, 0), (1, 256, 8, 0), (1, 640, 8, 1), (4, 384, 16, 0), (1, 640, 32, 0), (1, 100, 8, 0), (1, 500, 8, 0)]
+    one = [(1, 384, 32, 0), (1, 640, 8, 0)]
+    if _native.lib().dd_sm_count() != 148:
+        return
+    for sizes in one + two:
+        assert bool(_native.lib().dd_attn_fwd_two_tiles(*sizes)) == (sizes in two), sizes

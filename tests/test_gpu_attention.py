@@ -238,3 +238,21 @@ def test_backward_without_room_for_the_sums_of_one_pass(monkeypatch):
     for a, b in zip(got, want):
         # two ways with errors of 0.28 % (see above)
         assert (a.float() - b.float()).norm() < 8e-3 * b.float().norm()
+
+
+@pytest.mark.parametrize("batch,seq,Hq,Hkv,D", [(1, 384, 32, 8, 64), (2, 640, 4, 4, 128), (1, 1152, 3, 1, 128)])
+def test_forward_with_a_tile_per_cta(batch, seq, Hq, Hkv, D):
+    """Full attention over an odd number of tiles that all fit the SMs at once."""
+    from distdl_b200 import _native
+    from distdl_b200.ops.attention import _two_tiles, attention_forward
+    assert not _two_tiles(0, batch, seq, Hq, False)
+    torch.manual_seed(22)
+    q, k, v = (torch.randn(batch * seq, h, D, device="cuda", dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv))
+    out, lse = attention_forward(q, k, v, batch, seq, False)
+    assert _native.read_status()[0] == 0
+    four = lambda t: t.double().reshape(batch, seq, -1, D).transpose(1, 2)  # noqa: E731
+    K, V = (four(t).repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+    s = four(q) @ K.transpose(-1, -2) / math.sqrt(D)
+    # probabilities and output rounded to bf16: 0.28 % (see above)
+    assert (four(out) - s.softmax(-1) @ V).norm() < 5e-3 * (s.softmax(-1) @ V).norm()
+    assert (lse - s.logsumexp(-1)).abs().max() < 1e-3
