@@ -256,3 +256,106 @@ def test_forward_with_a_tile_per_cta(batch, seq, Hq, Hkv, D):
     # probabilities and output rounded to bf16: 0.28 % (see above)
     assert (four(out) - s.softmax(-1) @ V).norm() < 5e-3 * (s.softmax(-1) @ V).norm()
     assert (lse - s.logsumexp(-1)).abs().max() < 1e-3
+
+
+def _backward_errors(batch, seq, Hq, Hkv, D, causal, shift=0):
+    """Relative 2-norm errors of output and gradients against 64 bits, and whether a second run has the same bits."""
+    from distdl_b200 import _native
+    from distdl_b200.ops.attention import attention_backward, attention_forward
+    torch.manual_seed(23)
+    q, k, v, dout = (torch.randn(batch * seq, h, D, device="cuda", dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv, Hq))
+    out, lse = attention_forward(q, k, v, batch, seq, causal)
+    if shift:                                # an output that starts between two 16-byte units
+        out = torch.empty(out.numel() + shift, device="cuda", dtype=torch.bfloat16)[shift:].view(out.shape).copy_(out)
+    grads = attention_backward(dout, q, k, v, out, lse, batch, seq, causal)
+    again = attention_backward(dout, q, k, v, out, lse, batch, seq, causal)
+    assert _native.read_status()[0] == 0
+    leaves = [t.double().requires_grad_() for t in (q, k, v)]
+    Q, K, V = (t.reshape(batch, seq, -1, D).transpose(1, 2) for t in leaves)
+    s = Q @ K.repeat_interleave(Hq // Hkv, 1).transpose(-1, -2) / math.sqrt(D)
+    if causal:
+        s = s.masked_fill(torch.ones(seq, seq, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+    ref = (s.softmax(-1) @ V.repeat_interleave(Hq // Hkv, 1)).transpose(1, 2).reshape(out.shape)
+    want = [ref, *torch.autograd.grad(ref, leaves, dout.double())]
+    errors = [((t.double() - w).norm() / w.norm()).item() for t, w in zip((out, *grads), want)]
+    return errors, all(torch.equal(a, b) for a, b in zip(grads, again))
+
+
+@pytest.mark.parametrize("batch,seq,Hq,Hkv,D,causal,shift", [
+    (2, 512, 4, 4, 128, True, 0), (1, 384, 5, 5, 128, False, 0),
+    (4, 512, 32, 8, 128, True, 0),           # grouped heads, more key tiles than the one kernel takes
+    (1, 512, 8, 2, 128, False, 0), (2, 384, 6, 2, 128, False, 0),
+    (1, 512, 4, 2, 64, False, 0), (3, 384, 3, 3, 64, False, 0), (2, 256, 4, 4, 64, True, 0),
+    (1, 512, 4, 4, 128, True, 4), (1, 512, 4, 2, 64, False, 4)])
+def test_backward_in_two_kernels(batch, seq, Hq, Hkv, D, causal, shift):
+    """The same bounds as in one pass (see there), at sizes that the rule leaves to the two kernels."""
+    from distdl_b200.ops.attention import _one_pass
+    assert not _one_pass(batch, seq, Hq, Hkv, D, causal)
+    errors, same = _backward_errors(batch, seq, Hq, Hkv, D, causal, shift)
+    assert max(errors) < 5e-3, errors
+    assert same
+
+
+@pytest.mark.parametrize("batch,seq,Hq,Hkv,causal", [(2, 7, 2, 2, True), (3, 100, 4, 2, False), (2, 129, 4, 1, True),
+                                                     (1, 1000, 6, 3, False), (1, 641, 4, 4, True)])
+def test_ragged_lengths_at_head_dim_64(batch, seq, Hq, Hkv, causal):
+    errors, same = _backward_errors(batch, seq, Hq, Hkv, 64, causal)
+    assert max(errors) < 5e-3, errors
+    assert same
+
+
+def test_two_kernels_over_more_sequences_than_a_grid_dimension_holds(monkeypatch):
+    """The sequences around the limit have the bits of a call of their own, as in one pass (see above)."""
+    import importlib
+    A = importlib.import_module("distdl_b200.ops.attention")
+    monkeypatch.setattr(A, "_one_pass", lambda *sizes: 0)
+    torch.manual_seed(24)
+    B, S, D = 65537, 128, 64
+    q, k, v, dout = (torch.randn(B * S, 1, D, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    out, lse = A.attention_forward(q, k, v, B, S, True)
+    grads = A.attention_backward(dout, q, k, v, out, lse, B, S)
+    for b in (0, 65534, 65535, 65536):
+        sl = slice(b * S, (b + 1) * S)
+        one = A.attention_backward(dout[sl], q[sl], k[sl], v[sl], out[sl], lse[b:b + 1], 1, S)
+        assert all(torch.equal(a[sl], r) for a, r in zip(grads, one))
+
+
+@pytest.mark.parametrize("batch,seq,Hq,Hkv,D,causal", [(1, 128, 2, 2, 128, True), (2, 384, 6, 2, 64, False),
+                                                       (1, 512, 4, 1, 128, True), (2, 256, 3, 3, 64, True)])
+def test_kernels_behind_a_switch(batch, seq, Hq, Hkv, D, causal, monkeypatch):
+    """A tile per CTA forward, P and dS through shared memory backward."""
+    monkeypatch.setenv("DISTDL_ATTN_FWD2", "0")
+    monkeypatch.setenv("DISTDL_ATTN_BWD2", "0")
+    errors, same = _backward_errors(batch, seq, Hq, Hkv, D, causal)
+    assert max(errors) < 5e-3, errors
+    assert same
+
+
+def test_ragged_projection_differentiated_twice_and_in_batches():
+    """A gradient that is itself differentiated, and batched gradients, are the library's operators': the same as where the
+    forward pass was the library's too.  Two bf16 ways to the same numbers: 0.28 % each, 0.56 % after another pass."""
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+
+    from distdl_b200.ops import attention_packed
+    from distdl_b200.ops.attention import _reference
+    torch.manual_seed(25)
+    B, S, Hq, Hkv, D = 1, 100, 4, 2, 128
+    x = torch.randn(B * S, Hq + 2 * Hkv, D, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    douts = torch.randn(3, B * S, Hq, D, device="cuda", dtype=torch.bfloat16)
+    u = torch.randn_like(x)
+    y = attention_packed(x, Hq, Hkv, B, S)
+    assert type(y.grad_fn).__name__ == "_PackedAttnFnBackward"
+    w = x.detach().double().requires_grad_()
+    ref = _reference(w[:, :Hq], w[:, Hq:Hq + Hkv].repeat_interleave(2, 1), w[:, Hq + Hkv:].repeat_interleave(2, 1), B, S, True,
+                     1.0 / math.sqrt(D))
+    with sdpa_kernel(SDPBackend.MATH):                       # (the library's fused kernels have no second derivative)
+        g, = torch.autograd.grad(y, x, douts[0], create_graph=True)
+        gg, = torch.autograd.grad(g, x, u, retain_graph=True)
+        batched, = torch.autograd.grad(y, x, douts, is_grads_batched=True, retain_graph=True)
+    h, = torch.autograd.grad(ref, w, douts[0].double(), create_graph=True)
+    hh, = torch.autograd.grad(h, w, u.double(), retain_graph=True)
+    assert (g.double() - h).norm() < 1e-2 * h.norm()
+    assert (gg.double() - hh).norm() < 2e-2 * hh.norm()
+    for got, d in zip(batched, douts):
+        want, = torch.autograd.grad(ref, w, d.double(), retain_graph=True)
+        assert (got.double() - want).norm() < 1e-2 * want.norm()

@@ -231,3 +231,28 @@ def test_gemm_with_half_tiles(M, N, K, a_mn, b_mn):
     want = a.double() @ b.double().t() + before
     assert (acc.double() - want).norm() < 1e-5 * want.norm()
     assert _native.read_status()[0] == 0
+
+
+@pytest.mark.parametrize("B,M,N,K", [(3, 257, 136, 72), (2, 300, 40, 200), (5, 129, 264, 64)])
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_batched_gemm_with_half_tiles(B, M, N, K, a_mn, b_mn):
+    """Batches whose tiles fit one wave take 128 columns: remainders in every direction, both majors (bounds as above)."""
+    from distdl_b200 import _native
+    from distdl_b200.ops import gemm
+    torch.manual_seed(6)
+
+    def make(rows, cols, mn):
+        n, m = (cols, rows) if mn else (rows, cols)
+        st = torch.randn(B, n, (m + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)[:, :, :m]
+        return st.transpose(1, 2) if mn else st
+    a, b = make(M, K, a_mn), make(N, K, b_mn)
+    want = a.double() @ b.double().transpose(1, 2)
+    out = torch.full((B, M, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm(a, b, out=out[:, :, :N])
+    assert (out[:, :, :N].double() - want).norm() < 2.5e-3 * want.norm()
+    assert (out[:, :, N:] == 7).all()
+    acc = torch.randn(B, M, N, device="cuda")
+    before = acc.double()
+    gemm(a, b, out=acc, accumulate=True)
+    assert (acc.double() - want - before).norm() < 1e-5 * (want + before).norm()
+    assert _native.read_status()[0] == 0
