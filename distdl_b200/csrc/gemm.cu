@@ -87,6 +87,18 @@ split_reduce_kernel(const float* __restrict__ part, int split, long long part_st
     }
   }
 }
+
+// Columns of a pair's tile: 128 where the waves of half tiles are the shorter time.  A half tile costs 1.25 times as
+// much per column (its operands and what TMA brings are 192 bytes of shared memory a clock, a whole one's are 128).
+// Forward, in us, 256 -> 128 columns: 4096 x 1600 x 6400 74.8 -> 69.7, 3000 x 2048 x 5632 67.6 -> 63.5, 512 x 1024 x 512
+// 14.3 -> 11.2; but 4096 x 6400 x 1600 62.4 -> 71.7, 3000 x 11264 x 2048 98 -> 114.  Gradients that are added in fp32
+// are bound by their epilogue besides (3000 x 2048 x 5632 70.6 -> 79.9): only where there is one wave either way.
+bool half_tiles(int M, int N, int batch, bool f32, long long pairs, long long* whole, long long* half) {
+  const long long rows_of_tiles = (long long)((M + 2 * gemm2::BM - 1) / (2 * gemm2::BM)) * batch;
+  *whole = rows_of_tiles * ((N + 255) / 256);
+  *half = rows_of_tiles * ((N + 127) / 128);
+  return f32 ? *half <= pairs : (*half + pairs - 1) / pairs * 125 < (*whole + pairs - 1) / pairs * 200;
+}
 }  // namespace
 
 // D[b,m,n] (+)= sum_k A[b,m,k] B[b,n,k] (+ bias[n]);  bf16 operands, fp32 accumulation.
@@ -117,15 +129,8 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
     int ctas = current_sm_count() & ~1;
     if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas & ~1;
     if (ctas < 2) ctas = 2;
-    // Columns of a pair's tile: 128 where the waves of half tiles are the shorter time.  A half tile costs 1.25 times as
-    // much per column (its operands and what TMA brings are 192 bytes of shared memory a clock, a whole one's are 128).
-    // Forward, in us, 256 -> 128 columns: 4096 x 1600 x 6400 74.8 -> 69.7, 3000 x 2048 x 5632 67.6 -> 63.5, 512 x 1024 x 512
-    // 14.3 -> 11.2; but 4096 x 6400 x 1600 62.4 -> 71.7, 3000 x 11264 x 2048 98 -> 114.  Gradients that are added in fp32
-    // are bound by their epilogue besides (3000 x 2048 x 5632 70.6 -> 79.9): only where there is one wave either way.
-    const long long rows_of_tiles = (long long)((M + 2 * g2::BM - 1) / (2 * g2::BM)) * batch;
-    const long long whole = rows_of_tiles * ((N + 255) / 256), half = rows_of_tiles * ((N + 127) / 128), pairs = ctas / 2;
-    const bool narrow = rows == nullptr && ((flags & F_OUT_F32) ? half <= pairs
-                                            : (half + pairs - 1) / pairs * 125 < (whole + pairs - 1) / pairs * 200);
+    long long whole, half;
+    const bool narrow = half_tiles(M, N, batch, (flags & F_OUT_F32) != 0, ctas / 2, &whole, &half) && rows == nullptr;
     if (a_mn) rr = get_tensor_map_bf16_3d(&pa, A, M, K, batch, lda * 2, strideA * 2, 64, g2::BK);
     else      rr = get_tensor_map_bf16_3d(&pa, A, K, M, batch, lda * 2, strideA * 2, g2::BK, g2::BM);
     if (rr) return rr;
@@ -217,21 +222,27 @@ DD_API int dd_gemm_bf16_rows(const void* A, int a_mn, long long lda, long long s
 // Into how many parts dd_gemm_bf16_split should cut the contraction (1: not at all).  A GEMM with few output tiles
 // leaves SMs idle while each of its own walks all of K, and an SM takes in no more than about 85 GB/s, so that even
 // the read of the weights goes at a fifth of the memory rate with 16 tiles.  The parts run as a batch of the same
-// kernels into an fp32 workspace.  Measured: 33 x 4096 x 14336 split 8 ways 85.5 -> 29.0 us, 300 x 1600 x 6400 5 ways
-// 35.4 -> 19.0 us, 64 x 8 x 4096 16 ways 21.7 -> 9.7 us, error against fp64 2 to 10 times smaller (shorter sums).  A
-// k-block of 64 costs a CTA about 0.36 us, the parts and their sum about 5 us, the second launch 8 us on the host,
-// which a short GEMM does not hide: split from a gain of 8 us beyond both on.
+// kernels into an fp32 workspace.  Measured, each alone and with a cold L2: 33 x 4096 x 14336 split 8 ways 96 -> 42 us,
+// 64 x 8 x 4096 16 ways 29 -> 15, 300 x 1600 x 6400 5 ways 28.7 -> 25.6, error against fp64 2 to 10 times smaller (shorter
+// sums).  A k-block of 64 costs a CTA about 0.36 us, the parts and their sum about 5 us, the second launch 8 us on the host,
+// which a short GEMM does not hide: split from a gain of 8 us beyond both on.  A k-block of half tiles costs a pair 0.20 us:
+// nothing is split whose parts gain nothing over the product that takes them (1000 x 2048 x 14336, parts of whole tiles:
+// 55.3 us, 2 ways 58.3; 512 x 4096 x 11264 51.2, 2 ways 54.2).
 DD_API int dd_gemm_split(int M, int N, int K) {
   const int sms = current_sm_count(), num_k = K / 64;
   if (K % 64 || M <= 0 || N <= 0) return 1;
   const bool pair = M > BM;
   const long long tiles = (long long)((M + (pair ? 2 * BM - 1 : BM - 1)) / (pair ? 2 * BM : BM)) * ((N + BN - 1) / BN);
   const long long slots = pair ? sms / 2 : sms;
+  long long whole, half;
+  const double block = pair && half_tiles(M, N, 1, false, slots, &whole, &half) ? 0.20 : 0.36;
   int best = 1;
   double best_gain = 8.0;
   for (int s = 2; s <= 16 && tiles * s <= slots && num_k / s >= 4; ++s) {
     if (num_k % s) continue;
-    const double gain = 0.36 * (num_k - num_k / s) - 13.0 - (double)s * M * N * 8.0 / 6e6;
+    const double sum = 5.0 + (double)s * M * N * 8.0 / 6e6, gain = 0.36 * (num_k - num_k / s) - 8.0 - sum;
+    const double part = pair && half_tiles(M, N, s, true, slots, &whole, &half) ? 0.20 : 0.36;
+    if (block * num_k - part * (num_k / s) < sum) continue;
     if (gain > best_gain) { best_gain = gain; best = s; }
   }
   return best;

@@ -292,3 +292,16 @@ def test_rule_of_the_attention_forward():
         return
     for sizes in one + two:
         assert bool(_native.lib().dd_attn_fwd_two_tiles(*sizes)) == (sizes in two), sizes
+
+
+def test_rule_of_split_contractions():
+    """Both sides, at measured sizes: few tiles against a long contraction, but no parts of whole tiles where the product
+    as a whole takes half ones."""
+    import distdl_b200.ops.gemm  # noqa: F401  (declares the entry point)
+    from distdl_b200 import _native
+    if _native.lib().dd_sm_count() != 148:
+        return
+    for sizes in ((33, 4096, 14336), (64, 8, 4096), (300, 1600, 6400), (1000, 512, 14336), (200, 1024, 8192)):
+        assert _native.lib().dd_gemm_split(*sizes) > 1, sizes
+    for sizes in ((1000, 2048, 14336), (512, 4096, 11264), (700, 1600, 11264), (256, 6144, 14336), (128, 4096, 4096)):
+        assert _native.lib().dd_gemm_split(*sizes) == 1, sizes
