@@ -14,8 +14,9 @@
 // counter per query tile says how many have been added; key tile j adds its part when it says j.  The first one stores
 // (nothing has to be cleared), the last one adds what is there to its own part, scales and writes bf16.  CTAs take
 // their key tile from a ticket, in the order of the counters, so that whoever is waited for has started before; every
-// CTA sweeps the query tiles in the same (descending) order, so that the CTAs of a head follow one another at the
-// distance of one hand-off (1.5 us) and wait only at the start.
+// CTA sweeps the query tiles in the same (descending) order, so that the CTAs of a head follow one another at the distance
+// of one hand-over.  Causal sweeps grow shorter by a tile from one CTA to the next, which hides most of it; full ones do not:
+// 8 heads of 128, 4, 8 and 16 key tiles that start together, each call alone: causal 34, 54 and 87 us, full 60, 114 and 214.
 //
 // Every wait is bounded; a time-out records a status, tells the CTAs that would wait in turn, and falls through to
 // the release of the tensor memory.
@@ -52,7 +53,8 @@ static_assert(REGS_ISSUE + SOFTMAX_WARPS / 4 * REGS_SOFTMAX + REGS_DRAIN <= REGS
 constexpr int Q_STAGES = ROOMY ? 3 : 2, DO_STAGES = ROOMY ? 2 : 1, DS_BUFS = ROOMY ? 2 : 1;
 // dQ leaves in chunks of 32 columns through two buffers in shared memory, as bulk reductions: the TMA unit does them
 // beside the softmax warps' accesses, where 16-byte reductions from registers took 3 200 clocks a tile at D = 128 and
-// held up every other access of the SM (6 900 us instead of 5 780 at 1 x 16384, 32 / 8 heads of 128, causal).
+// held up every other access of the SM (at 1 x 16384, 32 / 8 heads of 128, causal, 6 900 us where bulk reductions took 5 780,
+// both in one run on a card below its power limit; the kernel as it is now takes 6 440 back to back, at the limit).
 constexpr int CHUNK_BYTES = BT * 32 * 4, CHUNKS = D / 32;
 static_assert(CHUNKS % 2 == 0, "a tile starts with the first buffer");
 
