@@ -99,6 +99,17 @@ bool half_tiles(int M, int N, int batch, bool f32, long long pairs, long long* w
   *half = rows_of_tiles * ((N + 127) / 128);
   return f32 ? *half <= pairs : (*half + pairs - 1) / pairs * 125 < (*whole + pairs - 1) / pairs * 200;
 }
+
+// Order of a pair kernel's tiles of 256 x 256 (see tile_coords).  Large products run at the power limit, where each byte
+// that is read again from memory costs clock: a panel of the operand with fewer rows is kept in L2 (up to 36 MB of it; 67
+// MB no longer stay) while the other one streams past it, but at least 8 tiles wide, so that the tiles in flight are about
+// square.  In us, back to back, 4 rows before -> now: 8192 x 28672 x 4096 1634 -> 1425 (8 rows 1527), 4096 x 50304 x 1600
+// 570 -> 517, 3000 x 32000 x 2048 341 -> 311; 8192 x 4096 x 28672 1619 -> 1511 by columns (8 rows 1529).
+int tile_group(int M, int N, int K) {
+  const int tiles = (min(M, N) + 255) / 256;
+  const int g = min(tiles, max(8, (int)(36000000ll / (512ll * K))));
+  return M <= N ? g : -g;
+}
 }  // namespace
 
 // D[b,m,n] (+)= sum_k A[b,m,k] B[b,n,k] (+ bias[n]);  bf16 operands, fp32 accumulation.
@@ -140,7 +151,10 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
     int err2 = 0;
     Params q;
     q.M = M; q.N = N; q.K = K; q.batch = batch;
-    q.D = D; q.ldd = ldd; q.strideD = strideD; q.bias = bias; q.flags = flags; q.group_m = 4;
+    q.D = D; q.ldd = ldd; q.strideD = strideD; q.bias = bias; q.flags = flags;
+    // (four rows: half tiles, 4096 x 1600 x 6400 76 us and 79 to 83 in the other orders; rows without work, so that the
+    // last ones of all columns come together and every pair gets its share of the live ones, 966 us and 1027)
+    q.group_m = narrow || (rows != nullptr && !bound_k) ? 4 : tile_group(M, N, K);
     q.status = device_status(&err2);
     q.rows = rows; q.bound_k = bound_k;
     if (err2) return err2;

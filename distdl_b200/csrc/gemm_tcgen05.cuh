@@ -55,7 +55,7 @@ struct Params {
   long long strideD;   // elements between batches
   const void* bias;
   int flags;
-  int group_m;         // tile-order grouping (rows of tiles swept per column sweep)
+  int group_m;         // tile-order grouping: rows of tiles swept per column sweep; -g: g columns per row sweep
   StatusRecord* status;
   // CTA-pair kernel, batched products: A's rows after the first rows[b] (on the device, null = all live) are zero;
   // with bound_k the terms of the contraction after the first rows[b] are.
@@ -77,8 +77,15 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
   const int per_batch = tiles_m * tiles_n;
   tb = tile / per_batch;
   int t = tile - tb * per_batch;
-  // grouped ordering: sweep group_m tile-rows for each tile-column, so that a
-  // wave of CTAs shares A rows and B columns in L2.
+  // grouped ordering: sweep group_m tile-rows for each tile-column (or -group_m tile-columns for each
+  // tile-row), so that a wave of CTAs shares A rows and B columns in L2.
+  if (group_m < 0) {
+    const int gs = -group_m * tiles_m, g = t / gs, r = t - g * gs;
+    const int first_n = -g * group_m, cols = min(-group_m, tiles_n - first_n);
+    tm = r / cols;
+    tn = first_n + r - tm * cols;
+    return;
+  }
   const int group_size = group_m * tiles_n;
   const int g = t / group_size;
   const int first_m = g * group_m;
