@@ -2,6 +2,7 @@
 #include <cstdlib>
 
 #include "gemm2_tcgen05.cuh"
+#include "gemm4_tcgen05.cuh"
 #include <cstring>
 
 #include "gemm_tcgen05.cuh"
@@ -39,6 +40,22 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
     configured[dev & 63] = true;
   }
   kern<<<grid, dd::gemm2::NUM_THREADS, bytes, stream>>>(ta, tb, td, p);
+  return (int)cudaGetLastError();
+}
+
+template <bool A_MN, bool B_MN>
+int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p,
+                const dd::gemm4::Plan& plan, int grid, cudaStream_t stream) {
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  auto kern = dd::gemm4::gemm4_bf16_kernel<A_MN, B_MN>;
+  if (!configured[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dd::gemm4::SMEM);
+    if (e != cudaSuccess) return (int)e;
+    configured[dev & 63] = true;
+  }
+  kern<<<grid, dd::gemm4::NUM_THREADS, dd::gemm4::SMEM, stream>>>(ta, tb, td, p, plan);
   return (int)cudaGetLastError();
 }
 
@@ -173,6 +190,22 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
                : get_tensor_map_bf16_3d(&pd, D, N, M, batch, ldd * 2, strideD * 2, 64, 32);
       if (rr) return rr;
       q.flags |= F_TMA_EPI;
+    }
+    // Tiles of 512 x 256 (gemm4_tcgen05.cuh) for at least a whole wave of them.  They bring a quarter less through L2, but
+    // pairs wait for the epilogue between tiles, and the order of tiles that keeps a panel in L2 is at its best with the
+    // smaller ones where the contraction is short.  In us, back to back, 256 rows -> 512 rows: K = 1600: 4096 x 50304
+    // 515 -> 531; K = 4096: 8192 x 28672 1441 -> 1448; K = 8192: 8192 x 8192 895 -> 842, weight gradient 28672 x 4096
+    // 1649 -> 1533; K = 14336: 8192 x 4096 768 -> 741; K = 128256: 8192 x 4096 7756 -> 6838.
+    if (!narrow && rows == nullptr && (q.flags & F_TMA_EPI) && K > 4096 && M > 256) {
+      const dd::gemm4::Plan w = dd::gemm4::make_plan(M, N, batch, ctas / 2);
+      if (w.full > 0) {
+        q.group_m = M <= N ? 8 : -16;
+        const int wgrid = 2 * (w.items < ctas / 2 ? w.items : ctas / 2);
+        if (a_mn && b_mn) return launch_wide<true, true>(pa, pb, pd, q, w, wgrid, ps);
+        if (a_mn) return launch_wide<true, false>(pa, pb, pd, q, w, wgrid, ps);
+        if (b_mn) return launch_wide<false, true>(pa, pb, pd, q, w, wgrid, ps);
+        return launch_wide<false, false>(pa, pb, pd, q, w, wgrid, ps);
+      }
     }
     if (narrow) {
       if (a_mn && b_mn) return launch_pair<true, true, 128>(pa, pb, pd, q, pgrid, ps);

@@ -256,3 +256,48 @@ def test_batched_gemm_with_half_tiles(B, M, N, K, a_mn, b_mn):
     gemm(a, b, out=acc, accumulate=True)
     assert (acc.double() - want - before).norm() < 1e-5 * (want + before).norm()
     assert _native.read_status()[0] == 0
+
+
+@pytest.mark.parametrize("B,M,N,K,ctas", [(1, 257, 200, 4104, 2), (1, 512, 456, 4160, 4), (1, 1000, 520, 4168, 4),
+                                          (3, 1288, 456, 4224, 6), (1, 5120, 1280, 4104, 0)])
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_gemm_with_wide_tiles(B, M, N, K, ctas, a_mn, b_mn):
+    """Contractions beyond 4096 take 512 x 256 per pair of CTAs: an odd number of 256-row blocks, a last wave in single
+    blocks, remainders in every direction, both majors.  bf16 results as above; fp32 sums of 16 terms, 264 of them cut
+    off at 2**-23, are off by less than 264 / 2 * 2**-23 = 1.6e-5."""
+    from distdl_b200 import _native
+    from distdl_b200.ops import gemm
+    torch.manual_seed(7)
+
+    def make(rows, cols, mn):
+        n, m = (cols, rows) if mn else (rows, cols)
+        st = torch.randn(B, n, (m + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)[:, :, :m]
+        st = st.transpose(1, 2) if mn else st
+        return st[0] if B == 1 else st
+    a, b = make(M, K, a_mn), make(N, K, b_mn)
+    bias = torch.randn(N, device="cuda", dtype=torch.bfloat16)
+    want = a.double() @ b.double().transpose(-1, -2)
+    out = torch.full((*a.shape[:-1], N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm(a, b, out=out[..., :N], bias=bias, max_ctas=ctas)
+    assert (out[..., :N].double() - want - bias.double()).norm() < 2.5e-3 * want.norm()
+    assert (out[..., N:] == 7).all()
+    acc = torch.randn(*a.shape[:-1], N, device="cuda")
+    before = acc.double()
+    gemm(a, b, out=acc, accumulate=True, max_ctas=ctas)
+    assert (acc.double() - want - before).norm() < 2e-5 * want.norm()
+    bias = torch.randn(N, device="cuda")
+    gemm(a, b, out=acc, bias=bias, max_ctas=ctas)
+    assert (acc.double() - want - bias.double()).norm() < 2e-5 * want.norm()
+    assert _native.read_status()[0] == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(2600, 2312, 64), (2312, 2600, 64), (2312, 2312, 5000)])
+def test_gemm_tile_order_covers_every_tile(M, N, K):
+    """Tiles by panels of rows and of columns, the last panel narrower than the others."""
+    from distdl_b200.ops import gemm
+    torch.manual_seed(9)
+    a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
+    out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    want = a.double() @ b.double().t()
+    assert (gemm(a, b, out=out).double() - want).norm() < 2.5e-3 * want.norm()
