@@ -169,9 +169,8 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
     Params q;
     q.M = M; q.N = N; q.K = K; q.batch = batch;
     q.D = D; q.ldd = ldd; q.strideD = strideD; q.bias = bias; q.flags = flags;
-    // (four rows: half tiles, 4096 x 1600 x 6400 76 us and 79 to 83 in the other orders; rows without work, so that the
-    // last ones of all columns come together and every pair gets its share of the live ones, 966 us and 1027)
-    q.group_m = narrow || (rows != nullptr && !bound_k) ? 4 : tile_group(M, N, K);
+    // (four rows of half tiles: 4096 x 1600 x 6400 76 us, 79 to 83 in the other orders)
+    q.group_m = narrow ? 4 : tile_group(M, N, K);
     q.status = device_status(&err2);
     q.rows = rows; q.bound_k = bound_k;
     if (err2) return err2;
@@ -195,8 +194,10 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
     // pairs wait for the epilogue between tiles, and the order of tiles that keeps a panel in L2 is at its best with the
     // smaller ones where the contraction is short.  In us, back to back, 256 rows -> 512 rows: K = 1600: 4096 x 50304
     // 515 -> 531; K = 4096: 8192 x 28672 1441 -> 1448; K = 8192: 8192 x 8192 895 -> 842, weight gradient 28672 x 4096
-    // 1649 -> 1533; K = 14336: 8192 x 4096 768 -> 741; K = 128256: 8192 x 4096 7756 -> 6838.
-    if (!narrow && rows == nullptr && (q.flags & F_TMA_EPI) && K > 4096 && M > 256) {
+    // 1649 -> 1533; K = 14336: 8192 x 4096 768 -> 741; K = 128256: 8192 x 4096 7756 -> 6838.  Entries with live rows take them at
+    // any K, because only this kernel deals the live blocks out evenly (figures there).
+    const bool by_rows = rows != nullptr && !bound_k;
+    if (!narrow && (q.flags & F_TMA_EPI) && (by_rows || (rows == nullptr && K > 4096)) && M > 256) {
       const dd::gemm4::Plan w = dd::gemm4::make_plan(M, N, batch, ctas / 2);
       if (w.full > 0) {
         q.group_m = M <= N ? 8 : -16;

@@ -291,6 +291,23 @@ def test_gemm_with_wide_tiles(B, M, N, K, ctas, a_mn, b_mn):
     assert _native.read_status()[0] == 0
 
 
+@pytest.mark.parametrize("counts", [(0, 1, 256, 257), (512, 513, 768, 1000), (1000, 0, 0, 999), (0, 0, 0, 0)])
+def test_wide_tiles_skip_zero_rows(counts):
+    """The same tiles with rows that are known to be zero: counts on and off the edges of blocks and tiles."""
+    from distdl_b200 import _native
+    from distdl_b200.ops import gemm
+    torch.manual_seed(8)
+    E, C, K, N = len(counts), 1000, 4168, 2824                 # 2 x 12 x 4 tiles: a whole wave and 22 in single blocks
+    rows = torch.tensor(counts, dtype=torch.int32, device="cuda")
+    keep = (torch.arange(C, device="cuda")[None] < rows[:, None])[..., None]
+    x = torch.where(keep, torch.randn(E, C, K, device="cuda"), torch.zeros((), device="cuda")).bfloat16()
+    w = torch.randn(E, N, K, device="cuda", dtype=torch.bfloat16)
+    for dt in (torch.bfloat16, torch.float32):
+        out = torch.full((E, C, N), float("nan"), device="cuda", dtype=dt)
+        assert torch.equal(gemm(x, w, out=out, rows=rows), gemm(x, w, out_dtype=dt))
+    assert _native.read_status()[0] == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(2600, 2312, 64), (2312, 2600, 64), (2312, 2312, 5000)])
 def test_gemm_tile_order_covers_every_tile(M, N, K):
     """Tiles by panels of rows and of columns, the last panel narrower than the others."""
