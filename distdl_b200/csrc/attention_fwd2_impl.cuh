@@ -110,6 +110,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bar->tmem_base;
+  grid_dependency_launch();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------

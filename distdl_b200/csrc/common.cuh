@@ -86,6 +86,13 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Programmatic dependent launch (launch_ahead in runtime.cuh).  wait: everything that was launched before has completed and
+// can be seen; nothing in global memory is read or written before it, and nothing through the read-only path after it (the
+// kernel may have started before that was written).  launch: the next kernel of the stream, if it is
+// launched ahead, may start where SMs become free (it waits in its turn).
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------- mbarrier ----------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

@@ -100,6 +100,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 __nv_bfloat16* __restrict__ xsum, const __nv_bfloat16* __restrict__ w,
                 const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y, float2* __restrict__ stats,
                 int rows, int d, float eps) {
+  grid_dependency_launch();
   __shared__ float red[kNormWarps * R];
   const int nvec = d >> 3;
   const float inv_d = 1.f / (float)d;
@@ -229,6 +230,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
                 const __nv_bfloat16* __restrict__ w, const float2* __restrict__ stats,
                 const __nv_bfloat16* __restrict__ dres_in, __nv_bfloat16* __restrict__ dx,
                 float* __restrict__ partial, int rows, int d) {
+  grid_dependency_launch();
   __shared__ float red[kNormWarps * 2 * R];
   const int nvec = d >> 3;
   const float inv_d = 1.f / (float)d;
@@ -379,6 +381,7 @@ __device__ __forceinline__ float fold_lane(const float* __restrict__ src, int np
 __global__ void __launch_bounds__(kRedCols * kRedLanes)
 norm_bwd_reduce_kernel(const float* __restrict__ partial, int nparts, int d,
                        float* __restrict__ dw, float* __restrict__ db, int accumulate) {
+  grid_dependency_launch();
   __shared__ float s_w[kRedLanes][kRedCols + 1], s_b[kRedLanes][kRedCols + 1];
   const int col = threadIdx.x, lane = threadIdx.y;
   const int c = blockIdx.x * kRedCols + col;
@@ -399,6 +402,7 @@ norm_bwd_reduce_kernel(const float* __restrict__ partial, int nparts, int d,
 // ---------------------------------------------------------------------------
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                                   long long rows, int F) {
+  grid_dependency_launch();
   const int fv = F >> 3;
   const long long total = rows * fv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -415,6 +419,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
 }
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ gu,
                                   __nv_bfloat16* __restrict__ dgu, long long rows, int F) {
+  grid_dependency_launch();
   const int fv = F >> 3;
   const long long total = rows * fv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -449,6 +454,7 @@ __device__ __forceinline__ float gelu_grad_f(float x) {
 }
 __global__ void gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                                 long long nvec) {
+  grid_dependency_launch();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec;
        i += (long long)gridDim.x * blockDim.x) {
     float a[8], o[8];
@@ -460,6 +466,7 @@ __global__ void gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat
 }
 __global__ void gelu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                 __nv_bfloat16* __restrict__ dx, long long nvec) {
+  grid_dependency_launch();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec;
        i += (long long)gridDim.x * blockDim.x) {
     float a[8], g[8], o[8];
@@ -479,6 +486,7 @@ __global__ void gelu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv
 // ---------------------------------------------------------------------------
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float2* __restrict__ cs, long long tokens,
                             int seq, int heads_total, int nheads, int hd, float sign) {
+  grid_dependency_launch();
   const int half = hd >> 1;
   const int hv = half >> 3;  // 8-element vectors per half head
   const long long total = tokens * nheads * hv;
@@ -622,6 +630,7 @@ __device__ __forceinline__ void softmax_step(const uint4& u, float& m, float& s)
 __global__ void __launch_bounds__(1024)
 xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
             float* __restrict__ loss, int V, int ld, float grad_scale) {
+  grid_dependency_launch();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   __nv_bfloat16* lr = logits + row * (long long)ld;

@@ -23,8 +23,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int gr
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = true;
   }
-  kern<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, p);
-  return (int)cudaGetLastError();
+  return launch_ahead(kern, grid, NUM_THREADS, SMEM_BYTES, stream, ta, tb, p);
 }
 template <bool A_MN, bool B_MN, int NB>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p, int grid,
@@ -39,8 +38,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = true;
   }
-  kern<<<grid, dd::gemm2::NUM_THREADS, bytes, stream>>>(ta, tb, td, p);
-  return (int)cudaGetLastError();
+  return launch_ahead(kern, grid, dd::gemm2::NUM_THREADS, bytes, stream, ta, tb, td, p);
 }
 
 template <bool A_MN, bool B_MN>
@@ -55,24 +53,24 @@ int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = true;
   }
-  kern<<<grid, dd::gemm4::NUM_THREADS, dd::gemm4::SMEM, stream>>>(ta, tb, td, p, plan);
-  return (int)cudaGetLastError();
+  return launch_ahead(kern, grid, dd::gemm4::NUM_THREADS, dd::gemm4::SMEM, stream, ta, tb, td, p, plan);
 }
 
 // Second half of a split contraction: D (+)= sum_s part[s] (+ bias), the parts in order (the same bits in every
 // run).  Bound by the read of the parts, which the GEMM has just left in L2; four columns per thread.
 __global__ void __launch_bounds__(256)
-split_reduce_kernel(const float* __restrict__ part, int split, long long part_stride, int ldw, const Params p) {
+split_reduce_kernel(const float* part, int split, long long part_stride, int ldw, const Params p) {
   const int quads = ldw >> 2;
   const long long total = (long long)p.M * quads;
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  grid_dependency_wait();
   if (i >= total) return;
   const int row = (int)(i / quads), col = (int)(i - (long long)row * quads) * 4;
   const float* src = part + (long long)row * ldw + col;
-  float4 s = __ldg(reinterpret_cast<const float4*>(src));
+  float4 s = *reinterpret_cast<const float4*>(src);
 #pragma unroll 4
   for (int k = 1; k < split; ++k) {
-    const float4 t = __ldg(reinterpret_cast<const float4*>(src + k * part_stride));
+    const float4 t = *reinterpret_cast<const float4*>(src + k * part_stride);
     s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
   }
   float v[4] = {s.x, s.y, s.z, s.w};
@@ -81,8 +79,8 @@ split_reduce_kernel(const float* __restrict__ part, int split, long long part_st
   for (int j = 0; j < 4; ++j) {
     if (col + j >= p.N) break;
     if (p.flags & F_BIAS)
-      v[j] += (p.flags & F_BIAS_F32) ? __ldg(reinterpret_cast<const float*>(p.bias) + col + j)
-                                     : __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(p.bias) + col + j));
+      v[j] += (p.flags & F_BIAS_F32) ? reinterpret_cast<const float*>(p.bias)[col + j]
+                                     : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col + j]);
   }
   const long long at = (long long)row * p.ldd + col;
   const bool vec = col + 4 <= p.N && p.ldd % 4 == 0 && (reinterpret_cast<uintptr_t>(p.D) & 15) == 0;
@@ -312,7 +310,6 @@ DD_API int dd_gemm_bf16_split(const void* A, int a_mn, long long lda, const void
   p.M = M; p.N = N; p.K = K; p.batch = 1;
   p.D = D; p.ldd = ldd; p.strideD = 0; p.bias = bias; p.flags = flags; p.group_m = 1; p.status = nullptr;
   const long long total = (long long)M * (ldw / 4);
-  split_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      ws, split, (long long)M * ldw, ldw, p);
-  return (int)cudaGetLastError();
+  return launch_ahead(split_reduce_kernel, (unsigned)((total + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream),
+                      ws, split, (long long)M * ldw, ldw, p);
 }

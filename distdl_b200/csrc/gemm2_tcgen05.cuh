@@ -163,12 +163,12 @@ __device__ __forceinline__ void epilogue_tma(const Params& q, const CUtensorMap*
           const float* bp = reinterpret_cast<const float*>(q.bias) + col0;
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (i < nv) r[i] = __float_as_uint(__uint_as_float(r[i]) + __ldg(bp + i));
+            if (i < nv) r[i] = __float_as_uint(__uint_as_float(r[i]) + bp[i]);
         } else {
           const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(q.bias) + col0;
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (i < nv) r[i] = __float_as_uint(__uint_as_float(r[i]) + __bfloat162float(__ldg(bp + i)));
+            if (i < nv) r[i] = __float_as_uint(__uint_as_float(r[i]) + __bfloat162float(bp[i]));
         }
       }
       if (n_add > 0 && write) {
@@ -238,7 +238,7 @@ __device__ __forceinline__ void pair_tile_coords(int tile, int tiles_m, int tile
 __device__ __forceinline__ int k_blocks(const Params& p, int tm, int tb) {
   int k = p.K;
   if (p.rows != nullptr) {
-    const int live = __ldg(p.rows + tb);
+    const int live = p.rows[tb];
     if (p.bound_k) k = max(0, min(k, live));
     else if (tm * 2 * BM >= live) k = 0;
   }
@@ -278,6 +278,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   cluster_sync();                                   // barriers of both CTAs are initialised
   tc_fence_after();
   const uint32_t tmem_base = ss->tmem_base;
+  grid_dependency_launch();
+  grid_dependency_wait();
 
   if (warp == 0) {
     // ------------------- TMA producer (both CTAs, own slices) -------------------

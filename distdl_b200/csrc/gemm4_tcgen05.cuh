@@ -121,7 +121,7 @@ struct Walk {
         dead = true;
         tb = 0;
       }
-      const int live = min(w.row_blocks, max(0, (__ldg(p.rows + tb) + BLK - 1) / BLK));
+      const int live = min(w.row_blocks, max(0, (p.rows[tb] + BLK - 1) / BLK));
       const int half = live >> 1, odd = live & 1, per = 2 * half + odd;      // slots of two columns
       const int n = dead ? (w.row_blocks - live) * w.tiles_n : per * ((w.tiles_n + 1) >> 1);
       if (at >= base + n) {
@@ -164,14 +164,14 @@ __device__ __forceinline__ void add_bias(const Params& q, int col0, uint32_t (&r
     const float* bp = reinterpret_cast<const float*>(q.bias) + col0;
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      if (i < nv) r[i] = __float_as_uint(__uint_as_float(r[i]) + __ldg(bp + i));
+      if (i < nv) r[i] = __float_as_uint(__uint_as_float(r[i]) + bp[i]);
     return;
   }
   const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(q.bias) + col0;
   if (nv == 32 && (reinterpret_cast<uintptr_t>(bp) & 15) == 0) {
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-      const uint4 u = __ldg(reinterpret_cast<const uint4*>(bp) + g);
+      const uint4 u = reinterpret_cast<const uint4*>(bp)[g];
       const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -184,7 +184,7 @@ __device__ __forceinline__ void add_bias(const Params& q, int col0, uint32_t (&r
   }
 #pragma unroll
   for (int i = 0; i < 32; ++i)
-    if (i < nv) r[i] = __float_as_uint(__uint_as_float(r[i]) + __bfloat162float(__ldg(bp + i)));
+    if (i < nv) r[i] = __float_as_uint(__uint_as_float(r[i]) + __bfloat162float(bp[i]));
 }
 
 // 128 bytes per row (w[0 .. 31] of lane = row) through the warp's box to columns col0 .. of D.
@@ -288,6 +288,8 @@ gemm4_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   cluster_sync();                                   // barriers of both CTAs are initialised
   tc_fence_after();
   const uint32_t tmem_base = ss->tmem_base;
+  grid_dependency_launch();
+  grid_dependency_wait();
 
   if (warp == 0) {
     // ------------------- TMA producer (both CTAs, own slices) -------------------

@@ -106,12 +106,12 @@ __device__ __forceinline__ void store_chunk(const Params& p, uint32_t (&acc)[32]
       const float* b = reinterpret_cast<const float*>(p.bias) + col0;
 #pragma unroll
       for (int i = 0; i < 32; ++i)
-        if (i < ncols_valid) v[i] += __ldg(b + i);
+        if (i < ncols_valid) v[i] += b[i];
     } else {
       const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(p.bias) + col0;
 #pragma unroll
       for (int i = 0; i < 32; ++i)
-        if (i < ncols_valid) v[i] += __bfloat162float(__ldg(b + i));
+        if (i < ncols_valid) v[i] += __bfloat162float(b[i]);
     }
   }
   if (p.flags & F_OUT_F32) {
@@ -197,6 +197,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ss->tmem_base;
+  grid_dependency_launch();
+  grid_dependency_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------

