@@ -12,6 +12,7 @@
 // with s = 1 / scale_factor (or in / out); nearest takes floor(i * s).
 // Counterpart of the reference's CPU-only C++ extension
 // (src/distdl/functional/interpolate/src/*.cpp).
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <type_traits>
@@ -249,7 +250,7 @@ __device__ inline A adjoint_weight(const InterpGeom& g, int d, int o, int i) {
 // Outputs that may take input i of dimension d: the inverse of the source coordinate at i - 1 and i + 1
 // with one output of slack on either side (rounding), the tail for the last input (coordinates beyond it are
 // clamped to it), clipped to the local outputs.
-__device__ inline void adjoint_candidates(const InterpGeom& g, int d, int i, int& lo, int& hi) {
+__host__ __device__ inline void adjoint_candidates(const InterpGeom& g, int d, int i, int& lo, int& hi) {
   const int ig = i + g.x_off[d], n_in = g.in_global[d], n_out = g.out_global[d];
   double step = g.scale[d], shift = 0.0;
   if (g.linear && g.align_corners) step = n_out > 1 ? (double)(n_in - 1) / (double)(n_out - 1) : 0.0;
@@ -304,14 +305,14 @@ __device__ __forceinline__ int adjoint_taps(const InterpGeom& g, int d, int i, i
   return n > K ? -1 : n > 0 ? n : 0;
 }
 
-// K: outputs per dimension whose weights a thread keeps: up to four in registers, unrolled, from a table that the
+// K: outputs per dimension whose weights a thread keeps: up to five in registers, unrolled, from a table that the
 // CTA fills together, as a window of outputs whose rows and columns lie at the same offsets for every thread; 32
 // in a thread's own (local) memory, for scales above two and outputs smaller than the window.
 template <typename T, int ND, int K>
 __global__ void __launch_bounds__(kThreads)
 interp_adjoint_kernel(const InterpGeom g, T* __restrict__ x, const T* __restrict__ y, long long BC) {
   using A = typename Acc<T>::type;
-  constexpr bool TABLE = K <= 4;
+  constexpr bool TABLE = K <= 5;
   constexpr int E = TABLE ? kMaxEntries(kThreads) : 1;
   __shared__ int s_lo[E], s_n[E];
   __shared__ A s_w[TABLE ? K : 1][E];
@@ -404,6 +405,276 @@ interp_adjoint_kernel(const InterpGeom g, T* __restrict__ x, const T* __restrict
   }
 }
 
+// Two and three dimensions march along the leading one (rows, or sheets): what a sheet of the smaller tensor gives is
+// the same for all the positions of the larger one before and behind it, so that a thread that holds one position of the
+// other dimensions reads every sheet once instead of once per output.  What bounded the kernels above there was the
+// number of loads: 8 per output of a volume and 64 per input in the adjoint (up-sampling by 1.5), now 3 and 27.
+// In us, forward: [1, 32, 46^3] -> 69^3 in fp32 51 -> 42, [4, 72, 34^3] -> 68^3 in bf16 277 -> 186, [8, 64, 128, 128] -> 256^2 in
+// bf16 76 -> 57.  The adjoint marches over volumes of 4-byte elements: the first of these 83 -> 58; in bf16 and over rows
+// the loads of a sheet wait for each other more than they save (65 -> 109 for the last), but not where a window of five
+// outputs is 125 of them: the second 407 -> 300 (909 with weights worked out on the way, as all of more than four were).
+constexpr int kLead = 32;            // leading positions per segment, at most
+constexpr long long kMarchFrom = 1 << 20;     // outputs of all planes; below, the tables take longer than the loads (10^3: 3.5 and 6.7 us)
+constexpr int kLeadOut = 5 * kLead + 16;      // outputs that may take the inputs of a segment (adjoint)
+
+struct Segments {
+  int count, len;                    // over the leading positions, blockIdx.z
+};
+
+// dimensions behind the leading one, as the spans above take them
+template <int ND> __device__ __forceinline__ void tail_of(const int* n, int* t) {
+  t[0] = 1;
+  t[1] = ND == 3 ? n[1] : 1;
+  t[2] = n[2];
+}
+
+// V consecutive outputs of one row per thread (V divides the row, so that a pair of bf16 leaves as one word).
+// I: offsets within a plane of x, 32 bits unless a plane is larger than that.
+template <typename T, int ND, int V, typename I>
+__global__ void __launch_bounds__(kThreads)
+interp_fwd_march_kernel(const InterpGeom g, const T* __restrict__ x, T* __restrict__ y, long long BC, const Segments sg) {
+  using A = typename Acc<T>::type;
+  constexpr int LEAD = 3 - ND, NR = ND == 3 ? 2 : 1;
+  __shared__ int s_i[2][kMaxEntries(kThreads * V)];
+  __shared__ A s_w[2][kMaxEntries(kThreads * V)];
+  __shared__ int l_i[2][kLead];
+  __shared__ A l_w[2][kLead];
+  int n[3];
+  tail_of<ND>(g.out_local, n);
+  const long long out_tail = (long long)n[1] * n[2];
+  const long long in_tail = (long long)(ND == 3 ? g.in_local[1] : 1) * g.in_local[2];
+  const Span sp = span_of(n, (int)blockDim.x * V);
+  for (int t = threadIdx.x; t < sp.cols + sp.rows; t += blockDim.x) {
+    int d, o, a[2];
+    span_entry(sp, n, t, d, o);
+    A lam = (A)0;
+    if (ND == 2 && d == 1) { a[0] = a[1] = 0; }                 // (no such dimension behind the leading one)
+    else source_index<A>(g, d, o, a[0], a[1], lam);
+    const A w[2] = {(A)1 - lam, lam};
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const bool in = a[s] >= 0 && a[s] < g.in_local[d];
+      s_i[s][t] = in ? a[s] : 0;
+      s_w[s][t] = in ? w[s] : (A)0;
+    }
+  }
+  __syncthreads();
+  const long long first = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * V;
+  const bool mine = first < out_tail;
+  int entry[3], o[3];
+  span_locate(sp, n, mine ? (int)threadIdx.x * V : 0, entry, o);
+  I at[NR][V][2];
+  Weight<A> wr[NR], wc[V][2];
+  I col[V][2];
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    const int e = entry[2] + v < sp.cols ? entry[2] + v : entry[2] + v - sp.cols;   // (V > 1: the row goes on)
+#pragma unroll
+    for (int s = 0; s < 2; ++s) { col[v][s] = s_i[s][e]; wc[v][s].set(s_w[s][e]); }
+  }
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const I row = ND == 3 ? (I)s_i[r][entry[1]] * g.in_local[2] : (I)0;
+    wr[r].set(ND == 3 ? s_w[r][entry[1]] : (A)1);
+#pragma unroll
+    for (int v = 0; v < V; ++v) { at[r][v][0] = row + col[v][0]; at[r][v][1] = row + col[v][1]; }
+  }
+  const long long xstep = gridDim.y * (in_tail * g.in_local[LEAD]), ystep = gridDim.y * (out_tail * g.out_local[LEAD]);
+  for (int z = blockIdx.z; z < sg.count; z += gridDim.z) {
+    const int o_first = z * sg.len, o_count = min(sg.len, g.out_local[LEAD] - o_first);
+    __syncthreads();
+    for (int t = threadIdx.x; t < o_count; t += blockDim.x) {
+      int a[2];
+      A lam;
+      source_index<A>(g, LEAD, o_first + t, a[0], a[1], lam);
+      const A w[2] = {(A)1 - lam, lam};
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const bool in = a[s] >= 0 && a[s] < g.in_local[LEAD];
+        l_i[s][t] = in ? a[s] : 0;
+        l_w[s][t] = in ? w[s] : (A)0;
+      }
+    }
+    __syncthreads();
+    if (!mine) continue;
+    const T* xb = x + blockIdx.y * (in_tail * g.in_local[LEAD]);
+    T* yb = y + blockIdx.y * (out_tail * g.out_local[LEAD]) + o_first * out_tail + first;
+    for (int left = planes_left(BC); left > 0; --left, xb += xstep, yb += ystep) {
+      A held[2][V];                                  // of the sheets number `sheet`
+      int sheet[2] = {-1, -1};
+      auto fetch = [&](int i, A (&v)[V]) {
+        const T* xs = xb + i * in_tail;
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+          v[j] = (A)0;
+#pragma unroll
+          for (int r = 0; r < NR; ++r) {
+            const A t = wc[j][1].add(wc[j][0].add((A)0, ld(xs + at[r][j][0])), ld(xs + at[r][j][1]));
+            v[j] = ND == 3 ? wr[r].add(v[j], t) : t;
+          }
+        }
+      };
+      T* yo = yb;
+      for (int t = 0; t < o_count; ++t, yo += out_tail) {
+        const int i0 = l_i[0][t], i1 = l_i[1][t];
+        if (i0 != sheet[0]) {
+          if (i0 == sheet[1]) {
+#pragma unroll
+            for (int j = 0; j < V; ++j) held[0][j] = held[1][j];
+          } else {
+            fetch(i0, held[0]);
+          }
+          sheet[0] = i0;
+        }
+        if (i1 != sheet[1]) {
+          if (i1 == i0) {
+#pragma unroll
+            for (int j = 0; j < V; ++j) held[1][j] = held[0][j];
+          } else {
+            fetch(i1, held[1]);
+          }
+          sheet[1] = i1;
+        }
+        Weight<A> w0, w1;
+        w0.set(l_w[0][t]);
+        w1.set(l_w[1][t]);
+        A acc[V];
+#pragma unroll
+        for (int j = 0; j < V; ++j) acc[j] = w1.add(w0.add((A)0, held[0][j]), held[1][j]);
+        if constexpr (V == 2) *reinterpret_cast<uint32_t*>(yo) = dd::pack_bf16x2(acc[0], acc[1]);
+        else st(yo, acc[0]);
+      }
+    }
+  }
+}
+
+// K: outputs per dimension behind the leading one that take an input, at most (as above).
+template <typename T, int K>
+__global__ void __launch_bounds__(kThreads)
+interp_adjoint_march_kernel(const InterpGeom g, T* __restrict__ x, const T* __restrict__ y, long long BC,
+                            const Segments sg) {
+  using A = typename Acc<T>::type;
+  constexpr int E = kMaxEntries(kThreads);
+  __shared__ int s_lo[E], s_n[E];
+  __shared__ A s_w[K][E];
+  __shared__ int l_a[kLeadOut];
+  __shared__ A l_w[2][kLeadOut];
+  int n[3];
+  tail_of<3>(g.in_local, n);
+  const long long in_tail = (long long)n[1] * n[2];
+  const long long out_tail = (long long)g.out_local[1] * g.out_local[2];
+  const int i_first = (int)blockIdx.z * sg.len, i_end = min(i_first + sg.len, g.in_local[0]);
+  int o_first, o_last, skip;
+  adjoint_candidates(g, 0, i_first, o_first, skip);
+  adjoint_candidates(g, 0, i_end - 1, skip, o_last);
+  const int o_count = min(o_last - o_first + 1, kLeadOut);      // (never cut: march_fits)
+  const Span sp = span_of(n, (int)blockDim.x);
+  for (int t = threadIdx.x; t < sp.cols + sp.rows; t += blockDim.x) {
+    int d, i;
+    span_entry(sp, n, t, d, i);
+    A w[K];
+    int lo = 0;
+    const int taps = adjoint_taps<A, K, true>(g, d, i, lo, w);
+    s_lo[t] = lo;
+    s_n[t] = taps;
+#pragma unroll
+    for (int j = 0; j < K; ++j) s_w[j][t] = w[j];
+  }
+  for (int t = threadIdx.x; t < o_count; t += blockDim.x) {
+    int a0, a1;
+    A lam;
+    source_index<A>(g, 0, o_first + t, a0, a1, lam);
+    l_a[t] = a0;
+    l_w[0][t] = (A)1 - lam;
+    l_w[1][t] = a1 == a0 ? (A)0 : lam;
+  }
+  __syncthreads();
+  const long long pos = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (pos >= in_tail) return;
+  int entry[3], i[3];
+  span_locate(sp, n, (int)threadIdx.x, entry, i);
+  const T* yb = y + blockIdx.y * (out_tail * g.out_local[0]);
+  T* xb = x + blockIdx.y * (in_tail * g.in_local[0]) + pos;
+  const long long xstep = gridDim.y * (in_tail * g.in_local[0]), ystep = gridDim.y * (out_tail * g.out_local[0]);
+  if (s_n[entry[2]] < 0 || s_n[entry[1]] < 0) {       // more than K outputs take this position
+    for (int left = planes_left(BC); left > 0; --left, xb += xstep, yb += ystep)
+      for (int il = i_first; il < i_end; ++il) {
+        int from[3], to[3];
+        i[0] = il;
+        for (int d = 0; d < 3; ++d) adjoint_candidates(g, d, i[d], from[d], to[d]);
+        st(xb + il * in_tail, adjoint_any<T>(g, yb, i, from, to));
+      }
+    return;
+  }
+  Weight<A> wc[K], wb[K];
+#pragma unroll
+  for (int c = 0; c < K; ++c) wc[c].set(s_w[c][entry[2]]);
+#pragma unroll
+  for (int b = 0; b < K; ++b) wb[b].set(s_w[b][entry[1]]);
+  yb += o_first * out_tail + (long long)s_lo[entry[1]] * g.out_local[2] + s_lo[entry[2]];
+  for (int left = planes_left(BC); left > 0; --left, xb += xstep, yb += ystep) {
+    A acc0 = (A)0, acc1 = (A)0;                      // of the inputs `cur` and cur + 1
+    int cur = i_first - 1;
+    A ahead[K][K];                                  // of the next sheet, on its way while this one is added up
+    auto fetch = [&](int t) {
+#pragma unroll
+      for (int b = 0; b < K; ++b)
+#pragma unroll
+        for (int c = 0; c < K; ++c) ahead[b][c] = ld(yb + t * out_tail + (long long)b * g.out_local[2] + c);
+    };
+    int t = 0;
+    while (t < o_count && l_a[t] < i_first - 1) ++t;
+    if (t < o_count) fetch(t);
+    for (; t < o_count; ++t) {
+      const int a = l_a[t];
+      while (cur < a && cur < i_end) {
+        if (cur >= i_first) st(xb + cur * in_tail, acc0);
+        acc0 = acc1;
+        acc1 = (A)0;
+        ++cur;
+      }
+      if (cur >= i_end) break;
+      A sum = (A)0;
+      A v[K][K];
+#pragma unroll
+      for (int b = 0; b < K; ++b)
+#pragma unroll
+        for (int c = 0; c < K; ++c) v[b][c] = ahead[b][c];
+      if (t + 1 < o_count) fetch(t + 1);
+#pragma unroll
+      for (int b = 0; b < K; ++b) {
+        A q = (A)0;
+#pragma unroll
+        for (int c = 0; c < K; ++c) q = wc[c].add(q, v[b][c]);
+        sum = wb[b].add(sum, q);
+      }
+      Weight<A> w0, w1;
+      w0.set(l_w[0][t]);
+      w1.set(l_w[1][t]);
+      acc0 = w0.add(acc0, sum);
+      acc1 = w1.add(acc1, sum);
+    }
+    for (; cur < i_end; ++cur) {
+      if (cur >= i_first) st(xb + cur * in_tail, acc0);
+      acc0 = acc1;
+      acc1 = (A)0;
+    }
+  }
+}
+
+// Segments of the leading dimension and groups of planes.  A CTA's tables take as long as tens of sheets, so that a segment
+// is long (kLead) unless that leaves SMs idle, and a CTA walks as many planes as about 2048 threads per SM allow.
+inline dim3 march_grid(long long positions, int lead, long long BC, int threads, Segments& sg) {
+  const long long bx = (positions + threads - 1) / threads;
+  const long long want = 148LL * 2048 / threads;
+  long long segs = std::max((lead + kLead - 1LL) / kLead, std::min((want + bx * BC - 1) / (bx * BC), (long long)(lead / 8)));
+  sg.len = (int)((lead + segs - 1) / segs);
+  sg.count = (lead + sg.len - 1) / sg.len;
+  const long long each = std::max(BC * bx * sg.count / want, 1LL);       // planes of a CTA
+  const long long by = std::min((BC + each - 1) / each, 65535LL);
+  return dim3((unsigned)bx, (unsigned)by, (unsigned)std::min(sg.count, 65535));
+}
+
 // CTAs over positions x groups of planes: about sixteen CTAs per SM in all, so that a thread keeps its indices
 // for as many planes as leave the GPU full
 inline dim3 plane_grid(long long positions, long long BC, int threads) {
@@ -417,6 +688,16 @@ inline int plane_threads(long long positions) {
   return positions >= kThreads ? kThreads : (int)((positions + 31) / 32 * 32);
 }
 
+// Whether the outputs that may take the inputs of a segment fit the adjoint's table: between the ends of the dimension
+// (len + 1) / step and a few, at the last input as many as lie beyond it.
+inline bool march_fits(const InterpGeom& g, const Segments& sg, double step) {
+  if (sg.count > 65535 || !(step > 0.0) || (sg.len + 1) / step + 8.0 > kLeadOut) return false;
+  int lo, hi, skip;
+  adjoint_candidates(g, 0, (sg.count - 1) * sg.len, lo, skip);
+  adjoint_candidates(g, 0, g.in_local[0] - 1, skip, hi);
+  return hi - lo < kLeadOut;
+}
+
 template <typename T, int ND>
 int run_cuda(int adjoint, const InterpGeom& g, T* x, T* y, long long BC, cudaStream_t s) {
   const long long in_plane = (long long)g.in_local[0] * g.in_local[1] * g.in_local[2];
@@ -427,6 +708,25 @@ int run_cuda(int adjoint, const InterpGeom& g, T* x, T* y, long long BC, cudaStr
     // weight zero
     if (in_plane <= 0) return (int)cudaMemsetAsync(y, 0, (size_t)(BC * out_plane) * sizeof(T), s);
     const bool small = in_plane < 0x7fffffffLL;
+    if constexpr (ND >= 2) {
+      if (BC * out_plane >= kMarchFrom) {
+        const long long tail = out_plane / g.out_local[3 - ND];
+        Segments sg;
+        if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+          if (small && g.out_local[2] % 2 == 0 && (reinterpret_cast<uintptr_t>(y) & 3) == 0) {
+            const int t = plane_threads(tail / 2);
+            const dim3 grid = march_grid(tail / 2, g.out_local[3 - ND], BC, t, sg);
+            interp_fwd_march_kernel<T, ND, 2, int><<<grid, t, 0, s>>>(g, x, y, BC, sg);
+            return (int)cudaGetLastError();
+          }
+        }
+        const int t = plane_threads(tail);
+        const dim3 grid = march_grid(tail, g.out_local[3 - ND], BC, t, sg);
+        if (small) interp_fwd_march_kernel<T, ND, 1, int><<<grid, t, 0, s>>>(g, x, y, BC, sg);
+        else       interp_fwd_march_kernel<T, ND, 1, long long><<<grid, t, 0, s>>>(g, x, y, BC, sg);
+        return (int)cudaGetLastError();
+      }
+    }
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
       if (small && g.out_local[2] % 2 == 0 && (reinterpret_cast<uintptr_t>(y) & 3) == 0) {
         const int t = plane_threads(out_plane / 2);
@@ -443,21 +743,41 @@ int run_cuda(int adjoint, const InterpGeom& g, T* x, T* y, long long BC, cudaStr
   if (out_plane <= 0) return (int)cudaMemsetAsync(x, 0, (size_t)(BC * in_plane) * sizeof(T), s);
   // outputs per input and dimension, as a hint: a position that has more takes the slow way by itself
   double per = 1.0;
+  double lead_step = 0.0;
   int least = g.out_local[2];                       // the smallest extent must hold a whole window
-  for (int d = 3 - ND; d < 3; ++d) {
+  for (int d = 2; d >= 3 - ND; --d) {
     if (g.out_local[d] < least) least = g.out_local[d];
     double step = g.scale[d];
     if (g.linear && g.align_corners)
       step = g.out_global[d] > 1 ? (double)(g.in_global[d] - 1) / (double)(g.out_global[d] - 1) : 0.0;
     const double n = step > 0.0 ? std::ceil((g.linear ? 2.0 : 1.0) / step - 1e-9) : (double)g.out_local[d];
     if (n > per) per = n;
+    lead_step = step;
+  }
+  const int K = per <= 2.0 && least >= 2 ? 2 : per <= 3.0 && least >= 3 ? 3 : per <= 4.0 && least >= 4 ? 4
+                : per <= 5.0 && least >= 5 ? 5 : 32;
+  if constexpr (ND == 3) {
+    const long long tail = in_plane / g.in_local[0];
+    const int t = plane_threads(tail);
+    Segments sg;
+    const dim3 grid = march_grid(tail, g.in_local[0], BC, t, sg);
+    if (BC * out_plane >= kMarchFrom && (sizeof(T) >= 4 || K == 5) && K <= 5 && march_fits(g, sg, lead_step)) {
+      if (K == 5) interp_adjoint_march_kernel<T, 5><<<grid, t, 0, s>>>(g, x, y, BC, sg);
+      if constexpr (sizeof(T) >= 4) {
+        if (K == 2)      interp_adjoint_march_kernel<T, 2><<<grid, t, 0, s>>>(g, x, y, BC, sg);
+        else if (K == 3) interp_adjoint_march_kernel<T, 3><<<grid, t, 0, s>>>(g, x, y, BC, sg);
+        else if (K == 4) interp_adjoint_march_kernel<T, 4><<<grid, t, 0, s>>>(g, x, y, BC, sg);
+      }
+      return (int)cudaGetLastError();
+    }
   }
   const int t = plane_threads(in_plane);
   const dim3 grid = plane_grid(in_plane, BC, t);
-  if (per <= 2.0 && least >= 2)      interp_adjoint_kernel<T, ND, 2><<<grid, t, 0, s>>>(g, x, y, BC);
-  else if (per <= 3.0 && least >= 3) interp_adjoint_kernel<T, ND, 3><<<grid, t, 0, s>>>(g, x, y, BC);
-  else if (per <= 4.0 && least >= 4) interp_adjoint_kernel<T, ND, 4><<<grid, t, 0, s>>>(g, x, y, BC);
-  else                 interp_adjoint_kernel<T, ND, 32><<<grid, t, 0, s>>>(g, x, y, BC);
+  if (K == 2)      interp_adjoint_kernel<T, ND, 2><<<grid, t, 0, s>>>(g, x, y, BC);
+  else if (K == 3) interp_adjoint_kernel<T, ND, 3><<<grid, t, 0, s>>>(g, x, y, BC);
+  else if (K == 4) interp_adjoint_kernel<T, ND, 4><<<grid, t, 0, s>>>(g, x, y, BC);
+  else if (K == 5) interp_adjoint_kernel<T, ND, 5><<<grid, t, 0, s>>>(g, x, y, BC);
+  else             interp_adjoint_kernel<T, ND, 32><<<grid, t, 0, s>>>(g, x, y, BC);
   return (int)cudaGetLastError();
 }
 

@@ -204,6 +204,37 @@ def test_interpolation_kernels_over_scales(mode, ac, n_in, n_out, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16])
+@pytest.mark.parametrize("mode,ac,planes,n_in,n_out", [
+    ("linear", False, 700, (35, 41), (70, 81)),          # rows: two segments of outputs, the last one shorter
+    ("linear", True, 90, (34, 17, 9), (68, 34, 18)),     # sheets: nearly half a step, so that five outputs take some inputs
+    ("linear", True, 40, (46, 23, 22), (69, 35, 33)),
+    ("linear", False, 300, (70, 33, 30), (35, 16, 15)),  # fewer outputs than inputs: inputs that none takes
+    ("nearest", False, 120, (33, 10, 9), (99, 21, 10))])
+def test_interpolation_marches_over_large_tensors(mode, ac, planes, n_in, n_out, dtype):
+    """From a million outputs on, a thread walks the sheets of a volume (rows of an image): segments and their ends,
+    sub-ranges of the output, infinities; against the CPU code in fp64 with the bounds of the test above."""
+    from distdl_b200.functional.interpolate import interpolate
+    torch.manual_seed(6)
+    tol = {torch.float32: 2e-6, torch.float64: 1e-13, torch.bfloat16: 8e-3}[dtype]
+    gi, go = list(n_in), list(n_out)
+    lo = [0] * len(gi)
+    hi = [n - 1 for n in go]
+    hi[-1] += go[-1] % 2                                   # an even extent at the end for some: pairs of bf16
+    x = torch.randn(1, planes, *gi).to(dtype)
+    args = (lo, gi, gi, lo, hi, go, None, mode, ac)
+    xc, xg = x.double().clone().requires_grad_(), x.cuda().requires_grad_()
+    yc, yg = interpolate(xc, *args), interpolate(xg, *args)
+    assert (yg.double().cpu() - yc).abs().max() <= tol * yc.abs().max()
+    dy = torch.randn(yc.shape).to(dtype)
+    yc.backward(dy.double())
+    yg.backward(dy.cuda())
+    assert (xg.grad.double().cpu() - xc.grad).abs().max() <= tol * (1 + xc.grad.abs().max())
+    bad = x.clone()
+    bad[:, :, -1] = float("inf")
+    assert torch.equal(interpolate(bad.cuda(), *args).isfinite().cpu(), interpolate(bad.double(), *args).isfinite())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16])
 @pytest.mark.parametrize("mode", ["linear", "nearest"])
 @pytest.mark.parametrize("n_in", [(0,), (0, 5), (4, 0), (0, 3, 4), (3, 0, 4), (3, 4, 0)])
 def test_interpolation_of_an_empty_slab(n_in, mode, dtype):
