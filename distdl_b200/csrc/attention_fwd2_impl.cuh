@@ -19,13 +19,15 @@
 //
 // Issue order per KV block j:  PV_0(j), S_0(j+1), PV_1(j), S_1(j+1); products of
 // one thread execute in order, so S_t(j+1) may overwrite P_t(j) right after PV_t(j)
-// was issued.  Causal: tile t of query pair qp sees blocks 0 .. 2 qp + t.
+// was issued (head dim 64: S_0(j+1), S_1(j+1), PV_0(j), PV_1(j)).  Causal: tile t of query pair qp sees blocks 0 .. 2 qp + t.
 // Any sequence length: rows behind the end of a sequence are read as zeros (the tensor maps end there), keys there are
 // masked in the last block, queries there are not stored, and a pair's second tile may not exist at all.
 // What bounds it: a tile's softmax (1 900 clocks a block, of which the exponentials alone 1 024) and its two products
 // (1 030) follow one another, and two tiles do not fill the tensor cores (56 % active at head dim 128).  So the chain is
 // kept short: the maximum in four chains, two values per fma / add instruction, and P_t V_j starts on three quarters of P_t.
-// Causal 1 x 16384, 32 / 8 heads of 128: 2 083 -> 1 947 us, full 1 x 4096, 16 heads 145 -> 136; head dim 64 1 609 -> 1 591.
+// Causal 1 x 16384, 32 / 8 heads of 128: 2 083 -> 1 947 us, full 1 x 4096, 16 heads 145 -> 136.
+// At head dim 64 P_t has columns of its own (OWN_P), and S_t(j + 1) is formed before P_t(j) V_j: full 1 x 16384, 16 heads
+// 1 609 -> 1 439 us, 8 x 1536 158 -> 142, causal 4 x 1024, 25 heads 43.0 -> 37.7.
 // All waits are bounded; a timeout drains and frees tensor memory.
 namespace DD_FWD2_NS {
 
@@ -33,6 +35,10 @@ constexpr int BQ = 128;
 constexpr int BKV = 128;
 constexpr int D = DD_HEAD_DIM;
 constexpr int KV_STAGES = 2;
+// Head dim 64 leaves half of O_t's columns to P_t, so that S_t(j + 1) need not wait for P_t(j) V_j: the tensor cores form it
+// while the softmax threads work on block j.
+constexpr bool OWN_P = D == 64;
+constexpr int P_COL = OWN_P ? 256 + 64 : 0;       // first column of P_0; P_1 128 further
 constexpr int P_SPLIT = 96;               // P_t V starts when this many columns of P_t are written
 constexpr int NUM_THREADS = 320;
 constexpr int Q_BYTES = BQ * D * 2;       // one query tile
@@ -45,6 +51,7 @@ struct Barriers {
   uint64_t k_full[KV_STAGES], k_empty[KV_STAGES];
   uint64_t v_full[KV_STAGES], v_empty[KV_STAGES];
   uint64_t s_full[2];      // S_t complete (tensor core -> softmax)
+  uint64_t s_free[2];      // S_t read into registers (softmax -> tensor core), 4 warps arrive; where P_t has columns of its own
   uint64_t p_most[2];      // the first P_SPLIT columns of P_t written, S_t consumed (softmax -> tensor core), 4 warps arrive
   uint64_t p_full[2];      // all of P_t written, 4 warps arrive
   uint64_t pv_done[2];     // O_t += P_t V complete
@@ -98,6 +105,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
     for (int t = 0; t < 2; ++t) {
       mbar_init(&bar->s_full[t], 1);
+      mbar_init(&bar->s_free[t], 4);
       mbar_init(&bar->p_most[t], 4);
       mbar_init(&bar->p_full[t], 4);
       mbar_init(&bar->pv_done[t], 1);
@@ -167,7 +175,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         const uint32_t v_addr = smem_u32(sV + st * KV_BYTES);
 #pragma unroll
         for (int kk = from / 16; kk < to / 16; ++kk)      // 16 kv rows = 8 columns of packed P
-          umma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8,
+          umma_f16_ts(tmem_base + 256 + t * 128, tmem_base + P_COL + t * 128 + kk * 8,
                       make_smem_desc_sw128(v_addr + kk * (16 * 128), BKV * 128, 1024), idesc_pv,
                       (j > 0 || kk > 0) ? 1u : 0u);
       };
@@ -176,15 +184,29 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         tc_fence_after();
         issue_S(0, 0);
         if (PAIRS || n1 > 0) issue_S(1, 0);
+        if (OWN_P) umma_commit(&bar->k_empty[0]);
       }
       for (int j = 0; j < blocks && ok; ++j) {
         const int st = j % KV_STAGES;
         const uint32_t ph = (j / KV_STAGES) & 1;
         const int stn = (j + 1) % KV_STAGES;
         const uint32_t phn = ((j + 1) / KV_STAGES) & 1;
+        bool k_next_ready = false;
+        if (OWN_P && j + 1 < blocks) {
+          for (int t = 0; t < 2 && ok; ++t) {
+            if (j + 1 >= (t == 0 ? n0 : n1)) continue;
+            if (!k_next_ready) ok = mbar_wait(&bar->k_full[stn], phn, &bar->abort_flag, p.status, 37);
+            k_next_ready = true;
+            if (ok) ok = mbar_wait(&bar->s_free[t], j & 1, &bar->abort_flag, p.status, 43);
+            if (!ok) break;
+            tc_fence_after();
+            issue_S(t, j + 1);
+          }
+          if (!ok) break;
+          umma_commit(&bar->k_empty[stn]);
+        }
         ok = mbar_wait(&bar->v_full[st], ph, &bar->abort_flag, p.status, 35);
         if (!ok) break;
-        bool k_next_ready = false;
         for (int t = 0; t < 2 && ok; ++t) {
           const int nt = t == 0 ? n0 : n1;
           if (j >= nt) continue;
@@ -197,7 +219,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           tc_fence_after();
           issue_PV(t, j, P_SPLIT, BKV);
           umma_commit(&bar->pv_done[t]);
-          if (j + 1 < nt) {
+          if (!OWN_P && j + 1 < nt) {
             if (!k_next_ready) {
               ok = mbar_wait(&bar->k_full[stn], phn, &bar->abort_flag, p.status, 37);
               if (!ok) break;
@@ -211,7 +233,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         // V_j is free once the products of both tiles are through; K_j was last read by
         // the S products of block j, which precede these commits in issue order
         umma_commit(&bar->v_empty[st]);
-        umma_commit(&bar->k_empty[st]);
+        if (!OWN_P) umma_commit(&bar->k_empty[st]);
       }
     }
   } else {
@@ -221,6 +243,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const int row = quarter * 32 + lane;            // row inside the tile
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
     const uint32_t tS = tmem_base + t * 128 + lane_off;
+    const uint32_t tP = tmem_base + P_COL + t * 128 + lane_off;
     const uint32_t tO = tmem_base + 256 + t * 128 + lane_off;
     const int nt = t == 0 ? n0 : n1;
     const float c = p.scale * 1.4426950408889634f;  // scores are exponentiated base 2
@@ -236,6 +259,11 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       tmem_ld_32x32(tS + 64, *reinterpret_cast<uint32_t(*)[32]>(s + 64));
       tmem_ld_32x32(tS + 96, *reinterpret_cast<uint32_t(*)[32]>(s + 96));
       tmem_ld_wait();
+      if (OWN_P) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar->s_free[t]);
+      }
       float top[4] = {m_ref, -INFINITY, -INFINITY, -INFINITY};      // four chains: one of 128 steps waits for itself
       const bool diag = p.causal && j == 2 * qp + t;
       if (diag || (!PAIRS && (j + 1) * BKV > p.S)) {
@@ -282,7 +310,12 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           sum2[i & 1] = add_f32x2(sum2[i & 1], pack_f32x2(p0, p1));
           packed[i] = pack_bf16x2(p0, p1);
         }
-        tmem_st_32x16(tS + ch * 16, packed);
+        if (OWN_P && ch == 0 && j > 0) {              // P_t(j - 1) has been read
+          ok = mbar_wait(&bar->pv_done[t], (j - 1) & 1, &bar->abort_flag, p.status, 44);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        tmem_st_32x16(tP + ch * 16, packed);
         if (ch == P_SPLIT / 32 - 1) {
           tmem_st_wait();
           tc_fence_before();
@@ -290,6 +323,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           if (lane == 0) mbar_arrive(&bar->p_most[t]);
         }
       }
+      if (!ok) break;
       const float2 sums = unpack_f32x2(add_f32x2(sum2[0], sum2[1]));
       const float lsum = sums.x + sums.y;
       l += lsum;
