@@ -800,6 +800,13 @@ inline int grid_for(long long work, int threads, int cap_mult = 16) {
   if (b < 1) b = 1;
   return (int)b;
 }
+// One vector per thread where tensors are larger than L2 and nothing is carried from one vector to the next: CTAs that end
+// and start keep memory busier than a grid that walks in strides.  In us, strides -> full: AdamW on 6.3e8 values 3 435 -> 3 089
+// (6.23 -> 6.92 TB/s), SwiGLU 8192 x 14336 121 -> 106 and backward 192 -> 172; but 3000 x 5632 16.4 -> 17.5, GELU of 2.6e7 18.4 -> 20.3.
+inline int grid_wide(long long work, int threads) {
+  const long long b = (work + threads - 1) / threads;
+  return b > 32768 ? (int)(b < 0x7fffffffLL ? b : 0x7fffffffLL) : grid_for(work, threads);
+}
 
 }  // namespace
 
@@ -884,22 +891,22 @@ DD_API int dd_norm_bwd(int rms, const void* dy, const void* x, const void* w, co
 
 DD_API int dd_swiglu_fwd(const void* gu, void* out, long long rows, int F, void* stream) {
   if (F % 8) return DD_ERR_BAD_ARG;
-  swiglu_fwd_kernel<<<grid_for(rows * (F / 8), 256), 256, 0, STREAM(stream)>>>(CBF(gu), BF(out), rows, F);
+  swiglu_fwd_kernel<<<grid_wide(rows * (F / 8), 256), 256, 0, STREAM(stream)>>>(CBF(gu), BF(out), rows, F);
   return (int)cudaGetLastError();
 }
 DD_API int dd_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long rows, int F, void* stream) {
   if (F % 8) return DD_ERR_BAD_ARG;
-  swiglu_bwd_kernel<<<grid_for(rows * (F / 8), 256), 256, 0, STREAM(stream)>>>(CBF(dout), CBF(gu), BF(dgu), rows, F);
+  swiglu_bwd_kernel<<<grid_wide(rows * (F / 8), 256), 256, 0, STREAM(stream)>>>(CBF(dout), CBF(gu), BF(dgu), rows, F);
   return (int)cudaGetLastError();
 }
 DD_API int dd_gelu_fwd(const void* x, void* y, long long n, void* stream) {
   if (n % 8) return DD_ERR_BAD_ARG;
-  gelu_fwd_kernel<<<grid_for(n / 8, 256), 256, 0, STREAM(stream)>>>(CBF(x), BF(y), n / 8);
+  gelu_fwd_kernel<<<grid_wide(n / 8, 256), 256, 0, STREAM(stream)>>>(CBF(x), BF(y), n / 8);
   return (int)cudaGetLastError();
 }
 DD_API int dd_gelu_bwd(const void* dy, const void* x, void* dx, long long n, void* stream) {
   if (n % 8) return DD_ERR_BAD_ARG;
-  gelu_bwd_kernel<<<grid_for(n / 8, 256), 256, 0, STREAM(stream)>>>(CBF(dy), CBF(x), BF(dx), n / 8);
+  gelu_bwd_kernel<<<grid_wide(n / 8, 256), 256, 0, STREAM(stream)>>>(CBF(dy), CBF(x), BF(dx), n / 8);
   return (int)cudaGetLastError();
 }
 DD_API int dd_rope(void* qkv, const void* cs, long long tokens, int seq, int heads_total, int nheads, int hd,
@@ -962,7 +969,7 @@ DD_API int dd_adamw(float* master, float* m, float* v, float* grad, void* param_
     return DD_ERR_ALIGN;
   if (reinterpret_cast<uintptr_t>(param_bf16) & 7) return DD_ERR_ALIGN;
   const float bc1 = 1.f - powf(beta1, (float)step), bc2 = 1.f - powf(beta2, (float)step);
-  adamw_kernel<<<grid_for((n + 3) / 4, 256), 256, 0, STREAM(stream)>>>(master, m, v, grad, BF(param_bf16), n, lr,
+  adamw_kernel<<<grid_wide((n + 3) / 4, 256), 256, 0, STREAM(stream)>>>(master, m, v, grad, BF(param_bf16), n, lr,
                                                                       beta1, beta2, eps, wd, bc1, bc2,
                                                                       grad_scale_ptr, grad_scale, zero_grad);
   return (int)cudaGetLastError();
@@ -974,17 +981,17 @@ DD_API int dd_sumsq_f32(const float* x, long long n, float* out, void* stream) {
 }
 DD_API int dd_add_bf16(const void* a, const void* b, void* y, long long n, void* stream) {
   if (n % 8) return DD_ERR_BAD_ARG;
-  add_bf16_kernel<<<grid_for(n / 8, 256), 256, 0, STREAM(stream)>>>(CBF(a), CBF(b), BF(y), n / 8);
+  add_bf16_kernel<<<grid_wide(n / 8, 256), 256, 0, STREAM(stream)>>>(CBF(a), CBF(b), BF(y), n / 8);
   return (int)cudaGetLastError();
 }
 DD_API int dd_cast_f32_bf16(const float* src, void* dst, long long n, float scale, void* stream) {
   if (n <= 0) return DD_OK;
-  cast_f32_bf16_kernel<<<grid_for(n, 256), 256, 0, STREAM(stream)>>>(src, BF(dst), n, scale);
+  cast_f32_bf16_kernel<<<grid_wide(n, 256), 256, 0, STREAM(stream)>>>(src, BF(dst), n, scale);
   return (int)cudaGetLastError();
 }
 DD_API int dd_cast_bf16_f32(const void* src, float* dst, long long n, float scale, int accumulate, void* stream) {
   if (n <= 0) return DD_OK;
-  cast_bf16_f32_kernel<<<grid_for(n, 256), 256, 0, STREAM(stream)>>>(CBF(src), dst, n, scale, accumulate);
+  cast_bf16_f32_kernel<<<grid_wide(n, 256), 256, 0, STREAM(stream)>>>(CBF(src), dst, n, scale, accumulate);
   return (int)cudaGetLastError();
 }
 

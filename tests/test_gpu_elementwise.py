@@ -397,3 +397,26 @@ def test_sum_of_squares_at_any_length_and_address(n, shift):
     sumsq_(x, out)
     want = x.double().pow(2).sum().item() + 2.0
     assert abs(out.item() - want) <= 512 * 2 ** -24 * want
+
+
+def test_wide_grids_match_narrow_ones():
+    """Beyond 32768 CTAs a thread takes one vector: the bits of AdamW and SwiGLU on parts that a grid in strides takes,
+    with a remainder behind the last vector."""
+    from distdl_b200 import ops
+    torch.manual_seed(0)
+    n = 4 * 256 * 32768 + 4 * 256 + 7
+    state = [torch.rand(n, device="cuda") for _ in range(4)] + [torch.zeros(n, device="cuda", dtype=torch.bfloat16)]
+    parts = [t.clone() for t in state]
+    kw = dict(lr=1e-3, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=3, grad_scale=0.5)
+    ops.adamw_step_(*state, **kw)
+    for lo in range(0, n, 1 << 23):
+        ops.adamw_step_(*[t[lo:lo + (1 << 23)] for t in parts], **kw)
+    assert all(torch.equal(a, b) for a, b in zip(state, parts)) and not state[3].any()
+    h = torch.randn(4099, 2 * 16400, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    dy = torch.randn(4099, 16400, device="cuda", dtype=torch.bfloat16)
+    y = ops.swiglu(h)
+    dh, = torch.autograd.grad(y, h, dy)
+    for rows in (slice(0, 1000), slice(3099, 4099)):
+        part = h.detach()[rows].clone().requires_grad_()
+        want = ops.swiglu(part)
+        assert torch.equal(y[rows], want) and torch.equal(dh[rows], torch.autograd.grad(want, part, dy[rows])[0])
