@@ -85,6 +85,8 @@ static bool split_in_one_pass(int nT, int group, long long kv_tiles, int Dh, int
 //   head dim 128, full     1 x 16384, 32: 16190 -> 13422 (16588 -> 13371); but 1 x 4096, 8: 261 -> 489; 1 x 16384, 8: 3113 -> 4063;
 //                          1 x 16384, 32 / 8: 13976 -> 14919 (13897 -> 14790)
 //   one key tile           64 x 128, 16 / 4 of 128: 118 -> 75
+// (The two at head dim 128 take 5 % less since their softmax threads work on two values per instruction: 2 x 4096, 32 / 8, causal
+// 973 -> 922 back to back.)
 // Hence one kernel where no more than a quarter of a head's key tiles start together, at head dim 128 for long sweeps only.
 // `words`: of scratch for the one kernel, on this device.
 DD_API int dd_attn_bwd_one_pass(int batch, int S, int Hq, int Hkv, int Dh, int causal, long long* words) {

@@ -489,6 +489,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const uint32_t ds_row = smem_u32(sdS) + cg * COLS / 64 * (BT * 128) + row * 128;
     const int unit0 = cg * COLS % 64 / 8;
     const float c = p.scale * kLog2e;
+    const uint64_t nc2 = pack_f32x2(-c, -c);
     bool ok = true;
     for (int it = 0; it < iters && ok; ++it) {
       const int st = it % Q_STAGES;
@@ -513,10 +514,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
         for (int g = 0; g < COLS / 4; ++g) {
           const float4 l = L4[g];
-          pr[4 * g] = exp2_mixed<POLY>(fmaf(__uint_as_float(s[4 * g]), c, -l.x), 4 * g);
-          pr[4 * g + 1] = exp2_mixed<POLY>(fmaf(__uint_as_float(s[4 * g + 1]), c, -l.y), 4 * g + 1);
-          pr[4 * g + 2] = exp2_mixed<POLY>(fmaf(__uint_as_float(s[4 * g + 2]), c, -l.z), 4 * g + 2);
-          pr[4 * g + 3] = exp2_mixed<POLY>(fmaf(__uint_as_float(s[4 * g + 3]), c, -l.w), 4 * g + 3);
+          // (two values per instruction, of l - s c: its negation comes with the exponential)
+          const float2 x = unpack_f32x2(fma_f32x2(pack_u32x2(s[4 * g], s[4 * g + 1]), nc2, pack_f32x2(l.x, l.y)));
+          const float2 z = unpack_f32x2(fma_f32x2(pack_u32x2(s[4 * g + 2], s[4 * g + 3]), nc2, pack_f32x2(l.z, l.w)));
+          pr[4 * g] = exp2_mixed<POLY>(-x.x, 4 * g);
+          pr[4 * g + 1] = exp2_mixed<POLY>(-x.y, 4 * g + 1);
+          pr[4 * g + 2] = exp2_mixed<POLY>(-z.x, 4 * g + 2);
+          pr[4 * g + 3] = exp2_mixed<POLY>(-z.y, 4 * g + 3);
         }
       }
       if (diag) {
@@ -564,10 +568,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           const float4 l = D4[ch / 4 + 2 * g], l2 = D4[ch / 4 + 2 * g + 1];
           const float* q = pr + ch + 8 * g;
           const uint32_t* d = dp + 8 * g;
-          const uint32_t w0 = pack_bf16x2(q[0] * (__uint_as_float(d[0]) - l.x), q[1] * (__uint_as_float(d[1]) - l.y));
-          const uint32_t w1 = pack_bf16x2(q[2] * (__uint_as_float(d[2]) - l.z), q[3] * (__uint_as_float(d[3]) - l.w));
-          const uint32_t w2 = pack_bf16x2(q[4] * (__uint_as_float(d[4]) - l2.x), q[5] * (__uint_as_float(d[5]) - l2.y));
-          const uint32_t w3 = pack_bf16x2(q[6] * (__uint_as_float(d[6]) - l2.z), q[7] * (__uint_as_float(d[7]) - l2.w));
+          const uint32_t w0 = scaled_diff_bf16x2(q[0], q[1], d[0], d[1], l.x, l.y);
+          const uint32_t w1 = scaled_diff_bf16x2(q[2], q[3], d[2], d[3], l.z, l.w);
+          const uint32_t w2 = scaled_diff_bf16x2(q[4], q[5], d[4], d[5], l2.x, l2.y);
+          const uint32_t w3 = scaled_diff_bf16x2(q[6], q[7], d[6], d[7], l2.z, l2.w);
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
                        ::"r"(out + (((unit0 + ch / 8 + g) ^ (row & 7)) << 4)), "r"(w0), "r"(w1), "r"(w2), "r"(w3)
                        : "memory");

@@ -348,6 +348,19 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
   asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t sub_f32x2(uint64_t a, uint64_t b) {
+  return fma_f32x2(b, pack_f32x2(-1.f, -1.f), a);
+}
+// p (d - l) of two values as a pair of bf16
+__device__ __forceinline__ uint32_t scaled_diff_bf16x2(float p0, float p1, uint32_t d0, uint32_t d1, float l0, float l1) {
+  const float2 v = unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1), sub_f32x2(pack_u32x2(d0, d1), pack_f32x2(l0, l1))));
+  return pack_bf16x2(v.x, v.y);
+}
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
