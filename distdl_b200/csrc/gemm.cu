@@ -26,8 +26,10 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int gr
   return launch_ahead(kern, grid, NUM_THREADS, SMEM_BYTES, stream, ta, tb, p);
 }
 template <bool A_MN, bool B_MN, int NB>
-int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p, int grid,
+int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p, int pairs,
                 cudaStream_t stream) {
+  const dd::gemm2::Plan plan = dd::gemm2::make_plan(p.M, p.N, p.batch, pairs, NB);
+  const int grid = 2 * (plan.items < pairs ? plan.items : pairs);
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -38,7 +40,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = true;
   }
-  return launch_ahead(kern, grid, dd::gemm2::NUM_THREADS, bytes, stream, ta, tb, td, p);
+  return launch_ahead(kern, grid, dd::gemm2::NUM_THREADS, bytes, stream, ta, tb, td, p, plan);
 }
 
 template <bool A_MN, bool B_MN>
@@ -105,14 +107,16 @@ split_reduce_kernel(const float* part, int split, long long part_stride, int ldw
 
 // Columns of a pair's tile: 128 where the waves of half tiles are the shorter time.  A half tile costs 1.25 times as
 // much per column (its operands and what TMA brings are 192 bytes of shared memory a clock, a whole one's are 128).
-// Forward, in us, 256 -> 128 columns: 4096 x 1600 x 6400 74.8 -> 69.7, 3000 x 2048 x 5632 67.6 -> 63.5, 512 x 1024 x 512
-// 14.3 -> 11.2; but 4096 x 6400 x 1600 62.4 -> 71.7, 3000 x 11264 x 2048 98 -> 114.  Gradients that are added in fp32
+// Forward, in us, 256 -> 128 columns: 4096 x 1600 x 6400 74.8 -> 69.7, 512 x 1024 x 512 14.3 -> 11.2; 3000 x 2048 x 5632, whose
+// last wave of whole tiles is short enough to be taken in halves, 59 -> 63.5; but 4096 x 6400 x 1600 62.4 -> 71.7, 3000 x 11264 x 2048 98 -> 114.  Gradients that are added in fp32
 // are bound by their epilogue besides (3000 x 2048 x 5632 70.6 -> 79.9): only where there is one wave either way.
 bool half_tiles(int M, int N, int batch, bool f32, long long pairs, long long* whole, long long* half) {
   const long long rows_of_tiles = (long long)((M + 2 * gemm2::BM - 1) / (2 * gemm2::BM)) * batch;
   *whole = rows_of_tiles * ((N + 255) / 256);
   *half = rows_of_tiles * ((N + 127) / 128);
-  return f32 ? *half <= pairs : (*half + pairs - 1) / pairs * 125 < (*whole + pairs - 1) / pairs * 200;
+  const long long rest = *whole % pairs;                       // (a last, short wave of whole tiles is taken in halves)
+  const long long waves = *whole / pairs * 200 + (rest == 0 ? 0 : *whole > pairs && rest * 2 <= pairs ? 125 : 200);
+  return f32 ? *half <= pairs : (*half + pairs - 1) / pairs * 125 < waves;
 }
 
 // Order of a pair kernel's tiles of 256 x 256 (see tile_coords).  Large products run at the power limit, where each byte
@@ -161,7 +165,7 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
     else      rr = get_tensor_map_bf16_3d(&pa, A, K, M, batch, lda * 2, strideA * 2, g2::BK, g2::BM);
     if (rr) return rr;
     if (b_mn) rr = get_tensor_map_bf16_3d(&pb, B, N, K, batch, ldb * 2, strideB * 2, 64, g2::BK);
-    else      rr = get_tensor_map_bf16_3d(&pb, B, K, N, batch, ldb * 2, strideB * 2, g2::BK, narrow ? 64 : g2::BNH);
+    else      rr = get_tensor_map_bf16_3d(&pb, B, K, N, batch, ldb * 2, strideB * 2, g2::BK, 64);
     if (rr) return rr;
     int err2 = 0;
     Params q;
@@ -172,8 +176,6 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
     q.status = device_status(&err2);
     q.rows = rows; q.bound_k = bound_k;
     if (err2) return err2;
-    const long long ptiles = narrow ? half : whole;
-    const int pgrid = 2 * ptiles < ctas ? (int)(2 * ptiles) : ctas;
     cudaStream_t ps = reinterpret_cast<cudaStream_t>(stream);
     // TMA epilogue where the output qualifies: bf16 store, fp32 store or fp32 add
     static const bool tma_epi = []() { const char* e = getenv("DISTDL_GEMM_TMA_EPI"); return !(e && e[0] == '0'); }();
@@ -207,15 +209,15 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
       }
     }
     if (narrow) {
-      if (a_mn && b_mn) return launch_pair<true, true, 128>(pa, pb, pd, q, pgrid, ps);
-      if (a_mn) return launch_pair<true, false, 128>(pa, pb, pd, q, pgrid, ps);
-      if (b_mn) return launch_pair<false, true, 128>(pa, pb, pd, q, pgrid, ps);
-      return launch_pair<false, false, 128>(pa, pb, pd, q, pgrid, ps);
+      if (a_mn && b_mn) return launch_pair<true, true, 128>(pa, pb, pd, q, ctas / 2, ps);
+      if (a_mn) return launch_pair<true, false, 128>(pa, pb, pd, q, ctas / 2, ps);
+      if (b_mn) return launch_pair<false, true, 128>(pa, pb, pd, q, ctas / 2, ps);
+      return launch_pair<false, false, 128>(pa, pb, pd, q, ctas / 2, ps);
     }
-    if (a_mn && b_mn) return launch_pair<true, true, 256>(pa, pb, pd, q, pgrid, ps);
-    if (a_mn) return launch_pair<true, false, 256>(pa, pb, pd, q, pgrid, ps);
-    if (b_mn) return launch_pair<false, true, 256>(pa, pb, pd, q, pgrid, ps);
-    return launch_pair<false, false, 256>(pa, pb, pd, q, pgrid, ps);
+    if (a_mn && b_mn) return launch_pair<true, true, 256>(pa, pb, pd, q, ctas / 2, ps);
+    if (a_mn) return launch_pair<true, false, 256>(pa, pb, pd, q, ctas / 2, ps);
+    if (b_mn) return launch_pair<false, true, 256>(pa, pb, pd, q, ctas / 2, ps);
+    return launch_pair<false, false, 256>(pa, pb, pd, q, ctas / 2, ps);
   }
   CUtensorMap ta, tb;
   int r;

@@ -135,13 +135,13 @@ template <int NB = BN>
 __device__ __forceinline__ void epilogue_tma(const Params& q, const CUtensorMap* map, uint32_t taddr, uint8_t* stage_w,
                                              int lane, int col_tile0, int row0, int tb, bool write,
                                              const __nv_bfloat16* const* add_src = nullptr, int n_add = 0,
-                                             long long add_ld = 0, bool zero = false) {
+                                             long long add_ld = 0, bool zero = false, int columns = NB) {
   const bool f32 = (q.flags & gemm::F_OUT_F32) != 0;
   const bool add = (q.flags & gemm::F_ACCUMULATE) != 0;
   const int round_cols = f32 ? 64 : 128;
   const int box_cols = round_cols / 2;
 #pragma unroll 1
-  for (int rd = 0; rd < NB / round_cols; ++rd) {
+  for (int rd = 0; rd < columns / round_cols; ++rd) {
     const int colr = col_tile0 + rd * round_cols;
     if (colr >= q.N) break;
     if (lane == 0) tma_store_wait_read();
@@ -231,6 +231,36 @@ __device__ __forceinline__ void pair_tile_coords(int tile, int tiles_m, int tile
   gemm::tile_coords(tile, tiles_m, tiles_n, group_m, tm, tn, tb);
 }
 
+// Work items of the pairs.  A last, partial wave that is no more than half a wave is taken in halves of 128 columns (items
+// from `full` on), which end after 0.63 of the time of a whole tile.  Back to back, us: 3000 x 2048 x 2048 (96 tiles on 74 pairs) 27 -> 23,
+// x 5632 65 -> 59, its weight gradient 67 -> 62, 3000 x 2048 x 32000 411 -> 349, weight gradient 6400 x 1600 of 4096 rows 87 -> 81.
+struct Plan {
+  int tiles_m, tiles_n, full, items;
+};
+inline Plan make_plan(int M, int N, int batch, int pairs, int NB) {
+  Plan w;
+  w.tiles_m = (M + 2 * BM - 1) / (2 * BM);
+  w.tiles_n = (N + NB - 1) / NB;
+  const int tiles = w.tiles_m * w.tiles_n * batch, rest = tiles % pairs;
+  w.full = NB == BN && tiles > pairs && rest * 2 <= pairs ? tiles - rest : tiles;
+  w.items = w.full + 2 * (tiles - w.full);
+  return w;
+}
+struct Item {
+  int tm, tn, tb;
+  int col0, columns;             // first column, NB or (from `full` on) half as many; none behind the matrix
+};
+template <int NB>
+__device__ __forceinline__ Item item_at(int j, const Params& p, const Plan& w) {
+  Item it;
+  const int rest = j - w.full;
+  pair_tile_coords(rest < 0 ? j : w.full + (rest >> 1), w.tiles_m, w.tiles_n, p.group_m, it.tm, it.tn, it.tb);
+  it.col0 = it.tn * NB + (rest < 0 ? 0 : (rest & 1) * (NB / 2));
+  it.columns = rest < 0 ? NB : NB / 2;
+  if (it.col0 >= p.N) it.columns = 0;
+  return it;
+}
+
 // Batched products with rows[b] live rows (see Params): a tile without live rows is neither loaded nor
 // multiplied, only its zeros are written, and with bound_k the contraction ends at the last k-block that has live
 // terms.  Eight experts' GEMMs, capacity 1280 for 1024 tokens on average, 4096 x 28672 and 14336 x 4096, forward
@@ -248,7 +278,7 @@ __device__ __forceinline__ int k_blocks(const Params& p, int tm, int tb) {
 template <bool A_MN, bool B_MN, int NB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                  const __grid_constant__ CUtensorMap tmap_d, const Params p) {
+                  const __grid_constant__ CUtensorMap tmap_d, const Params p, const Plan plan) {
   using T = Shape<NB>;
   constexpr int STAGES = T::NSTAGES, STAGE_BYTES = T::BYTES, BN = NB, BNH = T::NBH, TMEM_COLS = T::COLS;
   extern __shared__ uint8_t smem_raw[];
@@ -259,9 +289,6 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();          // 0 = leader
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM);
-  const int tiles_n = (p.N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n * p.batch;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&ss->full[s], 1); mbar_init(&ss->empty[s], 1); }
@@ -289,19 +316,20 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        int tm, tn, tb;
-        pair_tile_coords(tile, tiles_m, tiles_n, p.group_m, tm, tn, tb);
-        const int num_k = k_blocks(p, tm, tb);
-        const int m0 = tm * 2 * BM + (int)rank * BM;
-        const int n0 = tn * BN + (int)rank * BNH;
+      for (int j = pair; j < plan.items && ok; j += num_pairs) {
+        const Item it = item_at<NB>(j, p, plan);
+        if (it.columns == 0) continue;
+        const int tb = it.tb, num_k = k_blocks(p, it.tm, tb);
+        const int boxes = it.columns / 128;                       // of 64 rows of B that this CTA stages
+        const int m0 = it.tm * 2 * BM + (int)rank * BM;
+        const int n0 = it.col0 + (int)rank * (it.columns / 2);
         for (int k = 0; k < num_k; ++k) {
           ok = mbar_wait(&ss->empty[stage], phase ^ 1, &ss->abort_flag, p.status, 301);
           if (!ok) break;
           uint8_t* sa = tiles + stage * STAGE_BYTES;
           uint8_t* sb = sa + A_STAGE_BYTES;
           const uint32_t full_leader = mapa(smem_u32(&ss->full[stage]), 0);
-          if (rank == 0) mbar_expect_tx(&ss->full[stage], 2 * STAGE_BYTES);
+          if (rank == 0) mbar_expect_tx(&ss->full[stage], 2 * (A_STAGE_BYTES + boxes * (64 * BK * 2)));
           if (A_MN) {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j)
@@ -309,12 +337,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           } else {
             tma_load_3d_pair(sa, &tmap_a, full_leader, k * BK, m0, tb);
           }
-          if (B_MN) {
 #pragma unroll
-            for (int j = 0; j < BNH / 64; ++j)
-              tma_load_3d_pair(sb + j * (64 * BK * 2), &tmap_b, full_leader, n0 + j * 64, k * BK, tb);
-          } else {
-            tma_load_3d_pair(sb, &tmap_b, full_leader, k * BK, n0, tb);
+          for (int j = 0; j < BNH / 64; ++j) {
+            if (j >= boxes) break;
+            if (B_MN) tma_load_3d_pair(sb + j * (64 * BK * 2), &tmap_b, full_leader, n0 + j * 64, k * BK, tb);
+            else      tma_load_3d_pair(sb + j * (64 * BK * 2), &tmap_b, full_leader, k * BK, n0 + j * 64, tb);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -327,14 +354,16 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   } else if (warp == 1) {
     // ---------------------------- MMA issuer (leader) ---------------------------
     if (rank == 0 && elect_one()) {
-      constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      constexpr uint32_t idesc_whole = make_idesc_bf16(2 * BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      constexpr uint32_t idesc_half = make_idesc_bf16(2 * BM, BN / 2, A_MN ? 1 : 0, B_MN ? 1 : 0);
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        int tm, tn, tb;
-        pair_tile_coords(tile, tiles_m, tiles_n, p.group_m, tm, tn, tb);
-        const int num_k = k_blocks(p, tm, tb);
+      for (int j = pair; j < plan.items && ok; j += num_pairs) {
+        const Item it = item_at<NB>(j, p, plan);
+        if (it.columns == 0) continue;
+        const int num_k = k_blocks(p, it.tm, it.tb);
+        const uint32_t idesc = it.columns == NB ? idesc_whole : idesc_half;
         if (num_k == 0) continue;                      // (the epilogue writes zeros by itself)
         ok = mbar_wait(&ss->tmem_empty[acc], acc_phase ^ 1, &ss->abort_flag, p.status, 302);
         if (!ok) break;
@@ -369,9 +398,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     bool ok = true;
     const bool vec_ok = ((p.flags & gemm::F_OUT_F32) ? (p.ldd % 4 == 0) : (p.ldd % 8 == 0)) &&
                         ((reinterpret_cast<uintptr_t>(p.D) & 15) == 0) && ((p.strideD % 8) == 0);
-    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-      int tm, tn, tb;
-      pair_tile_coords(tile, tiles_m, tiles_n, p.group_m, tm, tn, tb);
+    for (int j = pair; j < plan.items && ok; j += num_pairs) {
+      const Item it = item_at<NB>(j, p, plan);
+      if (it.columns == 0) continue;
+      const int tm = it.tm, tb = it.tb;
       const bool zero = k_blocks(p, tm, tb) == 0;      // nothing is multiplied for this tile: no accumulator
       if (!zero) {
         ok = mbar_wait(&ss->tmem_full[acc], acc_phase, &ss->abort_flag, p.status, 304);
@@ -382,12 +412,12 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const long long row_off = (long long)tb * p.strideD + (long long)row * p.ldd;
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
       if (p.flags & gemm::F_TMA_EPI) {
-        epilogue_tma<NB>(p, &tmap_d, taddr, out_stage + quarter * OUT_WARP_BYTES, lane, tn * BN,
-                     tm * 2 * BM + (int)rank * BM + quarter * 32, tb, true, nullptr, 0, 0, zero);
+        epilogue_tma<NB>(p, &tmap_d, taddr, out_stage + quarter * OUT_WARP_BYTES, lane, it.col0,
+                     tm * 2 * BM + (int)rank * BM + quarter * 32, tb, true, nullptr, 0, 0, zero, it.columns);
       } else {
 #pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
-          const int col0 = tn * BN + c * 32;
+        for (int c = 0; c < it.columns / 32; ++c) {
+          const int col0 = it.col0 + c * 32;
           if (col0 >= p.N) break;
           uint32_t r[32];
           if (!zero) {

@@ -321,12 +321,10 @@ gemm4_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               tma_load_3d_pair(sa + h * SLICE, &tmap_a, full_leader, k * BK, m0, it.tb);
             }
           }
-          if (B_MN) {
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-              tma_load_3d_pair(sb + i * (SLICE / 2), &tmap_b, full_leader, n0 + i * 64, k * BK, it.tb);
-          } else {
-            tma_load_3d_pair(sb, &tmap_b, full_leader, k * BK, n0, it.tb);
+          for (int i = 0; i < 2; ++i) {                 // boxes of 64 rows or columns
+            if (B_MN) tma_load_3d_pair(sb + i * (SLICE / 2), &tmap_b, full_leader, n0 + i * 64, k * BK, it.tb);
+            else      tma_load_3d_pair(sb + i * (SLICE / 2), &tmap_b, full_leader, k * BK, n0 + i * 64, it.tb);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }

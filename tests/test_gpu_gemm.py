@@ -291,6 +291,35 @@ def test_gemm_with_wide_tiles(B, M, N, K, ctas, a_mn, b_mn):
     assert _native.read_status()[0] == 0
 
 
+@pytest.mark.parametrize("B,M,N,K,ctas", [(1, 256, 640, 136, 4), (1, 513, 264, 200, 8), (1, 1000, 500, 72, 14),
+                                          (3, 300, 256, 64, 10), (1, 2816, 2048, 64, 0), (1, 3000, 2048, 2048, 0)])
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_gemm_whose_last_wave_is_taken_in_halves(B, M, N, K, ctas, a_mn, b_mn):
+    """A last wave of no more than half as many tiles as pairs of CTAs: halves of 128 columns, some of them behind the
+    matrix; bf16 and fp32 results (bounds as above)."""
+    from distdl_b200 import _native
+    from distdl_b200.ops import gemm
+    torch.manual_seed(10)
+
+    def make(rows, cols, mn):
+        n, m = (cols, rows) if mn else (rows, cols)
+        st = torch.randn(B, n, (m + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)[:, :, :m]
+        st = st.transpose(1, 2) if mn else st
+        return st[0] if B == 1 else st
+    a, b = make(M, K, a_mn), make(N, K, b_mn)
+    want = a.double() @ b.double().transpose(-1, -2)
+    for pad in (8, 1):                                   # with TMA stores, and rows that do not start at 16 bytes
+        out = torch.full((*a.shape[:-1], N + pad), 7.0, device="cuda", dtype=torch.bfloat16)
+        gemm(a, b, out=out[..., :N], max_ctas=ctas)
+        assert (out[..., :N].double() - want).norm() < 2.5e-3 * want.norm()
+        assert (out[..., N:] == 7).all()
+    acc = torch.randn(*a.shape[:-1], N, device="cuda")
+    before = acc.double()
+    gemm(a, b, out=acc, accumulate=True, max_ctas=ctas)
+    assert (acc.double() - want - before).norm() < 1e-5 * want.norm()
+    assert _native.read_status()[0] == 0
+
+
 @pytest.mark.parametrize("counts", [(0, 1, 256, 257), (512, 513, 768, 1000), (1000, 0, 0, 999), (0, 0, 0, 0)])
 def test_wide_tiles_skip_zero_rows(counts):
     """The same tiles with rows that are known to be zero: counts on and off the edges of blocks and tiles."""
