@@ -13,7 +13,9 @@ using namespace dd::gemm;
 
 namespace {
 template <bool A_MN, bool B_MN>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int grid, cudaStream_t stream) {
+int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int ctas, cudaStream_t stream) {
+  const Plan plan = make_plan(p.M, p.N, p.batch, ctas);
+  const int grid = plan.items < ctas ? plan.items : ctas;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -23,7 +25,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int gr
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = true;
   }
-  return launch_ahead(kern, grid, NUM_THREADS, SMEM_BYTES, stream, ta, tb, p);
+  return launch_ahead(kern, grid, NUM_THREADS, SMEM_BYTES, stream, ta, tb, p, plan);
 }
 template <bool A_MN, bool B_MN, int NB>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p, int pairs,
@@ -225,7 +227,7 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
   else      r = get_tensor_map_bf16_3d(&ta, A, K, M, batch, lda * 2, strideA * 2, BK, BM);
   if (r) return r;
   if (b_mn) r = get_tensor_map_bf16_3d(&tb, B, N, K, batch, ldb * 2, strideB * 2, 64, BK);
-  else      r = get_tensor_map_bf16_3d(&tb, B, K, N, batch, ldb * 2, strideB * 2, BK, BN);
+  else      r = get_tensor_map_bf16_3d(&tb, B, K, N, batch, ldb * 2, strideB * 2, BK, 64);
   if (r) return r;
 
   int err = 0;
@@ -237,15 +239,13 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
   p.status = device_status(&err);
   if (err) return err;
 
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * batch;
   int ctas = current_sm_count();
   if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
-  const int grid = tiles < ctas ? tiles : ctas;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (a_mn && b_mn) return launch<true, true>(ta, tb, p, grid, s);
-  if (a_mn) return launch<true, false>(ta, tb, p, grid, s);
-  if (b_mn) return launch<false, true>(ta, tb, p, grid, s);
-  return launch<false, false>(ta, tb, p, grid, s);
+  if (a_mn && b_mn) return launch<true, true>(ta, tb, p, ctas, s);
+  if (a_mn) return launch<true, false>(ta, tb, p, ctas, s);
+  if (b_mn) return launch<false, true>(ta, tb, p, ctas, s);
+  return launch<false, false>(ta, tb, p, ctas, s);
 }
 }  // namespace
 

@@ -161,10 +161,41 @@ __device__ __forceinline__ void store_chunk(const Params& p, uint32_t (&acc)[32]
   }
 }
 
+// Work items: the tiles of whole waves, then those of a last, partial wave (or of the only one) in `parts` parts of their
+// columns, as many as there are CTAs for.  Few rows against many columns are bound by the read of B, of which one SM takes in
+// no more than about 85 GB/s.  Back to back, us: 33 x 6144 x 4096 (24 tiles on 148 SMs) 26.8 -> 16.8, 33 x 4096 x 4096 24.6 -> 13.3,
+// 100 x 2048 x 2048 17.5 -> 11.3; but halves behind whole waves, 1 x 128256 x 4096 (501 tiles), 197 -> 204.
+struct Plan {
+  int tiles_m, tiles_n, full, parts, items;
+};
+inline Plan make_plan(int M, int N, int batch, int ctas) {
+  Plan w;
+  w.tiles_m = (M + BM - 1) / BM;
+  w.tiles_n = (N + BN - 1) / BN;
+  const int tiles = w.tiles_m * w.tiles_n * batch, rest = tiles <= ctas ? tiles : tiles % ctas;
+  w.parts = rest * 4 <= ctas ? 4 : rest * 2 <= ctas && tiles <= ctas ? 2 : 1;
+  w.full = tiles - rest;
+  w.items = w.full + w.parts * rest;
+  return w;
+}
+struct Item {
+  int tm, tn, tb;
+  int col0, columns;             // first column and number of columns (none: behind the matrix)
+};
+__device__ __forceinline__ Item item_at(int j, const Params& p, const Plan& w) {
+  Item it;
+  const int rest = j - w.full;
+  tile_coords(rest < 0 ? j : w.full + rest / w.parts, w.tiles_m, w.tiles_n, p.group_m, it.tm, it.tn, it.tb);
+  it.columns = rest < 0 ? BN : BN / w.parts;
+  it.col0 = it.tn * BN + (rest < 0 ? 0 : rest % w.parts * it.columns);
+  if (it.col0 >= p.N) it.columns = 0;
+  return it;
+}
+
 template <bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const Params p) {
+                 const Params p, const Plan plan) {
   extern __shared__ uint8_t smem_raw[];
   // 128B-swizzled tiles must sit on 1024 B boundaries.
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -172,9 +203,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int tiles_m = (p.M + BM - 1) / BM;
-  const int tiles_n = (p.N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n * p.batch;
   const int num_k = (p.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -208,15 +236,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        int tm, tn, tb;
-        tile_coords(tile, tiles_m, tiles_n, p.group_m, tm, tn, tb);
+      for (int j = blockIdx.x; j < plan.items && ok; j += gridDim.x) {
+        const Item it = item_at(j, p, plan);
+        const int tm = it.tm, tb = it.tb, boxes = it.columns / 64;
+        if (boxes == 0) continue;
         for (int k = 0; k < num_k; ++k) {
           ok = mbar_wait(&ss->empty[stage], phase ^ 1, &ss->abort_flag, p.status, 1);
           if (!ok) break;
           uint8_t* sa = tiles + stage * STAGE_BYTES;
           uint8_t* sb = sa + A_STAGE_BYTES;
-          mbar_expect_tx(&ss->full[stage], STAGE_BYTES);
+          mbar_expect_tx(&ss->full[stage], A_STAGE_BYTES + boxes * (64 * BK * 2));
           if (A_MN) {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j)
@@ -224,12 +253,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           } else {
             tma_load_3d(sa, &tmap_a, &ss->full[stage], k * BK, tm * BM, tb);
           }
-          if (B_MN) {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              tma_load_3d(sb + j * (64 * BK * 2), &tmap_b, &ss->full[stage], tn * BN + j * 64, k * BK, tb);
-          } else {
-            tma_load_3d(sb, &tmap_b, &ss->full[stage], k * BK, tn * BN, tb);
+          for (int i = 0; i < BN / 64; ++i) {           // boxes of 64 rows or columns
+            if (i >= boxes) break;
+            if (B_MN) tma_load_3d(sb + i * (64 * BK * 2), &tmap_b, &ss->full[stage], it.col0 + i * 64, k * BK, tb);
+            else      tma_load_3d(sb + i * (64 * BK * 2), &tmap_b, &ss->full[stage], k * BK, it.col0 + i * 64, tb);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -244,13 +272,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   } else if (warp == 1) {
     // ------------------------------- MMA issuer -------------------------------
     if (elect_one()) {
-      constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int j = blockIdx.x; j < plan.items && ok; j += gridDim.x) {
+        const int columns = item_at(j, p, plan).columns;
+        if (columns == 0) continue;
+        const uint32_t idesc = make_idesc_bf16(BM, columns, A_MN ? 1 : 0, B_MN ? 1 : 0);
         ok = mbar_wait(&ss->tmem_empty[acc], acc_phase ^ 1, &ss->abort_flag, p.status, 2);
         if (!ok) break;
         tc_fence_after();
@@ -288,9 +318,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const bool vec_ok = ((p.flags & F_OUT_F32) ? (p.ldd % 4 == 0) : (p.ldd % 8 == 0)) &&
                         ((reinterpret_cast<uintptr_t>(p.D) & 15) == 0) &&
                         ((p.strideD % 8) == 0);
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-      int tm, tn, tb;
-      tile_coords(tile, tiles_m, tiles_n, p.group_m, tm, tn, tb);
+    for (int j = blockIdx.x; j < plan.items && ok; j += gridDim.x) {
+      const Item it = item_at(j, p, plan);
+      const int tm = it.tm, tb = it.tb;
+      if (it.columns == 0) continue;
       ok = mbar_wait(&ss->tmem_full[acc], acc_phase, &ss->abort_flag, p.status, 4);
       if (!ok) break;
       tc_fence_after();
@@ -298,8 +329,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       const long long row_off = (long long)tb * p.strideD + (long long)row * p.ldd;
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        const int col0 = tn * BN + c * 32;
+      for (int c = 0; c < it.columns / 32; ++c) {
+        const int col0 = it.col0 + c * 32;
         if (col0 >= p.N) break;  // uniform across the warp
         uint32_t r[32];
         tmem_ld_32x32(taddr + c * 32, r);

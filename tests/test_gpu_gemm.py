@@ -320,6 +320,33 @@ def test_gemm_whose_last_wave_is_taken_in_halves(B, M, N, K, ctas, a_mn, b_mn):
     assert _native.read_status()[0] == 0
 
 
+@pytest.mark.parametrize("B,M,N,K,ctas", [(1, 33, 1000, 136, 0), (1, 128, 264, 72, 3), (1, 77, 1160, 200, 4), (2, 20, 2312, 64, 4),
+                                          (1, 1, 520, 1600, 12)])
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_gemm_of_few_rows_in_parts_of_tiles(B, M, N, K, ctas, a_mn, b_mn):
+    """One row of tiles: quarters and halves of the only or of the last wave, some behind the matrix (bounds as above)."""
+    from distdl_b200 import _native
+    from distdl_b200.ops import gemm
+    torch.manual_seed(11)
+
+    def make(rows, cols, mn):
+        n, m = (cols, rows) if mn else (rows, cols)
+        st = torch.randn(B, n, (m + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)[:, :, :m]
+        st = st.transpose(1, 2) if mn else st
+        return st[0] if B == 1 else st
+    a, b = make(M, K, a_mn), make(N, K, b_mn)
+    want = a.double() @ b.double().transpose(-1, -2)
+    out = torch.full((*a.shape[:-1], N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm(a, b, out=out[..., :N], max_ctas=ctas)
+    assert (out[..., :N].double() - want).norm() < 2.5e-3 * want.norm()
+    assert (out[..., N:] == 7).all()
+    acc = torch.randn(*a.shape[:-1], N, device="cuda")
+    before = acc.double()
+    gemm(a, b, out=acc, accumulate=True, max_ctas=ctas)
+    assert (acc.double() - want - before).norm() < 1e-5 * want.norm()
+    assert _native.read_status()[0] == 0
+
+
 @pytest.mark.parametrize("counts", [(0, 1, 256, 257), (512, 513, 768, 1000), (1000, 0, 0, 999), (0, 0, 0, 0)])
 def test_wide_tiles_skip_zero_rows(counts):
     """The same tiles with rows that are known to be zero: counts on and off the edges of blocks and tiles."""
