@@ -374,3 +374,40 @@ def test_gemm_tile_order_covers_every_tile(M, N, K):
     out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
     want = a.double() @ b.double().t()
     assert (gemm(a, b, out=out).double() - want).norm() < 2.5e-3 * want.norm()
+
+
+def test_products_launched_ahead_are_ordered_on_streams_and_in_graphs():
+    """A chain of products, each of the one before it, right behind library kernels that write its operands: on a stream of
+    its own, and captured (twice the same bits as one kernel at a time)."""
+    from distdl_b200.ops import gemm, rms_norm
+    torch.manual_seed(12)
+    x = torch.randn(2048, 1024, device="cuda", dtype=torch.bfloat16)
+    ws = [torch.randn(1024, 1024, device="cuda", dtype=torch.bfloat16) / 32 for _ in range(4)]
+    one = torch.ones(1024, device="cuda", dtype=torch.bfloat16)
+
+    def chain(wait):
+        y = x.clone()
+        for i, w in enumerate(ws * 3):
+            y = gemm(y, w if i % 2 else w.t().contiguous().t())
+            wait()
+            y = rms_norm(y, one) if i % 3 == 0 else y.mul(1.25)
+            wait()
+            y = gemm(y[:100], w, out=torch.zeros(2048, 1024, device="cuda", dtype=torch.bfloat16)[:100]) if i == 11 else y
+            wait()
+        return y
+
+    want = chain(torch.cuda.synchronize)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        got = chain(lambda: None)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(lambda: None)
+    for _ in range(3):
+        got.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
