@@ -82,11 +82,20 @@ int run(const void* src, void* dst, const ShiftGeom& g, W fill, cudaStream_t s) 
 
 // ------------------------------------------------------------------ between channels-first and channels-last
 // The same shifted copy into or out of the layout [batch, n0, n1, n2, C] that the tensor-core convolutions work in,
-// so that padding, crop and change of layout are one pass, for 2-byte elements.  A CTA moves 64 positions of 32 words
-// (pairs of channels) through shared memory: channels-first side 64 positions at a time, channels-last side 16 bytes
-// per thread, both without bank conflicts (pitch 65).  [8, 64, 256, 256] bf16, padded by one: 48 us to channels-last,
-// 34 us back (the library's own conversion inside the convolution: 64 and 46 behind 31 and 26 for padding and crop).
-constexpr int kPos = 64, kWords = 32, kPitch = kPos + 1;
+// so that padding, crop and change of layout are one pass, for 2-byte elements.  A CTA moves 2048 words (pairs of channels)
+// through shared memory, W of each position: channels-first side consecutive positions, channels-last side 16 bytes per
+// thread, both without bank conflicts.  W follows the channels, because a CTA for 64 of them is idle where there are 8, and
+// positions are decoded in 32 bits where a plane allows it.  bf16, padded by one, us, to channels-last | back, 32 words and 64
+// bits -> now: [8, 64, 256, 256] 51 | 35 -> 51 | 33, [6, 8, 87^3] 131 | 187 -> 49 | 29, [8, 16, 300, 300] 27 | 37 -> 12 | 12, [4, 24, 60^3]
+// 41 | 47 -> 25 | 25 (the library's own conversion inside the convolution at the first size: 64 | 46 behind 31 | 26 for padding
+// and crop).
+template <int W>
+struct ChannelTile {
+  static constexpr int POS = 2048 / W;                       // positions
+  static constexpr int PITCH = POS + (W == 32 ? 1 : W == 16 ? 2 : W == 8 ? 4 : 0);
+  static constexpr int PER = POS > 256 ? POS / 256 : 1;      // positions of a thread on the channels-first side
+  static constexpr int STEP = POS > 256 ? 1 : 256 / POS;     // distance of its words there
+};
 
 // the pair of channels at p, zero outside
 __device__ __forceinline__ uint32_t gather_pair(const uint16_t* p, long long step, bool live) {
@@ -94,36 +103,40 @@ __device__ __forceinline__ uint32_t gather_pair(const uint16_t* p, long long ste
   return a | (b << 16);
 }
 
-// position of dst -> offset (in positions) inside a plane of src, -1 outside
-__device__ __forceinline__ long long source_position(const ShiftGeom& g, long long o) {
-  const long long row = o / g.out[2];
-  const int i2 = (int)(o - row * g.out[2]) - g.lo[2];
-  const int i1 = (int)(row % g.out[1]) - g.lo[1], i0 = (int)(row / g.out[1]) - g.lo[0];
+// position of dst -> offset (in positions) inside a plane of src, -1 outside.  I: unsigned where a plane has fewer than 2^31.
+template <typename I>
+__device__ __forceinline__ long long source_position(const ShiftGeom& g, I o) {
+  const I row = o / (I)g.out[2], sheet = row / (I)g.out[1];
+  const int i2 = (int)(o - row * (I)g.out[2]) - g.lo[2];
+  const int i1 = (int)(row - sheet * (I)g.out[1]) - g.lo[1], i0 = (int)sheet - g.lo[0];
   const bool live = i0 >= 0 && i0 < g.in[0] && i1 >= 0 && i1 < g.in[1] && i2 >= 0 && i2 < g.in[2];
   return live ? ((long long)i0 * g.in[1] + i1) * g.in[2] + i2 : -1;
 }
 
+template <int W, typename I>
 __global__ void __launch_bounds__(256)
 to_channels_last_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, const ShiftGeom g, int C) {
-  __shared__ uint32_t tile[kWords][kPitch];
+  using T = ChannelTile<W>;
+  __shared__ uint32_t tile[W][T::PITCH];
   const long long out_plane = (long long)g.out[0] * g.out[1] * g.out[2];
   const long long in_plane = (long long)g.in[0] * g.in[1] * g.in[2];
-  const long long p0 = blockIdx.x * (long long)kPos;
-  const int c0 = blockIdx.y * kWords * 2;
-  {
-    const int pos = threadIdx.x & (kPos - 1), w0 = threadIdx.x / kPos;
-    const long long at = p0 + pos < out_plane ? source_position(g, p0 + pos) : -1;
+  const long long p0 = blockIdx.x * (long long)T::POS;
+  const int c0 = blockIdx.y * W * 2, w0 = T::POS > 256 ? 0 : threadIdx.x / T::POS;
+#pragma unroll
+  for (int k = 0; k < T::PER; ++k) {
+    const int pos = (threadIdx.x & (T::POS - 1)) + 256 * k;
+    const long long at = p0 + pos < out_plane ? source_position<I>(g, (I)(p0 + pos)) : -1;
     const uint16_t* s = src + ((long long)blockIdx.z * C + c0 + w0 * 2) * in_plane + (at < 0 ? 0 : at);
 #pragma unroll
-    for (int w = w0; w < kWords; w += 256 / kPos) {
+    for (int w = w0; w < W; w += T::STEP) {
       if (c0 + w * 2 < C) tile[w][pos] = gather_pair(s, in_plane, at >= 0);
-      s += 256 / kPos * 2 * in_plane;
+      s += T::STEP * 2 * in_plane;
     }
   }
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < kPos * 8 / 256; ++k) {
-    const int idx = threadIdx.x + 256 * k, chunk = idx & 7, pos = idx >> 3, c = c0 + chunk * 8;
+  for (int k = 0; k < 2; ++k) {
+    const int idx = threadIdx.x + 256 * k, chunk = idx & (W / 4 - 1), pos = idx / (W / 4), c = c0 + chunk * 8;
     if (c >= C || p0 + pos >= out_plane) continue;
     const uint4 v = make_uint4(tile[chunk * 4][pos], tile[chunk * 4 + 1][pos], tile[chunk * 4 + 2][pos],
                                tile[chunk * 4 + 3][pos]);
@@ -131,36 +144,54 @@ to_channels_last_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__
   }
 }
 
+template <int W, typename I>
 __global__ void __launch_bounds__(256)
 from_channels_last_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, const ShiftGeom g, int C) {
-  __shared__ uint32_t tile[kWords][kPitch];
+  using T = ChannelTile<W>;
+  __shared__ uint32_t tile[W][T::PITCH];
   const long long out_plane = (long long)g.out[0] * g.out[1] * g.out[2];
   const long long in_plane = (long long)g.in[0] * g.in[1] * g.in[2];
-  const long long p0 = blockIdx.x * (long long)kPos;
-  const int c0 = blockIdx.y * kWords * 2;
+  const long long p0 = blockIdx.x * (long long)T::POS;
+  const int c0 = blockIdx.y * W * 2;
 #pragma unroll
-  for (int k = 0; k < kPos * 8 / 256; ++k) {
-    const int idx = threadIdx.x + 256 * k, chunk = idx & 7, pos = idx >> 3, c = c0 + chunk * 8;
+  for (int k = 0; k < 2; ++k) {
+    const int idx = threadIdx.x + 256 * k, chunk = idx & (W / 4 - 1), pos = idx / (W / 4), c = c0 + chunk * 8;
     if (c >= C || p0 + pos >= out_plane) continue;
-    const long long at = source_position(g, p0 + pos);
+    const long long at = source_position<I>(g, (I)(p0 + pos));
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (at >= 0) v = __ldg(reinterpret_cast<const uint4*>(src + ((long long)blockIdx.z * in_plane + at) * C + c));
     tile[chunk * 4][pos] = v.x; tile[chunk * 4 + 1][pos] = v.y;
     tile[chunk * 4 + 2][pos] = v.z; tile[chunk * 4 + 3][pos] = v.w;
   }
   __syncthreads();
-  const int pos = threadIdx.x & (kPos - 1), w0 = threadIdx.x / kPos;
-  if (p0 + pos >= out_plane) return;
-  uint16_t* d = dst + ((long long)blockIdx.z * C + c0 + w0 * 2) * out_plane + p0 + pos;
+  const int w0 = T::POS > 256 ? 0 : threadIdx.x / T::POS;
 #pragma unroll
-  for (int w = w0; w < kWords; w += 256 / kPos) {
-    if (c0 + w * 2 < C) {
-      const uint32_t v = tile[w][pos];
-      d[0] = (uint16_t)v;
-      d[out_plane] = (uint16_t)(v >> 16);
+  for (int k = 0; k < T::PER; ++k) {
+    const int pos = (threadIdx.x & (T::POS - 1)) + 256 * k;
+    if (p0 + pos >= out_plane) return;
+    uint16_t* d = dst + ((long long)blockIdx.z * C + c0 + w0 * 2) * out_plane + p0 + pos;
+#pragma unroll
+    for (int w = w0; w < W; w += T::STEP) {
+      if (c0 + w * 2 < C) {
+        const uint32_t v = tile[w][pos];
+        d[0] = (uint16_t)v;
+        d[out_plane] = (uint16_t)(v >> 16);
+      }
+      d += T::STEP * 2 * out_plane;
     }
-    d += 256 / kPos * 2 * out_plane;
   }
+}
+
+template <int W>
+int launch_channels(const uint16_t* src, uint16_t* dst, int to_last, int B, int C, const ShiftGeom& g, cudaStream_t s) {
+  const long long n = (long long)g.out[0] * g.out[1] * g.out[2];
+  const dim3 grid((unsigned)((n + ChannelTile<W>::POS - 1) / ChannelTile<W>::POS), (unsigned)((C + W * 2 - 1) / (W * 2)),
+                  (unsigned)B);
+  const bool small = n < 0x7fffffffLL;
+  auto kernel = to_last ? (small ? to_channels_last_kernel<W, unsigned> : to_channels_last_kernel<W, long long>)
+                        : (small ? from_channels_last_kernel<W, unsigned> : from_channels_last_kernel<W, long long>);
+  kernel<<<grid, 256, 0, s>>>(src, dst, g, C);
+  return (int)cudaGetLastError();
 }
 
 }  // namespace
@@ -191,10 +222,13 @@ DD_API int dd_shift_channels(const void* src, void* dst, int to_last, int B, int
     if (in[i] <= 0 || out[i] <= 0) return DD_ERR_BAD_ARG;
     g.in[i] = in[i]; g.out[i] = out[i]; g.lo[i] = lo[i];
   }
-  const long long n = (long long)out[0] * out[1] * out[2];
-  const dim3 grid((unsigned)((n + kPos - 1) / kPos), (unsigned)((C + kWords * 2 - 1) / (kWords * 2)), (unsigned)B);
   const uint16_t* from = reinterpret_cast<const uint16_t*>(src);
-  auto kernel = to_last ? to_channels_last_kernel : from_channels_last_kernel;
-  kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(from, reinterpret_cast<uint16_t*>(dst), g, C);
-  return (int)cudaGetLastError();
+  uint16_t* to = reinterpret_cast<uint16_t*>(dst);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  // as many words of a position as leave no more than a fifth of the threads without channels; 32 bytes or more, a sector
+  auto fits = [C](int w) { return (C + w * 2 - 1) / (w * 2) * (w * 2) * 4 <= C * 5; };
+  if (C <= 8) return launch_channels<4>(from, to, to_last, B, C, g, st);
+  if (fits(32)) return launch_channels<32>(from, to, to_last, B, C, g, st);
+  if (fits(16)) return launch_channels<16>(from, to, to_last, B, C, g, st);
+  return launch_channels<8>(from, to, to_last, B, C, g, st);
 }

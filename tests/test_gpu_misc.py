@@ -378,6 +378,20 @@ def test_padding_into_channels_last_and_back(space, pads, C, dtype):
     assert torch.equal(torch.autograd.grad(g.sum(), x)[0], torch.autograd.grad(gr.sum(), xr)[0])
 
 
+@pytest.mark.parametrize("space,C", [((2, 17, 19), 8), ((30, 21), 64), ((5, 300), 16), ((11, 13, 7), 40), ((33, 34), 48),
+                                     ((12, 31), 56), ((65, 3), 128)])
+def test_channel_tiles_follow_the_number_of_channels(space, C):
+    """Tiles of 4 to 32 pairs of channels, positions on and beyond their edges, channels that do not fill the last one."""
+    import torch.nn.functional as F
+
+    from distdl_b200.ops.pad import channels_first, pad_channels_last
+    torch.manual_seed(13)
+    x = torch.randn(2, C, *space, device="cuda").bfloat16()
+    pads = (1, 0, 2, 1) + ((1, 1) if len(space) == 3 else ())
+    y = pad_channels_last(x, pads)
+    assert torch.equal(y, F.pad(x, pads)) and torch.equal(channels_first(y), F.pad(x, pads))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("batch,space,cin,cout,kernel,stride,bias", [
     (2, (13, 17), 16, 24, 3, 1, True), (2, (12, 12), 8, 8, 1, 1, False), (2, (14, 14), 16, 16, 3, 2, False),
