@@ -112,13 +112,15 @@ split_reduce_kernel(const float* part, int split, long long part_stride, int ldw
 // Forward, in us, 256 -> 128 columns: 4096 x 1600 x 6400 74.8 -> 69.7, 512 x 1024 x 512 14.3 -> 11.2; 3000 x 2048 x 5632, whose
 // last wave of whole tiles is short enough to be taken in halves, 59 -> 63.5; but 4096 x 6400 x 1600 62.4 -> 71.7, 3000 x 11264 x 2048 98 -> 114.  Gradients that are added in fp32
 // are bound by their epilogue besides (3000 x 2048 x 5632 70.6 -> 79.9): only where there is one wave either way.
+long long whole_tile_waves(long long tiles, long long pairs) {      // in 200ths
+  const long long rest = tiles % pairs;                       // (a last, short wave of whole tiles is taken in halves)
+  return tiles / pairs * 200 + (rest == 0 ? 0 : tiles > pairs && rest * 2 <= pairs ? 125 : 200);
+}
 bool half_tiles(int M, int N, int batch, bool f32, long long pairs, long long* whole, long long* half) {
   const long long rows_of_tiles = (long long)((M + 2 * gemm2::BM - 1) / (2 * gemm2::BM)) * batch;
   *whole = rows_of_tiles * ((N + 255) / 256);
   *half = rows_of_tiles * ((N + 127) / 128);
-  const long long rest = *whole % pairs;                       // (a last, short wave of whole tiles is taken in halves)
-  const long long waves = *whole / pairs * 200 + (rest == 0 ? 0 : *whole > pairs && rest * 2 <= pairs ? 125 : 200);
-  return f32 ? *half <= pairs : (*half + pairs - 1) / pairs * 125 < waves;
+  return f32 ? *half <= pairs : (*half + pairs - 1) / pairs * 125 < whole_tile_waves(*whole, pairs);
 }
 
 // Order of a pair kernel's tiles of 256 x 256 (see tile_coords).  Large products run at the power limit, where each byte
@@ -198,10 +200,14 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
     // 515 -> 531; K = 4096: 8192 x 28672 1441 -> 1448; K = 8192: 8192 x 8192 895 -> 842, weight gradient 28672 x 4096
     // 1649 -> 1533; K = 14336: 8192 x 4096 768 -> 741; K = 128256: 8192 x 4096 7756 -> 6838.  Entries with live rows take them at
     // any K, because only this kernel deals the live blocks out evenly (figures there).
+    // Where their waves end later than those of the smaller tiles by more than the traffic gains, these stay: weight gradient
+    // 5184 x 1728 of 7716 rows, 147 tiles in two waves, or 77 in one of twice the length and one more; a training step that has it
+    // 8 680 -> 8 440 us, 9 030 with the larger tiles there.
     const bool by_rows = rows != nullptr && !bound_k;
     if (!narrow && (q.flags & F_TMA_EPI) && (by_rows || (rows == nullptr && K > 4096)) && M > 256) {
       const dd::gemm4::Plan w = dd::gemm4::make_plan(M, N, batch, ctas / 2);
-      if (w.full > 0) {
+      const long long pairs = ctas / 2, waves = (long long)(w.full + pairs - 1) / pairs * 400 + (w.items > w.full ? 200 : 0);
+      if (w.full > 0 && (by_rows || waves * 100 <= whole_tile_waves(whole, pairs) * 106)) {
         q.group_m = M <= N ? 8 : -16;
         const int wgrid = 2 * (w.items < ctas / 2 ? w.items : ctas / 2);
         if (a_mn && b_mn) return launch_wide<true, true>(pa, pb, pd, q, w, wgrid, ps);

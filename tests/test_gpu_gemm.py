@@ -259,7 +259,7 @@ def test_batched_gemm_with_half_tiles(B, M, N, K, a_mn, b_mn):
 
 
 @pytest.mark.parametrize("B,M,N,K,ctas", [(1, 257, 200, 4104, 2), (1, 512, 456, 4160, 4), (1, 1000, 520, 4168, 4),
-                                          (3, 1288, 456, 4224, 6), (1, 5120, 1280, 4104, 0)])
+                                          (3, 1288, 456, 4224, 6), (1, 2400, 200, 4160, 4)])
 @pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 0), (1, 1)])
 def test_gemm_with_wide_tiles(B, M, N, K, ctas, a_mn, b_mn):
     """Contractions beyond 4096 take 512 x 256 per pair of CTAs: an odd number of 256-row blocks, a last wave in single
