@@ -25,7 +25,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int ct
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = true;
   }
-  return launch_ahead(kern, grid, NUM_THREADS, SMEM_BYTES, stream, ta, tb, p, plan);
+  return launch_ahead(kern, grid, NUM_THREADS, SMEM_BYTES, stream, !(p.flags & F_ALONE), ta, tb, p, plan);
 }
 template <bool A_MN, bool B_MN, int NB>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p, int pairs,
@@ -42,7 +42,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = true;
   }
-  return launch_ahead(kern, grid, dd::gemm2::NUM_THREADS, bytes, stream, ta, tb, td, p, plan);
+  return launch_ahead(kern, grid, dd::gemm2::NUM_THREADS, bytes, stream, !(p.flags & F_ALONE), ta, tb, td, p, plan);
 }
 
 template <bool A_MN, bool B_MN>
@@ -57,7 +57,8 @@ int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = true;
   }
-  return launch_ahead(kern, grid, dd::gemm4::NUM_THREADS, dd::gemm4::SMEM, stream, ta, tb, td, p, plan);
+  return launch_ahead(kern, grid, dd::gemm4::NUM_THREADS, dd::gemm4::SMEM, stream, !(p.flags & F_ALONE), ta, tb, td, p,
+                      plan);
 }
 
 // Second half of a split contraction: D (+)= sum_s part[s] (+ bias), the parts in order (the same bits in every
@@ -140,8 +141,9 @@ int tile_group(int M, int N, int K) {
 //                 1 = MN-major (lda = elements between rows k)
 //   stride*     : elements between batches (ignored when batch == 1)
 //   flags       : dd::gemm::Flags
-//   max_ctas    : 0 = one CTA per SM; otherwise an upper bound (used to leave
-//                 SMs to a concurrent communication kernel)
+//   max_ctas    : 0 = one CTA per SM; otherwise an upper bound, which leaves
+//                 SMs to a concurrent communication kernel: until the product
+//                 has ended, the kernel behind it does not start on them either
 namespace {
 int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const void* B, int b_mn, long long ldb,
               long long strideB, void* D, long long ldd, long long strideD, const void* bias, int M, int N, int K,
@@ -154,6 +156,7 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
     strideB = (b_mn ? (long long)K : (long long)N) * ldb;
     strideD = (long long)M * ldd;
   }
+  if (max_ctas > 0 && max_ctas < current_sm_count()) flags |= F_ALONE;
   // CTA pairs (cta_group::2) unless disabled or the problem is a single tile row
   static const bool pair_ok = []() { const char* e = getenv("DISTDL_GEMM_PAIR"); return !(e && e[0] == '0'); }();
   if (pair_ok && M > BM) {
@@ -319,5 +322,5 @@ DD_API int dd_gemm_bf16_split(const void* A, int a_mn, long long lda, const void
   p.D = D; p.ldd = ldd; p.strideD = 0; p.bias = bias; p.flags = flags; p.group_m = 1; p.status = nullptr;
   const long long total = (long long)M * (ldw / 4);
   return launch_ahead(split_reduce_kernel, (unsigned)((total + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream),
-                      ws, split, (long long)M * ldw, ldw, p);
+                      true, ws, split, (long long)M * ldw, ldw, p);
 }

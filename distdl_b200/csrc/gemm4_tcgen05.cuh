@@ -288,7 +288,7 @@ gemm4_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   cluster_sync();                                   // barriers of both CTAs are initialised
   tc_fence_after();
   const uint32_t tmem_base = ss->tmem_base;
-  grid_dependency_launch();
+  if (!(p.flags & gemm::F_ALONE)) grid_dependency_launch();
   grid_dependency_wait();
 
   if (warp == 0) {

@@ -46,6 +46,7 @@ enum Flags : int {
   F_BIAS = 4,         // add bias[n] (bf16)
   F_BIAS_F32 = 8,     // bias is fp32
   F_TMA_EPI = 16,     // CTA-pair kernels: the tile leaves through shared memory + TMA (set by the host)
+  F_ALONE = 32,       // limited to some SMs: the next kernel may not start before the end (set by the host)
 };
 
 struct Params {
@@ -225,7 +226,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ss->tmem_base;
-  grid_dependency_launch();
+  if (!(p.flags & F_ALONE)) grid_dependency_launch();
   grid_dependency_wait();
 
   if (warp == 0) {

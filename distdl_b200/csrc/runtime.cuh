@@ -39,11 +39,13 @@ int current_sm_count();
 // barriers, tensor memory: 2 to 4 us) does not wait for the end of the kernel before it.  The products do so, and the kernels
 // that mostly come before one let it start.  A training step of four layers of 1600 columns, 2 x 4096 tokens, 306 launches:
 // 13 980 -> 13 720 us; four layers of 2048 columns, 3000 tokens: 7 180 -> 7 060.
+// ahead: false for a kernel that leaves SMs to other streams, which would otherwise hold its SMs before it can work on them.
 template <typename... P, typename... A>
-inline int launch_ahead(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A&... args) {
+inline int launch_ahead(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool ahead,
+                        const A&... args) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+  attr.val.programmaticStreamSerializationAllowed = ahead ? 1 : 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;

@@ -411,3 +411,35 @@ def test_products_launched_ahead_are_ordered_on_streams_and_in_graphs():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 131072, 2048), (4096, 16384, 2048), (4096, 8192, 4160)])
+def test_a_product_limited_to_some_sms_leaves_the_others_to_another_stream(M, N, K):
+    """``max_ctas``: the product behind a limited one must not settle on the SMs that the limit leaves free, so that work of
+    another stream ends while the limited one (milliseconds on four SMs) still runs.  One size for each kernel."""
+    from distdl_b200.ops import gemm
+    a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
+    c = torch.randn(2048, 512, device="cuda", dtype=torch.bfloat16)
+    outs = [torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    small = torch.empty(2048, 2048, device="cuda", dtype=torch.bfloat16)
+    side = torch.cuda.Stream()
+    start, end, other = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+
+    def both(record):
+        if record:
+            start.record()
+        gemm(a, b, out=outs[0], max_ctas=4)
+        gemm(a, b, out=outs[1])
+        with torch.cuda.stream(side):
+            gemm(c, c, out=small, max_ctas=64)
+            if record:
+                other.record()
+        if record:
+            end.record()
+    for record in (False, True):
+        torch.cuda.synchronize()
+        both(record)
+    torch.cuda.synchronize()
+    assert start.elapsed_time(other) < 0.5 * start.elapsed_time(end)
+    assert torch.equal(*outs)
