@@ -13,8 +13,7 @@ using namespace dd::gemm;
 
 namespace {
 template <bool A_MN, bool B_MN>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int ctas, cudaStream_t stream) {
-  const Plan plan = make_plan(p.M, p.N, p.batch, ctas);
+int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, const Plan& plan, int ctas, cudaStream_t stream) {
   const int grid = plan.items < ctas ? plan.items : ctas;
   static bool configured[64] = {false};
   int dev = 0;
@@ -29,8 +28,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int ct
 }
 template <bool A_MN, bool B_MN, int NB>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p, int pairs,
-                cudaStream_t stream) {
-  const dd::gemm2::Plan plan = dd::gemm2::make_plan(p.M, p.N, p.batch, pairs, NB);
+                const dd::gemm2::Plan& plan, cudaStream_t stream) {
   const int grid = 2 * (plan.items < pairs ? plan.items : pairs);
   static bool configured[64] = {false};
   int dev = 0;
@@ -134,6 +132,62 @@ int tile_group(int M, int N, int K) {
   const int g = min(tiles, max(8, (int)(36000000ll / (512ll * K))));
   return M <= N ? g : -g;
 }
+
+// Which kernel takes a product, with how many CTAs, its work items and the order of its tiles.
+enum Kernel : int { SINGLE, PAIR, PAIR_HALF, WIDE };
+struct Choice {
+  Kernel kernel;
+  int ctas, group_m;
+  Plan single;                       // (of the kernel that is taken; the others are not set)
+  dd::gemm2::Plan pair;
+  dd::gemm4::Plan wide;
+};
+
+// flags with F_TMA_EPI where the output allows it; rows: A has live rows or, with bound_k, live terms; a_span: bytes from the first
+// element of A to behind its last.
+Choice choose(int M, int N, int K, int batch, int flags, int max_ctas, bool rows, bool bound_k, long long a_span) {
+  Choice c = {};
+  const int sms = current_sm_count();
+  // CTA pairs (cta_group::2) unless disabled or the problem is a single tile row
+  static const bool pair_ok = []() { const char* e = getenv("DISTDL_GEMM_PAIR"); return !(e && e[0] == '0'); }();
+  if (!pair_ok || M <= BM) {
+    c.kernel = SINGLE;
+    c.ctas = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
+    c.group_m = 8;
+    c.single = make_plan(M, N, batch, c.ctas, a_span);
+    return c;
+  }
+  c.ctas = sms & ~1;
+  if (max_ctas > 0 && max_ctas < c.ctas) c.ctas = max_ctas & ~1;
+  if (c.ctas < 2) c.ctas = 2;
+  const int pairs = c.ctas / 2;
+  long long whole, half;
+  const bool narrow = half_tiles(M, N, batch, (flags & F_OUT_F32) != 0, pairs, &whole, &half) && !rows;
+  // Tiles of 512 x 256 (gemm4_tcgen05.cuh) for at least a whole wave of them.  They bring a quarter less through L2, but
+  // pairs wait for the epilogue between tiles, and the order of tiles that keeps a panel in L2 is at its best with the
+  // smaller ones where the contraction is short.  In us, back to back, 256 rows -> 512 rows: K = 1600: 4096 x 50304
+  // 515 -> 531; K = 4096: 8192 x 28672 1441 -> 1448; K = 8192: 8192 x 8192 895 -> 842, weight gradient 28672 x 4096
+  // 1649 -> 1533; K = 14336: 8192 x 4096 768 -> 741; K = 128256: 8192 x 4096 7756 -> 6838.  Entries with live rows take them at
+  // any K, because only this kernel deals the live blocks out evenly (figures there).
+  // Where their waves end later than those of the smaller tiles by more than the traffic gains, these stay: weight gradient
+  // 5184 x 1728 of 7716 rows, 147 tiles in two waves, or 77 in one of twice the length and one more; a training step that has it
+  // 8 680 -> 8 440 us, 9 030 with the larger tiles there.
+  const bool by_rows = rows && !bound_k;
+  if (!narrow && (flags & F_TMA_EPI) && (by_rows || (!rows && K > 4096)) && M > 256) {
+    c.wide = dd::gemm4::make_plan(M, N, batch, pairs);
+    const long long waves = (long long)(c.wide.full + pairs - 1) / pairs * 400 + (c.wide.items > c.wide.full ? 200 : 0);
+    if (c.wide.full > 0 && (by_rows || waves * 100 <= whole_tile_waves(whole, pairs) * 106)) {
+      c.kernel = WIDE;
+      c.group_m = M <= N ? 8 : -16;
+      return c;
+    }
+  }
+  c.kernel = narrow ? PAIR_HALF : PAIR;
+  // (four rows of half tiles: 4096 x 1600 x 6400 76 us, 79 to 83 in the other orders)
+  c.group_m = narrow ? 4 : tile_group(M, N, K);
+  c.pair = dd::gemm2::make_plan(M, N, batch, pairs, narrow ? 128 : 256);
+  return c;
+}
 }  // namespace
 
 // D[b,m,n] (+)= sum_k A[b,m,k] B[b,n,k] (+ bias[n]);  bf16 operands, fp32 accumulation.
@@ -147,7 +201,7 @@ int tile_group(int M, int N, int K) {
 namespace {
 int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const void* B, int b_mn, long long ldb,
               long long strideB, void* D, long long ldd, long long strideD, const void* bias, int M, int N, int K,
-              int batch, int flags, int max_ctas, const int* rows, int bound_k, void* stream) {
+              int batch, int flags, int max_ctas, const int* rows, int bound_k, void* stream, bool parts_of_k = false) {
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return DD_ERR_BAD_ARG;
   if ((lda % 8) || (ldb % 8)) return DD_ERR_ALIGN;
   if (batch > 1 && ((strideA % 8) || (strideB % 8))) return DD_ERR_ALIGN;
@@ -157,104 +211,62 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
     strideD = (long long)M * ldd;
   }
   if (max_ctas > 0 && max_ctas < current_sm_count()) flags |= F_ALONE;
-  // CTA pairs (cta_group::2) unless disabled or the problem is a single tile row
-  static const bool pair_ok = []() { const char* e = getenv("DISTDL_GEMM_PAIR"); return !(e && e[0] == '0'); }();
-  if (pair_ok && M > BM) {
-    CUtensorMap pa, pb;
-    int rr;
-    namespace g2 = dd::gemm2;
-    int ctas = current_sm_count() & ~1;
-    if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas & ~1;
-    if (ctas < 2) ctas = 2;
-    long long whole, half;
-    const bool narrow = half_tiles(M, N, batch, (flags & F_OUT_F32) != 0, ctas / 2, &whole, &half) && rows == nullptr;
-    if (a_mn) rr = get_tensor_map_bf16_3d(&pa, A, M, K, batch, lda * 2, strideA * 2, 64, g2::BK);
-    else      rr = get_tensor_map_bf16_3d(&pa, A, K, M, batch, lda * 2, strideA * 2, g2::BK, g2::BM);
-    if (rr) return rr;
-    if (b_mn) rr = get_tensor_map_bf16_3d(&pb, B, N, K, batch, ldb * 2, strideB * 2, 64, g2::BK);
-    else      rr = get_tensor_map_bf16_3d(&pb, B, K, N, batch, ldb * 2, strideB * 2, g2::BK, 64);
-    if (rr) return rr;
-    int err2 = 0;
-    Params q;
-    q.M = M; q.N = N; q.K = K; q.batch = batch;
-    q.D = D; q.ldd = ldd; q.strideD = strideD; q.bias = bias; q.flags = flags;
-    // (four rows of half tiles: 4096 x 1600 x 6400 76 us, 79 to 83 in the other orders)
-    q.group_m = narrow ? 4 : tile_group(M, N, K);
-    q.status = device_status(&err2);
-    q.rows = rows; q.bound_k = bound_k;
-    if (err2) return err2;
-    cudaStream_t ps = reinterpret_cast<cudaStream_t>(stream);
-    // TMA epilogue where the output qualifies: bf16 store, fp32 store or fp32 add
-    static const bool tma_epi = []() { const char* e = getenv("DISTDL_GEMM_TMA_EPI"); return !(e && e[0] == '0'); }();
-    CUtensorMap pd;
-    memset(&pd, 0, sizeof(pd));
-    const bool f32 = (flags & F_OUT_F32) != 0;
-    const long long es = f32 ? 4 : 2;
-    if (tma_epi && (f32 || !(flags & F_ACCUMULATE)) && (reinterpret_cast<uintptr_t>(D) & 15) == 0 &&
-        (ldd * es) % 16 == 0 && (strideD * es) % 16 == 0) {
-      rr = f32 ? get_tensor_map_f32_3d(&pd, D, N, M, batch, ldd * 4, strideD * 4, 32, 32)
-               : get_tensor_map_bf16_3d(&pd, D, N, M, batch, ldd * 2, strideD * 2, 64, 32);
-      if (rr) return rr;
-      q.flags |= F_TMA_EPI;
-    }
-    // Tiles of 512 x 256 (gemm4_tcgen05.cuh) for at least a whole wave of them.  They bring a quarter less through L2, but
-    // pairs wait for the epilogue between tiles, and the order of tiles that keeps a panel in L2 is at its best with the
-    // smaller ones where the contraction is short.  In us, back to back, 256 rows -> 512 rows: K = 1600: 4096 x 50304
-    // 515 -> 531; K = 4096: 8192 x 28672 1441 -> 1448; K = 8192: 8192 x 8192 895 -> 842, weight gradient 28672 x 4096
-    // 1649 -> 1533; K = 14336: 8192 x 4096 768 -> 741; K = 128256: 8192 x 4096 7756 -> 6838.  Entries with live rows take them at
-    // any K, because only this kernel deals the live blocks out evenly (figures there).
-    // Where their waves end later than those of the smaller tiles by more than the traffic gains, these stay: weight gradient
-    // 5184 x 1728 of 7716 rows, 147 tiles in two waves, or 77 in one of twice the length and one more; a training step that has it
-    // 8 680 -> 8 440 us, 9 030 with the larger tiles there.
-    const bool by_rows = rows != nullptr && !bound_k;
-    if (!narrow && (q.flags & F_TMA_EPI) && (by_rows || (rows == nullptr && K > 4096)) && M > 256) {
-      const dd::gemm4::Plan w = dd::gemm4::make_plan(M, N, batch, ctas / 2);
-      const long long pairs = ctas / 2, waves = (long long)(w.full + pairs - 1) / pairs * 400 + (w.items > w.full ? 200 : 0);
-      if (w.full > 0 && (by_rows || waves * 100 <= whole_tile_waves(whole, pairs) * 106)) {
-        q.group_m = M <= N ? 8 : -16;
-        const int wgrid = 2 * (w.items < ctas / 2 ? w.items : ctas / 2);
-        if (a_mn && b_mn) return launch_wide<true, true>(pa, pb, pd, q, w, wgrid, ps);
-        if (a_mn) return launch_wide<true, false>(pa, pb, pd, q, w, wgrid, ps);
-        if (b_mn) return launch_wide<false, true>(pa, pb, pd, q, w, wgrid, ps);
-        return launch_wide<false, false>(pa, pb, pd, q, w, wgrid, ps);
-      }
-    }
-    if (narrow) {
-      if (a_mn && b_mn) return launch_pair<true, true, 128>(pa, pb, pd, q, ctas / 2, ps);
-      if (a_mn) return launch_pair<true, false, 128>(pa, pb, pd, q, ctas / 2, ps);
-      if (b_mn) return launch_pair<false, true, 128>(pa, pb, pd, q, ctas / 2, ps);
-      return launch_pair<false, false, 128>(pa, pb, pd, q, ctas / 2, ps);
-    }
-    if (a_mn && b_mn) return launch_pair<true, true, 256>(pa, pb, pd, q, ctas / 2, ps);
-    if (a_mn) return launch_pair<true, false, 256>(pa, pb, pd, q, ctas / 2, ps);
-    if (b_mn) return launch_pair<false, true, 256>(pa, pb, pd, q, ctas / 2, ps);
-    return launch_pair<false, false, 256>(pa, pb, pd, q, ctas / 2, ps);
-  }
-  CUtensorMap ta, tb;
-  int r;
+  // TMA epilogue of the pair kernels where the output qualifies: bf16 store, fp32 store or fp32 add
+  static const bool tma_epi = []() { const char* e = getenv("DISTDL_GEMM_TMA_EPI"); return !(e && e[0] == '0'); }();
+  const bool f32 = (flags & F_OUT_F32) != 0;
+  const long long es = f32 ? 4 : 2;
+  const bool tma_out = tma_epi && (f32 || !(flags & F_ACCUMULATE)) && (reinterpret_cast<uintptr_t>(D) & 15) == 0 &&
+                       (ldd * es) % 16 == 0 && (strideD * es) % 16 == 0;
+  // (parts of one contraction: each reads a part of A of its own, and briefly)
+  const long long a_span = parts_of_k ? 1ll << 62 : 2 * ((batch - 1) * strideA + (a_mn ? (K - 1) * lda + M : (M - 1) * lda + K));
+  const Choice c = choose(M, N, K, batch, flags | (tma_out ? F_TMA_EPI : 0), max_ctas, rows != nullptr, bound_k != 0, a_span);
+  int err = 0, r;
+  Params p;
+  p.M = M; p.N = N; p.K = K; p.batch = batch;
+  p.D = D; p.ldd = ldd; p.strideD = strideD; p.bias = bias; p.flags = flags; p.group_m = c.group_m;
+  p.status = device_status(&err);
+  if (err) return err;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  CUtensorMap ta, tb, td;
+  static_assert(BM == dd::gemm2::BM && BK == dd::gemm2::BK && BM == dd::gemm4::BLK / 2 && BK == dd::gemm4::BK, "boxes of A");
   if (a_mn) r = get_tensor_map_bf16_3d(&ta, A, M, K, batch, lda * 2, strideA * 2, 64, BK);
   else      r = get_tensor_map_bf16_3d(&ta, A, K, M, batch, lda * 2, strideA * 2, BK, BM);
   if (r) return r;
   if (b_mn) r = get_tensor_map_bf16_3d(&tb, B, N, K, batch, ldb * 2, strideB * 2, 64, BK);
   else      r = get_tensor_map_bf16_3d(&tb, B, K, N, batch, ldb * 2, strideB * 2, BK, 64);
   if (r) return r;
-
-  int err = 0;
-  Params p;
-  p.M = M; p.N = N; p.K = K; p.batch = batch;
-  p.D = D; p.ldd = ldd; p.strideD = strideD;
-  p.bias = bias; p.flags = flags;
-  p.group_m = 8;
-  p.status = device_status(&err);
-  if (err) return err;
-
-  int ctas = current_sm_count();
-  if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (a_mn && b_mn) return launch<true, true>(ta, tb, p, ctas, s);
-  if (a_mn) return launch<true, false>(ta, tb, p, ctas, s);
-  if (b_mn) return launch<false, true>(ta, tb, p, ctas, s);
-  return launch<false, false>(ta, tb, p, ctas, s);
+  if (c.kernel == SINGLE) {
+    if (a_mn && b_mn) return launch<true, true>(ta, tb, p, c.single, c.ctas, s);
+    if (a_mn) return launch<true, false>(ta, tb, p, c.single, c.ctas, s);
+    if (b_mn) return launch<false, true>(ta, tb, p, c.single, c.ctas, s);
+    return launch<false, false>(ta, tb, p, c.single, c.ctas, s);
+  }
+  p.rows = rows; p.bound_k = bound_k;
+  memset(&td, 0, sizeof(td));
+  if (tma_out) {
+    r = f32 ? get_tensor_map_f32_3d(&td, D, N, M, batch, ldd * 4, strideD * 4, 32, 32)
+            : get_tensor_map_bf16_3d(&td, D, N, M, batch, ldd * 2, strideD * 2, 64, 32);
+    if (r) return r;
+    p.flags |= F_TMA_EPI;
+  }
+  const int pairs = c.ctas / 2;
+  if (c.kernel == WIDE) {
+    const int grid = 2 * (c.wide.items < pairs ? c.wide.items : pairs);
+    if (a_mn && b_mn) return launch_wide<true, true>(ta, tb, td, p, c.wide, grid, s);
+    if (a_mn) return launch_wide<true, false>(ta, tb, td, p, c.wide, grid, s);
+    if (b_mn) return launch_wide<false, true>(ta, tb, td, p, c.wide, grid, s);
+    return launch_wide<false, false>(ta, tb, td, p, c.wide, grid, s);
+  }
+  if (c.kernel == PAIR_HALF) {
+    if (a_mn && b_mn) return launch_pair<true, true, 128>(ta, tb, td, p, pairs, c.pair, s);
+    if (a_mn) return launch_pair<true, false, 128>(ta, tb, td, p, pairs, c.pair, s);
+    if (b_mn) return launch_pair<false, true, 128>(ta, tb, td, p, pairs, c.pair, s);
+    return launch_pair<false, false, 128>(ta, tb, td, p, pairs, c.pair, s);
+  }
+  if (a_mn && b_mn) return launch_pair<true, true, 256>(ta, tb, td, p, pairs, c.pair, s);
+  if (a_mn) return launch_pair<true, false, 256>(ta, tb, td, p, pairs, c.pair, s);
+  if (b_mn) return launch_pair<false, true, 256>(ta, tb, td, p, pairs, c.pair, s);
+  return launch_pair<false, false, 256>(ta, tb, td, p, pairs, c.pair, s);
 }
 }  // namespace
 
@@ -274,6 +286,19 @@ DD_API int dd_gemm_bf16_rows(const void* A, int a_mn, long long lda, long long s
                              int K, int batch, int flags, const int* rows, int bound_k, void* stream) {
   return gemm_bf16(A, a_mn, lda, strideA, B, b_mn, ldb, strideB, D, ldd, strideD, nullptr, M, N, K, batch, flags, 0, rows,
                    bound_k, stream);
+}
+
+// What the entries above would do with a contiguous A and an output that TMA can write, for tests: the kernel (0 single CTA, 1
+// pair, 2 pair with half tiles, 3 512 x 256 per pair), CTAs at most, order of tiles, whole tiles, work items, and parts of a tile
+// behind the whole ones.
+DD_API int dd_gemm_plan(int M, int N, int K, int batch, int flags, int max_ctas, int rows, int bound_k, int* out) {
+  if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return DD_ERR_BAD_ARG;
+  const Choice c = choose(M, N, K, batch, flags | F_TMA_EPI, max_ctas, rows != 0, bound_k != 0, 2ll * batch * M * K);
+  out[0] = c.kernel; out[1] = c.ctas; out[2] = c.group_m;
+  out[3] = c.kernel == SINGLE ? c.single.full : c.kernel == WIDE ? c.wide.full : c.pair.full;
+  out[4] = c.kernel == SINGLE ? c.single.items : c.kernel == WIDE ? c.wide.items : c.pair.items;
+  out[5] = c.kernel == SINGLE ? c.single.parts : 2;
+  return DD_OK;
 }
 
 // Into how many parts dd_gemm_bf16_split should cut the contraction (1: not at all).  A GEMM with few output tiles
@@ -315,7 +340,7 @@ DD_API int dd_gemm_bf16_split(const void* A, int a_mn, long long lda, const void
   const long long kc = K / split;
   const int ldw = (N + 3) & ~3;
   const int r = gemm_bf16(A, a_mn, lda, a_mn ? kc * lda : kc, B, b_mn, ldb, b_mn ? kc * ldb : kc, ws, ldw,
-                          (long long)M * ldw, nullptr, M, N, (int)kc, split, F_OUT_F32, 0, nullptr, 0, stream);
+                          (long long)M * ldw, nullptr, M, N, (int)kc, split, F_OUT_F32, 0, nullptr, 0, stream, true);
   if (r) return r;
   Params p;
   p.M = M; p.N = N; p.K = K; p.batch = 1;

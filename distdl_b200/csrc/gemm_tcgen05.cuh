@@ -166,15 +166,20 @@ __device__ __forceinline__ void store_chunk(const Params& p, uint32_t (&acc)[32]
 // columns, as many as there are CTAs for.  Few rows against many columns are bound by the read of B, of which one SM takes in
 // no more than about 85 GB/s.  Back to back, us: 33 x 6144 x 4096 (24 tiles on 148 SMs) 26.8 -> 16.8, 33 x 4096 x 4096 24.6 -> 13.3,
 // 100 x 2048 x 2048 17.5 -> 11.3; but halves behind whole waves, 1 x 128256 x 4096 (501 tiles), 197 -> 204.
+// An A of less than 128 KB from its first element to its last lies in few places of L2, where the CTAs wait for one another:
+// no more than 32 items there.  Whole tiles, halves, quarters, each alone with a cold L2: 4 x 4096 x 4096 34.8, 30.8, 38.9, 1 x 8192 x
+// 4096 39, 43, 47, 1 x 4096 x 8192 60, 53, 70 (8 rows, 128 KB: 60, 53, 49), 1 x 2048 x 4096 32.8, 28.7, 28.6; two of 1 x 4096 x 4096 39
+// and, in quarters, 45.
 struct Plan {
   int tiles_m, tiles_n, full, parts, items;
 };
-inline Plan make_plan(int M, int N, int batch, int ctas) {
+inline Plan make_plan(int M, int N, int batch, int ctas, long long a_span) {
   Plan w;
+  const int room = a_span < (128 << 10) && ctas > 32 ? 32 : ctas;
   w.tiles_m = (M + BM - 1) / BM;
   w.tiles_n = (N + BN - 1) / BN;
   const int tiles = w.tiles_m * w.tiles_n * batch, rest = tiles <= ctas ? tiles : tiles % ctas;
-  w.parts = rest * 4 <= ctas ? 4 : rest * 2 <= ctas && tiles <= ctas ? 2 : 1;
+  w.parts = rest * 4 <= room ? 4 : rest * 2 <= room && tiles <= ctas ? 2 : 1;
   w.full = tiles - rest;
   w.items = w.full + w.parts * rest;
   return w;

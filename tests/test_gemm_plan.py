@@ -1,0 +1,34 @@
+"""The rules that choose a GEMM's kernel, order of tiles and work items (``csrc/gemm.cu``), asked on the host for a GPU of 148
+SMs, which is what the library assumes without one."""
+import ctypes
+
+import pytest
+
+from distdl_b200 import _native
+
+pytestmark = pytest.mark.skipif(not _native.available(), reason="native library not built")
+SINGLE, PAIR, PAIR_HALF, WIDE = range(4)
+F_OUT_F32 = 1
+
+
+def plan(M, N, K, batch=1, flags=0, max_ctas=0, rows=0, bound_k=0):
+    out = (ctypes.c_int * 6)()
+    assert _native.lib().dd_gemm_plan(M, N, K, batch, flags, max_ctas, rows, bound_k, out) == 0
+    return dict(zip(("kernel", "ctas", "group", "full", "items", "parts"), out))
+
+
+@pytest.fixture(autouse=True)
+def on_148_sms():
+    if plan(4096, 4096, 64)["ctas"] != 148:
+        pytest.skip("figures for 148 SMs")
+
+
+@pytest.mark.parametrize("M,N,K,batch,items", [
+    (1, 4096, 4096, 1, 32), (4, 4096, 4096, 1, 32), (15, 4096, 4096, 1, 32), (16, 4096, 4096, 1, 64),  # 16 tiles: halves, then quarters
+    (1, 8192, 4096, 1, 32), (33, 8192, 4096, 1, 128), (1, 14336, 4096, 1, 56), (16, 14336, 4096, 1, 112),
+    (1, 2048, 4096, 1, 32), (1, 4096, 8192, 1, 32), (8, 4096, 8192, 1, 64), (32, 8192, 1024, 1, 32), (64, 8192, 1024, 1, 128),
+    (1, 4096, 4096, 2, 32), (16, 4096, 4096, 2, 128), (1, 2048, 2048, 4, 32)])
+def test_few_rows_that_lie_close_together_are_read_by_few_ctas(M, N, K, batch, items):
+    """An A of less than 128 KB in no more than 32 parts of tiles: in more, the CTAs wait for one another's reads of it."""
+    p = plan(M, N, K, batch)
+    assert p["kernel"] == SINGLE and p["items"] == items
