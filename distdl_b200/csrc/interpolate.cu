@@ -413,8 +413,8 @@ interp_adjoint_kernel(const InterpGeom g, T* __restrict__ x, const T* __restrict
 // bf16 76 -> 57.  The adjoint marches over volumes of 4-byte elements: the first of these 83 -> 58; in bf16 and over rows
 // the loads of a sheet wait for each other more than they save (65 -> 109 for the last), but not where a window of five
 // outputs is 125 of them: the second 407 -> 300 (909 with weights worked out on the way, as all of more than four were).
+// Which tensors are walked so: march_forward, march_adjoint.
 constexpr int kLead = 32;            // leading positions per segment, at most
-constexpr long long kMarchFrom = 1 << 20;     // outputs of all planes; below, the tables take longer than the loads (10^3: 3.5 and 6.7 us)
 constexpr int kLeadOut = 5 * kLead + 16;      // outputs that may take the inputs of a segment (adjoint)
 
 struct Segments {
@@ -698,6 +698,78 @@ inline bool march_fits(const InterpGeom& g, const Segments& sg, double step) {
   return hi - lo < kLeadOut;
 }
 
+// Source step per output along dimension d (0: all outputs take the same).
+inline double step_of(const InterpGeom& g, int d) {
+  if (!(g.linear && g.align_corners)) return g.scale[d];
+  return g.out_global[d] > 1 ? (double)(g.in_global[d] - 1) / (double)(g.out_global[d] - 1) : 0.0;
+}
+
+// Whether the forward walks sheets (or rows), of V outputs of esize bytes per thread.  That gains where a sheet is read by
+// several outputs of the leading dimension, so not where that grows by less than 1.4 (size kept, rows of 256, 2^24 outputs in
+// fp32: 1.15 times the time of the kernel above; halved, rows of 128 in bf16, 2^23: 1.6).  The threads of a CTA lie over one sheet: short
+// rows leave lanes without one, and whole tensors beyond L2 hide loads by themselves, so that the kernel above is the faster one
+// for rows.  Times the kernel's above, growing by 2 (by 1.5), outputs in all 2^20, 2^21, 2^23, 2^25:
+//   rows in bf16    of 32 0.98 1.24 2.01 2.07 (0.99 1.35 2.22 2.66), 64 0.80 0.90 1.31 1.42 (0.77 0.96 1.46 1.77), 128 0.54 0.76 0.92 1.02
+//                   (0.62 0.77 0.98 1.08), 160 0.58 0.61 0.84 0.80 (0.60 0.67 0.87 0.89), 256 0.49 0.51 0.72 0.72
+//   rows in fp32    of 32 0.81 1.11 1.54 1.70, 64 0.62 0.86 1.06 1.39 (0.64 0.87 1.16 1.49), 128 0.66 0.77 0.96 1.03 (0.63 0.78 1.05
+//                   1.15; 0.90 of 2^22), 384 0.60 0.67 0.93 1.21 (0.61 0.68 1.05 1.39), 512 0.52 0.58 0.80 1.00 (0.52 0.58 0.90 1.10);
+//                   of 260, half the lanes of two CTAs, 2^22 (1.09)
+//   sheets in bf16  of 6 x 6 1.24 - 1.26 1.06, 8 x 8 0.66 0.79 1.20 0.91 (0.68 0.84 1.31 1.10), 12 x 12 0.53 0.59 0.81 0.75 (0.60 0.66
+//                   0.92 0.96), 32 x 32 0.51 0.59 0.72 0.62
+//   sheets in fp32  of 6 x 6 0.98 - 1.07 1.18, 8 x 8 0.57 0.72 0.75 0.78 (0.63 0.74 0.81 0.91), 24 x 24 0.64 0.84 0.78 0.80 (0.65 0.88
+//                   0.88 1.01); in fp64 - 0.90 0.93 1.01 (- 0.99 1.06 1.05)
+// Below 2^20 the tables take longer than the loads (10^3: 3.5 and 6.7 us).
+inline bool march_forward(const InterpGeom& g, int nd, long long tail, long long outputs, int V, int esize) {
+  if (nd < 2 || outputs < (1 << 20) || step_of(g, 3 - nd) > 0.72) return false;
+  const long long threads = tail / V, per_cta = plane_threads(threads), lanes = (threads + per_cta - 1) / per_cta * per_cta;
+  const bool busy = threads * 5 >= lanes * 4;
+  if (nd == 3) return threads >= 64 && (esize <= 4 || (busy && outputs < (1 << 22)));
+  if (V == 2) return busy && (threads >= 72 || (threads >= 32 && outputs <= (1 << 21)));
+  return busy && ((threads >= 128 && outputs < (3 << 21)) || (threads >= 64 && outputs <= (1 << 21)));
+}
+
+// Outputs of a row per thread: a pair of bf16, where a row is whole pairs, leaves as one word.
+template <typename T>
+inline int forward_vector(const InterpGeom& g, bool small, const T* y) {
+  return std::is_same<T, __nv_bfloat16>::value && small && g.out_local[2] % 2 == 0 && (reinterpret_cast<uintptr_t>(y) & 3) == 0
+             ? 2 : 1;
+}
+
+// Outputs per input and dimension that a thread of the adjoint keeps weights for (32: in its own memory), as a hint: a position
+// that has more takes the slow way by itself.  per: of the dimension that has the most, where the ratio is no whole number.
+// Five cost a table of their own: 0.3 to 0.5 of the time in three dimensions, 0.4 to 0.8 in two, in one 0.6 to 0.95 for rows of 100
+// and more, but 1.1 to 1.4 for 12 to 40 inputs unless there are 2^22 outputs (0.8 to 0.98), in fp64 even then, and 1.2 for 3 x 14 and 4 x 4 x 4.
+inline int adjoint_window(const InterpGeom& g, int nd, long long outputs, int esize, double* per) {
+  double most = 1.0;
+  int least = g.out_local[2];                       // the smallest extent must hold a whole window
+  *per = 1.0;
+  for (int d = 2; d >= 3 - nd; --d) {
+    if (g.out_local[d] < least) least = g.out_local[d];
+    const double step = step_of(g, d), n = step > 0.0 ? (g.linear ? 2.0 : 1.0) / step : (double)g.out_local[d];
+    *per = std::max(*per, n);
+    most = std::max(most, step > 0.0 ? std::ceil(n - 1e-9) : n);
+  }
+  const bool five = (long long)g.in_local[0] * g.in_local[1] * g.in_local[2] >= 80 ||
+                    (esize <= 4 && (nd >= 2 || outputs >= (1 << 22)));
+  return most <= 2.0 && least >= 2 ? 2 : most <= 3.0 && least >= 3 ? 3 : most <= 4.0 && least >= 4 ? 4
+         : most <= 5.0 && least >= 5 && five ? 5 : 32;
+}
+
+// Whether the adjoint walks sheets, with K outputs per dimension that take an input, `per` of them where the ratio is no whole
+// number.  Nearest takes one and gains nothing (grown by 2, 2^20 outputs 1.3 to 1.9 times the time of the kernel above).  Times
+// the kernel's, in fp32, outputs in all 2^20, 2^21, 2^22, 2^23, 2^25:
+//   halved (K = 2)          32 x 32 inputs 0.90 0.80 0.77 0.75 0.82, 20 x 20 1.02 0.99 1.08 1.09 0.94; size kept, 24 x 24 0.79 - 1.25 - 1.55
+//   grown by 1.5 (K = 3)    7 x 7 0.60 0.82 1.02 1.27 1.20, 9 x 9 0.73 0.55 0.75 0.79 0.68, 16 x 16 0.78 0.56 0.81 0.98 1.17, 32 x 32 0.78 0.55
+//                           0.77 0.92 1.09 (fp64 - 0.56 - 0.83 0.75)
+//   grown by 2 (K = 4)      6 x 6 0.92 0.78 0.86 1.19 1.34, 7 x 7 0.88 0.68 0.81 0.91 0.98, 16 x 16 1.47 0.94 0.61 0.62 0.92
+//   the same with corners   (K = 5), bf16 as well: 5 x 5 1.09 1.15 1.60 1.85 1.67, 16 x 16 1.41 0.88 0.60 0.74 0.81
+inline bool march_adjoint(const InterpGeom& g, int K, double per, long long tail, long long outputs, int esize) {
+  if (!g.linear || outputs < (1 << 20) || K > 5 || (esize < 4 && K != 5)) return false;
+  if (K == 2) return tail >= 1024 && step_of(g, 0) >= 1.9;
+  if (K == 3) return tail >= 81 && (esize == 8 || outputs <= (1 << 23));
+  return tail >= 49 && (per < 3.4 || outputs >= (3 << 20));
+}
+
 template <typename T, int ND>
 int run_cuda(int adjoint, const InterpGeom& g, T* x, T* y, long long BC, cudaStream_t s) {
   const long long in_plane = (long long)g.in_local[0] * g.in_local[1] * g.in_local[2];
@@ -708,12 +780,13 @@ int run_cuda(int adjoint, const InterpGeom& g, T* x, T* y, long long BC, cudaStr
     // weight zero
     if (in_plane <= 0) return (int)cudaMemsetAsync(y, 0, (size_t)(BC * out_plane) * sizeof(T), s);
     const bool small = in_plane < 0x7fffffffLL;
+    const int V = forward_vector<T>(g, small, y);
     if constexpr (ND >= 2) {
-      if (BC * out_plane >= kMarchFrom) {
-        const long long tail = out_plane / g.out_local[3 - ND];
+      const long long tail = out_plane / g.out_local[3 - ND];
+      if (march_forward(g, ND, tail, BC * out_plane, V, (int)sizeof(T))) {
         Segments sg;
         if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-          if (small && g.out_local[2] % 2 == 0 && (reinterpret_cast<uintptr_t>(y) & 3) == 0) {
+          if (V == 2) {
             const int t = plane_threads(tail / 2);
             const dim3 grid = march_grid(tail / 2, g.out_local[3 - ND], BC, t, sg);
             interp_fwd_march_kernel<T, ND, 2, int><<<grid, t, 0, s>>>(g, x, y, BC, sg);
@@ -728,7 +801,7 @@ int run_cuda(int adjoint, const InterpGeom& g, T* x, T* y, long long BC, cudaStr
       }
     }
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-      if (small && g.out_local[2] % 2 == 0 && (reinterpret_cast<uintptr_t>(y) & 3) == 0) {
+      if (V == 2) {
         const int t = plane_threads(out_plane / 2);
         interp_fwd_kernel<T, ND, 2, int><<<plane_grid(out_plane / 2, BC, t), t, 0, s>>>(g, x, y, BC);
         return (int)cudaGetLastError();
@@ -741,27 +814,14 @@ int run_cuda(int adjoint, const InterpGeom& g, T* x, T* y, long long BC, cudaStr
   }
   if (BC * in_plane <= 0) return 0;
   if (out_plane <= 0) return (int)cudaMemsetAsync(x, 0, (size_t)(BC * in_plane) * sizeof(T), s);
-  // outputs per input and dimension, as a hint: a position that has more takes the slow way by itself
-  double per = 1.0;
-  double lead_step = 0.0;
-  int least = g.out_local[2];                       // the smallest extent must hold a whole window
-  for (int d = 2; d >= 3 - ND; --d) {
-    if (g.out_local[d] < least) least = g.out_local[d];
-    double step = g.scale[d];
-    if (g.linear && g.align_corners)
-      step = g.out_global[d] > 1 ? (double)(g.in_global[d] - 1) / (double)(g.out_global[d] - 1) : 0.0;
-    const double n = step > 0.0 ? std::ceil((g.linear ? 2.0 : 1.0) / step - 1e-9) : (double)g.out_local[d];
-    if (n > per) per = n;
-    lead_step = step;
-  }
-  const int K = per <= 2.0 && least >= 2 ? 2 : per <= 3.0 && least >= 3 ? 3 : per <= 4.0 && least >= 4 ? 4
-                : per <= 5.0 && least >= 5 ? 5 : 32;
+  double per;
+  const int K = adjoint_window(g, ND, BC * out_plane, (int)sizeof(T), &per);
   if constexpr (ND == 3) {
     const long long tail = in_plane / g.in_local[0];
     const int t = plane_threads(tail);
     Segments sg;
     const dim3 grid = march_grid(tail, g.in_local[0], BC, t, sg);
-    if (BC * out_plane >= kMarchFrom && (sizeof(T) >= 4 || K == 5) && K <= 5 && march_fits(g, sg, lead_step)) {
+    if (march_adjoint(g, K, per, tail, BC * out_plane, (int)sizeof(T)) && march_fits(g, sg, step_of(g, 0))) {
       if (K == 5) interp_adjoint_march_kernel<T, 5><<<grid, t, 0, s>>>(g, x, y, BC, sg);
       if constexpr (sizeof(T) >= 4) {
         if (K == 2)      interp_adjoint_march_kernel<T, 2><<<grid, t, 0, s>>>(g, x, y, BC, sg);
@@ -806,17 +866,8 @@ int run(int cuda, int adjoint, const InterpGeom& g, int nd, void* x, void* y, lo
   }
 }
 
-}  // namespace
-
-// nd in 1..3; all int arrays have nd entries; scale[d] = source step per output
-// index (1 / scale_factor, or in_global / out_global).  Forward: y = I(x).
-// Adjoint: x = I^T(y) (on the CPU x += I^T(y) into an x that the caller has zeroed).
-// dtype: 0 fp32, 1 fp64, 2 bf16 (CUDA only; weights and sums in fp32).
-DD_API int dd_interpolate(int cuda, int linear, int adjoint, int dtype, int nd, void* x, void* y, long long BC,
-                          const int* in_local, const int* out_local, const int* x_off, const int* y_off,
-                          const int* in_global, const int* out_global, const double* scale, int align_corners,
-                          void* stream) {
-  if (nd < 1 || nd > 3 || BC < 0) return DD_ERR_BAD_ARG;
+InterpGeom make_geom(int linear, int nd, const int* in_local, const int* out_local, const int* x_off, const int* y_off,
+                     const int* in_global, const int* out_global, const double* scale, int align_corners) {
   InterpGeom g;
   for (int d = 0; d < 3; ++d) {
     const int s = d - (3 - nd);     // leading dims are padded with extent 1
@@ -833,6 +884,21 @@ DD_API int dd_interpolate(int cuda, int linear, int adjoint, int dtype, int nd, 
   }
   g.align_corners = align_corners;
   g.linear = linear;
+  return g;
+}
+
+}  // namespace
+
+// nd in 1..3; all int arrays have nd entries; scale[d] = source step per output
+// index (1 / scale_factor, or in_global / out_global).  Forward: y = I(x).
+// Adjoint: x = I^T(y) (on the CPU x += I^T(y) into an x that the caller has zeroed).
+// dtype: 0 fp32, 1 fp64, 2 bf16 (CUDA only; weights and sums in fp32).
+DD_API int dd_interpolate(int cuda, int linear, int adjoint, int dtype, int nd, void* x, void* y, long long BC,
+                          const int* in_local, const int* out_local, const int* x_off, const int* y_off,
+                          const int* in_global, const int* out_global, const double* scale, int align_corners,
+                          void* stream) {
+  if (nd < 1 || nd > 3 || BC < 0) return DD_ERR_BAD_ARG;
+  const InterpGeom g = make_geom(linear, nd, in_local, out_local, x_off, y_off, in_global, out_global, scale, align_corners);
   // (an empty tensor has no address, and so has one without storage, which must not reach a kernel)
   long long n_in = BC, n_out = BC;
   for (int d = 0; d < 3; ++d) { n_in *= g.in_local[d]; n_out *= g.out_local[d]; }
@@ -840,4 +906,26 @@ DD_API int dd_interpolate(int cuda, int linear, int adjoint, int dtype, int nd, 
   if (dtype == 0) return run<float>(cuda, adjoint, g, nd, x, y, BC, stream);
   if (dtype == 1) return run<double>(cuda, adjoint, g, nd, x, y, BC, stream);
   return run<__nv_bfloat16>(cuda, adjoint, g, nd, x, y, BC, stream);
+}
+
+// Whether the call above walks sheets (or rows) on the GPU, for tests.
+DD_API int dd_interpolate_marches(int linear, int adjoint, int dtype, int nd, long long BC, const int* in_local,
+                                  const int* out_local, const int* x_off, const int* y_off, const int* in_global,
+                                  const int* out_global, const double* scale, int align_corners) {
+  if (nd < 1 || nd > 3) return 0;
+  const InterpGeom g = make_geom(linear, nd, in_local, out_local, x_off, y_off, in_global, out_global, scale, align_corners);
+  const long long in_plane = (long long)g.in_local[0] * g.in_local[1] * g.in_local[2];
+  const long long out_plane = (long long)g.out_local[0] * g.out_local[1] * g.out_local[2];
+  if (in_plane <= 0 || out_plane <= 0) return 0;
+  const int esize = dtype == 0 ? 4 : dtype == 1 ? 8 : 2;
+  if (!adjoint) {
+    const bool pairs = dtype == 2 && in_plane < 0x7fffffffLL && g.out_local[2] % 2 == 0;
+    return nd >= 2 && march_forward(g, nd, out_plane / g.out_local[3 - nd], BC * out_plane, pairs ? 2 : 1, esize);
+  }
+  double per;
+  const int K = adjoint_window(g, nd, BC * out_plane, esize, &per);
+  const long long tail = in_plane / g.in_local[0];
+  Segments sg;
+  march_grid(tail, g.in_local[0], BC, plane_threads(tail), sg);
+  return nd == 3 && march_adjoint(g, K, per, tail, BC * out_plane, esize) && march_fits(g, sg, step_of(g, 0));
 }

@@ -211,7 +211,7 @@ def test_interpolation_kernels_over_scales(mode, ac, n_in, n_out, dtype):
     ("linear", False, 300, (70, 33, 30), (35, 16, 15)),  # fewer outputs than inputs: inputs that none takes
     ("nearest", False, 120, (33, 10, 9), (99, 21, 10))])
 def test_interpolation_marches_over_large_tensors(mode, ac, planes, n_in, n_out, dtype):
-    """From a million outputs on, a thread walks the sheets of a volume (rows of an image): segments and their ends,
+    """A million outputs and more, most of which a thread takes sheet by sheet of a volume (row by row of an image):
     sub-ranges of the output, infinities; against the CPU code in fp64 with the bounds of the test above."""
     from distdl_b200.functional.interpolate import interpolate
     torch.manual_seed(6)
@@ -232,6 +232,49 @@ def test_interpolation_marches_over_large_tensors(mode, ac, planes, n_in, n_out,
     bad = x.clone()
     bad[:, :, -1] = float("inf")
     assert torch.equal(interpolate(bad.cuda(), *args).isfinite().cpu(), interpolate(bad.double(), *args).isfinite())
+
+
+@pytest.mark.parametrize("mode,ac,planes,n_in,n_out,forward,adjoint", [
+    ("linear", False, 110, (35, 81), (70, 162), "fp32 fp64 bf16", ""),       # rows: three segments, the last one shorter
+    ("linear", True, 140, (41, 120), (82, 161), "fp32 fp64 bf16", ""),       # rows of an odd length
+    ("nearest", False, 60, (33, 20, 9), (99, 21, 20), "fp32 bf16", ""),
+    ("linear", False, 70, (34, 12, 14), (51, 18, 21), "fp32 bf16", "fp32 fp64"),           # three outputs take an input
+    ("linear", False, 235, (33, 8, 8), (66, 16, 16), "fp32 fp64 bf16", "fp32 fp64"),            # four
+    ("linear", True, 85, (34, 17, 10), (68, 34, 20), "fp32 bf16", "fp32 fp64 bf16"),      # five
+    ("linear", False, 160, (70, 33, 34), (35, 16, 17), "", "fp32 fp64")])                      # two, of some none
+@pytest.mark.parametrize("slab", [False, True])
+def test_interpolation_sheet_by_sheet(mode, ac, planes, n_in, n_out, forward, adjoint, slab):
+    """Where the rules say that sheets (rows) are walked, whole tensors and slabs that begin and end inside, with a halo of
+    their own input: segments and their ends, infinities; against the CPU code in fp64 with the bounds of the test above."""
+    from test_interpolate_routes import marches
+
+    from distdl_b200.functional.interpolate import interpolate
+    for name, dtype, code in (("fp32", torch.float32, 0), ("fp64", torch.float64, 1), ("bf16", torch.bfloat16, 2)):
+        torch.manual_seed(6)
+        tol = {torch.float32: 2e-6, torch.float64: 1e-13, torch.bfloat16: 8e-3}[dtype]
+        gi, go = list(n_in), list(n_out)
+        lo, hi, x_lo, x_hi = [0] * len(gi), list(go), [0] * len(gi), list(gi)
+        if slab:                                          # the leading dimension cut off at both ends, the last at its end
+            lo[0], hi[0], hi[-1] = 3, go[0] - 2, go[-1] - 2
+            step = (gi[0] - 1) / (go[0] - 1) if ac else gi[0] / go[0]
+            at = lambda o: o * step if ac or mode == "nearest" else max(0.0, (o + 0.5) * step - 0.5)  # noqa: E731
+            x_lo[0], x_hi[0] = int(at(lo[0])), min(int(at(hi[0] - 1)) + 2, gi[0])
+        n_x, n_y = [b - a for a, b in zip(x_lo, x_hi)], [b - a for a, b in zip(lo, hi)]
+        route = dict(linear=int(mode == "linear"), corners=int(ac), x_off=x_lo, y_off=lo, in_global=gi, out_global=go)
+        assert marches(0, code, planes, n_x, n_y, **route) or name not in forward
+        assert marches(1, code, planes, n_x, n_y, **route) or name not in adjoint
+        x = torch.randn(1, planes, *n_x).to(dtype)
+        args = (x_lo, x_hi, gi, lo, hi, go, None, mode, ac)
+        xc, xg = x.double().clone().requires_grad_(), x.cuda().requires_grad_()
+        yc, yg = interpolate(xc, *args), interpolate(xg, *args)
+        assert (yg.double().cpu() - yc).abs().max() <= tol * yc.abs().max()
+        dy = torch.randn(yc.shape).to(dtype)
+        yc.backward(dy.double())
+        yg.backward(dy.cuda())
+        assert (xg.grad.double().cpu() - xc.grad).abs().max() <= tol * (1 + xc.grad.abs().max())
+        bad = x.clone()
+        bad[:, :, -1] = float("inf")
+        assert torch.equal(interpolate(bad.cuda(), *args).isfinite().cpu(), interpolate(bad.double(), *args).isfinite())
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16])
