@@ -800,9 +800,12 @@ inline int grid_for(long long work, int threads, int cap_mult = 16) {
   if (b < 1) b = 1;
   return (int)b;
 }
-// One vector per thread where tensors are larger than L2 and nothing is carried from one vector to the next: CTAs that end
-// and start keep memory busier than a grid that walks in strides.  In us, strides -> full: AdamW on 6.3e8 values 3 435 -> 3 089
-// (6.23 -> 6.92 TB/s), SwiGLU 8192 x 14336 121 -> 106 and backward 192 -> 172; but 3000 x 5632 16.4 -> 17.5, GELU of 2.6e7 18.4 -> 20.3.
+// One vector of 16 bytes per thread from 32769 CTAs of 256 on (a tensor of 134 MB or more of those read and written, beyond L2),
+// where nothing is carried from one vector to the next: CTAs that end and start keep memory busier than a grid that walks in
+// strides.  In us, strides -> full: AdamW on 6.3e8 values 3 435 -> 3 089 (6.23 -> 6.92 TB/s), SwiGLU 8192 x 14336 121 -> 106 and
+// backward 192 -> 172, gradient of GELU 2.1e8 217 -> 203, addition of 7.1e7 66 -> 61 and 4.2e8 392 -> 349; but 3000 x 5632 16.4 -> 17.5.
+// Not for GELU forward (2.1e8 131 -> 139) nor for the casts, whose threads take one value each: 1.0e7 fp32 -> bf16 7.5 -> 32.8, back 8.7
+// -> 36.0, added 12.3 -> 36.4, and 2.1e8 211 -> 735, 253 -> 767, 474 -> 817, since CTAs then cost more to start than what they move.
 inline int grid_wide(long long work, int threads) {
   const long long b = (work + threads - 1) / threads;
   return b > 32768 ? (int)(b < 0x7fffffffLL ? b : 0x7fffffffLL) : grid_for(work, threads);
@@ -901,7 +904,7 @@ DD_API int dd_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long 
 }
 DD_API int dd_gelu_fwd(const void* x, void* y, long long n, void* stream) {
   if (n % 8) return DD_ERR_BAD_ARG;
-  gelu_fwd_kernel<<<grid_wide(n / 8, 256), 256, 0, STREAM(stream)>>>(CBF(x), BF(y), n / 8);
+  gelu_fwd_kernel<<<grid_for(n / 8, 256), 256, 0, STREAM(stream)>>>(CBF(x), BF(y), n / 8);
   return (int)cudaGetLastError();
 }
 DD_API int dd_gelu_bwd(const void* dy, const void* x, void* dx, long long n, void* stream) {
@@ -986,12 +989,12 @@ DD_API int dd_add_bf16(const void* a, const void* b, void* y, long long n, void*
 }
 DD_API int dd_cast_f32_bf16(const float* src, void* dst, long long n, float scale, void* stream) {
   if (n <= 0) return DD_OK;
-  cast_f32_bf16_kernel<<<grid_wide(n, 256), 256, 0, STREAM(stream)>>>(src, BF(dst), n, scale);
+  cast_f32_bf16_kernel<<<grid_for(n, 256), 256, 0, STREAM(stream)>>>(src, BF(dst), n, scale);
   return (int)cudaGetLastError();
 }
 DD_API int dd_cast_bf16_f32(const void* src, float* dst, long long n, float scale, int accumulate, void* stream) {
   if (n <= 0) return DD_OK;
-  cast_bf16_f32_kernel<<<grid_wide(n, 256), 256, 0, STREAM(stream)>>>(CBF(src), dst, n, scale, accumulate);
+  cast_bf16_f32_kernel<<<grid_for(n, 256), 256, 0, STREAM(stream)>>>(CBF(src), dst, n, scale, accumulate);
   return (int)cudaGetLastError();
 }
 

@@ -2,6 +2,9 @@
 import pytest
 import torch
 
+from distdl_b200 import _native
+from distdl_b200.ops._util import stream_ptr
+
 pytestmark = pytest.mark.gpu
 
 
@@ -420,3 +423,46 @@ def test_wide_grids_match_narrow_ones():
         part = h.detach()[rows].clone().requires_grad_()
         want = ops.swiglu(part)
         assert torch.equal(y[rows], want) and torch.equal(dh[rows], torch.autograd.grad(want, part, dy[rows])[0])
+    n = 8 * 256 * 32768 + 8 * 256
+    a, b, y = (torch.randn(n, device="cuda").bfloat16() for _ in range(3))
+    _native.call("dd_add_bf16", a.data_ptr(), b.data_ptr(), y.data_ptr(), n, stream_ptr())
+    assert torch.equal(y, a + b)
+    x = a.requires_grad_()
+    y = ops.gelu(x)
+    dx, = torch.autograd.grad(y, x, b)
+    for part in (slice(0, 1 << 20), slice(n - (1 << 20), n)):
+        p = x.detach()[part].clone().requires_grad_()
+        want = ops.gelu(p)
+        assert torch.equal(y[part], want) and torch.equal(dx[part], torch.autograd.grad(want, p, b[part])[0])
+
+
+@pytest.mark.parametrize("cast", ["fp32 to bf16", "bf16 to fp32", "bf16 added to fp32"])
+def test_a_cast_takes_no_longer_than_its_parts(cast):
+    """16e6 values in one call against four calls of a quarter each, replayed from graphs: threads of one value each must not
+    bring a grid of as many CTAs (3.3 to 3.5 times as long; 1.8 where the sum is read as well)."""
+    n = 1 << 24
+    f, h = torch.randn(n, device="cuda"), torch.randn(n, device="cuda").bfloat16()
+
+    def run(lo, n):
+        if cast == "fp32 to bf16":
+            _native.call("dd_cast_f32_bf16", f[lo:].data_ptr(), h[lo:].data_ptr(), n, 1.0, stream_ptr())
+        else:
+            _native.call("dd_cast_bf16_f32", h[lo:].data_ptr(), f[lo:].data_ptr(), n, 1.0, int("added" in cast), stream_ptr())
+    run(0, n)
+    times = []
+    for part in (n, n // 4):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(5):
+                for lo in range(0, n, part):
+                    run(lo, part)
+        best = float("inf")
+        for _ in range(5):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            graph.replay()
+            end.record()
+            end.synchronize()
+            best = min(best, start.elapsed_time(end))
+        times.append(best)
+    assert times[0] < 1.2 * times[1]
