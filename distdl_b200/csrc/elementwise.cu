@@ -220,11 +220,13 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // dw/db partial sums per CTA go to `partial` ([gridDim.x][2][d] fp32, a scratch
 // buffer); norm_bwd_reduce_kernel folds them.  dx may alias dy.  WANT_DB: the
 // second half of a CTA's slice (db) is only accumulated and written when asked for.
-// If dres_in is given, it is added to dx (gradient of the residual stream).
+// RES: dres_in is added to dx (gradient of the residual stream).
 // Bound by the round trip of a group of rows (read, reduce over the CTA, write), so the next group is read meanwhile, and
 // the residual's gradient with it.  With the fold of dw and db, us: 8192 x 4096 75.8 -> 66.3, 3000 x 2048 16.4 -> 14.3, LayerNorm
-// 8192 x 8192 234 -> 146, 4096 x 1600 22.5 -> 21.1 (twice the rows per group, one group in flight before).
-template <bool RMS, int VEC, int R, bool WANT_DB>
+// 8192 x 8192 234 -> 146, 4096 x 1600 22.5 -> 21.1 (twice the rows per group, one group in flight before).  Without dres_in its
+// registers must not be there: 128 per thread are two CTAs per SM.  16384 x 2560 69 (before) -> 87 (with them) -> 60, LayerNorm 16384
+// x 424 33 -> 39 -> 34, 16384 x 2048 55 -> 65 -> 50, 16384 x 4096 154 -> 120 -> 81.
+template <bool RMS, int VEC, int R, bool WANT_DB, bool RES>
 __global__ void __launch_bounds__(kNormThreads)
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                 const __nv_bfloat16* __restrict__ w, const float2* __restrict__ stats,
@@ -267,7 +269,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
           const size_t at = (size_t)(row0 + r) * d + vi * 8;
           vdy[r][i] = *reinterpret_cast<const uint4*>(dy + at);
           vx[r][i] = *reinterpret_cast<const uint4*>(x + at);
-          if (dres_in != nullptr) vq[r][i] = *reinterpret_cast<const uint4*>(dres_in + at);
+          if (RES) vq[r][i] = *reinterpret_cast<const uint4*>(dres_in + at);
         }
       }
     }
@@ -322,7 +324,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
             const float xh = (xv[j] - mean[r]) * rstd[r];
             o[j] = rstd[r] * (dyv[j] * wv[i][j] - mg - xh * mgx);
           }
-          if (dres_in != nullptr) {
+          if (RES) {
             float q[8];
             unpack8(pq[r][i], q);
 #pragma unroll
@@ -838,15 +840,11 @@ static void launch_norm_fwd(int grid, cudaStream_t s, const void* x, const void*
 template <bool RMS, bool WANT_DB>
 static void launch_norm_bwd(int grid, cudaStream_t s, const void* dy, const void* x, const void* w, const void* stats,
                             const void* dres, void* dx, float* partial, int rows, int d) {
-  if (d <= 2048)
-    norm_bwd_kernel<RMS, 1, 2, WANT_DB><<<grid, kNormThreads, 0, s>>>(CBF(dy), CBF(x), CBF(w), (const float2*)stats,
-                                                                      CBF(dres), BF(dx), partial, rows, d);
-  else if (d <= 4096)
-    norm_bwd_kernel<RMS, 2, 1, WANT_DB><<<grid, kNormThreads, 0, s>>>(CBF(dy), CBF(x), CBF(w), (const float2*)stats,
-                                                                      CBF(dres), BF(dx), partial, rows, d);
-  else
-    norm_bwd_kernel<RMS, 4, 1, WANT_DB><<<grid, kNormThreads, 0, s>>>(CBF(dy), CBF(x), CBF(w), (const float2*)stats,
-                                                                      CBF(dres), BF(dx), partial, rows, d);
+  const bool res = dres != nullptr;
+  auto kernel = d <= 2048 ? (res ? norm_bwd_kernel<RMS, 1, 2, WANT_DB, true> : norm_bwd_kernel<RMS, 1, 2, WANT_DB, false>)
+                : d <= 4096 ? (res ? norm_bwd_kernel<RMS, 2, 1, WANT_DB, true> : norm_bwd_kernel<RMS, 2, 1, WANT_DB, false>)
+                            : (res ? norm_bwd_kernel<RMS, 4, 1, WANT_DB, true> : norm_bwd_kernel<RMS, 4, 1, WANT_DB, false>);
+  kernel<<<grid, kNormThreads, 0, s>>>(CBF(dy), CBF(x), CBF(w), (const float2*)stats, CBF(dres), BF(dx), partial, rows, d);
 }
 static void launch_norm_bwd_any(int rms, bool want_db, int grid, cudaStream_t s, const void* dy, const void* x,
                                 const void* w, const void* stats, const void* dres, void* dx, float* partial,
@@ -862,8 +860,9 @@ static void launch_norm_bwd_any(int rms, bool want_db, int grid, cudaStream_t s,
 
 // CTAs of the backward kernel = slices of its partial-sum scratch.
 DD_API int dd_norm_bwd_parts(int rows) {
-  // two CTAs per SM are resident (about 126 registers per thread): more of them would only run one after the
-  // other and write more partial sums (3000 x 2048: 592 CTAs 20.2 us, 296 19.5 us; 4096 x 1600 with bias 29.4 and 24.4 us)
+  // two CTAs per SM are resident up to 4096 columns (94 to 127 registers per thread; beyond, 156 to 208, one is): more of
+  // them would only run one after the other and write more partial sums (before the next rows were read ahead, 3000 x 2048: 592
+  // CTAs 20.2 us, 296 19.5 us; 4096 x 1600 with bias 29.4 and 24.4 us)
   const int groups = (rows + 1) / 2;
   return groups < 148 * 2 ? (groups > 0 ? groups : 1) : 148 * 2;
 }
