@@ -11,6 +11,7 @@
 // element, are single and meet in L1.  [8, 64, 256, 256] bf16 by one on every side: 31 us (fill and strided
 // copy: 98), the crop 26 us (strided copy: 81).
 #include "common.cuh"
+#include "runtime.cuh"
 
 namespace {
 
@@ -182,6 +183,16 @@ from_channels_last_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict
   }
 }
 
+// Words of a position that a CTA takes: as many as leave no more than a fifth of the threads without channels; 32 bytes or
+// more, a sector.  Into channels-last memory 32 of them where there are too few CTAs to fill the SMs ten times: each has fewer
+// positions to decode then, and idle threads cost nothing.  us, 32 words -> fewer: [1, 8, 80^2] 2.3 -> 3.5, [8, 8, 80^2] 3.3 -> 3.7, [4, 24,
+// 120^2] 4.1 -> 4.1; [8, 8, 120^2] 5.3 -> 3.9, [4, 24, 160^2] 5.7 -> 5.1.  Back it makes no difference (2.5 -> 2.3 for the first).
+int channel_words(int to_last, int B, int C, long long positions) {
+  auto fits = [C](int w) { return (C + w * 2 - 1) / (w * 2) * (w * 2) * 4 <= C * 5; };
+  if (to_last && (positions + 63) / 64 * ((C + 63) / 64) * B < 10LL * dd::current_sm_count()) return 32;
+  return C <= 8 ? 4 : fits(32) ? 32 : fits(16) ? 16 : 8;
+}
+
 template <int W>
 int launch_channels(const uint16_t* src, uint16_t* dst, int to_last, int B, int C, const ShiftGeom& g, cudaStream_t s) {
   const long long n = (long long)g.out[0] * g.out[1] * g.out[2];
@@ -225,10 +236,14 @@ DD_API int dd_shift_channels(const void* src, void* dst, int to_last, int B, int
   const uint16_t* from = reinterpret_cast<const uint16_t*>(src);
   uint16_t* to = reinterpret_cast<uint16_t*>(dst);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  // as many words of a position as leave no more than a fifth of the threads without channels; 32 bytes or more, a sector
-  auto fits = [C](int w) { return (C + w * 2 - 1) / (w * 2) * (w * 2) * 4 <= C * 5; };
-  if (C <= 8) return launch_channels<4>(from, to, to_last, B, C, g, st);
-  if (fits(32)) return launch_channels<32>(from, to, to_last, B, C, g, st);
-  if (fits(16)) return launch_channels<16>(from, to, to_last, B, C, g, st);
-  return launch_channels<8>(from, to, to_last, B, C, g, st);
+  const int words = channel_words(to_last, B, C, (long long)g.out[0] * g.out[1] * g.out[2]);
+  if (words == 4) return launch_channels<4>(from, to, to_last, B, C, g, st);
+  if (words == 8) return launch_channels<8>(from, to, to_last, B, C, g, st);
+  if (words == 16) return launch_channels<16>(from, to, to_last, B, C, g, st);
+  return launch_channels<32>(from, to, to_last, B, C, g, st);
+}
+
+// The words of a position that a CTA takes in the call above, for tests.
+DD_API int dd_shift_channels_words(int to_last, int B, int C, long long positions) {
+  return channel_words(to_last, B, C, positions);
 }

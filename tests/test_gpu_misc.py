@@ -422,9 +422,11 @@ def test_padding_into_channels_last_and_back(space, pads, C, dtype):
 
 
 @pytest.mark.parametrize("space,C", [((2, 17, 19), 8), ((30, 21), 64), ((5, 300), 16), ((11, 13, 7), 40), ((33, 34), 48),
-                                     ((12, 31), 56), ((65, 3), 128)])
+                                     ((12, 31), 56), ((65, 3), 128), ((330, 301), 8), ((17, 77, 79), 24), ((301, 333), 40),
+                                     ((221, 247), 88)])
 def test_channel_tiles_follow_the_number_of_channels(space, C):
-    """Tiles of 4 to 32 pairs of channels, positions on and beyond their edges, channels that do not fill the last one."""
+    """Tiles of 4 to 32 pairs of channels, positions on and beyond their edges, channels that do not fill the last one; the
+    narrow ones into channels-last memory only for the last sizes, back for all."""
     import torch.nn.functional as F
 
     from distdl_b200.ops.pad import channels_first, pad_channels_last
