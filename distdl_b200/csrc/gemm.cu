@@ -13,7 +13,8 @@ using namespace dd::gemm;
 
 namespace {
 template <bool A_MN, bool B_MN>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, const Plan& plan, int ctas, cudaStream_t stream) {
+int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, const Plan& plan, int ctas, bool ahead,
+           cudaStream_t stream) {
   const int grid = plan.items < ctas ? plan.items : ctas;
   static bool configured[64] = {false};
   int dev = 0;
@@ -24,7 +25,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, const 
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = true;
   }
-  return launch_ahead(kern, grid, NUM_THREADS, SMEM_BYTES, stream, !(p.flags & F_ALONE), ta, tb, p, plan);
+  return launch_ahead(kern, grid, NUM_THREADS, SMEM_BYTES, stream, ahead, ta, tb, p, plan);
 }
 template <bool A_MN, bool B_MN, int NB>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p, int pairs,
@@ -138,6 +139,7 @@ enum Kernel : int { SINGLE, PAIR, PAIR_HALF, WIDE };
 struct Choice {
   Kernel kernel;
   int ctas, group_m;
+  bool ahead;                        // launched ahead of the end of the kernel before it
   Plan single;                       // (of the kernel that is taken; the others are not set)
   dd::gemm2::Plan pair;
   dd::gemm4::Plan wide;
@@ -148,6 +150,7 @@ struct Choice {
 Choice choose(int M, int N, int K, int batch, int flags, int max_ctas, bool rows, bool bound_k, long long a_span) {
   Choice c = {};
   const int sms = current_sm_count();
+  c.ahead = !(max_ctas > 0 && max_ctas < sms);
   // CTA pairs (cta_group::2) unless disabled or the problem is a single tile row
   static const bool pair_ok = []() { const char* e = getenv("DISTDL_GEMM_PAIR"); return !(e && e[0] == '0'); }();
   if (!pair_ok || M <= BM) {
@@ -155,6 +158,11 @@ Choice choose(int M, int N, int K, int batch, int flags, int max_ctas, bool rows
     c.ctas = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
     c.group_m = 8;
     c.single = make_plan(M, N, batch, c.ctas, a_span);
+    // Many CTAs on an A that lies close together are slower on SMs that the product before leaves idle (they wait for one
+    // another's reads, see make_plan, more so the more uneven they lie).  Products of different weights in a chain, us, not ahead
+    // -> ahead: 1 x 14336 x 4096 (56 items) 36 -> 42, 8 x 24576 x 4096 49 -> 54, 1 x 50176 x 8192 162 -> 167; 1 x 12288 x 1024 (48 items)
+    // 12.5 -> 11.3, 33 x 14336 x 4096 (no such A) 29.5 -> 28.6.
+    if (a_span < kNearA && c.single.items > 48) c.ahead = false;
     return c;
   }
   c.ctas = sms & ~1;
@@ -236,10 +244,10 @@ int gemm_bf16(const void* A, int a_mn, long long lda, long long strideA, const v
   else      r = get_tensor_map_bf16_3d(&tb, B, K, N, batch, ldb * 2, strideB * 2, BK, 64);
   if (r) return r;
   if (c.kernel == SINGLE) {
-    if (a_mn && b_mn) return launch<true, true>(ta, tb, p, c.single, c.ctas, s);
-    if (a_mn) return launch<true, false>(ta, tb, p, c.single, c.ctas, s);
-    if (b_mn) return launch<false, true>(ta, tb, p, c.single, c.ctas, s);
-    return launch<false, false>(ta, tb, p, c.single, c.ctas, s);
+    if (a_mn && b_mn) return launch<true, true>(ta, tb, p, c.single, c.ctas, c.ahead, s);
+    if (a_mn) return launch<true, false>(ta, tb, p, c.single, c.ctas, c.ahead, s);
+    if (b_mn) return launch<false, true>(ta, tb, p, c.single, c.ctas, c.ahead, s);
+    return launch<false, false>(ta, tb, p, c.single, c.ctas, c.ahead, s);
   }
   p.rows = rows; p.bound_k = bound_k;
   memset(&td, 0, sizeof(td));
@@ -289,8 +297,8 @@ DD_API int dd_gemm_bf16_rows(const void* A, int a_mn, long long lda, long long s
 }
 
 // What the entries above would do with a contiguous A and an output that TMA can write, for tests: the kernel (0 single CTA, 1
-// pair, 2 pair with half tiles, 3 512 x 256 per pair), CTAs at most, order of tiles, whole tiles, work items, and parts of a tile
-// behind the whole ones.
+// pair, 2 pair with half tiles, 3 512 x 256 per pair), CTAs at most, order of tiles, whole tiles, work items, parts of a tile
+// behind the whole ones, and whether it is launched ahead.
 DD_API int dd_gemm_plan(int M, int N, int K, int batch, int flags, int max_ctas, int rows, int bound_k, int* out) {
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return DD_ERR_BAD_ARG;
   const Choice c = choose(M, N, K, batch, flags | F_TMA_EPI, max_ctas, rows != 0, bound_k != 0, 2ll * batch * M * K);
@@ -298,6 +306,7 @@ DD_API int dd_gemm_plan(int M, int N, int K, int batch, int flags, int max_ctas,
   out[3] = c.kernel == SINGLE ? c.single.full : c.kernel == WIDE ? c.wide.full : c.pair.full;
   out[4] = c.kernel == SINGLE ? c.single.items : c.kernel == WIDE ? c.wide.items : c.pair.items;
   out[5] = c.kernel == SINGLE ? c.single.parts : 2;
+  out[6] = c.ahead;
   return DD_OK;
 }
 

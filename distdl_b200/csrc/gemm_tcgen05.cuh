@@ -170,12 +170,13 @@ __device__ __forceinline__ void store_chunk(const Params& p, uint32_t (&acc)[32]
 // no more than 32 items there.  Whole tiles, halves, quarters, each alone with a cold L2: 4 x 4096 x 4096 34.8, 30.8, 38.9, 1 x 8192 x
 // 4096 39, 43, 47, 1 x 4096 x 8192 60, 53, 70 (8 rows, 128 KB: 60, 53, 49), 1 x 2048 x 4096 32.8, 28.7, 28.6; two of 1 x 4096 x 4096 39
 // and, in quarters, 45.
+constexpr long long kNearA = 128 << 10;
 struct Plan {
   int tiles_m, tiles_n, full, parts, items;
 };
 inline Plan make_plan(int M, int N, int batch, int ctas, long long a_span) {
   Plan w;
-  const int room = a_span < (128 << 10) && ctas > 32 ? 32 : ctas;
+  const int room = a_span < kNearA && ctas > 32 ? 32 : ctas;
   w.tiles_m = (M + BM - 1) / BM;
   w.tiles_n = (N + BN - 1) / BN;
   const int tiles = w.tiles_m * w.tiles_n * batch, rest = tiles <= ctas ? tiles : tiles % ctas;

@@ -12,9 +12,9 @@ F_OUT_F32 = 1
 
 
 def plan(M, N, K, batch=1, flags=0, max_ctas=0, rows=0, bound_k=0):
-    out = (ctypes.c_int * 6)()
+    out = (ctypes.c_int * 7)()
     assert _native.lib().dd_gemm_plan(M, N, K, batch, flags, max_ctas, rows, bound_k, out) == 0
-    return dict(zip(("kernel", "ctas", "group", "full", "items", "parts"), out))
+    return dict(zip(("kernel", "ctas", "group", "full", "items", "parts", "ahead"), out))
 
 
 @pytest.fixture(autouse=True)
@@ -32,3 +32,12 @@ def test_few_rows_that_lie_close_together_are_read_by_few_ctas(M, N, K, batch, i
     """An A of less than 128 KB in no more than 32 parts of tiles: in more, the CTAs wait for one another's reads of it."""
     p = plan(M, N, K, batch)
     assert p["kernel"] == SINGLE and p["items"] == items
+
+
+@pytest.mark.parametrize("M,N,K,max_ctas,ahead", [
+    (1, 14336, 4096, 0, 0), (8, 24576, 4096, 0, 0), (1, 4096, 4096, 0, 1), (1, 12288, 4096, 0, 1), (33, 14336, 4096, 0, 1),
+    (4096, 4096, 4096, 0, 1), (33, 14336, 4096, 64, 0), (4096, 4096, 4096, 64, 0), (8192, 8192, 8192, 64, 0),
+    (4096, 4096, 4096, 148, 1)])
+def test_products_that_are_launched_ahead(M, N, K, max_ctas, ahead):
+    """Not those that are limited to some SMs, nor many CTAs that read an A of less than 128 KB."""
+    assert plan(M, N, K, max_ctas=max_ctas)["ahead"] == ahead
