@@ -127,8 +127,12 @@ bool half_tiles(int M, int N, int batch, bool f32, long long pairs, long long* w
 // that is read again from memory costs clock: a panel of the operand with fewer rows is kept in L2 (up to 36 MB of it; 67
 // MB no longer stay) while the other one streams past it, but at least 8 tiles wide, so that the tiles in flight are about
 // square.  In us, back to back, 4 rows before -> now: 8192 x 28672 x 4096 1634 -> 1425 (8 rows 1527), 4096 x 50304 x 1600
-// 570 -> 517, 3000 x 32000 x 2048 341 -> 311; 8192 x 4096 x 28672 1619 -> 1511 by columns (8 rows 1529).
+// 570 -> 517, 3000 x 32000 x 2048 341 -> 311; 8192 x 4096 x 28672 1619 -> 1511 by columns (8 rows 1529).  A contraction of up to
+// 512 moves more of D than of its operands, which stay in L2 anyway, and memory takes whole rows of D sooner than strips of them:
+// four rows of tiles, 7582 x 9272 x 64 bf16 57 -> 62 us with a panel of thirty, x 256 60 -> 66, x 512 added in fp32 137 -> 143, but x
+// 1024 112 -> 106.
 int tile_group(int M, int N, int K) {
+  if (K <= 512) return 4;
   const int tiles = (min(M, N) + 255) / 256;
   const int g = min(tiles, max(8, (int)(36000000ll / (512ll * K))));
   return M <= N ? g : -g;

@@ -41,3 +41,11 @@ def test_few_rows_that_lie_close_together_are_read_by_few_ctas(M, N, K, batch, i
 def test_products_that_are_launched_ahead(M, N, K, max_ctas, ahead):
     """Not those that are limited to some SMs, nor many CTAs that read an A of less than 128 KB."""
     assert plan(M, N, K, max_ctas=max_ctas)["ahead"] == ahead
+
+
+@pytest.mark.parametrize("M,N,K,group", [(7582, 9272, 64, 4), (9272, 7584, 512, 4), (8192, 28672, 4096, 17), (4096, 50304, 1600, 16),
+                                         (28672, 8192, 4096, -17), (2304, 2816, 1024, 9), (16384, 16384, 16384, 8)])
+def test_order_of_tiles(M, N, K, group):
+    """Rows of D for short contractions, else a panel of up to 36 MB of the smaller operand."""
+    p = plan(M, N, K)
+    assert p["group"] == group and p["kernel"] in (PAIR, WIDE)
