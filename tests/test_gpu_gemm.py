@@ -258,16 +258,22 @@ def test_batched_gemm_with_half_tiles(B, M, N, K, a_mn, b_mn):
     assert _native.read_status()[0] == 0
 
 
-@pytest.mark.parametrize("B,M,N,K,ctas", [(1, 257, 200, 4104, 2), (1, 512, 456, 4160, 4), (1, 1000, 520, 4168, 4),
-                                          (3, 1288, 456, 4224, 6), (1, 2400, 200, 4160, 4)])
+@pytest.mark.parametrize("B,M,N,K,ctas", [
+    (1, 257, 200, 4104, 2), (1, 512, 456, 4160, 4), (1, 1000, 520, 4168, 4), (3, 1288, 456, 4224, 6), (1, 2400, 200, 4160, 4),
+    (3, 4300, 500, 4104, 18),        # 17 blocks: single ones before whole tiles, on either accumulator
+    (1, 4300, 500, 4160, 8),         # the single ones in a last wave of their own, which has none beyond them
+    (1, 6000, 5000, 4160, 0)])
 @pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 0), (1, 1)])
 def test_gemm_with_wide_tiles(B, M, N, K, ctas, a_mn, b_mn):
     """Contractions beyond 4096 take 512 x 256 per pair of CTAs: an odd number of 256-row blocks, a last wave in single
-    blocks, remainders in every direction, both majors.  bf16 results as above; fp32 sums of 16 terms, 264 of them cut
-    off at 2**-23, are off by less than 264 / 2 * 2**-23 = 1.6e-5."""
+    blocks, remainders in every direction, both majors, few pairs and all.  bf16 results as above; fp32 sums of 16 terms, 264
+    of them cut off at 2**-23, are off by less than 264 / 2 * 2**-23 = 1.6e-5."""
+    from test_gemm_plan import WIDE, plan
+
     from distdl_b200 import _native
     from distdl_b200.ops import gemm
     torch.manual_seed(7)
+    assert all(plan(M, N, K, B, flags, ctas)["kernel"] == WIDE for flags in (0, 1))
 
     def make(rows, cols, mn):
         n, m = (cols, rows) if mn else (rows, cols)
@@ -320,14 +326,19 @@ def test_gemm_whose_last_wave_is_taken_in_halves(B, M, N, K, ctas, a_mn, b_mn):
     assert _native.read_status()[0] == 0
 
 
-@pytest.mark.parametrize("B,M,N,K,ctas", [(1, 33, 1000, 136, 0), (1, 128, 264, 72, 3), (1, 77, 1160, 200, 4), (2, 20, 2312, 64, 4),
-                                          (1, 1, 520, 1600, 12)])
+@pytest.mark.parametrize("B,M,N,K,ctas,parts", [
+    (1, 33, 1000, 136, 0, 4), (1, 128, 264, 72, 3, 1), (1, 77, 1160, 200, 4, 4), (2, 20, 2312, 64, 4, 4), (1, 1, 520, 1600, 12, 4),
+    (1, 20, 264, 136, 4, 2), (1, 128, 14336, 1600, 0, 2), (1, 33, 10240, 2048, 0, 2)])
 @pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 0), (1, 1)])
-def test_gemm_of_few_rows_in_parts_of_tiles(B, M, N, K, ctas, a_mn, b_mn):
+def test_gemm_of_few_rows_in_parts_of_tiles(B, M, N, K, ctas, parts, a_mn, b_mn):
     """One row of tiles: quarters and halves of the only or of the last wave, some behind the matrix (bounds as above)."""
+    from test_gemm_plan import SINGLE, plan
+
     from distdl_b200 import _native
     from distdl_b200.ops import gemm
     torch.manual_seed(11)
+    p = plan(M, N, K, B, 0, ctas)
+    assert (p["kernel"], p["parts"]) == (SINGLE, parts)
 
     def make(rows, cols, mn):
         n, m = (cols, rows) if mn else (rows, cols)
@@ -347,13 +358,17 @@ def test_gemm_of_few_rows_in_parts_of_tiles(B, M, N, K, ctas, a_mn, b_mn):
     assert _native.read_status()[0] == 0
 
 
+@pytest.mark.parametrize("K", [4168, 256, 200, 64])          # 66 k-blocks, and no more than the ring of four holds
 @pytest.mark.parametrize("counts", [(0, 1, 256, 257), (512, 513, 768, 1000), (1000, 0, 0, 999), (0, 0, 0, 0)])
-def test_wide_tiles_skip_zero_rows(counts):
+def test_wide_tiles_skip_zero_rows(counts, K):
     """The same tiles with rows that are known to be zero: counts on and off the edges of blocks and tiles."""
+    from test_gemm_plan import WIDE, plan
+
     from distdl_b200 import _native
     from distdl_b200.ops import gemm
     torch.manual_seed(8)
-    E, C, K, N = len(counts), 1000, 4168, 2824                 # 2 x 12 x 4 tiles: a whole wave and 22 in single blocks
+    E, C, N = len(counts), 1000, 2824                          # 2 x 12 x 4 tiles: a whole wave and 22 in single blocks
+    assert plan(C, N, K, E, rows=1)["kernel"] == WIDE
     rows = torch.tensor(counts, dtype=torch.int32, device="cuda")
     keep = (torch.arange(C, device="cuda")[None] < rows[:, None])[..., None]
     x = torch.where(keep, torch.randn(E, C, K, device="cuda"), torch.zeros((), device="cuda")).bfloat16()
@@ -364,11 +379,18 @@ def test_wide_tiles_skip_zero_rows(counts):
     assert _native.read_status()[0] == 0
 
 
-@pytest.mark.parametrize("M,N,K", [(2600, 2312, 64), (2312, 2600, 64), (2312, 2312, 5000)])
-def test_gemm_tile_order_covers_every_tile(M, N, K):
-    """Tiles by panels of rows and of columns, the last panel narrower than the others."""
+@pytest.mark.parametrize("M,N,K,kernel,group", [
+    (2600, 2312, 64, 1, 4), (2312, 2600, 64, 1, 4), (2312, 2312, 5000, 1, 10), (4700, 5100, 4096, 1, 17),
+    (5100, 4700, 4096, 1, -17), (4608, 9472, 4160, 3, 8), (5000, 4300, 4160, 3, -16)])
+def test_gemm_tile_order_covers_every_tile(M, N, K, kernel, group):
+    """Tiles by panels of rows and of columns, in one panel and in several, the last one narrower than the others, with
+    tiles of 256 and of 512 rows."""
+    from test_gemm_plan import plan
+
     from distdl_b200.ops import gemm
     torch.manual_seed(9)
+    p = plan(M, N, K)
+    assert (p["kernel"], p["group"]) == (kernel, group)
     a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
     b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
     out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
