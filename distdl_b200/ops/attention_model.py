@@ -345,27 +345,33 @@ def dq_tile(Q, dO, K, V, lse2, delta, scale, causal_diag_at=None, softmax_warps=
     return tmem["dQ"] * scale
 
 
-def fwd_pair(Q, K, V, n, scale, diag=(None, None), row_warps=4, seed=0, grow_threshold=8.0, slow_warp=None):
+def fwd_pair(Q, K, V, n, scale, diag=(None, None), own_p=False, row_warps=4, seed=0, grow_threshold=8.0,
+             slow_warp=None, wait_pv=True):
     """The two-tile forward kernel for ONE pair of query tiles: ``Q`` = two ``[BQ, D]`` tiles, ``K`` /
-    ``V`` = lists of ``[BKV, D]`` blocks, ``n = (n0, n1)`` blocks seen by tile 0 / tile 1 (``n1 >= n0``),
-    ``diag[t]`` = the block on which tile ``t`` applies the causal mask.  Scores, probabilities and the
-    output accumulators live in "tensor memory"; the output is rescaled lazily (only when a row's
-    running maximum has grown by more than ``grow_threshold`` in base-2 exponent units).  Returns
-    ``(O, lse)`` with ``O`` = ``[2, BQ, D]`` and ``lse`` = ``[2, BQ]`` (natural logarithm)."""
+    ``V`` = lists of ``[BKV, D]`` blocks, ``n = (n0, n1)`` blocks seen by tile 0 / tile 1 (``n1 = 0`` where the sequence
+    has no second tile), ``diag[t]`` = the block on which tile ``t`` applies the causal mask.  Scores, probabilities and
+    the output accumulators live in "tensor memory"; the output is rescaled lazily (only when a row's
+    running maximum has grown by more than ``grow_threshold`` in base-2 exponent units), and the second product starts on
+    the first three quarters of ``P``.  ``own_p``: the schedule of head dim 64, where ``P`` has columns of its own and the
+    next block's scores are formed before the second product; else that of 128 (``P`` over ``S``).  ``wait_pv=False``
+    leaves out the wait of ``own_p`` for the product that reads the ``P`` of the block before.  Returns
+    ``(O, lse)`` with ``O`` = ``[2, BQ, D]`` and ``lse`` = ``[2, BQ]`` (natural logarithm; zeros for a tile that does not
+    exist)."""
     n0, n1 = n
+    blocks = max(n0, n1)
     BQ, D = Q[0].shape
     BKV = K[0].shape[0]
-    rows_per = BQ // row_warps
+    rows_per, most = BQ // row_warps, BKV * 3 // 4
     c = scale * 1.4426950408889634
     ST = 2
     bar = {"q_full": MBarrier(1, "q_full")}
     for name in ("k_full", "k_empty", "v_full", "v_empty"):
         bar[name] = [MBarrier(1, f"{name}[{s}]") for s in range(ST)]
-    bar["s_full"] = [MBarrier(1, f"s_full[{t}]") for t in range(2)]
-    bar["p_full"] = [MBarrier(row_warps, f"p_full[{t}]") for t in range(2)]
-    bar["pv_done"] = [MBarrier(1, f"pv_done[{t}]") for t in range(2)]
+    for name, count in (("s_full", 1), ("s_free", row_warps), ("p_most", row_warps), ("p_full", row_warps), ("pv_done", 1)):
+        bar[name] = [MBarrier(count, f"{name}[{t}]") for t in range(2)]
     smem = {"Q": [None, None], "K": [None] * ST, "V": [None] * ST}
     tmem = {"S": [np.zeros((BQ, BKV)), np.zeros((BQ, BKV))], "O": [np.zeros((BQ, D)), np.zeros((BQ, D))]}
+    tmem["P"] = [np.zeros((BQ, BKV)), np.zeros((BQ, BKV))] if own_p else tmem["S"]
     out, lse = np.zeros((2, BQ, D)), np.zeros((2, BQ))
     pipe = TensorPipe(random.Random(seed))
 
@@ -373,7 +379,7 @@ def fwd_pair(Q, K, V, n, scale, diag=(None, None), row_warps=4, seed=0, grow_thr
         rng = random.Random(seed + 1)
         smem["Q"] = [Q[0].copy(), Q[1].copy()]
         bar["q_full"].arrive()
-        for j in range(n1):
+        for j in range(blocks):
             st, ph = j % ST, (j // ST) & 1
             bar["k_empty"][st].wait(ph ^ 1)
             _jitter(rng)
@@ -392,50 +398,69 @@ def fwd_pair(Q, K, V, n, scale, diag=(None, None), row_warps=4, seed=0, grow_thr
             pipe.issue(lambda: tmem["S"][t].__setitem__(slice(None), smem["Q"][t] @ smem["K"][st].T))
             pipe.commit(bar["s_full"][t])
 
-        def issue_pv(t, j):
+        def issue_pv(t, j, lo, hi):
             st = j % ST
 
             def fn():
-                prod = tmem["S"][t] @ smem["V"][st]             # P from tensor memory
-                tmem["O"][t][:] = prod if j == 0 else tmem["O"][t] + prod
+                prod = tmem["P"][t][:, lo:hi] @ smem["V"][st][lo:hi]             # P from tensor memory
+                tmem["O"][t][:] = prod if j == 0 and lo == 0 else tmem["O"][t] + prod
             pipe.issue(fn)
-            pipe.commit(bar["pv_done"][t])
         bar["q_full"].wait(0)
         bar["k_full"][0].wait(0)
         issue_s(0, 0)
-        issue_s(1, 0)
-        for j in range(n1):
+        if n1 > 0:
+            issue_s(1, 0)
+        if own_p:
+            pipe.commit(bar["k_empty"][0])
+        for j in range(blocks):
             st, ph = j % ST, (j // ST) & 1
             stn, phn = (j + 1) % ST, ((j + 1) // ST) & 1
-            bar["v_full"][st].wait(ph)
             k_next_ready = False
+            if own_p and j + 1 < blocks:
+                for t in range(2):
+                    if j + 1 >= n[t]:
+                        continue
+                    if not k_next_ready:
+                        bar["k_full"][stn].wait(phn)
+                        k_next_ready = True
+                    bar["s_free"][t].wait(j & 1)
+                    _jitter(rng)
+                    issue_s(t, j + 1)
+                pipe.commit(bar["k_empty"][stn])
+            bar["v_full"][st].wait(ph)
             for t in range(2):
-                nt = n0 if t == 0 else n1
-                if j >= nt:
+                if j >= n[t]:
                     continue
+                bar["p_most"][t].wait(j & 1)
+                _jitter(rng)
+                issue_pv(t, j, 0, most)
                 bar["p_full"][t].wait(j & 1)
                 _jitter(rng)
-                issue_pv(t, j)
-                if j + 1 < nt:
+                issue_pv(t, j, most, BKV)
+                pipe.commit(bar["pv_done"][t])
+                if not own_p and j + 1 < n[t]:
                     if not k_next_ready:
                         bar["k_full"][stn].wait(phn)
                         k_next_ready = True
                     issue_s(t, j + 1)
             pipe.commit(bar["v_empty"][st])
-            pipe.commit(bar["k_empty"][st])
+            if not own_p:
+                pipe.commit(bar["k_empty"][st])
 
     def softmax(t, w):
         def run():
             rng = random.Random(seed + 10 + 4 * t + w)
             mine = slice(w * rows_per, (w + 1) * rows_per)
             rows = np.arange(w * rows_per, (w + 1) * rows_per)[:, None]
-            nt = n0 if t == 0 else n1
+            nt = n[t]
             m_ref = np.full(rows_per, -np.inf)
             l = np.zeros(rows_per)
             for j in range(nt):
                 bar["s_full"][t].wait(j & 1)
                 _jitter(rng)
-                s = tmem["S"][t][mine].copy()
+                s = tmem["S"][t][mine].copy()                    # tcgen05.ld: into registers
+                if own_p:
+                    bar["s_free"][t].arrive()
                 if diag[t] is not None and j == diag[t]:
                     s = np.where(np.arange(BKV)[None, :] > rows, -np.inf, s)
                 mx = np.maximum(m_ref, s.max(axis=1))
@@ -453,11 +478,17 @@ def fwd_pair(Q, K, V, n, scale, diag=(None, None), row_warps=4, seed=0, grow_thr
                 l = l + p.sum(axis=1)
                 if (t, w) == slow_warp:
                     time.sleep(0.01)                             # a warp that lags behind the others
-                tmem["S"][t][mine] = p                           # P over S, this warp's rows
+                if own_p and j > 0 and wait_pv:
+                    bar["pv_done"][t].wait((j - 1) & 1)          # P_t of block j - 1 has been read
+                tmem["P"][t][mine, :most] = p[:, :most]          # this warp's rows (head dim 128: over S)
+                bar["p_most"][t].arrive()
+                _jitter(rng)
+                tmem["P"][t][mine, most:] = p[:, most:]
                 bar["p_full"][t].arrive()
-            bar["pv_done"][t].wait((nt - 1) & 1)
-            out[t, mine] = tmem["O"][t][mine] / l[:, None]
-            lse[t, mine] = m_ref * scale + np.log(l)
+            if nt > 0:
+                bar["pv_done"][t].wait((nt - 1) & 1)
+                out[t, mine] = tmem["O"][t][mine] / l[:, None]
+                lse[t, mine] = m_ref * scale + np.log(l)
         return run
 
     try:

@@ -1,7 +1,7 @@
-"""The schedules of the attention backward kernels, run as a host model (one thread per role, the same
-barriers, parities and issue order as ``csrc/attention_bwd2_impl.cuh`` and ``csrc/attention_bwd3_impl.cuh``,
-random delays in every role):
-every sweep length must terminate and give the directly computed gradients."""
+"""The schedules of the attention kernels, run as a host model (one thread per role, the same
+barriers, parities and issue order as ``csrc/attention_fwd2_impl.cuh``, ``csrc/attention_bwd2_impl.cuh`` and
+``csrc/attention_bwd3_impl.cuh``, random delays in every role):
+every sweep length must terminate and give the directly computed results."""
 import numpy as np
 import pytest
 
@@ -108,20 +108,16 @@ def test_a_softmax_warp_that_lags_an_iteration_behind():
     assert not np.allclose(model.dq_tile(q, do, Ks, Vs, l2[0], dl[0], SCALE, slow_warp=1, ds_full_buffers=1), dQ)
 
 
-@pytest.mark.parametrize("qp,causal", [(0, True), (1, True), (3, True), (0, False), (2, False)])
-def test_forward_pair_schedule_terminates_and_matches(qp, causal):
-    """The two-tile forward kernel: both tiles alternate on the tensor pipe, the causal tiles see
-    different numbers of blocks (2 qp + 1 and 2 qp + 2), scores that grow from block to block force
-    the lazy rescale of the output accumulator."""
+def _pair_case(qp, causal, nkv, second=True):
     rng = np.random.default_rng(50 + qp)
-    nkv = 2 * qp + 2 if causal else 5
     n = (2 * qp + 1, 2 * qp + 2) if causal else (nkv, nkv)
+    n = n if second else (n[0], 0)
     diag = (2 * qp, 2 * qp + 1) if causal else (None, None)
     Q = _tiles(rng, 2)
     K = [rng.standard_normal((BT, D)) * (1 + 4 * j) for j in range(nkv)]        # later blocks score higher
     V = _tiles(rng, nkv)
     want_o, want_l = np.zeros((2, BT, D)), np.zeros((2, BT))
-    for t in range(2):
+    for t in range(2 if second else 1):
         s = np.concatenate([Q[t] @ K[j].T for j in range(n[t])], axis=1) * SCALE
         if causal:
             cols = np.arange(n[t] * BT)[None, :]
@@ -130,14 +126,43 @@ def test_forward_pair_schedule_terminates_and_matches(qp, causal):
         e = np.exp(s - m)
         want_o[t] = (e / e.sum(axis=1, keepdims=True)) @ np.concatenate(V[:n[t]], axis=0)
         want_l[t] = (m + np.log(e.sum(axis=1, keepdims=True)))[:, 0]
+    return (Q, K, V, n, SCALE, diag), want_o, want_l
+
+
+@pytest.mark.parametrize("own_p", [False, True])
+@pytest.mark.parametrize("qp,causal,nkv,second", [(0, True, 2, True), (1, True, 4, True), (3, True, 8, True), (2, True, 6, False),
+                                                  (0, False, 1, True), (0, False, 5, True), (2, False, 2, False)])
+def test_forward_pair_schedule_terminates_and_matches(qp, causal, nkv, second, own_p):
+    """The two-tile forward kernel, with the schedules of head dim 128 and 64: both tiles alternate on the tensor pipe, the
+    causal tiles see different numbers of blocks (2 qp + 1 and 2 qp + 2), a sequence may end before the second tile, scores
+    that grow from block to block force the lazy rescale of the output accumulator."""
+    args, want_o, want_l = _pair_case(qp, causal, nkv, second)
     for seed in range(3):
-        o, lse = model.fwd_pair(Q, K, V, n, SCALE, diag=diag, seed=seed, grow_threshold=2.0)
-        assert np.allclose(o, want_o, rtol=1e-9, atol=1e-9), (qp, causal, seed)
+        o, lse = model.fwd_pair(*args, own_p=own_p, seed=seed, grow_threshold=2.0)
+        assert np.allclose(o, want_o, rtol=1e-9, atol=1e-9), seed
         assert np.allclose(lse, want_l, rtol=1e-9, atol=1e-9)
-    # one softmax warp of tile 1 lagging: S of the next block is only issued after all four warps of a tile
-    # have written their probabilities, so nobody can run ahead of it
-    o, lse = model.fwd_pair(Q, K, V, n, SCALE, diag=diag, grow_threshold=2.0, slow_warp=(1, 2))
+    # one softmax warp lagging: the next S is only issued after all four warps of a tile have read their scores (at head
+    # dim 128: written their probabilities), so nobody is a whole block ahead of it
+    o, lse = model.fwd_pair(*args, own_p=own_p, grow_threshold=2.0, slow_warp=(1 if second else 0, 2))
     assert np.allclose(o, want_o, rtol=1e-9, atol=1e-9) and np.allclose(lse, want_l, rtol=1e-9, atol=1e-9)
+
+
+def test_probabilities_written_before_they_were_read_are_caught():
+    """Without the wait for the second product of the block before, a P with columns of its own is overwritten early: the
+    output is wrong, or whoever waits for a phase that has gone by never sees it."""
+    args, want_o, _ = _pair_case(0, False, 9)
+    old_limit, model.WAIT_LIMIT_S = model.WAIT_LIMIT_S, 0.5
+    try:
+        wrong = 0
+        for seed in range(4):
+            try:
+                o, _ = model.fwd_pair(*args, own_p=True, seed=seed, grow_threshold=1e9, wait_pv=False)
+                wrong += not np.allclose(o, want_o)
+            except model.PipelineStuck:
+                wrong += 1
+        assert wrong
+    finally:
+        model.WAIT_LIMIT_S = old_limit
 
 
 def _one_pass_case(nT, heads, causal, seed):
