@@ -328,7 +328,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
             float q[8];
             unpack8(pq[r][i], q);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] += q[j];
+            for (int j = 0; j < 8; ++j) o[j] = __fadd_rn(o[j], q[j]);      // (a sum of its own, as with separate operators)
           }
           store8(dx + (size_t)(row0 + r) * d + vi * 8, o);
         }
