@@ -1,4 +1,5 @@
 // C entry point of the tcgen05 GEMM.
+#include <algorithm>
 #include <cstdlib>
 
 #include "gemm2_tcgen05.cuh"
@@ -138,6 +139,28 @@ int tile_group(int M, int N, int K) {
   return M <= N ? g : -g;
 }
 
+// Whether entries with live rows take tiles of 512 x 256.  Only that kernel deals the live blocks out evenly, but at a coarser
+// grain and, tile for tile, some 5 % slower where both are even.  The counts are on the device: it is reckoned with four fifths
+// of the rows live, what a capacity of 1.25 leaves on average.  With an even number of row blocks the others' tiles lie on every
+// other pair, so that pairs with a dead block in each period wait for those without; there from 12 waves or 3e11 operations on.
+// Products of 1e12 run at the power limit, where the bytes that wide tiles leave out count (8 x 1280, 990 to 1055 rows live, 28672 x
+// 4096, 4096 x 14336, 14336 x 4096, 4096 x 28672: 1754 -> 1666, 959 -> 860, 945 -> 838, 1761 -> 1509 us).  Contractions of up
+// to 512 are bound by what is stored, which this kernel does in two sets of warps.  1142 products of 4 to 16 entries of 257 to
+// 3000 rows, time against 256-row tiles in groups of four rows: capacities filled to 0.8 0.92, at random 0.93, to 0.03 0.92, full
+// 0.94; with the wide tiles in all of them 0.98, 0.95, 0.99, 1.04, and up to 2.1 for one (8 x 320 x 4096 x 14336 333 -> 406 us).
+// Back to back for half a second, 245 products from 5e10 operations on, 0.97 and, with the wide tiles in all, 1.00, up to 1.56.
+bool live_rows_wide(int M, int N, int K, int batch, long long pairs) {
+  const long long blocks = (M + 255) / 256, cols = (N + 255) / 256;
+  const long long live = std::min(blocks, (M * 4ll + 5 * 256 - 1) / (5 * 256));
+  const long long longest = blocks % 2 == 0 && live < blocks ? (live + 1) / 2 * 2 : live;      // live blocks as if all pairs had the most
+  const long long tiles = batch * longest * cols;
+  if (K <= 512) return tiles >= 4 * pairs;
+  const double flops = 2.0 * batch * M * N * K;
+  if (live == blocks || flops >= 1e12) return live < blocks;
+  const long long waves = (tiles + pairs - 1) / pairs, wide = (batch * live * ((cols + 1) / 2) + pairs - 1) / pairs * 2;
+  return (tiles >= 12 * pairs || flops >= 3e11) && wide * 100 < waves * 95;
+}
+
 // Which kernel takes a product, with how many CTAs, its work items and the order of its tiles.
 enum Kernel : int { SINGLE, PAIR, PAIR_HALF, WIDE };
 struct Choice {
@@ -179,12 +202,12 @@ Choice choose(int M, int N, int K, int batch, int flags, int max_ctas, bool rows
   // pairs wait for the epilogue between tiles, and the order of tiles that keeps a panel in L2 is at its best with the
   // smaller ones where the contraction is short.  In us, back to back, 256 rows -> 512 rows: K = 1600: 4096 x 50304
   // 515 -> 531; K = 4096: 8192 x 28672 1441 -> 1448; K = 8192: 8192 x 8192 895 -> 842, weight gradient 28672 x 4096
-  // 1649 -> 1533; K = 14336: 8192 x 4096 768 -> 741; K = 128256: 8192 x 4096 7756 -> 6838.  Entries with live rows take them at
-  // any K, because only this kernel deals the live blocks out evenly (figures there).
+  // 1649 -> 1533; K = 14336: 8192 x 4096 768 -> 741; K = 128256: 8192 x 4096 7756 -> 6838.
   // Where their waves end later than those of the smaller tiles by more than the traffic gains, these stay: weight gradient
   // 5184 x 1728 of 7716 rows, 147 tiles in two waves, or 77 in one of twice the length and one more; a training step that has it
   // 8 680 -> 8 440 us, 9 030 with the larger tiles there.
-  const bool by_rows = rows && !bound_k;
+  // Entries with live rows: live_rows_wide.
+  const bool by_rows = rows && !bound_k && live_rows_wide(M, N, K, batch, pairs);
   if (!narrow && (flags & F_TMA_EPI) && (by_rows || (!rows && K > 4096)) && M > 256) {
     c.wide = dd::gemm4::make_plan(M, N, batch, pairs);
     const long long waves = (long long)(c.wide.full + pairs - 1) / pairs * 400 + (c.wide.items > c.wide.full ? 200 : 0);
@@ -195,8 +218,9 @@ Choice choose(int M, int N, int K, int batch, int flags, int max_ctas, bool rows
     }
   }
   c.kernel = narrow ? PAIR_HALF : PAIR;
-  // (four rows of half tiles: 4096 x 1600 x 6400 76 us, 79 to 83 in the other orders)
-  c.group_m = narrow ? 4 : tile_group(M, N, K);
+  // (four rows of half tiles: 4096 x 1600 x 6400 76 us, 79 to 83 in the other orders; and by columns, tiles without live rows
+  // follow one another on the same pairs: 16 x 1698 x 576 x 10496, 7 to 81 rows live, 72 us by rows, 150 by columns)
+  c.group_m = narrow || (rows && !bound_k && M > N) ? 4 : tile_group(M, N, K);
   c.pair = dd::gemm2::make_plan(M, N, batch, pairs, narrow ? 128 : 256);
   return c;
 }
@@ -317,10 +341,13 @@ DD_API int dd_gemm_plan(int M, int N, int K, int batch, int flags, int max_ctas,
 // Into how many parts dd_gemm_bf16_split should cut the contraction (1: not at all).  A GEMM with few output tiles
 // leaves SMs idle while each of its own walks all of K, and an SM takes in no more than about 85 GB/s, so that even
 // the read of the weights goes at a fifth of the memory rate with 16 tiles.  The parts run as a batch of the same
-// kernels into an fp32 workspace.  Measured, each alone and with a cold L2: 33 x 4096 x 14336 split 8 ways 96 -> 42 us,
-// 64 x 8 x 4096 16 ways 29 -> 15, 300 x 1600 x 6400 5 ways 28.7 -> 25.6, error against fp64 2 to 10 times smaller (shorter
+// kernels into an fp32 workspace.  Measured, each alone and with a cold L2: 33 x 4096 x 14336 split 8 ways 79 -> 40 us,
+// 33 x 64 x 4096 16 ways 25.6 -> 13.3, 200 x 2048 x 8192 8 ways 33.7 -> 27.6, error against fp64 2 to 10 times smaller (shorter
 // sums).  A k-block of 64 costs a CTA about 0.36 us, the parts and their sum about 5 us, the second launch 8 us on the host,
-// which a short GEMM does not hide: split from a gain of 8 us beyond both on.  A k-block of half tiles costs a pair 0.20 us:
+// which a short GEMM does not hide: split from a gain of 8 us beyond both on.  That is reckoned for whole tiles; up to 128 rows
+// halves of tiles cost 0.34 and quarters 0.29, so that the device gains less there than the rule says: 8 us or more at 150 of 164
+// sizes of 33 and 128 rows that are split, 3 to 8 at most others (128 x 6144 x 6144 6 ways 43.2 -> 39.9), nothing at 128 x 14336
+// x 11264.  A k-block of half tiles costs a pair 0.20 us:
 // nothing is split whose parts gain nothing over the product that takes them (1000 x 2048 x 14336, parts of whole tiles:
 // 55.3 us, 2 ways 58.3; 512 x 4096 x 11264 51.2, 2 ways 54.2).
 DD_API int dd_gemm_split(int M, int N, int K) {

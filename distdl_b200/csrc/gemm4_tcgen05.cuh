@@ -93,9 +93,8 @@ inline Plan make_plan(int M, int N, int batch, int pairs) {
 //
 // Batched products with rows[b] live rows (see Params): only blocks with live rows are dealt out, in slots of two blocks
 // (a tile, or the last, odd block of two neighbouring columns), so that every pair gets as many; the blocks without live
-// rows follow, whose zeros the epilogue writes.  In us back to back, eight
-// experts of 990 to 1061 rows in 1280, against 256-row tiles dealt out with the empty ones: 28672 x 4096 1747 -> 1678, 4096
-// x 14336 951 -> 852, 14336 x 4096 886 -> 849, 4096 x 28672 2041 -> 1760.
+// rows follow, whose zeros the epilogue writes.  In us back to back, against 256-row tiles dealt out with the empty ones: eight
+// experts of about 256 rows in 320, 28672 x 4096 622 -> 489, 14336 x 4096 356 -> 333.
 struct Walk {
   int at, sub = 0, tb = 0, base = 0;
   bool dead = false;

@@ -49,3 +49,18 @@ def test_order_of_tiles(M, N, K, group):
     """Rows of D for short contractions, else a panel of up to 36 MB of the smaller operand."""
     p = plan(M, N, K)
     assert p["group"] == group and p["kernel"] in (PAIR, WIDE)
+
+
+@pytest.mark.parametrize("M,N,K,batch,kernel", [
+    (320, 28672, 4096, 8, WIDE), (320, 14336, 4096, 8, WIDE), (960, 16384, 3072, 8, WIDE),       # dead blocks on every other pair
+    (320, 4096, 8192, 8, PAIR), (640, 4096, 14336, 8, PAIR),                                     # ... in too few waves, or few of them
+    (1280, 28672, 4096, 8, WIDE), (1280, 4096, 14336, 8, WIDE),                                  # at the power limit
+    (1280, 11264, 2048, 8, PAIR), (1000, 28672, 4096, 8, PAIR), (2560, 2048, 5632, 4, PAIR),    # an odd number of blocks, or all live
+    (1000, 2824, 512, 8, WIDE), (1000, 2824, 512, 4, PAIR)])
+def test_entries_with_live_rows_take_wide_tiles_only_where_those_are_faster(M, N, K, batch, kernel):
+    assert plan(M, N, K, batch, rows=1)["kernel"] == kernel
+
+
+def test_live_rows_of_narrow_products_by_rows():
+    """By columns, the tiles without live rows would follow one another on the same pairs."""
+    assert plan(1698, 576, 10496, 16, rows=1)["group"] == 4 and plan(1698, 576, 10496, 16)["group"] < 0

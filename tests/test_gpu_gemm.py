@@ -358,17 +358,21 @@ def test_gemm_of_few_rows_in_parts_of_tiles(B, M, N, K, ctas, parts, a_mn, b_mn)
     assert _native.read_status()[0] == 0
 
 
-@pytest.mark.parametrize("K", [4168, 256, 200, 64])          # 66 k-blocks, and no more than the ring of four holds
+@pytest.mark.parametrize("C,K,N,kernel", [
+    (1000, 4168, 2824, 1), (1000, 512, 2824, 3), (1000, 256, 2824, 3),      # 256-row tiles; eight k-blocks, four as the ring has
+    (1000, 200, 2824, 3), (1000, 64, 2824, 3), (300, 1032, 14336, 3)])
 @pytest.mark.parametrize("counts", [(0, 1, 256, 257), (512, 513, 768, 1000), (1000, 0, 0, 999), (0, 0, 0, 0)])
-def test_wide_tiles_skip_zero_rows(counts, K):
-    """The same tiles with rows that are known to be zero: counts on and off the edges of blocks and tiles."""
-    from test_gemm_plan import WIDE, plan
+def test_wide_tiles_skip_zero_rows(counts, C, K, N, kernel):
+    """Rows that are known to be zero, with tiles of 512 rows where the rule takes them: counts on and off the edges of blocks
+    and tiles."""
+    from test_gemm_plan import plan
 
     from distdl_b200 import _native
     from distdl_b200.ops import gemm
     torch.manual_seed(8)
-    E, C, N = len(counts), 1000, 2824                          # 2 x 12 x 4 tiles: a whole wave and 22 in single blocks
-    assert plan(C, N, K, E, rows=1)["kernel"] == WIDE
+    counts = [min(c, C) for c in counts + counts[::-1]]
+    E = len(counts)
+    assert plan(C, N, K, E, rows=1)["kernel"] == kernel
     rows = torch.tensor(counts, dtype=torch.int32, device="cuda")
     keep = (torch.arange(C, device="cuda")[None] < rows[:, None])[..., None]
     x = torch.where(keep, torch.randn(E, C, K, device="cuda"), torch.zeros((), device="cuda")).bfloat16()
