@@ -86,7 +86,9 @@ static bool split_in_one_pass(int nT, int group, long long kv_tiles, int Dh, int
 //                          1 x 16384, 32 / 8: 13976 -> 14919 (13897 -> 14790)
 //   one key tile           64 x 128, 16 / 4 of 128: 118 -> 75
 // (The two at head dim 128 take 5 % less since their softmax threads work on two values per instruction: 2 x 4096, 32 / 8, causal
-// 973 -> 922 back to back.)
+// 973 -> 922 back to back.  Measured again, one batch, 485 sizes that take the one kernel: 0.80 of the time of the two on average,
+// cold; 26 are slower by 3 to 12 %, most of them groups over two key tiles in full attention, 256 tokens, 48 / 16 of 128 39.9 -> 40.2,
+// 192 / 24 81 -> 91, and 8192 tokens, 8 / 4 of 128, causal 400 -> 441.)
 // Hence one kernel where no more than a quarter of a head's key tiles start together, at head dim 128 for long sweeps only.
 // `words`: of scratch for the one kernel, on this device.
 DD_API int dd_attn_bwd_one_pass(int batch, int S, int Hq, int Hkv, int Dh, int causal, long long* words) {
