@@ -147,8 +147,10 @@ int tile_group(int M, int N, int K) {
 // 4096, 4096 x 14336, 14336 x 4096, 4096 x 28672: 1754 -> 1666, 959 -> 860, 945 -> 838, 1761 -> 1509 us).  Contractions of up
 // to 512 are bound by what is stored, which this kernel does in two sets of warps.  1142 products of 4 to 16 entries of 257 to
 // 3000 rows, time against 256-row tiles in groups of four rows: capacities filled to 0.8 0.92, at random 0.93, to 0.03 0.92, full
-// 0.94; with the wide tiles in all of them 0.98, 0.95, 0.99, 1.04, and up to 2.1 for one (8 x 320 x 4096 x 14336 333 -> 406 us).
-// Back to back for half a second, 245 products from 5e10 operations on, 0.97 and, with the wide tiles in all, 1.00, up to 1.56.
+// 0.94; with the wide tiles in all of them 0.98, 0.95, 0.99, 1.04, and up to 2.1 for one; back to back for half a second, 245
+// products from 5e10 operations on, 0.97 and, with the wide tiles in all, 1.00, up to 1.56.  Four fifths of 320 rows are one block,
+// but of 8 entries with 246 to 266 live rows half have two, 4096 x 14336 327 -> 406 us: the wide tiles are reckoned with half of
+// the last block on average.
 bool live_rows_wide(int M, int N, int K, int batch, long long pairs) {
   const long long blocks = (M + 255) / 256, cols = (N + 255) / 256;
   const long long live = std::min(blocks, (M * 4ll + 5 * 256 - 1) / (5 * 256));
@@ -157,7 +159,9 @@ bool live_rows_wide(int M, int N, int K, int batch, long long pairs) {
   if (K <= 512) return tiles >= 4 * pairs;
   const double flops = 2.0 * batch * M * N * K;
   if (live == blocks || flops >= 1e12) return live < blocks;
-  const long long waves = (tiles + pairs - 1) / pairs, wide = (batch * live * ((cols + 1) / 2) + pairs - 1) / pairs * 2;
+  const long long mean = std::min(blocks * 1280, M * 4ll + 640);       // live blocks of an entry, in parts of 1280
+  const long long slots = (batch * cols * mean + 2 * 1280 - 1) / (2 * 1280);
+  const long long waves = (tiles + pairs - 1) / pairs, wide = (slots + pairs - 1) / pairs * 2;
   return (tiles >= 12 * pairs || flops >= 3e11) && wide * 100 < waves * 95;
 }
 

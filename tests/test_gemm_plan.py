@@ -54,6 +54,7 @@ def test_order_of_tiles(M, N, K, group):
 @pytest.mark.parametrize("M,N,K,batch,kernel", [
     (320, 28672, 4096, 8, WIDE), (320, 14336, 4096, 8, WIDE), (960, 16384, 3072, 8, WIDE),       # dead blocks on every other pair
     (320, 4096, 8192, 8, PAIR), (640, 4096, 14336, 8, PAIR),                                     # ... in too few waves, or few of them
+    (320, 4096, 14336, 8, PAIR), (320, 4096, 28672, 8, PAIR),                                    # ... once a block is live in part
     (1280, 28672, 4096, 8, WIDE), (1280, 4096, 14336, 8, WIDE),                                  # at the power limit
     (1280, 11264, 2048, 8, PAIR), (1000, 28672, 4096, 8, PAIR), (2560, 2048, 5632, 4, PAIR),    # an odd number of blocks, or all live
     (1000, 2824, 512, 8, WIDE), (1000, 2824, 512, 4, PAIR)])
