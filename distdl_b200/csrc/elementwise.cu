@@ -223,7 +223,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // RES: dres_in is added to dx (gradient of the residual stream).
 // Bound by the round trip of a group of rows (read, reduce over the CTA, write), so the next group is read meanwhile, and
 // the residual's gradient with it.  With the fold of dw and db, us: 8192 x 4096 75.8 -> 66.3, 3000 x 2048 16.4 -> 14.3, LayerNorm
-// 8192 x 8192 234 -> 146, 4096 x 1600 22.5 -> 21.1 (twice the rows per group, one group in flight before).  Without dres_in its
+// 8192 x 8192 230 -> 132, 4096 x 1600 22.5 -> 21.1 (twice the rows per group, one group in flight before).  Without dres_in its
 // registers must not be there: 128 per thread are two CTAs per SM.  16384 x 2560 69 (before) -> 87 (with them) -> 60, LayerNorm 16384
 // x 424 33 -> 39 -> 34, 16384 x 2048 55 -> 65 -> 50, 16384 x 4096 154 -> 120 -> 81.
 template <bool RMS, int VEC, int R, bool WANT_DB, bool RES>

@@ -64,6 +64,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor = None, *, bias: to
     ``rows`` (int32 ``[batch]`` on the device, for 3-D operands without a bias) promises that ``a[b]`` is zero after
     its first ``rows[b]`` rows, or, with ``bound_k``, that the terms of the contraction after the first ``rows[b]``
     are zero: the result is the same, the work on those zeros is left out.
+
+    ``max_ctas`` below the number of SMs leaves the others to work of other streams; the next product does not start on
+    them before this one has ended.
     """
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16, "bf16 operands required"
     assert a.dim() == b.dim() and a.dim() in (2, 3)
